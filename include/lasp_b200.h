@@ -183,6 +183,25 @@ LASP_B200_API int lasp_b200_bwd_dkv(const lasp_problem* p, const lasp_bwd_args* 
  * lasp_b200_bwd_grads without its dQ launch (on the fp32 path: all of lasp_b200_bwd_grads). */
 LASP_B200_API int lasp_b200_bwd_dkv_walk(const lasp_problem* p, const lasp_bwd_args* a, void* stream);
 
+/* The two composite calls with options, for a host that keeps its own synchronisation words and drives the
+ * slices of wide heads itself (lasp_forward / lasp_backward, lasp/lasp_fuse.py:356-475). */
+enum {
+  LASP_ACCUMULATE_QK = 1, /* add to what dq, dk hold (rounded to the tensors' type) instead of overwriting it */
+  LASP_ACCUMULATE_V = 2   /* the same for o and dv; both on the tensor-core path only (LASP_ERR_PATH otherwise) */
+};
+typedef struct {
+  uint32_t* sync;      /* 4 KB of device memory, zeroed once: the words the CTAs of a launch synchronise through,
+                        * used instead of the first 4 KB of ws, which then need no zeroing.  Calls that share a
+                        * block must not overlap on the GPU (one block per stream).  NULL = those of ws. */
+  int32_t keep_states; /* forward: leave the states the backward pass reads in ws (0: nothing is kept) */
+  int32_t accumulate;  /* LASP_ACCUMULATE_* */
+} lasp_call_options;
+LASP_B200_API int lasp_b200_forward_opt(const lasp_problem* p, const lasp_fwd_args* a, const lasp_call_options* opt,
+                                        void* stream);
+/* fwd_ws must come from lasp_b200_forward_opt of the same problem with keep_states */
+LASP_B200_API int lasp_b200_backward_opt(const lasp_problem* p, const lasp_bwd_args* a, const lasp_call_options* opt,
+                                         void* stream);
+
 /* x_out = exp(-s_h n) x_in + x_local on (b,h,d,e) fp32 states; x_in may be NULL.
  * Replaces the torch glue KV = block_decay*KV + kv, lasp/lasp_naive.py:565,614. */
 LASP_B200_API int lasp_b200_state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,

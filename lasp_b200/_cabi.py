@@ -53,6 +53,10 @@ class BwdArgs(C.Structure):
                 ("ws", C.c_void_p), ("ws_bytes", C.c_size_t)]
 
 
+class CallOptions(C.Structure):   # lasp_call_options
+    _fields_ = [("sync", C.c_void_p), ("keep_states", C.c_int32), ("accumulate", C.c_int32)]
+
+
 class ExchangeArgs(C.Structure):
     _fields_ = [(n, C.c_int32) for n in ("ranks", "position", "reverse", "phase")] + \
                [("s", C.c_void_p), ("ws", C.c_void_p), ("ws_bytes", C.c_size_t)] + \
@@ -82,6 +86,8 @@ SIGNATURES = {
     "lasp_b200_bwd_dq": (C.c_int, [_PP, _BP, C.c_void_p]),
     "lasp_b200_bwd_dkv": (C.c_int, [_PP, _BP, C.c_void_p]),
     "lasp_b200_bwd_dkv_walk": (C.c_int, [_PP, _BP, C.c_void_p]),
+    "lasp_b200_forward_opt": (C.c_int, [_PP, _FP, C.POINTER(CallOptions), C.c_void_p]),
+    "lasp_b200_backward_opt": (C.c_int, [_PP, _BP, C.POINTER(CallOptions), C.c_void_p]),
     "lasp_b200_state_combine": (C.c_int, [C.c_int] * 5 + [C.c_void_p] * 5),
     "lasp_b200_read_status": (C.c_int, [C.POINTER(C.c_int32), C.c_int, C.c_void_p]),
     "lasp_b200_copy_status_async": (C.c_int, [C.c_void_p, C.c_void_p]),

@@ -163,6 +163,14 @@ int check_bwd(const lasp_problem* p, const lasp_bwd_args* a, lasp::Dims* m, bool
   return LASP_OK;
 }
 
+int check_options(const lasp::Dims& m, const lasp_call_options* opt) {
+  if (!opt) return LASP_ERR_NULL;
+  if (!aligned16(opt->sync)) return LASP_ERR_ALIGN;
+  if (opt->accumulate & ~(LASP_ACCUMULATE_QK | LASP_ACCUMULATE_V)) return LASP_ERR_SHAPE;
+  if (opt->accumulate && !m.walk) return LASP_ERR_PATH;   // the TMA stores of the walk kernels add
+  return LASP_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -210,6 +218,8 @@ size_t lasp_b200_bwd_workspace_bytes(const lasp_problem* p) { return lasp_b200_f
 
 namespace {
 
+constexpr lasp_call_options kPlainCall = {nullptr, 1, 0};
+
 int fwd_chunk_states(const lasp::Dims& m, const lasp_fwd_args* a, cudaStream_t cs) {
   if (lasp::has_qk_preprocessing(m)) return LASP_ERR_PATH;
   if (m.walk) return cuda_fail(lasp::walk_span_totals(m, a->k, a->v, a->s, lasp::ws_local(a->ws, m), false, cs));
@@ -222,11 +232,12 @@ int fwd_scan(const lasp::Dims& m, const lasp_fwd_args* a, cudaStream_t cs) {
                                      false, cs));
 }
 
-int fwd_output(const lasp::Dims& m, const lasp_fwd_args* a, cudaStream_t cs) {
+int fwd_output(const lasp::Dims& m, const lasp_fwd_args* a, const lasp_call_options& opt, cudaStream_t cs) {
   if (lasp::has_qk_preprocessing(m)) return LASP_ERR_PATH;
   if (m.walk)
     return cuda_fail(lasp::walk_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_walk_border(a->ws, m),
-                                           lasp::ws_walk_sync(a->ws), a->o, cs));
+                                           opt.sync ? opt.sync : lasp::ws_walk_sync(a->ws), a->o,
+                                           (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
   return cuda_fail(lasp::simt_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_prefix(a->ws, m), a->o, cs));
 }
 
@@ -242,15 +253,16 @@ int bwd_scan(const lasp::Dims& m, const lasp_bwd_args* a, cudaStream_t cs) {
                                      a->dkv_out, true, cs));
 }
 
-int bwd_grads(const lasp::Dims& m, const lasp_bwd_args* a, cudaStream_t cs) {
+int bwd_grads(const lasp::Dims& m, const lasp_bwd_args* a, const lasp_call_options& opt, cudaStream_t cs) {
   if (lasp::has_qk_preprocessing(m)) return LASP_ERR_PATH;
   if (m.walk) {
     // dQ walks forward over the border states the forward pass left in its workspace; dK, dV walk backward
+    const bool add_qk = (opt.accumulate & LASP_ACCUMULATE_QK) != 0, add_v = (opt.accumulate & LASP_ACCUMULATE_V) != 0;
     int st = cuda_fail(lasp::walk_bwd_dq(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->fwd_ws, m),
-                                          lasp::ws_walk_sync(a->fwd_ws), a->dq, cs));
+                                         opt.sync ? nullptr : lasp::ws_walk_sync(a->fwd_ws), false, a->dq, add_qk, cs));
     if (st != LASP_OK) return st;
     return cuda_fail(lasp::walk_bwd_dkv(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->ws, m), a->dk,
-                                        a->dv, cs));
+                                        a->dv, add_qk, add_v, cs));
   }
   return cuda_fail(lasp::simt_bwd_grads(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_prefix(a->fwd_ws, m),
                                         lasp::ws_prefix(a->ws, m), a->dq, a->dk, a->dv, cs));
@@ -276,21 +288,28 @@ int lasp_b200_fwd_scan(const lasp_problem* p, const lasp_fwd_args* a, void* stre
 int lasp_b200_fwd_output(const lasp_problem* p, const lasp_fwd_args* a, void* stream) {
   lasp::Dims m;
   int st = check_fwd(p, a, &m, true);
-  return st != LASP_OK ? st : fwd_output(m, a, static_cast<cudaStream_t>(stream));
+  return st != LASP_OK ? st : fwd_output(m, a, kPlainCall, static_cast<cudaStream_t>(stream));
 }
 
-int lasp_b200_forward(const lasp_problem* p, const lasp_fwd_args* a, void* stream) {
+int lasp_b200_forward_opt(const lasp_problem* p, const lasp_fwd_args* a, const lasp_call_options* opt, void* stream) {
   lasp::Dims m;
   int st = check_fwd(p, a, &m, true);
   if (st != LASP_OK) return st;
+  if ((st = check_options(m, opt)) != LASP_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   if (fusable(m))
-    return cuda_fail(lasp::walk_fwd_fused(m, a->q, a->k, a->v, a->s, a->kv_in, a->kv_out, lasp::ws_walk_sync(a->ws),
-                                          lasp::ws_walk_totals(a->ws), lasp::ws_walk_border(a->ws, m), a->o, nullptr,
-                                          cs));
+    return cuda_fail(lasp::walk_fwd_fused(m, a->q, a->k, a->v, a->s, a->kv_in, a->kv_out,
+                                          opt->sync ? opt->sync : lasp::ws_walk_sync(a->ws),
+                                          lasp::ws_walk_totals(a->ws),
+                                          opt->keep_states ? lasp::ws_walk_border(a->ws, m) : nullptr, a->o, nullptr,
+                                          (opt->accumulate & LASP_ACCUMULATE_V) != 0, cs));
   if ((st = fwd_chunk_states(m, a, cs)) != LASP_OK) return st;
   if ((st = fwd_scan(m, a, cs)) != LASP_OK) return st;
-  return fwd_output(m, a, cs);
+  return fwd_output(m, a, *opt, cs);
+}
+
+int lasp_b200_forward(const lasp_problem* p, const lasp_fwd_args* a, void* stream) {
+  return lasp_b200_forward_opt(p, a, &kPlainCall, stream);
 }
 
 // ---- backward -------------------------------------------------------------
@@ -309,7 +328,7 @@ int lasp_b200_bwd_scan(const lasp_problem* p, const lasp_bwd_args* a, void* stre
 int lasp_b200_bwd_grads(const lasp_problem* p, const lasp_bwd_args* a, void* stream) {
   lasp::Dims m;
   int st = check_bwd(p, a, &m, true);
-  return st != LASP_OK ? st : bwd_grads(m, a, static_cast<cudaStream_t>(stream));
+  return st != LASP_OK ? st : bwd_grads(m, a, kPlainCall, static_cast<cudaStream_t>(stream));
 }
 
 // The two launches of the tensor-core backward, separately (the fp32 path has one gradient kernel: there
@@ -319,7 +338,7 @@ int lasp_b200_bwd_dq(const lasp_problem* p, const lasp_bwd_args* a, void* stream
   int st = check_bwd(p, a, &m, true);
   if (st != LASP_OK || !m.walk) return st;
   return cuda_fail(lasp::walk_bwd_dq(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->fwd_ws, m),
-                                          lasp::ws_walk_sync(a->fwd_ws), a->dq,
+                                          lasp::ws_walk_sync(a->fwd_ws), false, a->dq, false,
                                      static_cast<cudaStream_t>(stream)));
 }
 
@@ -328,10 +347,10 @@ int lasp_b200_bwd_dkv_walk(const lasp_problem* p, const lasp_bwd_args* a, void* 
   int st = check_bwd(p, a, &m, true);
   if (st != LASP_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  if (!m.walk) return bwd_grads(m, a, cs);
+  if (!m.walk) return bwd_grads(m, a, kPlainCall, cs);
   if (lasp::has_qk_preprocessing(m)) return LASP_ERR_PATH;
   return cuda_fail(lasp::walk_bwd_dkv(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->ws, m), a->dk, a->dv,
-                                      cs));
+                                      false, false, cs));
 }
 
 int lasp_b200_bwd_dkv(const lasp_problem* p, const lasp_bwd_args* a, void* stream) {
@@ -341,27 +360,33 @@ int lasp_b200_bwd_dkv(const lasp_problem* p, const lasp_bwd_args* a, void* strea
   if (!fusable(m)) return lasp_b200_backward(p, a, stream);
   return cuda_fail(lasp::walk_bwd_dkv_fused(m, a->q, a->k, a->v, a->d_o, a->s, a->dkv_in, a->dkv_out,
                                             lasp::ws_walk_sync(a->ws), lasp::ws_walk_totals(a->ws), a->dk, a->dv,
-                                            nullptr, static_cast<cudaStream_t>(stream)));
+                                            nullptr, false, false, static_cast<cudaStream_t>(stream)));
 }
 
-int lasp_b200_backward(const lasp_problem* p, const lasp_bwd_args* a, void* stream) {
+int lasp_b200_backward_opt(const lasp_problem* p, const lasp_bwd_args* a, const lasp_call_options* opt, void* stream) {
   lasp::Dims m;
   int st = check_bwd(p, a, &m, true);
   if (st != LASP_OK) return st;
+  if ((st = check_options(m, opt)) != LASP_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   if (fusable(m)) {
-    // dQ walks forward over the border states the forward pass kept; dK, dV walk backward in one fused launch
-    if ((st = cuda_fail(lasp::walk_bwd_dq(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->fwd_ws, m),
-                                          lasp::ws_walk_sync(a->fwd_ws), a->dq,
-                                          cs))) != LASP_OK)
-      return st;
+    // dQ walks forward over the border states the forward pass kept; dK, dV walk backward in one fused launch.
+    // (With synchronisation words of the caller's the forward's workspace does not say how the sequences were cut.)
+    const bool add_qk = (opt->accumulate & LASP_ACCUMULATE_QK) != 0, add_v = (opt->accumulate & LASP_ACCUMULATE_V) != 0;
+    st = cuda_fail(lasp::walk_bwd_dq(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->fwd_ws, m),
+                                     opt->sync ? nullptr : lasp::ws_walk_sync(a->fwd_ws), m.nc > 1, a->dq, add_qk, cs));
+    if (st != LASP_OK) return st;
     return cuda_fail(lasp::walk_bwd_dkv_fused(m, a->q, a->k, a->v, a->d_o, a->s, a->dkv_in, a->dkv_out,
-                                              lasp::ws_walk_sync(a->ws), lasp::ws_walk_totals(a->ws), a->dk, a->dv,
-                                              nullptr, cs));
+                                              opt->sync ? opt->sync : lasp::ws_walk_sync(a->ws),
+                                              lasp::ws_walk_totals(a->ws), a->dk, a->dv, nullptr, add_qk, add_v, cs));
   }
   if ((st = bwd_chunk_states(m, a, cs)) != LASP_OK) return st;
   if ((st = bwd_scan(m, a, cs)) != LASP_OK) return st;
-  return bwd_grads(m, a, cs);
+  return bwd_grads(m, a, *opt, cs);
+}
+
+int lasp_b200_backward(const lasp_problem* p, const lasp_bwd_args* a, void* stream) {
+  return lasp_b200_backward_opt(p, a, &kPlainCall, stream);
 }
 
 int lasp_b200_state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
@@ -401,7 +426,7 @@ int lasp_b200_forward_linked(const lasp_problem* p, const lasp_fwd_args* a, cons
   if ((st = check_link(x)) != LASP_OK) return st;
   if (lasp_b200_linked_ok(p) != 1) return LASP_ERR_PATH;
   return cuda_fail(lasp::walk_fwd_fused(m, a->q, a->k, a->v, a->s, nullptr, nullptr, lasp::ws_walk_sync(a->ws),
-                                        lasp::ws_walk_totals(a->ws), lasp::ws_walk_border(a->ws, m), a->o, x,
+                                        lasp::ws_walk_totals(a->ws), lasp::ws_walk_border(a->ws, m), a->o, x, false,
                                         static_cast<cudaStream_t>(stream)));
 }
 
@@ -414,7 +439,7 @@ int lasp_b200_bwd_dkv_linked(const lasp_problem* p, const lasp_bwd_args* a, cons
   if (lasp_b200_linked_ok(p) != 1) return LASP_ERR_PATH;
   return cuda_fail(lasp::walk_bwd_dkv_fused(m, a->q, a->k, a->v, a->d_o, a->s, nullptr, nullptr,
                                             lasp::ws_walk_sync(a->ws), lasp::ws_walk_totals(a->ws), a->dk, a->dv, x,
-                                            static_cast<cudaStream_t>(stream)));
+                                            false, false, static_cast<cudaStream_t>(stream)));
 }
 
 int lasp_b200_exchange_scan(const lasp_problem* p, const lasp_exchange_args* a, void* stream) {

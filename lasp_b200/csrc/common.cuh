@@ -114,16 +114,19 @@ bool tensor_path_supported(const Dims& m);
 cudaError_t walk_span_totals(const Dims& m, const void* a, const void* bten, const float* s, float* totals,
                              bool reverse, cudaStream_t st);
 cudaError_t walk_fwd_output(const Dims& m, const void* q, const void* k, const void* v, const float* s,
-                            const float* prefix, uint32_t* sync, void* o, cudaStream_t st);
+                            const float* prefix, uint32_t* sync, void* o, bool add_o, cudaStream_t st);
 cudaError_t walk_fwd_fused(const Dims& m, const void* q, const void* k, const void* v, const float* s,
                            const float* x_in, float* x_out, uint32_t* sync, float* totals, float* prefix, void* o,
-                           const lasp_exchange_args* link, cudaStream_t st);
+                           const lasp_exchange_args* link, bool add_o, cudaStream_t st);
+// fwd_sync: the forward's synchronisation words, which say how it cut the sequences; NULL: `even` says it
 cudaError_t walk_bwd_dq(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, const float* s,
-                        const float* prefix, const uint32_t* fwd_sync, void* dq, cudaStream_t st);
+                        const float* prefix, const uint32_t* fwd_sync, bool even, void* dq, bool add_dq, cudaStream_t st);
 cudaError_t walk_bwd_dkv(const Dims& m, const void* q, const void* k, const void* v, const void* d_o,
-                         const float* s, const float* suffix, void* dk, void* dv, cudaStream_t st);
+                         const float* s, const float* suffix, void* dk, void* dv, bool add_dk, bool add_dv,
+                         cudaStream_t st);
 cudaError_t walk_bwd_dkv_fused(const Dims& m, const void* q, const void* k, const void* v, const void* d_o,
                                const float* s, const float* x_in, float* x_out, uint32_t* sync, float* totals,
-                               void* dk, void* dv, const lasp_exchange_args* link, cudaStream_t st);
+                               void* dk, void* dv, const lasp_exchange_args* link, bool add_dk, bool add_dv,
+                               cudaStream_t st);
 
 }  // namespace lasp

@@ -110,6 +110,20 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void*
                "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
+// the same, added to what the destination holds (in the map's element type, rounded to nearest even)
+__device__ __forceinline__ void tma_add_4d(const CUtensorMap* map, const void* smem_src, int c0, int c1, int c2,
+                                           int c3) {
+  asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"(map), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
+__device__ __forceinline__ void tma_store_or_add_4d(const CUtensorMap* map, const void* smem_src, int c0, int c1, int c2,
+                                                    int c3, int add) {
+  if (add)
+    tma_add_4d(map, smem_src, c0, c1, c2, c3);
+  else
+    tma_store_4d(map, smem_src, c0, c1, c2, c3);
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all but the newest `pending` store groups of this thread have finished READING shared memory
 template <int pending>

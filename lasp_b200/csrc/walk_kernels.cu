@@ -414,6 +414,7 @@ struct WalkArgs {
   int all_totals;      // fused: the last span of a sequence computes its total too
   int coop;            // fused: every CTA has exactly one span and the CTAs synchronise (several spans per
                        // sequence, or a link)
+  int add_out, add_out2;       // the stores of OUT (dK, dV) add to what the tensors hold
   long long wait_clocks;
   int32_t* fault;
   Link link;           // fused: hand the rank state over inside the launch (link.ranks > 0)
@@ -603,7 +604,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
         if (i >= 2) {
           // the output of tile i-2 is staged in Y's buffer: store it, then reuse the buffer
           wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
-          tma_store_4d(&map_out, sy[p], 0, out_row.get(p), 0, out_bh.get(p));
+          tma_store_or_add_4d(&map_out, sy[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
           bulk_commit();
           bulk_wait_read<0>();
         }
@@ -615,7 +616,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
       for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
         const int p = j & 1, u = j >> 1;
         wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
-        tma_store_4d(&map_out, sy[p], 0, out_row.get(p), 0, out_bh.get(p));
+        tma_store_or_add_4d(&map_out, sy[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
         bulk_commit();
       }
       bulk_wait_all<0>();
@@ -1147,8 +1148,8 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
         if (i >= 2) {
           // dK and dV of tile i-2 are staged in this parity's K and V buffers
           wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
-          tma_store_4d(&map_dk, sk[p], 0, out_row.get(p), 0, out_bh.get(p));
-          tma_store_4d(&map_dv, sv[p], 0, out_row.get(p), 0, out_bh.get(p));
+          tma_store_or_add_4d(&map_dk, sk[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
+          tma_store_or_add_4d(&map_dv, sv[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
           bulk_commit();
           bulk_wait_read<0>();
         }
@@ -1172,8 +1173,8 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
       for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
         const int p = j & 1, u = j >> 1;
         wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
-        tma_store_4d(&map_dk, sk[p], 0, out_row.get(p), 0, out_bh.get(p));
-        tma_store_4d(&map_dv, sv[p], 0, out_row.get(p), 0, out_bh.get(p));
+        tma_store_or_add_4d(&map_dk, sk[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
+        tma_store_or_add_4d(&map_dv, sv[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
         bulk_commit();
       }
       bulk_wait_all<0>();
@@ -1512,10 +1513,19 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-template <typename F>
-cudaError_t opt_in_smem(F* fn, size_t bytes) {
-  cudaError_t err = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err != cudaSuccess) g_failed_step = "cudaFuncSetAttribute(max dynamic shared memory)";
+// once per kernel and device (the attribute call costs the host about as much as a launch)
+template <auto fn>
+cudaError_t opt_in_smem(size_t bytes) {
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err == cudaSuccess && dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (err != cudaSuccess)
+    g_failed_step = "cudaFuncSetAttribute(max dynamic shared memory)";
+  else if (dev >= 0 && dev < 64)
+    done[dev] = true;
   return err;
 }
 
@@ -1551,7 +1561,7 @@ cudaError_t launch_span_totals(const Dims& m, const void* a, const void* bten, c
   int32_t* fault = nullptr;
   if ((err = fault_word_address(&fault)) != cudaSuccess) return err;
   const size_t smem = (size_t)3 * C * (D + E) * 2 + 1024;
-  if ((err = opt_in_smem(k_span_totals<D, E>, smem)) != cudaSuccess) return err;
+  if ((err = opt_in_smem<k_span_totals<D, E>>(smem)) != cudaSuccess) return err;
   const int items = m.b * m.h * m.nc;
   k_span_totals<D, E><<<grid_for(items), 320, smem, st>>>(ma, mb, s, totals, m.h, m.n, m.tiles, m.span, m.nc, items,
                                                           reverse ? 1 : 0, fault);
@@ -1585,7 +1595,7 @@ cudaError_t launch_walk_out_pre(const Dims& m, const void* x, const void* y, con
   if ((err = seq_map(&mo, out, m, WZ, DQ ? m.pitch_d : m.pitch_e, DQ ? "dq" : "o")) != cudaSuccess) return err;
   if ((err = fault_word_address(&a.fault)) != cudaSuccess) return err;
   const size_t smem = (size_t)7 * kBuf + 1024;
-  if ((err = opt_in_smem(k_walk_out<D, E, DQ, FUSED, PRE, LINK>, smem)) != cudaSuccess) return err;
+  if ((err = opt_in_smem<k_walk_out<D, E, DQ, FUSED, PRE, LINK>>(smem)) != cudaSuccess) return err;
   a.h = m.h, a.n = m.n, a.tiles = m.tiles, a.span = m.span, a.nspans = m.nc, a.items = m.b * m.h * m.nc;
   a.wait_clocks = kFlagWaitClocks;
   a.qk_scale = m.qk_scale, a.elu = m.qk_map, a.raw_pitch = m.pitch_d;
@@ -1619,7 +1629,7 @@ cudaError_t launch_walk_dkv_pre(const Dims& m, const void* q, const void* k, con
   if ((err = fault_word_address(&a.fault)) != cudaSuccess) return err;
   a.raw = k;   // for the chain rule of a folded k preprocessing
   const size_t smem = (size_t)7 * kBuf + 1024;
-  if ((err = opt_in_smem(k_walk_dkv<D, E, FUSED, PRE, LINK>, smem)) != cudaSuccess) return err;
+  if ((err = opt_in_smem<k_walk_dkv<D, E, FUSED, PRE, LINK>>(smem)) != cudaSuccess) return err;
   a.h = m.h, a.n = m.n, a.tiles = m.tiles, a.span = m.span, a.nspans = m.nc, a.items = m.b * m.h * m.nc;
   a.wait_clocks = kFlagWaitClocks;
   a.qk_scale = m.qk_scale, a.elu = m.qk_map, a.raw_pitch = m.pitch_d;
@@ -1697,8 +1707,9 @@ cudaError_t walk_span_totals(const Dims& m, const void* a, const void* bten, con
 }
 
 cudaError_t walk_fwd_output(const Dims& m, const void* q, const void* k, const void* v, const float* s,
-                            const float* prefix, uint32_t* sync, void* o, cudaStream_t st) {
+                            const float* prefix, uint32_t* sync, void* o, bool add_o, cudaStream_t st) {
   WalkArgs a = {};
+  a.add_out = add_o;
   a.s = s, a.p0 = prefix, a.sync = sync;   // sync: only the word that says how the sequences were cut
 #define LASP_CALL(DD, EE) launch_walk_out<DD, EE, false, false>(m, q, k, v, o, a, st)
   LASP_DISPATCH_DE(m, LASP_CALL);
@@ -1724,8 +1735,9 @@ static Link make_link(const lasp_exchange_args* x) {
 
 cudaError_t walk_fwd_fused(const Dims& m, const void* q, const void* k, const void* v, const float* s,
                            const float* x_in, float* x_out, uint32_t* sync, float* totals, float* prefix, void* o,
-                           const lasp_exchange_args* link, cudaStream_t st) {
+                           const lasp_exchange_args* link, bool add_o, cudaStream_t st) {
   WalkArgs a = {};
+  a.add_out = add_o;
   a.link = make_link(link);
   a.s = s, a.x_in = x_in, a.x_out = x_out, a.sync = sync, a.totals = totals, a.p0_save = prefix;
 #define LASP_CALL(DD, EE) launch_walk_out<DD, EE, false, true>(m, q, k, v, o, a, st)
@@ -1734,9 +1746,11 @@ cudaError_t walk_fwd_fused(const Dims& m, const void* q, const void* k, const vo
 }
 
 cudaError_t walk_bwd_dq(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, const float* s,
-                        const float* prefix, const uint32_t* fwd_sync, void* dq, cudaStream_t st) {
+                        const float* prefix, const uint32_t* fwd_sync, bool even, void* dq, bool add_dq, cudaStream_t st) {
   WalkArgs a = {};
-  a.s = s, a.p0 = prefix, a.even_word = fwd_sync + kSyncEven;   // cut the sequences as the forward pass did
+  a.add_out = add_dq;
+  a.s = s, a.p0 = prefix, a.even = even;   // the sequences are cut as the forward pass did
+  if (fwd_sync != nullptr) a.even_word = fwd_sync + kSyncEven;
   a.raw = q;                                                    // for the chain rule of a folded q preprocessing
 #define LASP_CALL(DD, EE) launch_walk_out<DD, EE, true, false>(m, d_o, v, k, dq, a, st)
   LASP_DISPATCH_DE(m, LASP_CALL);
@@ -1744,8 +1758,10 @@ cudaError_t walk_bwd_dq(const Dims& m, const void* q, const void* k, const void*
 }
 
 cudaError_t walk_bwd_dkv(const Dims& m, const void* q, const void* k, const void* v, const void* d_o,
-                         const float* s, const float* suffix, void* dk, void* dv, cudaStream_t st) {
+                         const float* s, const float* suffix, void* dk, void* dv, bool add_dk, bool add_dv,
+                         cudaStream_t st) {
   WalkArgs a = {};
+  a.add_out = add_dk, a.add_out2 = add_dv;
   a.s = s, a.p0 = suffix;
 #define LASP_CALL(DD, EE) launch_walk_dkv<DD, EE, false>(m, q, k, v, d_o, dk, dv, a, st)
   LASP_DISPATCH_DE(m, LASP_CALL);
@@ -1754,8 +1770,10 @@ cudaError_t walk_bwd_dkv(const Dims& m, const void* q, const void* k, const void
 
 cudaError_t walk_bwd_dkv_fused(const Dims& m, const void* q, const void* k, const void* v, const void* d_o,
                                const float* s, const float* x_in, float* x_out, uint32_t* sync, float* totals,
-                               void* dk, void* dv, const lasp_exchange_args* link, cudaStream_t st) {
+                               void* dk, void* dv, const lasp_exchange_args* link, bool add_dk, bool add_dv,
+                               cudaStream_t st) {
   WalkArgs a = {};
+  a.add_out = add_dk, a.add_out2 = add_dv;
   a.link = make_link(link);
   a.s = s, a.x_in = x_in, a.x_out = x_out, a.sync = sync, a.totals = totals;
 #define LASP_CALL(DD, EE) launch_walk_dkv<DD, EE, true>(m, q, k, v, d_o, dk, dv, a, st)
