@@ -1,5 +1,5 @@
-"""Shared machinery of the five operators: head-dim slicing, the single-device
-autograd function and the sequence-parallel autograd function.
+"""Shared machinery of the five operators: the way to the native single-device operator, head-dim slicing and
+the sequence-parallel autograd function.
 
 The kernels are reached through ``ENGINE`` (module ``lasp_b200.engine``, the
 ctypes launcher of the CUDA library).  The host-logic tests replace ``ENGINE``
@@ -120,92 +120,6 @@ def _check_shapes(q, k, v, s):
         raise ValueError(f"batch x heads = {q.shape[0] * q.shape[1]} exceeds 65535")
 
 
-class LightningAttention(torch.autograd.Function):
-    """Single-device op: O = ((Q K^T) * M) V.  Interface of LightningAttention,
-    lasp/lightning_attention.py:396-504; gradients for q, k, v only.
-
-    Head dimensions wider than 128 are cut here, inside the function, the way the reference's wrapper cuts
-    them (lasp/lightning_attention.py:510-531: a sum over 128-wide q,k slices; v slices side by side) - but
-    the slices' results go straight into their place in o, dq, dk, dv.  Slicing outside, through autograd,
-    builds a full-size zero tensor per slice and adds them up: at d = e = 256 that costs more memory traffic
-    than the operator itself.
-    """
-
-    @staticmethod
-    def forward(ctx, q, k, v, s, qk_scale=1.0, feature_map=None):
-        _check_shapes(q, k, v, s)
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        d, e = q.shape[-1], v.shape[-1]
-        ctx.pre = (qk_scale, feature_map)
-        ctx.save_for_backward(q, k, v, s)
-        if d <= MAX_HEAD_SLICE and e <= MAX_HEAD_SLICE:
-            plan = _plan_for(q, v, qk_scale=qk_scale, feature_map=feature_map)
-            fw = ENGINE.Forward(plan, q, k, v, s)
-            ctx.pairs = None
-            ctx.plan, ctx.fwd_ws = plan, fw.ws
-            return fw.run()
-        o = torch.empty(*q.shape[:3], e, dtype=q.dtype, device=q.device)
-        # Where the kernels take a row pitch (tensor-core path), a slice is read and written where it lies in the
-        # wide tensors; otherwise it is copied out and back.
-        in_place = _slices_in_place(q, v, qk_scale, feature_map)
-        ctx.in_place = in_place
-        ctx.pairs = []                                   # (q/k slice, v slice, plan, forward workspace)
-        # in place, every tensor of a call has the wide tensors' row pitch: later contributions to a slice of o land
-        # in a slice of a second wide tensor and are added from there
-        more = torch.empty_like(o) if (in_place and len(_cuts(d)) > 1) else None
-        for e0, e1 in _cuts(e):
-            vs = v[..., e0:e1] if in_place else v[..., e0:e1].contiguous()
-            for i, (d0, d1) in enumerate(_cuts(d)):
-                qs, ks = (q[..., d0:d1], k[..., d0:d1]) if in_place else (q[..., d0:d1].contiguous(), k[..., d0:d1].contiguous())
-                plan = _slice_plan(q, v, d1 - d0, e1 - e0, qk_scale, feature_map, in_place)
-                first = i == 0
-                fw = ENGINE.Forward(plan, qs, ks, vs, s,
-                                    o=None if not in_place else (o if first else more)[..., e0:e1])
-                part = fw.run()
-                if not first:
-                    o[..., e0:e1] += part
-                elif not in_place:
-                    o[..., e0:e1] = part
-                ctx.pairs.append(((d0, d1), (e0, e1), plan, fw.ws))
-        return o
-
-    @staticmethod
-    def backward(ctx, do):
-        q, k, v, s = ctx.saved_tensors
-        do = do.contiguous()
-        if ctx.pairs is None:
-            bw = ENGINE.Backward(ctx.plan, q, k, v, do, s, ctx.fwd_ws)
-            dq, dk, dv = bw.run()
-            return dq, dk, dv, None, None, None
-        in_place = ctx.in_place
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        # (as in forward: later contributions go through second wide tensors with the same row pitch)
-        mq, mk, mv = (torch.empty_like(t) for t in (q, k, v)) if in_place else (None, None, None)
-        seen_d, seen_e = set(), set()
-        cut = (lambda t, lo, hi: t[..., lo:hi]) if in_place else (lambda t, lo, hi: t[..., lo:hi].contiguous())
-        for (d0, d1), (e0, e1), plan, fwd_ws in ctx.pairs:
-            new_d, new_e = d0 not in seen_d, e0 not in seen_e
-            # a q/k slice collects from every v slice, a v slice from every q/k slice: the first contribution is
-            # written in place (where the kernels can), the later ones are added
-            bw = ENGINE.Backward(plan, cut(q, d0, d1), cut(k, d0, d1), cut(v, e0, e1), cut(do, e0, e1), s, fwd_ws,
-                                 dq=None if not in_place else (dq if new_d else mq)[..., d0:d1],
-                                 dk=None if not in_place else (dk if new_d else mk)[..., d0:d1],
-                                 dv=None if not in_place else (dv if new_e else mv)[..., e0:e1])
-            gq, gk, gv = bw.run()
-            if not new_d:
-                dq[..., d0:d1] += gq
-                dk[..., d0:d1] += gk
-            elif not in_place:
-                dq[..., d0:d1] = gq
-                dk[..., d0:d1] = gk
-            if not new_e:
-                dv[..., e0:e1] += gv
-            elif not in_place:
-                dv[..., e0:e1] = gv
-            seen_d.add(d0), seen_e.add(e0)
-        return dq, dk, dv, None, None, None
-
-
 def _slice_plan(q, v, wd, we, qk_scale, feature_map, in_place):
     b, h, n = q.shape[:3]
     pitches = dict(pitch_d=q.shape[-1], pitch_e=v.shape[-1]) if in_place else {}
@@ -223,6 +137,31 @@ def _slices_in_place(q, v, qk_scale, feature_map) -> bool:
     except (ENGINE.LaspStatusError, TypeError):
         return False
     return True
+
+
+_QK_MAPS = {None: 0, "elu1": 1}
+_attention = None   # lasp_b200._torch_ops.attention, looked up at the first call
+
+
+def _load_attention():
+    global _attention
+    try:
+        from . import _torch_ops
+    except ImportError as exc:
+        from ._cabi import LaspLibraryError
+        raise LaspLibraryError("the native operator lasp_b200/_torch_ops.so is missing or does not load: build it with "
+                               f"`python -m lasp_b200.build` (there is no fallback): {exc}") from exc
+    _attention = _torch_ops.attention
+    return _attention
+
+
+def lightning(q, k, v, s, qk_scale=1.0, feature_map=None):
+    """Single-device op: O = ((Q K^T) * M) V on qk_scale * map(q), qk_scale * map(k).  Interface of
+    LightningAttention, lasp/lightning_attention.py:396-504; gradients for q, k, v only.  Everything between this
+    call and the kernels is native code (csrc/torch_ops.cpp)."""
+    if feature_map not in _QK_MAPS:
+        raise ValueError(f"unknown feature map {feature_map!r}; use None or 'elu1'")
+    return (_attention or _load_attention())(q, k, v, s, float(qk_scale), _QK_MAPS[feature_map])
 
 
 class SequenceParallelAttention(torch.autograd.Function):
@@ -254,9 +193,7 @@ class SequenceParallelAttention(torch.autograd.Function):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         b, h, n, d = q.shape
         e = v.shape[-1]
-        for name, buf in (("KV", KV), ("DKV", DKV)):
-            if tuple(buf.shape) != (b, h, d, e) or buf.dtype != torch.float32 or not buf.is_contiguous():
-                raise ValueError(f"{name} must be a contiguous float32 tensor of shape {(b, h, d, e)}")
+        _check_state_buffers(q, v, KV, DKV)
         group = get_sequence_parallel_group()
         rank = get_sequence_parallel_rank()
         last = get_sequence_parallel_world_size() - 1
@@ -342,7 +279,34 @@ class SequenceParallelAttention(torch.autograd.Function):
         return bw.dq, bw.dk, bw.dv, None, None, None, None, None, None
 
 
+def _check_state_buffers(q, v, KV, DKV):
+    shape = (q.shape[0], q.shape[1], q.shape[3], v.shape[3])
+    for name, buf in (("KV", KV), ("DKV", DKV)):
+        if tuple(buf.shape) != shape or buf.dtype != torch.float32 or not buf.is_contiguous():
+            raise ValueError(f"{name} must be a contiguous float32 tensor of shape {shape}")
+
+
+def _alone(q) -> bool:
+    """A rank that is its whole sequence-parallel group (a purely data-parallel job) has nobody to exchange a
+    state with: the operator is the single-device one, in one launch forward and two backward instead of the
+    phase-by-phase schedule's three and four."""
+    return q.is_cuda and get_sequence_parallel_world_size() == 1
+
+
+def sequence_parallel_slice(q, k, v, s, KV, DKV, overlap: bool):
+    """The autograd function itself (head dimensions of one slice at most)."""
+    if q.dim() == 4 and v.dim() == 4 and max(q.shape[-1], v.shape[-1]) <= MAX_HEAD_SLICE and _alone(q):
+        _check_shapes(q, k, v, s)
+        _check_state_buffers(q, v, KV, DKV)
+        return lightning(q, k, v, s)
+    return SequenceParallelAttention.apply(q, k, v, s, KV, DKV, overlap)
+
+
 def sequence_parallel(q, k, v, s, KV, DKV, overlap: bool):
+    if _alone(q):
+        _check_shapes(q, k, v, s)
+        _check_state_buffers(q, v, KV, DKV)
+        return lightning(q, k, v, s)
     return sliced_apply(lambda qs, ks, vs, kv, dkv: SequenceParallelAttention.apply(qs, ks, vs, s, kv, dkv, overlap),
                         q, k, v, (KV, DKV))
 
@@ -358,15 +322,17 @@ def lightning_attn_fused(q, k, v, s, qk_scale: float = 1.0, feature_map=None):
     between.  ``feature_map``: None or "elu1" (elu(x) + 1); ``qk_scale``: c.  Problems whose kernels cannot
     do this (fp32 path, head dims other than 64 / 128 per slice, more spans than SMs) get the same result from
     torch operations in front of the operator."""
-    if (qk_scale == 1.0 and feature_map is None) or not kernels_preprocess(*_slice_like(q, v), qk_scale, feature_map):
-        return LightningAttention.apply(preprocess_qk(q, qk_scale, feature_map), preprocess_qk(k, qk_scale, feature_map), v, s)
-    return LightningAttention.apply(q, k, v, s, qk_scale, feature_map)
+    return lightning(q, k, v, s, qk_scale, feature_map)
 
 
 def sequence_parallel_fused(q, k, v, s, KV, DKV, qk_scale: float = 1.0, feature_map=None):
     """``lasp_fuse_parallel`` on c * map(q), c * map(k) with the preprocessing inside the kernels where the
     rank's launches are the fused ones that hand the state over themselves; torch operations otherwise."""
     qs, vs = _slice_like(q, v)
+    if _alone(q):
+        _check_shapes(q, k, v, s)
+        _check_state_buffers(q, v, KV, DKV)
+        return lightning(q, k, v, s, qk_scale, feature_map)
     in_kernel = (qk_scale != 1.0 or feature_map is not None) and kernels_preprocess(qs, vs, qk_scale, feature_map)
     if in_kernel and get_sequence_parallel_world_size() > 1:
         b, h, n, d = qs.shape

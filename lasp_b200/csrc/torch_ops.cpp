@@ -1,0 +1,359 @@
+// The single-device operator as PyTorch sees it: argument checks, head-dimension slices, allocation, the C-ABI
+// calls and the autograd node, in native code.  The kernels of an ordinary layer take tens of microseconds; the same
+// steps as a Python autograd function with ctypes calls took the host about 210 us for a forward and a backward
+// pass (57 us for a forward pass alone) and set the pace of every call below about 50 MB of inputs.
+//
+// Interface of LightningAttention, lasp/lightning_attention.py:396-504, with the wrapper's head-dimension slicing
+// (:510-531: a sum over 128-wide q,k slices, v slices side by side): every 128-wide slice pair is read and written
+// where it lies in the wide tensors (row pitch in the problem), later contributions to a slice of o, dq, dk, dv
+// are added by the kernels' own stores.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAGraphsUtils.cuh>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <nvtx3/nvToolsExt.h>
+
+#include <cmath>
+#include <cstdlib>
+#include <cstring>
+#include <deque>
+#include <mutex>
+#include <utility>
+#include <vector>
+
+#include "lasp_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+constexpr int64_t kSlice = 128;      // widest q/k (d) or v (e) slice one kernel call takes
+constexpr int64_t kSyncBytes = 4096; // synchronisation words of a launch (lasp_call_options.sync)
+
+struct Range {   // NVTX range around a library call (LASP_B200_NVTX=1)
+  bool on;
+  explicit Range(const char* name) : on(enabled()) {
+    if (on) nvtxRangePushA(name);
+  }
+  ~Range() {
+    if (on) nvtxRangePop();
+  }
+  static bool enabled() {
+    static const bool v = [] {
+      const char* e = std::getenv("LASP_B200_NVTX");
+      return e && e[0] == '1';
+    }();
+    return v;
+  }
+};
+
+// A negative status becomes lasp_b200._cabi.LaspStatusError, on whatever thread this is (autograd's workers too).
+void check_status(const char* fn, int status) {
+  if (status >= 0) return;
+  std::string text = lasp_b200_strerror(status);
+  if (status == LASP_ERR_CUDA) text += std::string(": ") + lasp_b200_last_cuda_error();
+  PyGILState_STATE gil = PyGILState_Ensure();
+  PyObject* mod = PyImport_ImportModule("lasp_b200._cabi");
+  PyObject* cls = mod ? PyObject_GetAttrString(mod, "LaspStatusError") : nullptr;
+  PyObject* exc = cls ? PyObject_CallFunction(cls, "sis", fn, status, text.c_str()) : nullptr;
+  if (exc) PyErr_SetObject(cls, exc);
+  Py_XDECREF(exc);
+  Py_XDECREF(cls);
+  Py_XDECREF(mod);
+  python_error err;
+  err.persist();
+  PyGILState_Release(gil);
+  throw err;
+}
+
+int32_t lasp_dtype_of(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return LASP_F32;
+    case at::kBFloat16: return LASP_BF16;
+    case at::kHalf: return LASP_F16;
+    default: TORCH_CHECK_TYPE(false, "unsupported dtype ", t, "; use float32, bfloat16 or float16");
+  }
+}
+
+int32_t requested_path() {   // env LASP_B200_PATH, looked at on every call as the Python launcher does
+  const char* p = std::getenv("LASP_B200_PATH");
+  if (!p || !*p || !std::strcmp(p, "auto")) return LASP_PATH_AUTO;
+  if (!std::strcmp(p, "simt")) return LASP_PATH_SIMT;
+  if (!std::strcmp(p, "tensor")) return LASP_PATH_TENSOR;
+  TORCH_CHECK_VALUE(false, "unknown kernel path '", p, "'; use auto, simt or tensor");
+}
+
+// The 4 KB of synchronisation words of the current stream's launches: zeroed once, then kept consistent by the
+// kernels.  Launches of one stream do not overlap, so they share a block; a capturing stream gets a block per call,
+// zeroed by the graph itself, because the graph may be replayed anywhere.  At most kMaxBlocks are kept, the oldest
+// going first; a block comes from its stream's allocator pool, so giving it back is ordered behind its last use.
+Tensor sync_words(const at::Device& device, const at::cuda::CUDAStream& stream) {
+  const auto fresh = [&] { return at::zeros({kSyncBytes}, at::TensorOptions().dtype(at::kByte).device(device)); };
+  if (at::cuda::currentStreamCaptureStatusMayInitCtx() != at::cuda::CaptureStatus::None) return fresh();
+  struct Block {
+    int64_t device;
+    unsigned long long stream;
+    Tensor words;
+  };
+  constexpr size_t kMaxBlocks = 64;
+  static std::mutex lock;
+  static auto* blocks = new std::deque<Block>;   // never destroyed: the process may end after the CUDA context
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetId(stream.stream(), &id));   // unique, unlike a handle that a later stream may reuse
+  std::lock_guard<std::mutex> guard(lock);
+  for (const Block& b : *blocks)
+    if (b.stream == id && b.device == device.index()) return b.words;
+  if (blocks->size() >= kMaxBlocks) blocks->pop_front();
+  blocks->push_back({device.index(), id, fresh()});
+  return blocks->back().words;
+}
+
+struct Shape {
+  int64_t b, h, n, d, e;
+};
+
+Shape check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s) {
+  TORCH_CHECK_VALUE(q.dim() == 4 && k.sizes() == q.sizes() && v.dim() == 4 && v.sizes().slice(0, 3) == q.sizes().slice(0, 3),
+                    "expected q,k (b,h,n,d) and v (b,h,n,e); got ", q.sizes(), ", ", k.sizes(), ", ", v.sizes());
+  TORCH_CHECK_TYPE(k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(), "q, k, v must share one dtype");
+  TORCH_CHECK_VALUE(s.numel() == q.size(1), "decay tensor has ", s.numel(), " entries for ", q.size(1), " heads");
+  for (const auto& [name, width] : {std::pair<const char*, int64_t>{"q/k", q.size(3)}, {"v", v.size(3)}})
+    TORCH_CHECK_VALUE(width % 16 == 0, "head dimension of ", name, " is ", width, ": it must be a multiple of 16 (wider than ",
+                      kSlice, ": cut in ", kSlice, "-wide slices)");
+  TORCH_CHECK_VALUE(q.size(0) * q.size(1) <= 65535, "batch x heads = ", q.size(0) * q.size(1), " exceeds 65535");
+  lasp_dtype_of(q.scalar_type());
+  for (const Tensor* t : {&q, &k, &v})
+    TORCH_CHECK(t->is_cuda(), "lasp_b200 runs on CUDA tensors only (there is no CPU fallback); got a tensor on ", t->device());
+  return {q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
+}
+
+lasp_problem problem_of(const Shape& m, int64_t d, int64_t e, int32_t dtype, double scale, int64_t map, bool pitched) {
+  TORCH_CHECK_VALUE(m.n <= INT32_MAX, "sequence of ", m.n, " tokens is too long");
+  lasp_problem p = {};
+  p.b = (int32_t)m.b, p.h = (int32_t)m.h, p.n = (int32_t)m.n, p.d = (int32_t)d, p.e = (int32_t)e;
+  p.dtype = dtype, p.path = requested_path();
+  p.qk_map = (int32_t)map, p.qk_scale = (float)scale;
+  if (pitched) p.pitch_d = (int32_t)m.d, p.pitch_e = (int32_t)m.e;
+  return p;
+}
+
+// One 128-wide slice pair of the head dimensions: columns [d0, d1) of q,k and [e0, e1) of v.
+struct Pair {
+  int64_t d0, d1, e0, e1;
+  lasp_problem problem;
+  size_t ws_bytes;
+};
+
+// How a call is cut: `in_place` = the kernels take the slices where they lie in the wide tensors.
+struct Cut {
+  std::vector<Pair> pairs;
+  bool in_place = false;
+};
+
+bool resolve(lasp_problem& p) {
+  const int path = lasp_b200_resolve_path(&p);
+  if (path < 0) return false;
+  p.path = path;
+  return true;
+}
+
+Cut cut_call(const Shape& m, int32_t dtype, double scale, int64_t map) {
+  Cut c;
+  const auto fill = [&](bool pitched) {
+    c.pairs.clear();
+    for (int64_t e0 = 0; e0 < m.e; e0 += kSlice)
+      for (int64_t d0 = 0; d0 < m.d; d0 += kSlice) {
+        Pair p{d0, std::min(d0 + kSlice, m.d), e0, std::min(e0 + kSlice, m.e), {}, 0};
+        p.problem = problem_of(m, p.d1 - p.d0, p.e1 - p.e0, dtype, scale, map, pitched);
+        if (!resolve(p.problem)) {
+          if (pitched) return false;
+          check_status("lasp_b200_resolve_path", lasp_b200_resolve_path(&p.problem));
+        }
+        p.ws_bytes = lasp_b200_fwd_workspace_bytes(&p.problem);
+        c.pairs.push_back(p);
+      }
+    return true;
+  };
+  const bool wide = m.d > kSlice || m.e > kSlice;
+  c.in_place = wide && fill(true);
+  if (!c.in_place) fill(false);
+  return c;
+}
+
+char* column(const Tensor& t, int64_t col) { return static_cast<char*>(t.data_ptr()) + col * t.element_size(); }
+
+// A slice as a kernel call wants it: in place, or (kernels without a row pitch) a copy of its own.
+struct Slice {
+  Tensor copy;
+  void* ptr;
+};
+Slice slice_of(const Tensor& t, int64_t lo, int64_t hi, bool whole) {
+  if (whole) return {Tensor(), column(t, lo)};
+  Tensor c = t.slice(3, lo, hi).contiguous();
+  void* p = c.data_ptr();
+  return {std::move(c), p};
+}
+
+std::vector<Tensor> run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s, const Shape& m,
+                                double scale, int64_t map, bool keep) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  const Cut cut = cut_call(m, lasp_dtype_of(q.scalar_type()), scale, map);
+  const bool sliced = cut.pairs.size() > 1, whole = !sliced || cut.in_place;
+  Tensor o = at::empty({m.b, m.h, m.n, m.e}, q.options());
+  const Tensor sync = sync_words(q.device(), stream);
+  std::vector<Tensor> out{o};
+  Tensor ws;
+  for (const Pair& p : cut.pairs) {
+    // (nothing is kept without a backward pass: the slices then share a workspace)
+    if (keep || !ws.defined() || (size_t)ws.numel() < p.ws_bytes)
+      ws = at::empty({(int64_t)p.ws_bytes}, q.options().dtype(at::kByte));
+    if (keep) out.push_back(ws);
+    const Slice qs = slice_of(q, p.d0, p.d1, whole), ks = slice_of(k, p.d0, p.d1, whole), vs = slice_of(v, p.e0, p.e1, whole);
+    Tensor part = whole ? Tensor() : at::empty({m.b, m.h, m.n, p.e1 - p.e0}, q.options());
+    lasp_fwd_args a = {};
+    a.q = qs.ptr, a.k = ks.ptr, a.v = vs.ptr, a.s = s.const_data_ptr<float>();
+    a.o = whole ? column(o, p.e0) : part.data_ptr();
+    a.ws = ws.data_ptr(), a.ws_bytes = (size_t)ws.numel();
+    lasp_call_options opt = {};
+    opt.sync = static_cast<uint32_t*>(sync.data_ptr());
+    opt.keep_states = keep ? 1 : 0;
+    opt.accumulate = whole && p.d0 > 0 ? LASP_ACCUMULATE_V : 0;
+    Range range("lasp_b200_forward");
+    check_status("lasp_b200_forward", lasp_b200_forward_opt(&p.problem, &a, &opt, stream.stream()));
+    if (!whole) {
+      Tensor dst = o.slice(3, p.e0, p.e1);
+      if (p.d0 > 0)
+        dst.add_(part);
+      else
+        dst.copy_(part);
+    }
+  }
+  return out;
+}
+
+class Lightning : public torch::autograd::Function<Lightning> {
+ public:
+  static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s,
+                        double scale, int64_t map) {
+    const Shape m{q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
+    std::vector<Tensor> out = run_forward(q, k, v, s, m, scale, map, true);
+    variable_list saved{q, k, v, s};
+    saved.insert(saved.end(), out.begin() + 1, out.end());
+    ctx->save_for_backward(std::move(saved));
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["map"] = map;
+    return out[0];
+  }
+
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list saved = ctx->get_saved_variables();
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &s = saved[3];
+    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+    const Tensor d_o = grads[0].contiguous();
+    const Shape m{q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
+    const c10::cuda::CUDAGuard guard(q.device());
+    const auto stream = at::cuda::getCurrentCUDAStream();
+    const Cut cut = cut_call(m, lasp_dtype_of(q.scalar_type()), ctx->saved_data["scale"].toDouble(),
+                             ctx->saved_data["map"].toInt());
+    const bool sliced = cut.pairs.size() > 1, whole = !sliced || cut.in_place;
+    Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options()), dv = at::empty(v.sizes(), v.options());
+    const Tensor sync = sync_words(q.device(), stream);
+    Tensor ws;
+    for (size_t i = 0; i < cut.pairs.size(); ++i) {
+      const Pair& p = cut.pairs[i];
+      const Tensor& fwd_ws = saved[4 + i];
+      if (!ws.defined() || (size_t)ws.numel() < p.ws_bytes)
+        ws = at::empty({(int64_t)p.ws_bytes}, q.options().dtype(at::kByte));
+      const Slice qs = slice_of(q, p.d0, p.d1, whole), ks = slice_of(k, p.d0, p.d1, whole), vs = slice_of(v, p.e0, p.e1, whole),
+                  ds = slice_of(d_o, p.e0, p.e1, whole);
+      Tensor pq, pk, pv;
+      if (!whole) {
+        pq = at::empty({m.b, m.h, m.n, p.d1 - p.d0}, q.options());
+        pk = at::empty({m.b, m.h, m.n, p.d1 - p.d0}, q.options());
+        pv = at::empty({m.b, m.h, m.n, p.e1 - p.e0}, q.options());
+      }
+      lasp_bwd_args a = {};
+      a.q = qs.ptr, a.k = ks.ptr, a.v = vs.ptr, a.d_o = ds.ptr, a.s = s.const_data_ptr<float>();
+      a.dq = whole ? column(dq, p.d0) : pq.data_ptr();
+      a.dk = whole ? column(dk, p.d0) : pk.data_ptr();
+      a.dv = whole ? column(dv, p.e0) : pv.data_ptr();
+      a.fwd_ws = fwd_ws.data_ptr(), a.fwd_ws_bytes = (size_t)fwd_ws.numel();
+      a.ws = ws.data_ptr(), a.ws_bytes = (size_t)ws.numel();
+      lasp_call_options opt = {};
+      opt.sync = static_cast<uint32_t*>(sync.data_ptr());
+      // a q/k slice collects from every v slice, a v slice from every q/k slice
+      if (whole) opt.accumulate = (p.e0 > 0 ? LASP_ACCUMULATE_QK : 0) | (p.d0 > 0 ? LASP_ACCUMULATE_V : 0);
+      {
+        Range range("lasp_b200_backward");
+        check_status("lasp_b200_backward", lasp_b200_backward_opt(&p.problem, &a, &opt, stream.stream()));
+      }
+      if (!whole) {
+        const auto put = [](Tensor dst, const Tensor& part, bool add) { add ? dst.add_(part) : dst.copy_(part); };
+        put(dq.slice(3, p.d0, p.d1), pq, p.e0 > 0);
+        put(dk.slice(3, p.d0, p.d1), pk, p.e0 > 0);
+        put(dv.slice(3, p.e0, p.e1), pv, p.d0 > 0);
+      }
+    }
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor preprocess(const Tensor& x, double scale, int64_t map) {   // what a caller would write in front of the operator
+  Tensor y = map ? at::elu(x) + 1.0 : x;
+  return scale == 1.0 ? y : y * scale;
+}
+
+Tensor attention(Tensor q, Tensor k, Tensor v, const Tensor& ed, double scale, int64_t map) {
+  const Shape m = check_inputs(q, k, v, ed);
+  if (scale != 1.0 || map != 0) {
+    // kernels that cannot take the preprocessing over get preprocessed tensors
+    lasp_problem p = problem_of(m, std::min(m.d, kSlice), std::min(m.e, kSlice), lasp_dtype_of(q.scalar_type()), scale, map, false);
+    if (!resolve(p)) q = preprocess(q, scale, map), k = preprocess(k, scale, map), scale = 1.0, map = 0;
+  }
+  Tensor s = ed.detach().reshape({-1});
+  if (s.device() != q.device() || s.scalar_type() != at::kFloat) s = s.to(q.device(), at::kFloat);
+  s = s.contiguous();
+  q = q.contiguous(), k = k.contiguous(), v = v.contiguous();
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
+    return Lightning::apply(q, k, v, s, scale, map);
+  return run_forward(q, k, v, s, m, scale, map, false)[0];
+}
+
+// attention(q, k, v, s, qk_scale, map) -> o
+PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK_TYPE(nargs == 6, "attention(q, k, v, s, qk_scale, map) takes 6 arguments");
+  for (int i = 0; i < 4; ++i)
+    TORCH_CHECK_TYPE(THPVariable_Check(args[i]), "q, k, v and the decay rates must be tensors");
+  const double scale = PyFloat_AsDouble(args[4]);
+  const long map = PyLong_AsLong(args[5]);
+  if (PyErr_Occurred()) return nullptr;
+  const Tensor &q = THPVariable_Unpack(args[0]), &k = THPVariable_Unpack(args[1]), &v = THPVariable_Unpack(args[2]),
+               &s = THPVariable_Unpack(args[3]);
+  Tensor o;
+  {
+    pybind11::gil_scoped_release no_gil;
+    o = attention(q, k, v, s, scale, map);
+  }
+  return THPVariable_Wrap(std::move(o));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef kMethods[] = {
+    {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention)), METH_FASTCALL,
+     "attention(q, k, v, s, qk_scale, map) -> o: decay-masked causal linear attention on scale * map(q), scale * map(k)"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_torch_ops", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__torch_ops(void) { return PyModule_Create(&kModule); }

@@ -6,11 +6,11 @@ kernels compute positions themselves.  The outgoing state always starts from a
 defined value (the reference's kernel reads an uninitialised buffer there,
 lasp/lasp_cache.py:104-106,438).
 """
-from ._core import SequenceParallelAttention, sequence_parallel
+from ._core import sequence_parallel, sequence_parallel_slice
 
 
 def lasp_cache_(q, k, v, s, array, KV, DKV):
-    return SequenceParallelAttention.apply(q, k, v, s, KV, DKV, False)
+    return sequence_parallel_slice(q, k, v, s, KV, DKV, False)
 
 
 def lasp_cache(q, k, v, ed, array, KV, DKV):

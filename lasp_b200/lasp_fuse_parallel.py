@@ -6,11 +6,11 @@ rank state is posted before the chunk-state kernel and the send right after
 the scan, so neighbouring ranks overlap everything but the scan.  No
 world-wide barrier is issued (the reference calls one per forward, :1094).
 """
-from ._core import SequenceParallelAttention, sequence_parallel
+from ._core import sequence_parallel, sequence_parallel_slice
 
 
 def lasp_fuse_parallel_(q, k, v, s, KV, DKV):
-    return SequenceParallelAttention.apply(q, k, v, s, KV, DKV, True)
+    return sequence_parallel_slice(q, k, v, s, KV, DKV, True)
 
 
 def lasp_fuse_parallel(q, k, v, ed, KV, DKV):

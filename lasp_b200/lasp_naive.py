@@ -5,7 +5,7 @@ here, the KV state is received before the local kernels run and sent after.
 """
 import torch
 
-from ._core import SequenceParallelAttention, sequence_parallel
+from ._core import sequence_parallel, sequence_parallel_slice
 
 
 def lasp_naive_(q, k, v, s):
@@ -13,7 +13,7 @@ def lasp_naive_(q, k, v, s):
     e = v.shape[-1]
     KV = torch.empty(b, h, d, e, dtype=torch.float32, device=q.device)
     DKV = torch.empty(b, h, d, e, dtype=torch.float32, device=q.device)
-    return SequenceParallelAttention.apply(q, k, v, s, KV, DKV, False)
+    return sequence_parallel_slice(q, k, v, s, KV, DKV, False)
 
 
 def lasp_naive(q, k, v, ed):

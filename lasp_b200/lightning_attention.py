@@ -3,9 +3,7 @@
 Drop-in for ``lasp/lightning_attention.py`` of the reference: ``lightning_attn``
 (:510-531) and ``lightning_attn_`` (= the autograd function's ``apply``, :507).
 """
-from ._core import LightningAttention
-
-lightning_attn_ = LightningAttention.apply
+from ._core import lightning as lightning_attn_
 
 
 def lightning_attn(q, k, v, ed):
