@@ -64,7 +64,7 @@ typedef enum { LASP_F32 = 0, LASP_BF16 = 1, LASP_F16 = 2 } lasp_dtype;
 /* which kernels run: AUTO picks TENSOR when the problem qualifies */
 typedef enum {
   LASP_PATH_AUTO = 0,
-  LASP_PATH_SIMT = 1,   /* fp32 FFMA kernels: any dtype, d,e multiples of 16 up to 128, any n */
+  LASP_PATH_SIMT = 1,   /* full-precision kernels: any dtype, d,e multiples of 16 up to 128, any n */
   LASP_PATH_TENSOR = 2  /* tcgen05/TMEM/TMA kernels: bf16, d,e in {64,128}, n >= 128 (a ragged tail is fine) */
 } lasp_path;
 
@@ -86,7 +86,7 @@ typedef struct {
   /* Elements from one token's row to the next in q,k,dq,dk (pitch_d) and in v,o,do,dv (pitch_e); 0 = d / e, i.e.
    * tensors of their own.  Larger values let a call work in place on a 128-wide slice of the head dimension of
    * wider tensors (the slicing of lasp/lightning_attention.py:510-531 without a copy per slice): pass the address
-   * of the slice's first column.  Multiples of 8; tensor-core path only (LASP_ERR_PATH otherwise). */
+   * of the slice's first column.  Multiples of 8. */
   int32_t pitch_d, pitch_e;
 } lasp_problem;
 
@@ -187,7 +187,7 @@ LASP_B200_API int lasp_b200_bwd_dkv_walk(const lasp_problem* p, const lasp_bwd_a
  * slices of wide heads itself (lasp_forward / lasp_backward, lasp/lasp_fuse.py:356-475). */
 enum {
   LASP_ACCUMULATE_QK = 1, /* add to what dq, dk hold (rounded to the tensors' type) instead of overwriting it */
-  LASP_ACCUMULATE_V = 2   /* the same for o and dv; both on the tensor-core path only (LASP_ERR_PATH otherwise) */
+  LASP_ACCUMULATE_V = 2   /* the same for o and dv */
 };
 typedef struct {
   uint32_t* sync;      /* 4 KB of device memory, zeroed once: the words the CTAs of a launch synchronise through,
@@ -195,6 +195,8 @@ typedef struct {
                         * block must not overlap on the GPU (one block per stream).  NULL = those of ws. */
   int32_t keep_states; /* forward: leave the states the backward pass reads in ws (0: nothing is kept) */
   int32_t accumulate;  /* LASP_ACCUMULATE_* */
+  int32_t alone;       /* no rank state in either direction of this problem (kv_in, kv_out, dkv_in, dkv_out NULL in
+                        * the forward AND the backward call): states at the sequence's ends are skipped */
 } lasp_call_options;
 LASP_B200_API int lasp_b200_forward_opt(const lasp_problem* p, const lasp_fwd_args* a, const lasp_call_options* opt,
                                         void* stream);

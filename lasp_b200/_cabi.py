@@ -54,7 +54,7 @@ class BwdArgs(C.Structure):
 
 
 class CallOptions(C.Structure):   # lasp_call_options
-    _fields_ = [("sync", C.c_void_p), ("keep_states", C.c_int32), ("accumulate", C.c_int32)]
+    _fields_ = [("sync", C.c_void_p), ("keep_states", C.c_int32), ("accumulate", C.c_int32), ("alone", C.c_int32)]
 
 
 class ExchangeArgs(C.Structure):

@@ -19,7 +19,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "liblasp_b200.so")
 TORCH_OPS = os.path.join(PKG, "_torch_ops.so")   # the operator as PyTorch calls it, on top of LIB
-SOURCES = ["api.cu", "simt_kernels.cu", "fault_word.cu", "walk_kernels.cu", "relay_kernels.cu", "static_scratch.cu"]
+SOURCES = ["api.cu", "split_kernels.cu", "state_kernels.cu", "fault_word.cu", "walk_kernels.cu", "relay_kernels.cu", "static_scratch.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -85,7 +85,7 @@ def build_torch_ops(force: bool = False) -> None:
     include = [os.path.join(ROOT, "include"), os.path.join(base, "include"),
                os.path.join(base, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
                sysconfig.get_paths()["include"]]
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-o", TORCH_OPS, src]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wno-interference-size", "-o", TORCH_OPS, src]
     cmd += [x for d in include for x in ("-I", d)]
     cmd += ["-L", PKG, "-l:liblasp_b200.so", "-L", os.path.join(base, "lib"), "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
             "-ltorch_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]

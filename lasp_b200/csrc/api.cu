@@ -1,5 +1,5 @@
 // extern "C" entry points of liblasp_b200.so: argument validation, workspace
-// layout and the choice between the tensor-core and the fp32 kernels.
+// layout and the choice between the walk kernels and the full-precision kernels.
 #include <stdio.h>
 #include <string.h>
 
@@ -101,8 +101,7 @@ int make_dims(const lasp_problem* p, lasp::Dims* m) {
   m->path = path;
   if (path == LASP_PATH_SIMT) {
     if (lasp::has_qk_preprocessing(*m)) return LASP_ERR_PATH;   // folded into the tensor-core kernels only
-    if (m->pitch_d != m->d || m->pitch_e != m->e) return LASP_ERR_PATH;   // slices in place: TMA tensor maps only
-    m->chunk = lasp::kSimtChunk;
+    m->chunk = lasp::kTensorTile;
     m->nc = (p->n + m->chunk - 1) / m->chunk;
     return LASP_OK;
   }
@@ -127,6 +126,7 @@ int make_dims(const lasp_problem* p, lasp::Dims* m) {
 
 size_t workspace_bytes(const lasp::Dims& m) {
   size_t s = lasp::state_elems(m);
+  if (!m.walk) s = (size_t)m.b * m.h * ((m.n + lasp::kAbiChunk - 1) / lasp::kAbiChunk) * m.d * m.e;
   size_t bytes = 2 * s * 4;  // local + prefix states
   if (m.walk) bytes += lasp::kWalkSyncBytes;
   return (bytes + 255) & ~(size_t)255;
@@ -163,11 +163,11 @@ int check_bwd(const lasp_problem* p, const lasp_bwd_args* a, lasp::Dims* m, bool
   return LASP_OK;
 }
 
-int check_options(const lasp::Dims& m, const lasp_call_options* opt) {
+int check_options(const lasp_call_options* opt, bool rank_state) {
   if (!opt) return LASP_ERR_NULL;
   if (!aligned16(opt->sync)) return LASP_ERR_ALIGN;
+  if (opt->alone && rank_state) return LASP_ERR_SHAPE;
   if (opt->accumulate & ~(LASP_ACCUMULATE_QK | LASP_ACCUMULATE_V)) return LASP_ERR_SHAPE;
-  if (opt->accumulate && !m.walk) return LASP_ERR_PATH;   // the TMA stores of the walk kernels add
   return LASP_OK;
 }
 
@@ -204,7 +204,7 @@ int lasp_b200_resolve_path(const lasp_problem* p) {
 int lasp_b200_chunk_tokens(const lasp_problem* p) {
   lasp::Dims m;
   int st = make_dims(p, &m);
-  return st != LASP_OK ? st : m.chunk;
+  return st != LASP_OK ? st : m.walk ? m.chunk : lasp::kAbiChunk;
 }
 
 size_t lasp_b200_fwd_workspace_bytes(const lasp_problem* p) {
@@ -218,12 +218,15 @@ size_t lasp_b200_bwd_workspace_bytes(const lasp_problem* p) { return lasp_b200_f
 
 namespace {
 
-constexpr lasp_call_options kPlainCall = {nullptr, 1, 0};
+// a single chunk with no rank state: nothing to carry from chunk to chunk
+bool stateless(const lasp::Dims& m, const lasp_call_options& opt) { return !m.walk && m.nc == 1 && opt.alone; }
 
-int fwd_chunk_states(const lasp::Dims& m, const lasp_fwd_args* a, cudaStream_t cs) {
+constexpr lasp_call_options kPlainCall = {nullptr, 1, 0, 0};
+
+int fwd_chunk_states(const lasp::Dims& m, const lasp_fwd_args* a, const lasp_call_options& opt, cudaStream_t cs) {
   if (lasp::has_qk_preprocessing(m)) return LASP_ERR_PATH;
   if (m.walk) return cuda_fail(lasp::walk_span_totals(m, a->k, a->v, a->s, lasp::ws_local(a->ws, m), false, cs));
-  return cuda_fail(lasp::simt_chunk_states(m, a->k, a->v, a->s, lasp::ws_local(a->ws, m), false, cs));
+  return cuda_fail(lasp::split_chunk_states(m, a->k, a->v, a->s, lasp::ws_local(a->ws, m), false, opt.alone != 0, cs));
 }
 
 int fwd_scan(const lasp::Dims& m, const lasp_fwd_args* a, cudaStream_t cs) {
@@ -238,13 +241,14 @@ int fwd_output(const lasp::Dims& m, const lasp_fwd_args* a, const lasp_call_opti
     return cuda_fail(lasp::walk_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_walk_border(a->ws, m),
                                            opt.sync ? opt.sync : lasp::ws_walk_sync(a->ws), a->o,
                                            (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
-  return cuda_fail(lasp::simt_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_prefix(a->ws, m), a->o, cs));
+  return cuda_fail(lasp::split_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_prefix(a->ws, m), a->o, opt.alone != 0,
+                                          (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
 }
 
-int bwd_chunk_states(const lasp::Dims& m, const lasp_bwd_args* a, cudaStream_t cs) {
+int bwd_chunk_states(const lasp::Dims& m, const lasp_bwd_args* a, const lasp_call_options& opt, cudaStream_t cs) {
   if (lasp::has_qk_preprocessing(m)) return LASP_ERR_PATH;
   if (m.walk) return cuda_fail(lasp::walk_span_totals(m, a->q, a->d_o, a->s, lasp::ws_local(a->ws, m), true, cs));
-  return cuda_fail(lasp::simt_chunk_states(m, a->q, a->d_o, a->s, lasp::ws_local(a->ws, m), true, cs));
+  return cuda_fail(lasp::split_chunk_states(m, a->q, a->d_o, a->s, lasp::ws_local(a->ws, m), true, opt.alone != 0, cs));
 }
 
 int bwd_scan(const lasp::Dims& m, const lasp_bwd_args* a, cudaStream_t cs) {
@@ -264,8 +268,10 @@ int bwd_grads(const lasp::Dims& m, const lasp_bwd_args* a, const lasp_call_optio
     return cuda_fail(lasp::walk_bwd_dkv(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->ws, m), a->dk,
                                         a->dv, add_qk, add_v, cs));
   }
-  return cuda_fail(lasp::simt_bwd_grads(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_prefix(a->fwd_ws, m),
-                                        lasp::ws_prefix(a->ws, m), a->dq, a->dk, a->dv, cs));
+  return cuda_fail(lasp::split_bwd_grads(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_prefix(a->fwd_ws, m),
+                                         lasp::ws_prefix(a->ws, m), a->dq, a->dk, a->dv, opt.alone != 0,
+                                         (opt.accumulate & LASP_ACCUMULATE_QK) != 0,
+                                         (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
 }
 
 }  // namespace
@@ -276,7 +282,7 @@ extern "C" {
 int lasp_b200_fwd_chunk_states(const lasp_problem* p, const lasp_fwd_args* a, void* stream) {
   lasp::Dims m;
   int st = check_fwd(p, a, &m, false);
-  return st != LASP_OK ? st : fwd_chunk_states(m, a, static_cast<cudaStream_t>(stream));
+  return st != LASP_OK ? st : fwd_chunk_states(m, a, kPlainCall, static_cast<cudaStream_t>(stream));
 }
 
 int lasp_b200_fwd_scan(const lasp_problem* p, const lasp_fwd_args* a, void* stream) {
@@ -295,7 +301,7 @@ int lasp_b200_forward_opt(const lasp_problem* p, const lasp_fwd_args* a, const l
   lasp::Dims m;
   int st = check_fwd(p, a, &m, true);
   if (st != LASP_OK) return st;
-  if ((st = check_options(m, opt)) != LASP_OK) return st;
+  if ((st = check_options(opt, a->kv_in || a->kv_out)) != LASP_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   if (fusable(m))
     return cuda_fail(lasp::walk_fwd_fused(m, a->q, a->k, a->v, a->s, a->kv_in, a->kv_out,
@@ -303,8 +309,10 @@ int lasp_b200_forward_opt(const lasp_problem* p, const lasp_fwd_args* a, const l
                                           lasp::ws_walk_totals(a->ws),
                                           opt->keep_states ? lasp::ws_walk_border(a->ws, m) : nullptr, a->o, nullptr,
                                           (opt->accumulate & LASP_ACCUMULATE_V) != 0, cs));
-  if ((st = fwd_chunk_states(m, a, cs)) != LASP_OK) return st;
-  if ((st = fwd_scan(m, a, cs)) != LASP_OK) return st;
+  if (!stateless(m, *opt)) {
+    if ((st = fwd_chunk_states(m, a, *opt, cs)) != LASP_OK) return st;
+    if ((st = fwd_scan(m, a, cs)) != LASP_OK) return st;
+  }
   return fwd_output(m, a, *opt, cs);
 }
 
@@ -316,7 +324,7 @@ int lasp_b200_forward(const lasp_problem* p, const lasp_fwd_args* a, void* strea
 int lasp_b200_bwd_chunk_states(const lasp_problem* p, const lasp_bwd_args* a, void* stream) {
   lasp::Dims m;
   int st = check_bwd(p, a, &m, false);
-  return st != LASP_OK ? st : bwd_chunk_states(m, a, static_cast<cudaStream_t>(stream));
+  return st != LASP_OK ? st : bwd_chunk_states(m, a, kPlainCall, static_cast<cudaStream_t>(stream));
 }
 
 int lasp_b200_bwd_scan(const lasp_problem* p, const lasp_bwd_args* a, void* stream) {
@@ -367,7 +375,7 @@ int lasp_b200_backward_opt(const lasp_problem* p, const lasp_bwd_args* a, const 
   lasp::Dims m;
   int st = check_bwd(p, a, &m, true);
   if (st != LASP_OK) return st;
-  if ((st = check_options(m, opt)) != LASP_OK) return st;
+  if ((st = check_options(opt, a->dkv_in || a->dkv_out)) != LASP_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   if (fusable(m)) {
     // dQ walks forward over the border states the forward pass kept; dK, dV walk backward in one fused launch.
@@ -380,8 +388,10 @@ int lasp_b200_backward_opt(const lasp_problem* p, const lasp_bwd_args* a, const 
                                               opt->sync ? opt->sync : lasp::ws_walk_sync(a->ws),
                                               lasp::ws_walk_totals(a->ws), a->dk, a->dv, nullptr, add_qk, add_v, cs));
   }
-  if ((st = bwd_chunk_states(m, a, cs)) != LASP_OK) return st;
-  if ((st = bwd_scan(m, a, cs)) != LASP_OK) return st;
+  if (!stateless(m, *opt)) {
+    if ((st = bwd_chunk_states(m, a, *opt, cs)) != LASP_OK) return st;
+    if ((st = bwd_scan(m, a, cs)) != LASP_OK) return st;
+  }
   return bwd_grads(m, a, *opt, cs);
 }
 

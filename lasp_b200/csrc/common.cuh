@@ -13,7 +13,7 @@ namespace lasp {
 // and nc the number of states kept per sequence.  The chunk-state phase writes
 // the LOCAL states, the scan reads them and writes the PREFIX states (exclusive,
 // seeded with the incoming rank state) that the output / gradient kernels read:
-//   SIMT path        : one state per 64-token chunk, fp32 (b,h,nc,d,e):
+//   FULL PRECISION : one state per 128-token chunk, fp32:
 //                      [0, S*4) prefix states, [S*4, 2*S*4) local states
 //   TENSOR path      : one state per SPAN of `span` 128-token tiles (a few per
 //                      sequence; inside a span the state lives on chip):
@@ -23,8 +23,9 @@ namespace lasp {
 //                      [4096, 4096 + S*4)   local states: fp32 span totals
 //                      [4096 + S*4, + S*4)  prefix states: fp32 states at the span borders
 // The running prefix inside the scan is always fp32.
-constexpr int kSimtChunk = 64;    // the reference's block size
 constexpr int kTensorTile = 128;  // one tcgen05 M=128 tile
+constexpr int kAbiChunk = 64;     // the reference's block size: what the C ABI reports and sizes the full-precision
+                                  // path's workspace by (its chunks are two of these)
 
 struct Dims {
   int b, h, n, d, e;
@@ -47,10 +48,10 @@ int sm_count();
 
 inline size_t state_elems(const Dims& m) { return (size_t)m.b * m.h * m.nc * m.d * m.e; }
 
-// Span states of the walk kernels are kept in global memory in "lane order": the float4 holding
+// The states in a workspace are kept in "lane order": the float4 holding
 // columns 4g..4g+3 of row r of a d x e state sits at float4 index g*d + r, so that the 32 rows a warp
 // owns are contiguous for each of its accesses.  Rank states handed in and out by the caller stay
-// row-major; `rows` > 0 on the elementwise kernels below selects the conversion (0 = plain row-major).
+// row-major.
 __host__ __device__ inline int lane_order_to_row_major(int f4, int rows, int cols) {
   const int g = f4 / rows, r = f4 - g * rows;
   return r * (cols / 4) + g;
@@ -91,15 +92,17 @@ cudaError_t fault_word_address(int32_t** out);
 extern thread_local const char* g_failed_step;
 
 // ---- launchers implemented in the .cu files (return cudaError_t) -----------
-cudaError_t simt_chunk_states(const Dims& m, const void* a, const void* bten, const float* s, float* states,
-                              bool backward, cudaStream_t st);
+// Full-precision path (split_kernels.cu).  `alone`: no rank state comes in or goes out, so the states at the
+// sequence's ends are zero or unread.
+cudaError_t split_chunk_states(const Dims& m, const void* a, const void* bten, const float* s, float* states,
+                               bool backward, bool alone, cudaStream_t st);
+cudaError_t split_fwd_output(const Dims& m, const void* q, const void* k, const void* v, const float* s,
+                             const float* prefix, void* o, bool alone, bool add_o, cudaStream_t st);
+cudaError_t split_bwd_grads(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, const float* s,
+                            const float* prefix, const float* suffix, void* dq, void* dk, void* dv, bool alone,
+                            bool add_qk, bool add_v, cudaStream_t st);
 cudaError_t scan_states(const Dims& m, const float* s, const float* local, float* prefix, const float* x_in,
                         float* x_out, bool reverse, cudaStream_t st);
-cudaError_t simt_fwd_output(const Dims& m, const void* q, const void* k, const void* v, const float* s,
-                            const float* prefix, void* o, cudaStream_t st);
-cudaError_t simt_bwd_grads(const Dims& m, const void* q, const void* k, const void* v, const void* d_o,
-                           const float* s, const float* prefix, const float* suffix, void* dq, void* dk,
-                           void* dv, cudaStream_t st);
 cudaError_t state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
                           const float* x_local, float* x_out, cudaStream_t st);
 

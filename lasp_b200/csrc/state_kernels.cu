@@ -1,0 +1,96 @@
+// Elementwise kernels on the fp32 d x e states: the scan over the chunks (or spans) of a sequence and the update of
+// a rank state.
+#include "common.cuh"
+
+namespace lasp {
+namespace {
+
+// ---------------------------------------------------------------------------
+// scan over chunks, elementwise in (d,e).  forward: exclusive prefix seeded
+// with x_in; reverse: exclusive suffix.  k_scan reads the fp32 local states
+// and writes the prefix states to a second array.  Loads of a batch of chunks are issued before the
+// dependent recurrence so that their latencies overlap.
+// ---------------------------------------------------------------------------
+constexpr int kScanBatch = 8;
+
+__global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const float* __restrict__ local,
+                                              float* __restrict__ prefix, const float* __restrict__ x_in,
+                                              float* __restrict__ x_out, int h,
+                                              int n, int de, int nc, int chunk, int reverse, int rows,
+                                              int cols) {
+  const int bh = blockIdx.y;
+  const int el = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (el >= de) return;
+  // where this float4 of a state in lane order lives in the caller's row-major rank states
+  const int ext = lane_order_to_row_major(el / 4, rows, cols) * 4;
+  const float sh = s[bh % h];
+  const float full = expf(-sh * (float)chunk);
+  const int last_len = n - (nc - 1) * chunk;
+  const float tail = expf(-sh * (float)last_len);
+  float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (x_in) p = *reinterpret_cast<const float4*>(x_in + (size_t)bh * de + ext);
+  const float* base = local + (size_t)bh * nc * de + el;
+  float* out = prefix + (size_t)bh * nc * de + el;
+  for (int i0 = 0; i0 < nc; i0 += kScanBatch) {
+    float4 loc[kScanBatch];
+#pragma unroll
+    for (int u = 0; u < kScanBatch; ++u) {
+      const int i = i0 + u;
+      if (i < nc) loc[u] = *reinterpret_cast<const float4*>(base + (size_t)(reverse ? nc - 1 - i : i) * de);
+    }
+#pragma unroll
+    for (int u = 0; u < kScanBatch; ++u) {
+      const int i = i0 + u;
+      if (i < nc) {
+        const int c = reverse ? nc - 1 - i : i;
+        const float dec = (c == nc - 1) ? tail : full;
+        *reinterpret_cast<float4*>(out + (size_t)c * de) = p;
+        p.x = fmaf(dec, p.x, loc[u].x);
+        p.y = fmaf(dec, p.y, loc[u].y);
+        p.z = fmaf(dec, p.z, loc[u].z);
+        p.w = fmaf(dec, p.w, loc[u].w);
+      }
+    }
+  }
+  if (x_out) *reinterpret_cast<float4*>(x_out + (size_t)bh * de + ext) = p;
+}
+
+__global__ void __launch_bounds__(256) k_state_combine(const float* __restrict__ s, const float* __restrict__ x_in,
+                                                       const float* __restrict__ x_local, float* __restrict__ x_out,
+                                                       int h, int de, int n) {
+  const int bh = blockIdx.y;
+  const int el = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (el >= de) return;
+  const float dec = expf(-s[bh % h] * (float)n);
+  float4 loc = *reinterpret_cast<const float4*>(x_local + (size_t)bh * de + el);
+  if (x_in) {
+    float4 p = *reinterpret_cast<const float4*>(x_in + (size_t)bh * de + el);
+    loc.x = fmaf(dec, p.x, loc.x);
+    loc.y = fmaf(dec, p.y, loc.y);
+    loc.z = fmaf(dec, p.z, loc.z);
+    loc.w = fmaf(dec, p.w, loc.w);
+  }
+  *reinterpret_cast<float4*>(x_out + (size_t)bh * de + el) = loc;
+}
+
+}  // namespace
+
+cudaError_t scan_states(const Dims& m, const float* s, const float* local, float* prefix, const float* x_in,
+                        float* x_out, bool reverse, cudaStream_t st) {
+  const int de = m.d * m.e;
+  dim3 grid((de / 4 + 255) / 256, m.b * m.h);
+  k_scan<<<grid, 256, 0, st>>>(s, local, prefix, x_in, x_out, m.h, m.n, de, m.nc, m.chunk, reverse ? 1 : 0, m.d,
+                               m.e);
+  return cudaGetLastError();
+}
+
+
+cudaError_t state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
+                          const float* x_local, float* x_out, cudaStream_t st) {
+  const int de = d * e;
+  dim3 grid((de / 4 + 255) / 256, b * h);
+  k_state_combine<<<grid, 256, 0, st>>>(s, x_in, x_local, x_out, h, de, n);
+  return cudaGetLastError();
+}
+
+}  // namespace lasp

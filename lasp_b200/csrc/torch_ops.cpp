@@ -145,17 +145,12 @@ lasp_problem problem_of(const Shape& m, int64_t d, int64_t e, int32_t dtype, dou
   return p;
 }
 
-// One 128-wide slice pair of the head dimensions: columns [d0, d1) of q,k and [e0, e1) of v.
+// One 128-wide slice pair of the head dimensions: columns [d0, d1) of q,k and [e0, e1) of v, where they lie in the
+// wide tensors.
 struct Pair {
   int64_t d0, d1, e0, e1;
   lasp_problem problem;
   size_t ws_bytes;
-};
-
-// How a call is cut: `in_place` = the kernels take the slices where they lie in the wide tensors.
-struct Cut {
-  std::vector<Pair> pairs;
-  bool in_place = false;
 };
 
 bool resolve(lasp_problem& p) {
@@ -165,77 +160,46 @@ bool resolve(lasp_problem& p) {
   return true;
 }
 
-Cut cut_call(const Shape& m, int32_t dtype, double scale, int64_t map) {
-  Cut c;
-  const auto fill = [&](bool pitched) {
-    c.pairs.clear();
-    for (int64_t e0 = 0; e0 < m.e; e0 += kSlice)
-      for (int64_t d0 = 0; d0 < m.d; d0 += kSlice) {
-        Pair p{d0, std::min(d0 + kSlice, m.d), e0, std::min(e0 + kSlice, m.e), {}, 0};
-        p.problem = problem_of(m, p.d1 - p.d0, p.e1 - p.e0, dtype, scale, map, pitched);
-        if (!resolve(p.problem)) {
-          if (pitched) return false;
-          check_status("lasp_b200_resolve_path", lasp_b200_resolve_path(&p.problem));
-        }
-        p.ws_bytes = lasp_b200_fwd_workspace_bytes(&p.problem);
-        c.pairs.push_back(p);
-      }
-    return true;
-  };
+std::vector<Pair> slice_pairs(const Shape& m, int32_t dtype, double scale, int64_t map) {
+  std::vector<Pair> pairs;
   const bool wide = m.d > kSlice || m.e > kSlice;
-  c.in_place = wide && fill(true);
-  if (!c.in_place) fill(false);
-  return c;
+  for (int64_t e0 = 0; e0 < m.e; e0 += kSlice)
+    for (int64_t d0 = 0; d0 < m.d; d0 += kSlice) {
+      Pair p{d0, std::min(d0 + kSlice, m.d), e0, std::min(e0 + kSlice, m.e), {}, 0};
+      p.problem = problem_of(m, p.d1 - p.d0, p.e1 - p.e0, dtype, scale, map, wide);
+      if (!resolve(p.problem)) check_status("lasp_b200_resolve_path", lasp_b200_resolve_path(&p.problem));
+      p.ws_bytes = lasp_b200_fwd_workspace_bytes(&p.problem);
+      pairs.push_back(p);
+    }
+  return pairs;
 }
 
 char* column(const Tensor& t, int64_t col) { return static_cast<char*>(t.data_ptr()) + col * t.element_size(); }
-
-// A slice as a kernel call wants it: in place, or (kernels without a row pitch) a copy of its own.
-struct Slice {
-  Tensor copy;
-  void* ptr;
-};
-Slice slice_of(const Tensor& t, int64_t lo, int64_t hi, bool whole) {
-  if (whole) return {Tensor(), column(t, lo)};
-  Tensor c = t.slice(3, lo, hi).contiguous();
-  void* p = c.data_ptr();
-  return {std::move(c), p};
-}
 
 std::vector<Tensor> run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s, const Shape& m,
                                 double scale, int64_t map, bool keep) {
   const c10::cuda::CUDAGuard guard(q.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
-  const Cut cut = cut_call(m, lasp_dtype_of(q.scalar_type()), scale, map);
-  const bool sliced = cut.pairs.size() > 1, whole = !sliced || cut.in_place;
   Tensor o = at::empty({m.b, m.h, m.n, m.e}, q.options());
   const Tensor sync = sync_words(q.device(), stream);
   std::vector<Tensor> out{o};
   Tensor ws;
-  for (const Pair& p : cut.pairs) {
+  for (const Pair& p : slice_pairs(m, lasp_dtype_of(q.scalar_type()), scale, map)) {
     // (nothing is kept without a backward pass: the slices then share a workspace)
     if (keep || !ws.defined() || (size_t)ws.numel() < p.ws_bytes)
       ws = at::empty({(int64_t)p.ws_bytes}, q.options().dtype(at::kByte));
     if (keep) out.push_back(ws);
-    const Slice qs = slice_of(q, p.d0, p.d1, whole), ks = slice_of(k, p.d0, p.d1, whole), vs = slice_of(v, p.e0, p.e1, whole);
-    Tensor part = whole ? Tensor() : at::empty({m.b, m.h, m.n, p.e1 - p.e0}, q.options());
     lasp_fwd_args a = {};
-    a.q = qs.ptr, a.k = ks.ptr, a.v = vs.ptr, a.s = s.const_data_ptr<float>();
-    a.o = whole ? column(o, p.e0) : part.data_ptr();
+    a.q = column(q, p.d0), a.k = column(k, p.d0), a.v = column(v, p.e0), a.s = s.const_data_ptr<float>();
+    a.o = column(o, p.e0);
     a.ws = ws.data_ptr(), a.ws_bytes = (size_t)ws.numel();
     lasp_call_options opt = {};
     opt.sync = static_cast<uint32_t*>(sync.data_ptr());
     opt.keep_states = keep ? 1 : 0;
-    opt.accumulate = whole && p.d0 > 0 ? LASP_ACCUMULATE_V : 0;
+    opt.accumulate = p.d0 > 0 ? LASP_ACCUMULATE_V : 0;   // a v slice collects from every q/k slice
+    opt.alone = 1;
     Range range("lasp_b200_forward");
     check_status("lasp_b200_forward", lasp_b200_forward_opt(&p.problem, &a, &opt, stream.stream()));
-    if (!whole) {
-      Tensor dst = o.slice(3, p.e0, p.e1);
-      if (p.d0 > 0)
-        dst.add_(part);
-      else
-        dst.copy_(part);
-    }
   }
   return out;
 }
@@ -262,46 +226,29 @@ class Lightning : public torch::autograd::Function<Lightning> {
     const Shape m{q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
     const c10::cuda::CUDAGuard guard(q.device());
     const auto stream = at::cuda::getCurrentCUDAStream();
-    const Cut cut = cut_call(m, lasp_dtype_of(q.scalar_type()), ctx->saved_data["scale"].toDouble(),
-                             ctx->saved_data["map"].toInt());
-    const bool sliced = cut.pairs.size() > 1, whole = !sliced || cut.in_place;
     Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options()), dv = at::empty(v.sizes(), v.options());
     const Tensor sync = sync_words(q.device(), stream);
     Tensor ws;
-    for (size_t i = 0; i < cut.pairs.size(); ++i) {
-      const Pair& p = cut.pairs[i];
+    const std::vector<Pair> pairs = slice_pairs(m, lasp_dtype_of(q.scalar_type()), ctx->saved_data["scale"].toDouble(),
+                                                ctx->saved_data["map"].toInt());
+    for (size_t i = 0; i < pairs.size(); ++i) {
+      const Pair& p = pairs[i];
       const Tensor& fwd_ws = saved[4 + i];
       if (!ws.defined() || (size_t)ws.numel() < p.ws_bytes)
         ws = at::empty({(int64_t)p.ws_bytes}, q.options().dtype(at::kByte));
-      const Slice qs = slice_of(q, p.d0, p.d1, whole), ks = slice_of(k, p.d0, p.d1, whole), vs = slice_of(v, p.e0, p.e1, whole),
-                  ds = slice_of(d_o, p.e0, p.e1, whole);
-      Tensor pq, pk, pv;
-      if (!whole) {
-        pq = at::empty({m.b, m.h, m.n, p.d1 - p.d0}, q.options());
-        pk = at::empty({m.b, m.h, m.n, p.d1 - p.d0}, q.options());
-        pv = at::empty({m.b, m.h, m.n, p.e1 - p.e0}, q.options());
-      }
       lasp_bwd_args a = {};
-      a.q = qs.ptr, a.k = ks.ptr, a.v = vs.ptr, a.d_o = ds.ptr, a.s = s.const_data_ptr<float>();
-      a.dq = whole ? column(dq, p.d0) : pq.data_ptr();
-      a.dk = whole ? column(dk, p.d0) : pk.data_ptr();
-      a.dv = whole ? column(dv, p.e0) : pv.data_ptr();
+      a.q = column(q, p.d0), a.k = column(k, p.d0), a.v = column(v, p.e0), a.d_o = column(d_o, p.e0);
+      a.s = s.const_data_ptr<float>();
+      a.dq = column(dq, p.d0), a.dk = column(dk, p.d0), a.dv = column(dv, p.e0);
       a.fwd_ws = fwd_ws.data_ptr(), a.fwd_ws_bytes = (size_t)fwd_ws.numel();
       a.ws = ws.data_ptr(), a.ws_bytes = (size_t)ws.numel();
       lasp_call_options opt = {};
       opt.sync = static_cast<uint32_t*>(sync.data_ptr());
       // a q/k slice collects from every v slice, a v slice from every q/k slice
-      if (whole) opt.accumulate = (p.e0 > 0 ? LASP_ACCUMULATE_QK : 0) | (p.d0 > 0 ? LASP_ACCUMULATE_V : 0);
-      {
-        Range range("lasp_b200_backward");
-        check_status("lasp_b200_backward", lasp_b200_backward_opt(&p.problem, &a, &opt, stream.stream()));
-      }
-      if (!whole) {
-        const auto put = [](Tensor dst, const Tensor& part, bool add) { add ? dst.add_(part) : dst.copy_(part); };
-        put(dq.slice(3, p.d0, p.d1), pq, p.e0 > 0);
-        put(dk.slice(3, p.d0, p.d1), pk, p.e0 > 0);
-        put(dv.slice(3, p.e0, p.e1), pv, p.d0 > 0);
-      }
+      opt.accumulate = (p.e0 > 0 ? LASP_ACCUMULATE_QK : 0) | (p.d0 > 0 ? LASP_ACCUMULATE_V : 0);
+      opt.alone = 1;
+      Range range("lasp_b200_backward");
+      check_status("lasp_b200_backward", lasp_b200_backward_opt(&p.problem, &a, &opt, stream.stream()));
     }
     return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
   }

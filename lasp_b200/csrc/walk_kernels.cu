@@ -5,7 +5,7 @@
 // consecutive tiles; a span is the unit of work of a persistent CTA.  Per direction:
 //
 //   k_span_totals   T_span = sum over the span's tokens of decay * a_j b_j^T  (a,b = k,v or q,do)
-//   (scan over the few span totals of a sequence: k_scan of simt_kernels.cu, seeded with the rank's
+//   (scan over the few span totals of a sequence: k_scan of state_kernels.cu, seeded with the rank's
 //    incoming state; gives every span its fp32 state at the span border)
 //   k_walk_out      walks a span first to last tile with the d x e state in registers (fp32) and in
 //                   shared memory (bf16 MMA operand):  OUT = (X Y^T . M) Z + diag(lambda^r) X op(P),
