@@ -67,17 +67,9 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after ~1e9 clocks (about half a second) and returns
-// false, so a lost arrival becomes a reported fault instead of a hung GPU.
-constexpr long long kWaitClocks = 1000000000LL;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (clock64() - t0 > kWaitClocks) return false;
-  }
-  return true;
-}
+// Waits give up after ~1e9 clocks (about half a second), so that a lost arrival becomes a reported fault instead of a
+// hung GPU.
+constexpr uint32_t kWaitClocks = 1000000000u;
 
 // ---------------------------------------------------------------------------
 // TMA: 3-D tiled load global -> shared, completion counted on an mbarrier
@@ -139,6 +131,16 @@ __device__ __forceinline__ void bulk_wait_all() {
 __device__ __forceinline__ void named_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// registers per thread of the calling warpgroup (all four warps): given back / taken from what the block was
+// launched with.  The warpgroups' shares must add up to no more than that.
+template <int regs>
+__device__ __forceinline__ void set_regs_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(regs));
+}
+template <int regs>
+__device__ __forceinline__ void set_regs_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(regs));
+}
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
@@ -170,6 +172,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
         "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+// 32 lanes x 16 consecutive 32-bit columns
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
 }
@@ -215,25 +227,30 @@ __host__ __device__ constexpr uint32_t umma_idesc(uint32_t m, uint32_t n, bool a
   return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
          ((n >> 3) << 17) | ((m >> 4) << 24);
 }
-// one MMA of shape M x N x 16; accumulate = 0 overwrites the accumulator
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                     uint32_t accumulate) {
+// One MMA of shape M x N x 16; accumulate = 0 overwrites the accumulator.  A descriptor is passed as its two words: the
+// steps of a product differ in the address field of the low one only.
+struct SmemDesc {
+  uint32_t lo, hi;
+};
+__device__ __forceinline__ void umma(uint32_t d_tmem, SmemDesc a, SmemDesc b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "mov.b64 da, {%1, %2};\n\t"
+      "mov.b64 db, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
+      ::"r"(d_tmem), "r"(a.lo), "r"(a.hi), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // The same with the A operand in tensor memory: lane = row of A, and each 32-bit column holds two
 // consecutive K elements (bf16), so one instruction (16 K elements) reads 8 columns from a_tmem on.
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
+__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, SmemDesc b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(b.lo), "r"(b.hi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // the mbarrier gets one arrival when every MMA issued so far by this thread has completed
@@ -242,40 +259,38 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// Operand views of a swizzled tile (see the tile format above).
-struct Operand {
-  uint32_t addr;   // shared address of the tile
-  uint32_t rows;   // rows of the tile (slab stride = rows * 128 bytes)
-  bool mn_major;   // false: rows = M/N index, cols = K;  true: rows = K index, cols = M/N
-};
-// descriptor for k-step `ks` (16 K elements each)
-__device__ __forceinline__ uint64_t operand_desc(const Operand& op, uint32_t ks) {
-  if (!op.mn_major) {
-    // K runs along columns: 4 k-steps per slab, 32 bytes each inside the swizzle atom
-    const uint32_t a = op.addr + (ks >> 2) * op.rows * kSlabRowBytes + (ks & 3) * 32;
-    return umma_desc(a, 16, 1024);
-  }
-  // K runs along rows: 16 rows = 2048 bytes per k-step
-  return umma_desc(op.addr + ks * 16 * kSlabRowBytes, op.rows * kSlabRowBytes, 1024);
+// Operand views of a swizzled tile of `rows` rows (slab stride rows * 128 bytes; see the tile format above):
+// mn_major = false: rows are the M or N index, columns K;  true: rows are the K index, columns M or N.
+__device__ __forceinline__ SmemDesc operand_desc(uint32_t addr, uint32_t rows, bool mn_major) {
+  const uint64_t d = umma_desc(addr, mn_major ? rows * kSlabRowBytes : 16, 1024);
+  return {(uint32_t)d, (uint32_t)(d >> 32)};
 }
-// D[128 x n] (+)= A x B over `ksteps` k-steps; issued by ONE thread
-__device__ __forceinline__ void umma_gemm(uint32_t d_tmem, const Operand& a, const Operand& b, uint32_t n,
-                                          uint32_t ksteps, bool accumulate) {
-  const uint32_t idesc = umma_idesc(128, n, a.mn_major, b.mn_major);
-  for (uint32_t ks = 0; ks < ksteps; ++ks)
-    umma(d_tmem, operand_desc(a, ks), operand_desc(b, ks), idesc, (accumulate || ks > 0) ? 1u : 0u);
+// ... advanced to k-step ks (16 K elements): along K-major columns four steps of 32 bytes per slab, along MN-major
+// rows 16 rows = 2048 bytes per step
+__device__ __forceinline__ SmemDesc operand_step(SmemDesc d, uint32_t rows, bool mn_major, uint32_t ks) {
+  return {d.lo + (mn_major ? ks * 128 : (ks >> 2) * rows * 8 + (ks & 3) * 2), d.hi};
 }
-
-// D[128 x n] (+)= A x B over 8 k-steps with A = a 128 x 128 bf16 matrix in tensor memory.  `split`:
-// K elements 0..63 sit in columns [0, 32) and 64..127 in columns [64, 96) of the region at a_tmem (what
-// packing an fp32 accumulator in place, half by half, leaves); otherwise in columns [0, 64).
-__device__ __forceinline__ void umma_gemm_ts(uint32_t d_tmem, uint32_t a_tmem, bool split, const Operand& b,
-                                             uint32_t n, bool accumulate) {
-  const uint32_t idesc = umma_idesc(128, n, false, b.mn_major);
-  for (uint32_t ks = 0; ks < 8; ++ks) {
-    const uint32_t col = split ? (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8) : ks * 8;
-    umma_ts(d_tmem, a_tmem + col, operand_desc(b, ks), idesc, (accumulate || ks > 0) ? 1u : 0u);
-  }
+// D[128 x N] (+)= A x B over K; issued by ONE thread
+template <bool A_MN, bool B_MN, int N, int K>
+__device__ __forceinline__ void umma_gemm(uint32_t d_tmem, uint32_t a_addr, uint32_t a_rows, uint32_t b_addr,
+                                          uint32_t b_rows, bool accumulate) {
+  constexpr uint32_t idesc = umma_idesc(128, N, A_MN, B_MN);
+  const SmemDesc a = operand_desc(a_addr, a_rows, A_MN), b = operand_desc(b_addr, b_rows, B_MN);
+#pragma unroll
+  for (uint32_t ks = 0; ks < K / 16; ++ks)
+    umma(d_tmem, operand_step(a, a_rows, A_MN, ks), operand_step(b, b_rows, B_MN, ks), idesc, (accumulate || ks > 0) ? 1u : 0u);
+}
+// D[128 x N] (+)= A x B over 128 K elements with A = a bf16 matrix in tensor memory, K elements 0..63 in columns
+// [0, 32) and 64..127 in columns [SECOND, SECOND + 32) of the region at a_tmem (what packing an fp32 accumulator in
+// place, half by half, leaves)
+template <bool B_MN, int N, int SECOND>
+__device__ __forceinline__ void umma_gemm_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_addr, uint32_t b_rows, bool accumulate) {
+  constexpr uint32_t idesc = umma_idesc(128, N, false, B_MN);
+  const SmemDesc b = operand_desc(b_addr, b_rows, B_MN);
+#pragma unroll
+  for (uint32_t ks = 0; ks < 8; ++ks)
+    umma_ts(d_tmem, a_tmem + (ks < 4 ? ks * 8 : SECOND + (ks - 4) * 8), operand_step(b, b_rows, B_MN, ks), idesc,
+            (accumulate || ks > 0) ? 1u : 0u);
 }
 
 // ---------------------------------------------------------------------------

@@ -163,28 +163,11 @@ __device__ __forceinline__ void store_state_terms(uint8_t* tiles, const Raw<floa
   }
 }
 
-// 32 lanes x 16 consecutive 32-bit columns
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
-// One operand of a product in shared memory: `tiles` holds its terms, `stride` bytes apart.
+// One operand of a product in shared memory: its terms lie `stride` bytes apart.
 struct TermOperand {
   uint32_t addr, stride, rows;
   bool mn_major;
-  __device__ __forceinline__ uint64_t desc(int term) const {
-    return umma_desc(addr + term * stride, mn_major ? rows * kSlabRowBytes : 16, 1024);
-  }
-  // advance to K step 4 kq + u, in descriptor units of 16 bytes
-  __device__ __forceinline__ uint64_t step(int kq, int u) const {
-    return mn_major ? (uint64_t)((4 * kq + u) * 128) : (uint64_t)(kq * (int)(rows * 8) + u * 2);
-  }
+  __device__ __forceinline__ SmemDesc desc(int term) const { return operand_desc(addr + term * stride, rows, mn_major); }
 };
 // D[128 x n] = A B: every kept product of terms, the smallest first; issued by one thread
 template <int NA, int NB, int CUT>
@@ -197,12 +180,12 @@ __device__ __forceinline__ void issue_terms(uint32_t d_tmem, const TermOperand& 
     for (int i = 0; i < NA; ++i) {
       const int j = sum - i;
       if (j < 0 || j >= NB) continue;
-      const uint64_t da = a.desc(i), db = b.desc(j);
+      const SmemDesc da = a.desc(i), db = b.desc(j);
 #pragma unroll 1
       for (int kq = 0; kq < ksteps / 4; ++kq) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          umma(d_tmem, da + a.step(kq, u), db + b.step(kq, u), idesc, acc);
+          umma(d_tmem, operand_step(da, a.rows, a.mn_major, 4 * kq + u), operand_step(db, b.rows, b.mn_major, 4 * kq + u), idesc, acc);
           acc = 1;
         }
       }
@@ -221,14 +204,14 @@ __device__ __forceinline__ void issue_terms_ts(uint32_t d_tmem, uint32_t t_s, ui
     for (int i = 0; i < NA; ++i) {
       const int j = sum - i;
       if (j < 0 || j >= NB) continue;
-      const uint64_t db = b.desc(j);
+      const SmemDesc db = b.desc(j);
 #pragma unroll 1
       for (int kq = 0; kq < C / 64; ++kq) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int ks = 4 * kq + u;
           const uint32_t ta = i == 2 ? t_lo + 8 * ks : t_s + 32 * (ks >> 1) + 8 * (ks & 1) + 16 * i;
-          umma_ts(d_tmem, ta, db + b.step(kq, u), idesc, acc);
+          umma_ts(d_tmem, ta, operand_step(db, b.rows, b.mn_major, ks), idesc, acc);
           acc = 1;
         }
       }

@@ -14,13 +14,19 @@ constexpr int C = kTensorTile;  // 128 tokens per tile
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr uint32_t kNoAcc = 0xFFFFFFFFu;
 
-// bounded wait that records a fault once and makes later waits of the CTA no-ops
+// Bounded wait that records a fault once and lets later waits of the CTA give up at once.  There are some thirty of
+// these in a walk kernel: the code that a wait normally runs is one probe, and 32-bit clocks keep the rest short.
 __device__ __forceinline__ void wait_or_fault(uint64_t* bar, uint32_t parity, volatile int* dead, int32_t* fault,
                                               int32_t code) {
-  if (*dead) return;
-  if (!mbar_wait(bar, parity)) {
-    *dead = 1;
-    atomicOr(fault, code);
+  if (mbar_try_wait(bar, parity)) return;
+  const uint32_t t0 = clock();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*dead) return;
+    if ((uint32_t)clock() - t0 > kWaitClocks) {
+      *dead = 1;
+      atomicOr(fault, code);
+      return;
+    }
   }
 }
 
@@ -34,6 +40,13 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 }
 
 __device__ __forceinline__ float decay_pow(float sl2, int k) { return exp2f(-sl2 * (float)k); }
+
+// Tiles that a decay rate s reaches over: a token s * tokens >= 27.6 away has a weight below 1e-12 (exchange_layout.h
+// draws the same line between ranks).  At least one; no limit without decay.
+__device__ __forceinline__ int reach_tiles(float s) {
+  const float r = 27.6f / (s * (float)C);
+  return s > 0.f && r < 1e6f ? (int)r + 1 : 1 << 20;
+}
 
 // acc (32 columns) *= f, in tensor memory
 __device__ __forceinline__ void scale_tmem32(uint32_t taddr, float f) {
@@ -213,6 +226,28 @@ __device__ __forceinline__ void scale_row_pieces(uint8_t* tile, int row, int fir
   }
 }
 
+// dst row = w * src row, the same pieces of two tiles of C rows
+template <int CHUNKS>
+__device__ __forceinline__ void copy_row_pieces(uint8_t* dst, const uint8_t* src, int row, int first, float w, int lane) {
+  uint4 v[CHUNKS];
+#pragma unroll
+  for (int q = 0; q < CHUNKS; ++q) {
+    const int piece = first + ((q + lane) & (CHUNKS - 1));
+    v[q] = *reinterpret_cast<const uint4*>(src + (piece >> 3) * C * 128 + row * 128 + (piece & 7) * 16);
+  }
+#pragma unroll
+  for (int q = 0; q < CHUNKS; ++q) {
+    const int piece = first + ((q + lane) & (CHUNKS - 1));
+    uint32_t* u = reinterpret_cast<uint32_t*>(&v[q]);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u[t]));
+      u[t] = pack_bf16(f.x * w, f.y * w);
+    }
+    *reinterpret_cast<uint4*>(dst + (piece >> 3) * C * 128 + row * 128 + (piece & 7) * 16) = v[q];
+  }
+}
+
 // stage_row32 with the chain rule of the folded q,k preprocessing x' = c * map(x): the 32 accumulator values
 // (a gradient with respect to x') are multiplied by c * map'(x) on their way to the staging tile, x read from
 // the raw tensor (`raw` points at column 0 of this thread's row).
@@ -244,45 +279,56 @@ __device__ __forceinline__ void stage_row32_chain(uint32_t taddr, uint8_t* tile,
   }
 }
 
+// How the sequences of a launch are cut into spans of tiles; `base`, `extra` and `magic` are what the kernels would
+// otherwise divide for at every item (three integer divisions, inlined wherever a role steps through its tiles, were a
+// third of a walk kernel's code).
+struct SpanCut {
+  int items, nspans, span, tiles;
+  int base, extra;   // tiles / nspans and the remainder
+  uint32_t magic;    // it / nspans = (it * magic) >> 32 with 64-bit arithmetic while items * nspans < 2^32
+};
+inline SpanCut make_span_cut(int items, int nspans, int span, int tiles) {
+  return {items, nspans, span, tiles, tiles / nspans, tiles % nspans, nspans > 1 ? (uint32_t)(0x100000000ull / nspans) + 1 : 0};
+}
+
 // The work of a persistent CTA: items blockIdx.x, blockIdx.x + gridDim.x, ...; an item is one span of
 // consecutive tiles of one (batch, head) sequence, walked first to last tile or last to first.
 // Spans: `span` tiles each, the last one of a sequence whatever is left (even = false), or - for a
 // kernel whose CTAs wait for one another - the tiles shared out evenly, spans differing by one tile at
 // most, with the longer spans where the walk starts: there nobody has to wait for anybody's total, and the
 // spans with the longest look-back get the fewest tiles (even = true).
+template <bool BACKWARDS>
 struct TileWalk {
-  int items, nspans, span, tiles, stride;
-  bool backwards;
+  const SpanCut& c;
   bool even;
-  int it, bh, t, t0, t1;  // current item, its sequence, current tile, the item's tile range [t0, t1)
+  int it, bh, sp, t, t0, t1;  // current item, its sequence and span, current tile, the item's tile range [t0, t1)
 
   // first tile of span sp (sp = nspans: one past the last tile)
-  __device__ __forceinline__ int span_t0(int sp) const {
-    if (!even) return min(sp * span, tiles);
-    const int base = tiles / nspans, extra = tiles - base * nspans;   // `extra` spans have base + 1 tiles
-    return backwards ? sp * base + max(0, sp - (nspans - extra)) : sp * base + min(sp, extra);
+  __device__ __forceinline__ int span_t0(int s) const {
+    if (!even) return min(s * c.span, c.tiles);
+    // `extra` spans have base + 1 tiles
+    return s * c.base + (BACKWARDS ? max(0, s - (c.nspans - c.extra)) : min(s, c.extra));
   }
   __device__ __forceinline__ bool load() {
-    if (it >= items) return false;
-    bh = it / nspans;
-    const int sp = it - bh * nspans;
+    if (it >= c.items) return false;
+    bh = c.nspans == 1 ? it : (int)(((uint64_t)(uint32_t)it * c.magic) >> 32);
+    sp = it - bh * c.nspans;
     t0 = span_t0(sp);
     t1 = span_t0(sp + 1);
-    t = backwards ? t1 - 1 : t0;
+    t = BACKWARDS ? t1 - 1 : t0;
     return true;
   }
-  __device__ __forceinline__ bool start(int first_item, int item_stride) {
-    it = first_item;
-    stride = item_stride;
+  __device__ __forceinline__ bool start() {
+    it = blockIdx.x;
     return load();
   }
   __device__ __forceinline__ bool next() {
-    if (backwards ? (--t >= t0) : (++t < t1)) return true;
-    it += stride;
+    if (BACKWARDS ? (--t >= t0) : (++t < t1)) return true;
+    it += gridDim.x;
     return load();
   }
-  __device__ __forceinline__ bool first_of_item() const { return backwards ? t == t1 - 1 : t == t0; }
-  __device__ __forceinline__ bool last_of_item() const { return backwards ? t == t0 : t == t1 - 1; }
+  __device__ __forceinline__ bool first_of_item() const { return BACKWARDS ? t == t1 - 1 : t == t0; }
+  __device__ __forceinline__ bool last_of_item() const { return BACKWARDS ? t == t0 : t == t1 - 1; }
 };
 
 }  // namespace tc

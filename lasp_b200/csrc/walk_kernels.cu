@@ -30,11 +30,15 @@ namespace {
 using namespace tc;
 
 #ifdef LASP_TRACE
-__device__ long long g_trace[160 * 64];
-#define TRACE(slot) do { if (blockIdx.x < 160 && (slot) < 64) g_trace[blockIdx.x * 64 + (slot)] = clock64(); } while (0)
+constexpr int kTraceSlots = 256;
+__device__ long long g_trace[160 * kTraceSlots];
+#define TRACE(slot) do { if (blockIdx.x < 160 && (slot) < kTraceSlots) g_trace[blockIdx.x * kTraceSlots + (slot)] = clock64(); } while (0)
 __device__ __forceinline__ long long gtime() { long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
-#define GTRACE(slot) do { if (blockIdx.x < 160) g_trace[blockIdx.x * 64 + (slot)] = gtime(); } while (0)
+#define GTRACE(slot) do { if (blockIdx.x < 160) g_trace[blockIdx.x * kTraceSlots + (slot)] = gtime(); } while (0)
+#define TRACE_VAL(slot, v) do { if (blockIdx.x < 160) g_trace[blockIdx.x * kTraceSlots + (slot)] = (v); } while (0)
+__device__ __forceinline__ uint32_t smid() { uint32_t v; asm volatile("mov.u32 %0, %%smid;" : "=r"(v)); return v; }
 #else
+#define TRACE_VAL(slot, v) do {} while (0)
 #define TRACE(slot) do {} while (0)
 #define GTRACE(slot) do {} while (0)
 #endif
@@ -51,6 +55,10 @@ struct TmemPair {
   uint32_t base;
   __device__ __forceinline__ uint32_t operator[](int p) const { return base + p * 128; }
 };
+template <int G>
+struct Group {   // a worker group as a compile-time constant: 0 = A, 1 = B
+  static constexpr int value = G;
+};
 struct IntPair {
   int a, b;
   __device__ __forceinline__ int get(int p) const { return p ? b : a; }
@@ -58,7 +66,14 @@ struct IntPair {
     if (p) b = v; else a = v;
   }
 };
-constexpr int kWorkers = 256;     // warps 2..9
+constexpr int kWorkers = 256;     // threads of one group of eight worker warps
+// The walk kernels run five warpgroups: producer and issuer in the first (its other two warps idle), two for each
+// worker group.  They are launched with 96 registers a thread (640 x 96 = 61440) and share them out anew: 64 + 2 x 72
+// + 2 x 136 per warpgroup of 128 threads, the state being held by group B.
+constexpr int kFirstWorker = 128;
+constexpr int kThreads = kFirstWorker + 2 * kWorkers;
+constexpr int kRegsFront = 64, kRegsA = 72, kRegsB = 136;
+static_assert(128 * kRegsFront + kWorkers * kRegsA + kWorkers * kRegsB <= kThreads * 96, "registers of the launch");
 
 // Global-memory image of a d x e span state in lane order (see common.cuh): this thread's part is row
 // `row`, columns [col0, col0 + N).
@@ -74,13 +89,18 @@ __device__ __forceinline__ void load_state(const float* state, int row, int col0
 template <int N, int ROWS>
 __device__ __forceinline__ void fma_state(const float* state, int row, int col0, float dec, float (&P)[N]) {
   const float4* src = reinterpret_cast<const float4*>(state) + (size_t)(col0 / 4) * ROWS + row;
-  float4 v[N / 4];
+  constexpr int kBatch = N / 4 < 8 ? N / 4 : 8;   // loads in flight per thread (registers)
 #pragma unroll
-  for (int q = 0; q < N / 4; ++q) v[q] = __ldcg(src + (size_t)q * ROWS);   // written by another CTA of this launch
+  for (int q0 = 0; q0 < N / 4; q0 += kBatch) {
+    float4 v[kBatch];
 #pragma unroll
-  for (int q = 0; q < N / 4; ++q) {
-    P[4 * q] = fmaf(dec, v[q].x, P[4 * q]), P[4 * q + 1] = fmaf(dec, v[q].y, P[4 * q + 1]);
-    P[4 * q + 2] = fmaf(dec, v[q].z, P[4 * q + 2]), P[4 * q + 3] = fmaf(dec, v[q].w, P[4 * q + 3]);
+    for (int u = 0; u < kBatch; ++u) v[u] = __ldcg(src + (size_t)(q0 + u) * ROWS);   // written by another CTA of this launch
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int q = q0 + u;
+      P[4 * q] = fmaf(dec, v[u].x, P[4 * q]), P[4 * q + 1] = fmaf(dec, v[u].y, P[4 * q + 1]);
+      P[4 * q + 2] = fmaf(dec, v[u].z, P[4 * q + 2]), P[4 * q + 3] = fmaf(dec, v[u].w, P[4 * q + 3]);
+    }
   }
 }
 template <int N, int ROWS>
@@ -111,8 +131,8 @@ template <int D, int E>
 __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ CUtensorMap map_a,
                                                         const __grid_constant__ CUtensorMap map_b,
                                                         const float* __restrict__ s, float* __restrict__ totals,
-                                                        int h, int n, int tiles, int span, int nspans, int items,
-                                                        int reverse, int32_t* fault) {
+                                                        int h, int n, const __grid_constant__ SpanCut cut,
+                                                              int reverse, int32_t* fault) {
   constexpr int kStages = 3;
   constexpr int kA = C * D * 2, kB = C * E * 2;
   extern __shared__ uint8_t smem_raw[];
@@ -142,12 +162,12 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  TileWalk w{items, nspans, span, tiles, 0, false, false};
+  TileWalk<false> w{cut, false};
 
   if (warp == 0) {
     if (lane == 0) {
       int g = 0;
-      for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++g) {
+      for (bool ok = w.start(); ok; ok = w.next(), ++g) {
         const int j = g % kStages, use = g / kStages;
         if (use >= 1) wait_or_fault(&empty[j], (use - 1) & 1, &dead, fault, kFaultMmaWait);
         uint8_t* sa = smem + j * (kA + kB);
@@ -159,7 +179,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
   } else if (warp == 1) {
     if (lane == 0) {
       int g = 0, li = -1;
-      for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++g) {
+      for (bool ok = w.start(); ok; ok = w.next(), ++g) {
         const int j = g % kStages, use = g / kStages;
         if (w.first_of_item()) {
           ++li;
@@ -168,8 +188,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
         wait_or_fault(&scaled[j], use & 1, &dead, fault, kFaultTmaWait);
         tc_fence_after_sync();
         uint8_t* sa = smem + j * (kA + kB);
-        umma_gemm(tmem + 128 * (li & 1), Operand{smem_u32(sa), C, true}, Operand{smem_u32(sa + kA), C, true}, E, C / 16,
-                  !w.first_of_item());
+        umma_gemm<true, true, E, C>(tmem + 128 * (li & 1), smem_u32(sa), C, smem_u32(sa + kA), C, !w.first_of_item());
         umma_commit(&empty[j]);
         if (w.last_of_item()) umma_commit(&acc_full[li & 1]);
       }
@@ -177,7 +196,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
   } else if (warp < 6) {
     const int row = tid - 64;  // the token of the tile this thread scales
     int g = 0;
-    for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++g) {
+    for (bool ok = w.start(); ok; ok = w.next(), ++g) {
       const int j = g % kStages, use = g / kStages;
       const float sl2 = s[w.bh % h] * kLog2e;
       const int pos = w.t * C + row;
@@ -192,7 +211,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
     const int row = (warp & 3) * 32 + lane;  // tensor-memory lane = row of the state; warps 6..9 -> quarters 2,3,0,1
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     int li = -1;
-    for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next()) {
+    for (bool ok = w.start(); ok; ok = w.next()) {
       if (!w.last_of_item()) continue;
       ++li;
       wait_or_fault(&acc_full[li & 1], (li >> 1) & 1, &dead, fault, kFaultMmaWait);
@@ -403,7 +422,8 @@ struct WalkArgs {
                        // [kSyncFlags + kSyncSecondBank + sequence] "sequence total written" flags (4 KB in all)
   const float* x_in;   // fused: incoming rank state (b,h,d,e) or NULL
   float* x_out;        // fused: outgoing rank state (b,h,d,e) or NULL
-  int h, n, tiles, span, nspans, items;
+  int h, n;
+  SpanCut cut;
   float qk_scale;      // q and k enter as qk_scale * map(q), qk_scale * map(k)
   int elu;             // map = elu(x) + 1 (otherwise the identity)
   const void* raw;     // backward with a map or a scale: the raw q (dQ walk) or k (dK/dV walk) for the chain rule
@@ -438,30 +458,35 @@ __device__ __forceinline__ void write_state_operand(uint8_t* tile, int rows, int
 //
 //   DQ = false: X,Y = Q,K (width D), Z,OUT = V,O (width E), op(P) = P
 //   DQ = true : X,Y = dO,V (width E), Z,OUT = K,dQ (width D), op(P) = P^T
-// P is the d x e state in both: fp32 in the registers of the eight worker warps (thread = one row and
+// P is the d x e state in both: fp32 in the registers of the eight group-B warps (thread = one row and
 // half of the columns) and bf16 in shared memory as the operand of X op(P).
 //
 // Shared memory: X, Y, Z double buffered and the state operand, seven 32 KB buffers.  A buffer's life
 // inside a tile:  X: tile -> free after S and O2
-//                 Y: tile -> (after S) rows scaled in place -> free after L -> staging tile of OUT
-//                 Z: tile -> free after L and O1
+//                 Y: tile -> (after S) rows scaled in place -> free after L
+//                 Z: tile -> free after L and O1 -> staging tile of OUT
+// (OUT is staged over Z, which is the last one read: X and Y of the tile after next are on their way early)
 // Tensor memory: S (two buffers; the masked scores are packed to bf16 over S itself and feed O1 as its A
 // operand from tensor memory), O (X op(P), rows scaled by lambda^r in place, += S_m Z), L = the state update.
 //   warp 0 (one lane)  producer: loads, and the TMA stores of the finished staging tiles
-//   warp 1 (one lane)  tensor-core issuer
-//   warps 2-9          mask, row scaling, state update, epilogue
+//   warps 1-3 (one lane each)  tensor-core issuers
+//   warps 4-11  (A)    mask of the scores, epilogue
+//   warps 12-19 (B)    the state chain: scaling of Y's rows, of O2's rows, state update
+// Two groups because one group of eight warps doing all of it was the serial chain of a tile: 5300 clocks against
+// the 5600 that its bytes take at the measured HBM rate, with nothing left to make up for the ramps of a launch.
 //
 // FUSED = false: the state of every span at its border comes from the scan (a.p0).
 // FUSED = true : one launch does everything.  With more than one span per sequence every CTA has
 //   exactly one span (a cooperative launch, all CTAs resident).  It first sums its own span,
 //   T = sum_c lambda^(span end - c) k_c v_c^T, streaming K and V once through the Y and Z buffers, writes
 //   T to global memory and raises a flag; then it adds up the totals of the spans before it (and the
-//   incoming rank state) with their decays - that is its border state - and walks.  The K and V tiles
-//   are read again by the walk (they are in L2 by then).  The last span of a sequence needs no total
-//   unless a.all_totals; the outgoing rank state is the state after the last tile of the last span.
+//   incoming rank state) with their decays - that is its border state - and walks.  The last span of a sequence
+//   needs no total unless a.all_totals; the outgoing rank state is the state after the last tile of the last span.
+//   Tokens and totals that the head's decay has brought below 1e-12 are left out of the sums (reach_tiles: the same
+//   line as for the ranks of a group), so on a long sequence only the tiles next to the border are read twice.
 // ---------------------------------------------------------------------------
 template <int D, int E, bool DQ, bool FUSED, bool PRE, bool LINK>
-__global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUtensorMap map_x,
+__global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant__ CUtensorMap map_x,
                                                      const __grid_constant__ CUtensorMap map_y,
                                                      const __grid_constant__ CUtensorMap map_z,
                                                      const __grid_constant__ CUtensorMap map_out,
@@ -476,8 +501,8 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
   const BufPair sy{smem + 2 * kBuf};
   const BufPair sz{smem + 4 * kBuf};
   uint8_t* sp = smem + 6 * kBuf;
-  __shared__ uint64_t x_full[2], y_full[2], z_full[2], s_full[2], sm_ready[2], o_full[2], o2_full[2], staged[2];
-  __shared__ uint64_t p_ready, l_free, o_free, ys_ready, o2s_ready, l_full;
+  __shared__ uint64_t x_full[2], y_full[2], z_full[2], s_full[2], sm_ready[2], o_full[2], o2_full[2], l_full[2], staged[2];
+  __shared__ uint64_t p_ready, l_free, o_free, ys_ready, o2s_ready;
   __shared__ uint64_t mapped[2];   // with a feature map: the workers have mapped the tile's X, Y (dQ: Z) in place
   __shared__ uint64_t ring_full[2], ring_scaled[2], ring_empty[2], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x, even_s;
@@ -505,8 +530,9 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
       mbar_init(&sm_ready[p], kWorkers);
       mbar_init(&o_full[p], 1);
       mbar_init(&o2_full[p], 1);
+      mbar_init(&l_full[p], 1);
       mbar_init(&staged[p], kWorkers);
-      mbar_init(&mapped[p], kWorkers);
+      mbar_init(&mapped[p], 2 * kWorkers);
       mbar_init(&ring_full[p], 1);
       mbar_init(&ring_scaled[p], kWorkers);
       mbar_init(&ring_empty[p], 1);
@@ -516,7 +542,6 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
     mbar_init(&o_free, kWorkers);
     mbar_init(&ys_ready, kWorkers);
     mbar_init(&o2s_ready, kWorkers);
-    mbar_init(&l_full, 1);
     mbar_init(&sum_done, 1);
     fence_mbar_init();
     prefetch_tensormap(&map_x);
@@ -528,13 +553,13 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
       step_s = a.coop ? ss + 1 : 0;                              // this launch among those on the workspace
       step_x = LINK && a.link.ranks > 0 ? sx_ + 1 : 0;           // this hand-over in the group
     }
-    TileWalk w0{a.items, a.nspans, a.span, a.tiles, 0, false, ev != 0};
-    if (w0.start(blockIdx.x, gridDim.x)) {
-      const int sp0 = w0.it - w0.bh * a.nspans;
-      if (FUSED && a.coop && (sp0 < a.nspans - 1 || a.all_totals)) {   // first stage of the span-total ring
+    TileWalk<false> w0{a.cut, ev != 0};
+    if (w0.start()) {
+      const int sp0 = w0.sp;
+      if (FUSED && a.coop && (sp0 < a.cut.nspans - 1 || a.all_totals)) {   // first stage of the span-total ring
         mbar_expect_tx(&ring_full[0], C * (WX + WZ) * 2);
-        tma_load_4d(smem + 2 * kBuf, &map_y, &ring_full[0], 0, w0.t0 * C, 0, w0.bh);
-        tma_load_4d(smem + 4 * kBuf, &map_z, &ring_full[0], 0, w0.t0 * C, 0, w0.bh);
+        tma_load_4d(smem + 2 * kBuf, &map_y, &ring_full[0], 0, (w0.t1 - 1) * C, 0, w0.bh);
+        tma_load_4d(smem + 4 * kBuf, &map_z, &ring_full[0], 0, (w0.t1 - 1) * C, 0, w0.bh);
         early_ring = true;
       } else {                                                          // X of the first tile of the walk
         mbar_expect_tx(&x_full[0], C * WX * 2);
@@ -548,254 +573,250 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  if (tid == 64) TRACE(0);
-  if (tid == 64) GTRACE(57);
+  if (tid == kFirstWorker) TRACE(0);
+  if (tid == kFirstWorker) GTRACE(57);
   const TmemPair t_s{tmem};
   const uint32_t t_o = tmem + 256, t_l = tmem + 384;
-  TileWalk w{a.items, a.nspans, a.span, a.tiles, 0, false, even_s != 0};
-  // the span-total phase: only with several spans per sequence, and then this CTA has one span
-  bool sums = false;
-  int sum_t0 = 0, sum_t1 = 0, my_bh = 0, my_sp = 0;
+  TileWalk<false> w{a.cut, even_s != 0};
+  // the span-total phase: only with several spans per sequence, and then this CTA has one span.  The tiles are
+  // summed from the span's end backwards, as far as the head's decay reaches.
+  int sums = 0, sum_t1 = 0, my_bh = 0;
   if constexpr (FUSED) {
-    if (a.coop && w.start(blockIdx.x, gridDim.x)) {
+    if (a.coop && w.start()) {
       my_bh = w.bh;
-      my_sp = w.it - w.bh * a.nspans;
-      sum_t0 = w.t0;
       sum_t1 = w.t1;
-      sums = my_sp < a.nspans - 1 || a.all_totals;
+      if (w.sp < a.cut.nspans - 1 || a.all_totals) sums = min(w.t1 - w.t0, reach_tiles(a.s[my_bh % a.h]));
     }
   }
 
-  if (warp == 0) {
-    if (lane == 0) {
-      int x_issued = early_x;
-      if (sums) {
-        for (int t = sum_t0, g = 0; t < sum_t1; ++t, ++g) {
-          const int j = g & 1;
-          if (g >= 2) wait_or_fault(&ring_empty[j], ((g >> 1) - 1) & 1, &dead, fault, kFaultMmaWait);
-          if (!(g == 0 && early_ring)) {
-            mbar_expect_tx(&ring_full[j], C * (WX + WZ) * 2);
-            tma_load_4d(sy[j], &map_y, &ring_full[j], 0, t * C, 0, my_bh);
-            tma_load_4d(sz[j], &map_z, &ring_full[j], 0, t * C, 0, my_bh);
-          }
-          if (g == 1 || t == sum_t1 - 1) {
-            // X of the first two tiles of the walk can come in during the sums - behind the first ring
-            // stages, which every CTA of the launch asks for at the same moment and the sums wait for
-            for (bool ok = x_issued == 0 && w.start(blockIdx.x, gridDim.x); ok && x_issued < 2; ok = w.next(), ++x_issued) {
-              mbar_expect_tx(&x_full[x_issued], C * WX * 2);
-              tma_load_4d(sx[x_issued], &map_x, &x_full[x_issued], 0, w.t * C, 0, w.bh);
+  const int wid = (tid - kFirstWorker) & (kWorkers - 1);   // 0..255 inside the group
+  const int row = (warp & 3) * 32 + lane;      // tensor-memory lane quarter of this warp
+  const int half = wid >> 7;
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+  constexpr int kHalfE = E / 2;
+  // q and k enter as c * map(q), c * map(k): the map is applied to the tiles in shared memory, c is folded
+  // into factors that exist anyway (dQ: the state already carries k's c)
+  // (PRE = false: instantiations without any of this, for callers who bring q and k as they are)
+  const float c = PRE ? a.qk_scale : 1.f;
+  const bool elu = PRE && a.elu != 0;
+  // brings tile j (buffers of parity j & 1) through the feature map once its loads have landed, each group its share
+  auto map_tile = [&](int j, auto group) {
+    constexpr int grp = decltype(group)::value;
+    const int q = j & 1, uq = (j >> 1) & 1;
+    if constexpr (!DQ) {
+      wait_or_fault(grp ? &y_full[q] : &x_full[q], uq, &dead, fault, kFaultTmaWait);
+      scale_row_pieces<WX / 16, true>(grp ? sy[q] : sx[q], row, half * (WX / 16), 1.f, lane);
+    } else {
+      wait_or_fault(&z_full[q], uq, &dead, fault, kFaultTmaWait);
+      scale_row_pieces<WZ / 32, true>(sz[q], row, (2 * half + grp) * (WZ / 32), 1.f, lane);
+    }
+    fence_async_smem();
+    mbar_arrive(&mapped[q]);
+  };
+  auto span_total = [&](auto group) {
+    constexpr int grp = decltype(group)::value;
+    if (sums == 0) return;
+    // ---- this span's total, written where the CTAs of the later spans find it; the groups take the stages in turn
+    const float sl2 = a.s[my_bh % a.h] * kLog2e;
+    const int span_end = min(sum_t1 * C, a.n);
+#pragma unroll 1
+    for (int g = grp; g < sums; g += 2) {
+      const int j = g & 1, t = sum_t1 - 1 - g;
+      wait_or_fault(&ring_full[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
+      const float wt = c * decay_pow(sl2, max(span_end - (t * C + row), 0));
+      if (elu)
+        scale_row_pieces<WX / 16, true>(sy[j], row, half * (WX / 16), wt, lane);
+      else
+        scale_row_pieces<WX / 16>(sy[j], row, half * (WX / 16), wt, lane);
+      fence_async_smem();
+      mbar_arrive(&ring_scaled[j]);
+    }
+    wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
+    if (tid == kFirstWorker) TRACE(59);
+    tc_fence_after_sync();
+    const int c0 = half * kHalfE + grp * 32;
+    if (row < D && grp * 32 < kHalfE) {
+      uint32_t r[32];
+      tmem_ld32(t_l + lane_base + c0, r);
+      tmem_ld_wait();
+      store_state32<D>(a.totals + (size_t)blockIdx.x * D * E, row, c0, r);
+    }
+    tc_fence_before_sync();
+    named_sync(2, 2 * kWorkers);   // every worker's part of the total is written ...
+    if (tid == kFirstWorker) {
+      __threadfence();             // ... and visible to the other CTAs before the flag is
+      st_volatile_u32(a.sync + kSyncFlags + blockIdx.x, step_s);
+    }
+    if (tid == kFirstWorker) TRACE(60);
+  };
+  // The three kinds of warps part for good here: each branch sets its registers and is compiled for them.
+  if (warp < kFirstWorker / 32) {
+    set_regs_dec<kRegsFront>();
+    if (warp == 0) {
+      if (lane == 0) {
+        int x_issued = early_x;
+        if (sums > 0) {
+#pragma unroll 1
+          for (int g = 0; g < sums; ++g) {
+            const int j = g & 1, t = sum_t1 - 1 - g;
+            if (g >= 2) wait_or_fault(&ring_empty[j], ((g >> 1) - 1) & 1, &dead, fault, kFaultMmaWait);
+            if (!(g == 0 && early_ring)) {
+              mbar_expect_tx(&ring_full[j], C * (WX + WZ) * 2);
+              tma_load_4d(sy[j], &map_y, &ring_full[j], 0, t * C, 0, my_bh);
+              tma_load_4d(sz[j], &map_z, &ring_full[j], 0, t * C, 0, my_bh);
+            }
+            if (g == 1 || g == sums - 1) {
+              // X of the first two tiles of the walk can come in during the sums - behind the first ring
+              // stages, which every CTA of the launch asks for at the same moment and the sums wait for
+#pragma unroll 1
+              for (bool ok = x_issued == 0 && w.start(); ok && x_issued < 2; ok = w.next(), ++x_issued) {
+                mbar_expect_tx(&x_full[x_issued], C * WX * 2);
+                tma_load_4d(sx[x_issued], &map_x, &x_full[x_issued], 0, w.t * C, 0, w.bh);
+              }
             }
           }
+          wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);   // the MMAs have read every ring stage
         }
-        wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);   // the MMAs have read every ring stage
-      }
-      int i = 0;
-      IntPair out_row{0, 0}, out_bh{0, 0};
-      for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++i) {
-        const int p = i & 1, u = i >> 1;
-        if (i >= x_issued) {
-          if (i >= 2) wait_or_fault(&o2_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);  // S, O2 of tile i-2 read X
-          mbar_expect_tx(&x_full[p], C * WX * 2);
-          tma_load_4d(sx[p], &map_x, &x_full[p], 0, w.t * C, 0, w.bh);
+        int i = 0;
+        IntPair out_row{0, 0}, out_bh{0, 0};
+#pragma unroll 1
+        for (bool ok = w.start(); ok; ok = w.next(), ++i) {
+          const int p = i & 1, u = i >> 1;
+          if (i >= x_issued) {
+            if (i >= 2) {   // S, O2 of tile i-2 read X
+              wait_or_fault(&s_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
+              wait_or_fault(&o2_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
+            }
+            mbar_expect_tx(&x_full[p], C * WX * 2);
+            tma_load_4d(sx[p], &map_x, &x_full[p], 0, w.t * C, 0, w.bh);
+          }
+          if (i >= 2) wait_or_fault(&l_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);   // S, L of tile i-2 read Y
+          mbar_expect_tx(&y_full[p], C * WX * 2);
+          tma_load_4d(sy[p], &map_y, &y_full[p], 0, w.t * C, 0, w.bh);
+          if (i >= 2) {
+            // the output of tile i-2 is staged in Z's buffer: store it, then reuse the buffer
+            wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
+            tma_store_or_add_4d(&map_out, sz[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
+            bulk_commit();
+            bulk_wait_read<0>();
+          }
+          mbar_expect_tx(&z_full[p], C * WZ * 2);
+          tma_load_4d(sz[p], &map_z, &z_full[p], 0, w.t * C, 0, w.bh);
+          out_row.set(p, w.t * C);
+          out_bh.set(p, w.bh);
         }
-        if (i >= 2) wait_or_fault(&o_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);     // L, O1 of tile i-2 read Z
-        mbar_expect_tx(&z_full[p], C * WZ * 2);
-        tma_load_4d(sz[p], &map_z, &z_full[p], 0, w.t * C, 0, w.bh);
-        if (i >= 2) {
-          // the output of tile i-2 is staged in Y's buffer: store it, then reuse the buffer
-          wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
-          tma_store_or_add_4d(&map_out, sy[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
+#pragma unroll 1
+        for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
+          const int p = j & 1, u = j >> 1;
+          wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
+          tma_store_or_add_4d(&map_out, sz[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
           bulk_commit();
-          bulk_wait_read<0>();
         }
-        mbar_expect_tx(&y_full[p], C * WX * 2);
-        tma_load_4d(sy[p], &map_y, &y_full[p], 0, w.t * C, 0, w.bh);
-        out_row.set(p, w.t * C);
-        out_bh.set(p, w.bh);
+        bulk_wait_all<0>();
       }
-      for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
-        const int p = j & 1, u = j >> 1;
-        wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
-        tma_store_or_add_4d(&map_out, sy[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
-        bulk_commit();
-      }
-      bulk_wait_all<0>();
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      if (sums) {
-        for (int t = sum_t0, g = 0; t < sum_t1; ++t, ++g) {
+    } else if (lane == 0) {
+      // Three issuing threads, so that no product waits behind another one's issue (eight instructions of 64 tensor
+      // clocks each take the issuing thread about as long) and none of them has to poll for what is ready:
+      //   warp 1  the span total; O2 = X op(P), then O1 = S_m Z on top of the row-scaled O2
+      //   warp 2  L = K^T diag(w) V (d x e), the scaled rows being Y's
+      //   warp 3  S = X Y^T of the next tile
+      const bool map_xy = PRE && a.elu && !DQ, map_z = PRE && a.elu && DQ;
+      if (warp == 1 && sums > 0) {
+#pragma unroll 1
+        for (int g = 0; g < sums; ++g) {
           const int j = g & 1;
           wait_or_fault(&ring_scaled[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
           tc_fence_after_sync();
-          umma_gemm(t_l, Operand{smem_u32(sy[j]), C, true}, Operand{smem_u32(sz[j]), C, true}, E, C / 16, g > 0);
+          umma_gemm<true, true, E, C>(t_l, smem_u32(sy[j]), C, smem_u32(sz[j]), C, g > 0);
           umma_commit(&ring_empty[j]);
         }
         umma_commit(&sum_done);
       }
       int total = 0;
-      for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next()) ++total;
-      // Per tile: O2 = X op(P) as soon as the state operand exists; L once Y's rows are scaled; O1 = S_m Z
-      // (S_m read from tensor memory) on top of the row-scaled O2 once both are ready; and S of the next
-      // tile whenever its inputs are there, so that the next tile's mask never waits.
-      auto issue_s = [&](int j) {
-        const int q = j & 1;
-        tc_fence_after_sync();
-        umma_gemm(t_s[q], Operand{smem_u32(sx[q]), C, false}, Operand{smem_u32(sy[q]), C, false}, C, WX / 16, false);
-        umma_commit(&s_full[q]);
-      };
-      const bool map_xy = PRE && a.elu && !DQ, map_z = PRE && a.elu && DQ;
-      if (total > 0) {
-        wait_or_fault(&x_full[0], 0, &dead, fault, kFaultTmaWait);
-        wait_or_fault(&y_full[0], 0, &dead, fault, kFaultTmaWait);
-        if (map_xy) wait_or_fault(&mapped[0], 0, &dead, fault, kFaultMmaWait);
-        issue_s(0);
-      }
-      for (int i = 0; i < total; ++i) {
-        const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
-        const int q = (i + 1) & 1, uq = (i + 1) >> 1;
-        // the four products of the tile go out as their inputs become ready, in whatever order that is
-        bool need_o2 = true, need_l = true, need_o1 = true, need_s = i + 1 < total;
-        const long long t0 = clock64();
-        while ((need_o2 || need_l || need_o1 || need_s) && !dead) {
-          // O1 = S_m Z on top of the row-scaled O2, the masked scores read from tensor memory.  It goes out
-          // after L: the commit behind it then also covers L's reads of Y and Z, which is what frees them
-          if (need_o1 && !need_o2 && !need_l && mbar_test_wait(&sm_ready[p], ph) && mbar_test_wait(&o2s_ready, one) &&
-              mbar_test_wait(&z_full[p], ph) && (!map_z || mbar_test_wait(&mapped[p], ph))) {
-            TRACE(32 + i * 5 + 3);
-            tc_fence_after_sync();
-            umma_gemm_ts(t_o, t_s[p], true, Operand{smem_u32(sz[p]), C, true}, WZ, true);
-            umma_commit(&o_full[p]);
-            need_o1 = false;
-            continue;
-          }
-          // L = K^T diag(w) V (d x e), the scaled rows being Y's; the state update has read the previous L
-          if (need_l && mbar_test_wait(&ys_ready, one) && mbar_test_wait(&z_full[p], ph) &&
-              (!map_z || mbar_test_wait(&mapped[p], ph)) && (i < 1 || mbar_test_wait(&l_free, one ^ 1))) {
-            TRACE(32 + i * 5 + 1);
-            tc_fence_after_sync();
-            if constexpr (!DQ)
-              umma_gemm(t_l, Operand{smem_u32(sy[p]), C, true}, Operand{smem_u32(sz[p]), C, true}, E, C / 16, false);
-            else
-              umma_gemm(t_l, Operand{smem_u32(sz[p]), C, true}, Operand{smem_u32(sy[p]), C, true}, E, C / 16, false);
-            umma_commit(&l_full);
-            need_l = false;
-            continue;
-          }
-          // O2 = X op(P): the state operand of this tile is written, the epilogue has drained O
-          if (need_o2 && mbar_test_wait(&p_ready, one) && (i < 1 || mbar_test_wait(&o_free, one ^ 1))) {
-            TRACE(32 + i * 5 + 0);
-            tc_fence_after_sync();
-            if constexpr (!DQ)  // X P: the state tile as [K = d rows] x [N = e columns]
-              umma_gemm(t_o, Operand{smem_u32(sx[p]), C, false}, Operand{smem_u32(sp), D, true}, E, D / 16, false);
-            else                // X P^T: the state tile as [N = d rows] x [K = e columns]
-              umma_gemm(t_o, Operand{smem_u32(sx[p]), C, false}, Operand{smem_u32(sp), D, false}, D, E / 16, false);
-            umma_commit(&o2_full[p]);
-            need_o2 = false;
-            continue;
-          }
-          // S of the next tile; S[q] held the masked scores of tile i-1: its O1 must have read them
-          if (need_s && mbar_test_wait(&x_full[q], uq & 1) && mbar_test_wait(&y_full[q], uq & 1) &&
-              (!map_xy || mbar_test_wait(&mapped[q], uq & 1)) && (i + 1 < 2 || mbar_test_wait(&o_full[q], (uq - 1) & 1))) {
-            TRACE(32 + i * 5 + 2);
-            issue_s(i + 1);
-            need_s = false;
-            continue;
-          }
-          if (clock64() - t0 > kWaitClocks) {
-            dead = 1;
-            atomicOr(fault, kFaultMmaWait);
-          }
+#pragma unroll 1
+      for (bool ok = w.start(); ok; ok = w.next()) ++total;
+      if (warp == 1) {
+#pragma unroll 1
+        for (int i = 0; i < total; ++i) {
+          const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
+          // the state operand of this tile is written, the epilogue has drained O
+          wait_or_fault(&p_ready, one, &dead, fault, kFaultMmaWait);
+          if (i >= 1) wait_or_fault(&o_free, one ^ 1, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&x_full[p], ph, &dead, fault, kFaultTmaWait);
+          if (map_xy) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 0 : 999);
+          tc_fence_after_sync();
+          if constexpr (!DQ)  // X P: the state tile as [K = d rows] x [N = e columns]
+            umma_gemm<false, true, E, D>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false);
+          else                // X P^T: the state tile as [N = d rows] x [K = e columns]
+            umma_gemm<false, false, D, E>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false);
+          umma_commit(&o2_full[p]);
+          // the masked scores are read from tensor memory
+          wait_or_fault(&sm_ready[p], ph, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&z_full[p], ph, &dead, fault, kFaultTmaWait);
+          if (map_z) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&o2s_ready, one, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 3 : 999);
+          tc_fence_after_sync();
+          umma_gemm_ts<true, WZ, 64>(t_o, t_s[p], smem_u32(sz[p]), C, true);
+          umma_commit(&o_full[p]);
         }
-      }
-    }
-  } else {
-    const int cw = warp - 2;                     // 0..7
-    const int row = (warp & 3) * 32 + lane;      // tensor-memory lane quarter of this warp
-    const int half = cw >> 2;
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    constexpr int kHalfE = E / 2;
-    float P[kHalfE];  // this thread's part of the state: row `row`, columns [half * E/2, (half+1) * E/2)
-    float sl2 = 0.f, lam = 1.f;
-    // q and k enter as c * map(q), c * map(k): the map is applied to the tiles in shared memory, c is folded
-    // into factors that exist anyway (dQ: the state already carries k's c)
-    // (PRE = false: instantiations without any of this, for callers who bring q and k as they are)
-    const float c = PRE ? a.qk_scale : 1.f;
-    const float c_mask = DQ ? c : c * c, c_o2 = DQ ? 1.f : c;
-    const bool elu = PRE && a.elu != 0;
-    // brings tile j (buffers of parity j & 1) through the feature map once its loads have landed
-    auto map_tile = [&](int j) {
-      const int q = j & 1, uq = (j >> 1) & 1;
-      if constexpr (!DQ) {
-        wait_or_fault(&x_full[q], uq, &dead, fault, kFaultTmaWait);
-        wait_or_fault(&y_full[q], uq, &dead, fault, kFaultTmaWait);
-        scale_row_pieces<WX / 16, true>(sx[q], row, half * (WX / 16), 1.f, lane);
-        scale_row_pieces<WX / 16, true>(sy[q], row, half * (WX / 16), 1.f, lane);
+      } else if (warp == 2) {
+#pragma unroll 1
+        for (int i = 0; i < total; ++i) {
+          const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
+          wait_or_fault(&z_full[p], ph, &dead, fault, kFaultTmaWait);
+          if (map_z) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
+          if (i >= 1) wait_or_fault(&l_free, one ^ 1, &dead, fault, kFaultMmaWait);   // the state update has read the previous L
+          wait_or_fault(&ys_ready, one, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 1 : 999);
+          tc_fence_after_sync();
+          if constexpr (!DQ)
+            umma_gemm<true, true, E, C>(t_l, smem_u32(sy[p]), C, smem_u32(sz[p]), C, false);
+          else
+            umma_gemm<true, true, E, C>(t_l, smem_u32(sz[p]), C, smem_u32(sy[p]), C, false);
+          umma_commit(&l_full[p]);
+        }
       } else {
-        wait_or_fault(&z_full[q], uq, &dead, fault, kFaultTmaWait);
-        scale_row_pieces<WZ / 16, true>(sz[q], row, half * (WZ / 16), 1.f, lane);
-      }
-      fence_async_smem();
-      mbar_arrive(&mapped[q]);
-    };
-    if (sums) {
-      // ---- this span's total, written where the CTAs of the later spans find it
-      sl2 = a.s[my_bh % a.h] * kLog2e;
-      const int span_end = min(sum_t1 * C, a.n);
-      for (int t = sum_t0, g = 0; t < sum_t1; ++t, ++g) {
-        const int j = g & 1;
-        wait_or_fault(&ring_full[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
-        const float wt = c * decay_pow(sl2, max(span_end - (t * C + row), 0));
-        if (elu)
-          scale_row_pieces<WX / 16, true>(sy[j], row, half * (WX / 16), wt, lane);
-        else
-          scale_row_pieces<WX / 16>(sy[j], row, half * (WX / 16), wt, lane);
-        fence_async_smem();
-        mbar_arrive(&ring_scaled[j]);
-      }
-      wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
-      if (tid == 64) TRACE(59);
-      tc_fence_after_sync();
-      if (row < D) {
-#pragma unroll
-        for (int c0 = 0; c0 < kHalfE; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(t_l + lane_base + half * kHalfE + c0, r);
-          tmem_ld_wait();
-          store_state32<D>(a.totals + (size_t)blockIdx.x * D * E, row, half * kHalfE + c0, r);
+#pragma unroll 1
+        for (int i = 0; i < total; ++i) {
+          const int p = i & 1, ph = (i >> 1) & 1;
+          if (i >= 2) wait_or_fault(&o_full[p], ph ^ 1, &dead, fault, kFaultMmaWait);   // O1 of tile i-2 has read S_m
+          wait_or_fault(&x_full[p], ph, &dead, fault, kFaultTmaWait);
+          wait_or_fault(&y_full[p], ph, &dead, fault, kFaultTmaWait);
+          if (map_xy) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 2 : 999);
+          tc_fence_after_sync();
+          umma_gemm<false, false, C, WX>(t_s[p], smem_u32(sx[p]), C, smem_u32(sy[p]), C, false);
+          umma_commit(&s_full[p]);
         }
       }
-      tc_fence_before_sync();
-      named_sync(1, kWorkers);   // every worker's part of the total is written ...
-      if (tid == 64) {
-        __threadfence();         // ... and visible to the other CTAs before the flag is
-        st_volatile_u32(a.sync + kSyncFlags + blockIdx.x, step_s);
-      }
-      if (tid == 64) TRACE(60);
     }
+  } else if (warp < (kFirstWorker + kWorkers) / 32) {
+    set_regs_dec<kRegsA>();
+    const Group<0> grp;
+    span_total(grp);
     int total = 0;
     if (elu) {
-      for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next()) ++total;
-      if (total > 0) map_tile(0);
+#pragma unroll 1
+      for (bool ok = w.start(); ok; ok = w.next()) ++total;
+      if (total > 0) map_tile(0, grp);
     }
+    // ---- group A
+    const float c_mask = DQ ? c : c * c;
+    float sl2 = 0.f, lam = 1.f;
     int i = 0;
-    for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++i) {
-      const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
-      const int len = min(C, a.n - w.t * C);     // tokens really in the tile
+#pragma unroll 1
+    for (bool ok = w.start(); ok; ok = w.next(), ++i) {
+      const int p = i & 1, ph = (i >> 1) & 1;
       if (w.first_of_item()) {
         sl2 = a.s[w.bh % a.h] * kLog2e;
         lam = exp2f(-sl2);
       }
-      if (tid == 64) TRACE(1 + i * 6 + 0);
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 0 : 999);
       wait_or_fault(&s_full[p], ph, &dead, fault, kFaultMmaWait);
-      wait_or_fault(&y_full[p], ph, &dead, fault, kFaultTmaWait);  // completed long ago: makes Y's bytes visible here
-      if (tid == 64) TRACE(1 + i * 6 + 1);
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 1 : 999);
       tc_fence_after_sync();
-      // state chain first: scale Y's rows so that L can run under the mask
-      scale_row_pieces<WX / 16>(sy[p], row, half * (WX / 16), c * decay_pow(sl2, max(len - row, 0)), lane);
-      fence_async_smem();
-      mbar_arrive(&ys_ready);
-      if (tid == 64) TRACE(1 + i * 6 + 2);
       // masked scores, packed to bf16 in place: they are the A operand of O1 straight from tensor memory
 #pragma unroll 1
       for (int cc = 0; cc < 2; ++cc) {
@@ -806,15 +827,72 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&sm_ready[p]);
-      if (tid == 64) TRACE(1 + i * 6 + 3);
-      if (elu && i + 1 < total) map_tile(i + 1);   // the next tile's S can then go out under this tile's work
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 2 : 999);
+      if (elu && i + 1 < total) map_tile(i + 1, grp);   // the next tile's S can then go out under this tile's work
+      // epilogue: OUT staged in Z's buffer, once L and O1 have read it
+      wait_or_fault(&l_full[p], ph, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&o_full[p], ph, &dead, fault, kFaultMmaWait);
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 3 : 999);
+      tc_fence_after_sync();
+      if (DQ && (elu || c != 1.f)) {
+        // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
+        const int len = min(C, a.n - w.t * C);     // tokens really in the tile
+        const bool live = row < len;
+        const __nv_bfloat16* raw =
+            static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
+#pragma unroll 1
+        for (int cc = 0; cc < WZ / 64; ++cc) {
+          const int col0 = half * (WZ / 2) + cc * 32;
+          stage_row32_chain(t_o + lane_base + col0, sz[p], row, col0, raw, c, elu && live);
+        }
+      } else {
+#pragma unroll 1
+        for (int cc = 0; cc < WZ / 64; ++cc) {
+          const int col0 = half * (WZ / 2) + cc * 32;
+          stage_row32(t_o + lane_base + col0, kNoAcc, 0.f, sz[p], row, col0);
+        }
+      }
+      tc_fence_before_sync();
+      mbar_arrive(&o_free);
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 4 : 999);
+      fence_async_smem();
+      mbar_arrive(&staged[p]);
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 5 : 999);
+    }
+  } else {
+    set_regs_inc<kRegsB>();
+    const Group<1> grp;
+    span_total(grp);
+    int total = 0;
+    if (elu) {
+#pragma unroll 1
+      for (bool ok = w.start(); ok; ok = w.next()) ++total;
+      if (total > 0) map_tile(0, grp);
+    }
+    // ---- group B
+    const float c_o2 = DQ ? 1.f : c;
+    float P[kHalfE];  // this thread's part of the state: row `row`, columns [half * E/2, (half+1) * E/2)
+    float sl2 = 0.f;
+    int i = 0;
+#pragma unroll 1
+    for (bool ok = w.start(); ok; ok = w.next(), ++i) {
+      const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
+      const int len = min(C, a.n - w.t * C);     // tokens really in the tile
+      if (w.first_of_item()) sl2 = a.s[w.bh % a.h] * kLog2e;
+      wait_or_fault(&s_full[p], ph, &dead, fault, kFaultMmaWait);   // S has read Y
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 0 : 999);
+      wait_or_fault(&y_full[p], ph, &dead, fault, kFaultTmaWait);   // completed long ago: makes Y's bytes visible here
+      scale_row_pieces<WX / 16>(sy[p], row, half * (WX / 16), c * decay_pow(sl2, max(len - row, 0)), lane);
+      fence_async_smem();
+      mbar_arrive(&ys_ready);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 1 : 999);
+      if (elu && i + 1 < total) map_tile(i + 1, grp);
       if (__builtin_expect(w.first_of_item(), 0)) {   // once per span: kept out of the tiles' straight-line code
-        // the state at the span border (the score work above does not need it, so the wait for the other
-        // CTAs' totals hides behind it); the O2 MMA that read the operand tile of the previous item has completed
+        // the state at the span border; the O2 MMA that read the operand tile of the previous item has completed
         if constexpr (!FUSED) {
           if (row < D) load_state<kHalfE, D, false>(a.p0 + (size_t)w.it * D * E, row, half * kHalfE, P);
         } else {
-          const int sp_idx = w.it - w.bh * a.nspans;
+          const int sp_idx = w.sp;
           const size_t mine = (size_t)row * E + half * kHalfE;
           // incoming rank state, decayed from the first token of the sequence to the first of the span
           if (a.x_in != nullptr && row < D) {
@@ -829,28 +907,33 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
 #pragma unroll
             for (int j = 0; j < kHalfE; ++j) P[j] = 0.f;
           }
-          // totals of the spans before this one (each decayed to its own end); one thread per flag
-          if (tid - 64 < sp_idx && !dead) {
-            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.nspans + (tid - 64), step_s, a.wait_clocks)) {
+          // totals of the spans before this one (each decayed to its own end) that still reach this one; one
+          // thread per flag
+          const int reach = reach_tiles(a.s[w.bh % a.h]);
+          int first = sp_idx;
+          while (first > 0 && w.t0 - w.span_t0(first) < reach) --first;
+          if (wid < sp_idx && wid >= first && !dead) {
+            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + wid, step_s, a.wait_clocks)) {
               dead = 1;
               atomicOr(fault, kFaultFlagWait);
             }
           }
           named_sync(1, kWorkers);
-          for (int j = 0; j < sp_idx; ++j) {   // each total is decayed to the end of its span
+#pragma unroll 1
+          for (int j = first; j < sp_idx; ++j) {   // each total is decayed to the end of its span
             if (row < D)
-              fma_state<kHalfE, D>(a.totals + (size_t)(w.bh * a.nspans + j) * D * E, row, half * kHalfE,
+              fma_state<kHalfE, D>(a.totals + (size_t)(w.bh * a.cut.nspans + j) * D * E, row, half * kHalfE,
                                    decay_pow(sl2, (w.t0 - w.span_t0(j + 1)) * C), P);
           }
-          if (tid == 64) TRACE(61);
+          if (wid == 0) TRACE(61);
           if (LINK && a.link.ranks > 0) {
             // hand-over of the rank state inside the launch.  P holds the local part of the border state.
             const float sn = a.s[w.bh % a.h] * (float)a.n;
-            const long long elems = (long long)(a.items / a.nspans) * D * E;
+            const long long elems = (long long)(a.cut.items / a.cut.nspans) * D * E;
             const size_t seq_off = (size_t)w.bh * D * E;
             const int n_dst = a.link.ranks - 1 - a.link.me;
             if (n_dst > 0) {
-              const int owner = w.bh * a.nspans + a.nspans - 1;   // the CTA that owns the end of the sequence
+              const int owner = w.bh * a.cut.nspans + a.cut.nspans - 1;   // the CTA that owns the end of the sequence
               const bool far = n_dst > 1 && xl::reaches(sn, 1);   // the state reaches beyond the next rank
               uint32_t* ready = a.sync + kSyncFlags + kSyncSecondBank + w.bh;
               if (w.it == owner && far) {
@@ -859,7 +942,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
                   link_make_total<kHalfE, D>(a.totals + (size_t)owner * D * E, row, half * kHalfE,
                                              decay_pow(sl2, a.n - w.t0 * C), P);
                 named_sync(1, kWorkers);
-                if (tid == 64) {
+                if (wid == 0) {
                   __threadfence();
                   st_volatile_u32(ready, step_s);
                 }
@@ -867,12 +950,12 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
               if (far || w.it == owner) {
                 // the readers of the ranks after this one have acknowledged the slots' previous use
                 if (!dead) {
-                  bool ok = true;
-                  if (xl::needs_ack_wait(step_x) && tid - 64 < n_dst)
-                    ok = wait_flag_ge(a.link.my_acks + xl::ack_index(a.link.me + 1 + (tid - 64), 0), step_x - 2,
-                                      a.link.wait_clocks);
-                  if (far && tid == 64 + xl::kMaxRanks && w.it != owner) ok = wait_flag_eq(ready, step_s, a.wait_clocks);
-                  if (!ok) {
+                  bool ok2 = true;
+                  if (xl::needs_ack_wait(step_x) && wid < n_dst)
+                    ok2 = wait_flag_ge(a.link.my_acks + xl::ack_index(a.link.me + 1 + wid, 0), step_x - 2,
+                                       a.link.wait_clocks);
+                  if (far && wid == xl::kMaxRanks && w.it != owner) ok2 = wait_flag_eq(ready, step_s, a.wait_clocks);
+                  if (!ok2) {
                     dead = 1;
                     atomicOr(fault, kFaultRelayWait);
                   }
@@ -881,21 +964,21 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
                 if (row < D) {
                   if (far)   // several destinations: every CTA of the sequence sends its share
                     link_send_part<kHalfE, D>(a.link, step_x, elems, seq_off, row, half * kHalfE,
-                                              a.totals + (size_t)owner * D * E, sn, sp_idx, a.nspans);
+                                              a.totals + (size_t)owner * D * E, sn, sp_idx, a.cut.nspans);
                   else       // the next rank only: straight from the owner's registers
                     link_send_next<kHalfE, D>(a.link, step_x, elems, seq_off, row, half * kHalfE,
                                               decay_pow(sl2, a.n - w.t0 * C), P, a.totals + (size_t)owner * D * E);
                 }
               }
             }
-            if (tid == 64) TRACE(62);
+            if (wid == 0) TRACE(62);
             if (a.link.me > 0 && row < D) {
               // what the ranks before this one sent, decayed from the first token of the sequence to the span
               if (!link_receive<kHalfE, D>(a.link, step_x, elems, seq_off, row, half * kHalfE,
                                            decay_pow(sl2, w.t0 * C), P, sn))
                 atomicOr(fault, kFaultRelayWait);
             }
-            if (tid == 64) TRACE(55);
+            if (wid == 0) TRACE(55);
           }
         }
         if (row < D) write_state_operand<kHalfE>(sp, D, row, half * kHalfE, P);
@@ -907,6 +990,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
       }
       // O2's rows take their decay lambda^row in tensor memory; O1 then accumulates on top
       wait_or_fault(&o2_full[p], ph, &dead, fault, kFaultMmaWait);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 2 : 999);
       tc_fence_after_sync();
       {
         const float qd = c_o2 * decay_pow(sl2, row);
@@ -916,66 +1000,43 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&o2s_ready);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 3 : 999);
       // state: P <- lambda^len P + L
-      wait_or_fault(&l_full, one, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&l_full[p], ph, &dead, fault, kFaultMmaWait);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 4 : 999);
       tc_fence_after_sync();
       if (row < D) {
         const float lam_c = decay_pow(sl2, len);
 #pragma unroll
-        for (int c0 = 0; c0 < kHalfE; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(t_l + lane_base + half * kHalfE + c0, r);
+        for (int c0 = 0; c0 < kHalfE; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(t_l + lane_base + half * kHalfE + c0, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) P[c0 + j] = fmaf(lam_c, P[c0 + j], __uint_as_float(r[j]));
+          for (int j = 0; j < 16; ++j) P[c0 + j] = fmaf(lam_c, P[c0 + j], __uint_as_float(r[j]));
         }
       }
       tc_fence_before_sync();
       mbar_arrive(&l_free);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 5 : 999);
       if (!w.last_of_item()) {
         if (row < D) write_state_operand<kHalfE>(sp, D, row, half * kHalfE, P);
         fence_async_smem();
         mbar_arrive(&p_ready);
       } else if constexpr (FUSED) {
         // the state after the last tile of the sequence is the outgoing rank state
-        if (a.x_out != nullptr && w.t == a.tiles - 1 && row < D) {
+        if (a.x_out != nullptr && w.t == a.cut.tiles - 1 && row < D) {
           float4* dst = reinterpret_cast<float4*>(a.x_out + (size_t)w.bh * D * E + (size_t)row * E + half * kHalfE);
 #pragma unroll
           for (int q = 0; q < kHalfE / 4; ++q) dst[q] = make_float4(P[4 * q], P[4 * q + 1], P[4 * q + 2], P[4 * q + 3]);
         }
       }
-      if (tid == 64) TRACE(1 + i * 6 + 4);
-      // epilogue: OUT staged in Y's buffer (the L MMA has read the scaled rows)
-      wait_or_fault(&o_full[p], ph, &dead, fault, kFaultMmaWait);
-      tc_fence_after_sync();
-      if (DQ && (elu || c != 1.f)) {
-        // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
-        const bool live = row < len;
-        const __nv_bfloat16* raw =
-            static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
-#pragma unroll 1
-        for (int cc = 0; cc < WZ / 64; ++cc) {
-          const int col0 = half * (WZ / 2) + cc * 32;
-          stage_row32_chain(t_o + lane_base + col0, sy[p], row, col0, raw, c, elu && live);
-        }
-      } else {
-#pragma unroll 1
-        for (int cc = 0; cc < WZ / 64; ++cc) {
-          const int col0 = half * (WZ / 2) + cc * 32;
-          stage_row32(t_o + lane_base + col0, kNoAcc, 0.f, sy[p], row, col0);
-        }
-      }
-      tc_fence_before_sync();
-      mbar_arrive(&o_free);
-      fence_async_smem();
-      mbar_arrive(&staged[p]);
-      if (tid == 64) TRACE(1 + i * 6 + 5);
     }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 64) TRACE(63);
-  if (tid == 64) GTRACE(58);
+  if (tid == kFirstWorker) TRACE(63);
+  if (tid == kFirstWorker) { GTRACE(58); TRACE_VAL(54, smid()); }
   if (warp == 2) tmem_dealloc(tmem, 512);
   if constexpr (!DQ) {   // how this pass cut the sequences, for the dQ walk over the border states it leaves
     if (tid == 0 && blockIdx.x == 0 && a.sync != nullptr) st_volatile_u32(a.sync + kSyncEven, even_s);
@@ -1005,39 +1066,43 @@ __global__ void __launch_bounds__(320, 1) k_walk_out(const __grid_constant__ CUt
 //   dV = S_m^T dO + diag(lambda^(len-c)) K Dn
 //   Dn <- lambda^len Dn + Q^T diag(lambda^r) dO          (len = tokens in the tile, 128 but for a ragged tail)
 //
-// Shared memory: Q, dO (single buffers), K, V (double buffered), the state operand: seven 32 KB buffers.
-//   K : tile -> (after phase A) S_m  -> (after phase B) staging tile of dK
-//   V : tile -> (after phase A) dS_m -> (after phase B) staging tile of dV
-//   Dn: state operand -> (after phase A) row-scaled copy of Q for the state update -> new state operand
+// Shared memory: Q, dO double buffered, K, V, the state operand: seven 32 KB buffers.
+//   Q, dO: tile -> (after the last product that reads them) staging tiles of dK, dV
+//   K, V : free after the four products of the next lines that read them, so the next tile's are on their way early
+//   Dn   : state operand -> (after the state products) row-scaled copy of Q for the state update -> new state operand
 // Tensor memory, four 128-column regions:
-//   T_S : S = Q K^T            -> (masked into shared memory) -> L = Q_s^T dO, the state update
-//   T_dS: dS = dO V^T          -> (masked into shared memory)
+//   T_S : S^T = K Q^T   -> masked and packed to bf16 in place, queries 0..63 in columns [0,32), 64..127 in [96,128),
+//                          the A operand of S_m^T dO; the columns between hold the left half of L = Q_s^T dO
+//   T_dS: dS^T = V dO^T -> the same for dS_m^T Q and the right half of L
 //   T_dK: V Dn^T, rows scaled  -> += dS_m^T Q                  = dK
 //   T_dV: K Dn, rows scaled    -> += S_m^T dO                  = dV
-// Per tile the issuer runs phase A (four products), L as soon as the workers have copied Q and masked S,
-// and phase B once dS is masked and the two state products are scaled; the workers update the state
-// while phase B runs and then stage dK and dV for the TMA stores.
+// Roles as in k_walk_out:
+//   warp 0 producer;  warp 1 state products, then the two products on top of them;  warp 2 L;  warp 3 S^T, dS^T
+//   warps 4-11 (A)  masks, epilogue;  warps 12-19 (B)  scaling, copy of Q, state update
+// With one group of eight warps, masked scores in shared memory and Q, dO single buffered, a tile was a chain of
+// 9300 clocks in which products and workers took turns; its bytes take 8400 at the measured HBM rate.
 //
 // FUSED: as in k_walk_out - the CTA first sums its span, T = sum_r lambda^(r - span start) q_r do_r^T,
-// through the K and V buffers, publishes it, adds up the totals of the LATER spans of its sequence (and
+// through the Q and dO buffers, publishes it, adds up the totals of the LATER spans of its sequence (and
 // the incoming rank state) and walks; the outgoing rank state is the state after the first tile of the
 // sequence.
 // ---------------------------------------------------------------------------
 template <int D, int E, bool FUSED, bool PRE, bool LINK>
-__global__ void __launch_bounds__(320, 1) k_walk_dkv(
+__global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
     const __grid_constant__ CUtensorMap map_dk, const __grid_constant__ CUtensorMap map_dv,
     const __grid_constant__ WalkArgs a) {
+  if (threadIdx.x == 0) GTRACE(56);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint8_t* sq = smem;
-  uint8_t* sdo = smem + kBuf;
-  const BufPair sk{smem + 2 * kBuf};
-  const BufPair sv{smem + 4 * kBuf};
+  const BufPair sq{smem};
+  const BufPair sdo{smem + 2 * kBuf};
+  uint8_t* sk = smem + 4 * kBuf;
+  uint8_t* sv = smem + 5 * kBuf;
   uint8_t* sdn = smem + 6 * kBuf;
-  __shared__ uint64_t kv_full[2], staged[2];
-  __shared__ uint64_t qdo_full, dn_ready, a_done, ms_ready, sm_ready, b_done, l_done, e_free, l_free;
+  __shared__ uint64_t qdo_full[2], staged[2];
+  __shared__ uint64_t kv_full, dn_ready, st_done, s_done, ds_done, sm_ready, dsm_ready, qs_ready, scaled, l_done, l_free, b_done, e_free;
   __shared__ uint64_t mapped;   // with a feature map: the workers have mapped the tile's Q and K in place
   __shared__ uint64_t ring_full[2], ring_scaled[2], ring_empty[2], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x;
@@ -1045,7 +1110,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int32_t* fault = a.fault;
   // thread 0 is also the producer: its first loads go out before the CTA-wide barrier (see k_walk_out)
-  bool early_ring = false, early_kv = false;
+  bool early_ring = false, early_q = false;
   if (tid == 0) {
     dead = 0;
     uint32_t ss = 0, sx_ = 0;   // in flight while the barriers are set up
@@ -1054,23 +1119,27 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
       if (LINK && a.link.ranks > 0) sx_ = ld_volatile_u32(a.link.counters);
     }
     for (int p = 0; p < 2; ++p) {
-      mbar_init(&kv_full[p], 1);
+      mbar_init(&qdo_full[p], 1);
       mbar_init(&staged[p], kWorkers);
       mbar_init(&ring_full[p], 1);
       mbar_init(&ring_scaled[p], kWorkers);
       mbar_init(&ring_empty[p], 1);
     }
-    mbar_init(&qdo_full, 1);
-    mbar_init(&mapped, kWorkers);
-    mbar_init(&dn_ready, kWorkers);
-    mbar_init(&a_done, 1);
-    mbar_init(&ms_ready, kWorkers);
-    mbar_init(&sm_ready, kWorkers);
-    mbar_init(&b_done, 1);
+    mbar_init(&mapped, 2 * kWorkers);
+    mbar_init(&kv_full, 1);
+    mbar_init(&st_done, 1);
+    mbar_init(&s_done, 1);
+    mbar_init(&ds_done, 1);
     mbar_init(&l_done, 1);
-    mbar_init(&e_free, kWorkers);
-    mbar_init(&l_free, kWorkers);
+    mbar_init(&b_done, 1);
     mbar_init(&sum_done, 1);
+    mbar_init(&dn_ready, kWorkers);
+    mbar_init(&sm_ready, kWorkers);
+    mbar_init(&dsm_ready, kWorkers);
+    mbar_init(&qs_ready, kWorkers);
+    mbar_init(&scaled, kWorkers);
+    mbar_init(&l_free, kWorkers);
+    mbar_init(&e_free, kWorkers);
     fence_mbar_init();
     prefetch_tensormap(&map_q);
     prefetch_tensormap(&map_k);
@@ -1082,20 +1151,16 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
       step_s = a.coop ? ss + 1 : 0;                              // this launch among those on the workspace
       step_x = LINK && a.link.ranks > 0 ? sx_ + 1 : 0;           // this hand-over in the group
     }
-    TileWalk w0{a.items, a.nspans, a.span, a.tiles, 0, true, a.even != 0};
-    if (w0.start(blockIdx.x, gridDim.x)) {
-      const int sp0 = w0.it - w0.bh * a.nspans;
-      if (FUSED && a.coop && (sp0 > 0 || a.all_totals)) {   // first stage of the span-total ring: Q, dO
-        mbar_expect_tx(&ring_full[0], C * (D + E) * 2);
-        tma_load_4d(smem + 2 * kBuf, &map_q, &ring_full[0], 0, w0.t0 * C, 0, w0.bh);
-        tma_load_4d(smem + 4 * kBuf, &map_do, &ring_full[0], 0, w0.t0 * C, 0, w0.bh);
-        early_ring = true;
-      } else {                                               // K, V of the first tile of the walk
-        mbar_expect_tx(&kv_full[0], C * (D + E) * 2);
-        tma_load_4d(smem + 2 * kBuf, &map_k, &kv_full[0], 0, w0.t * C, 0, w0.bh);
-        tma_load_4d(smem + 4 * kBuf, &map_v, &kv_full[0], 0, w0.t * C, 0, w0.bh);
-        early_kv = true;
-      }
+    TileWalk<true> w0{a.cut, a.even != 0};
+    if (w0.start()) {
+      const bool ring = FUSED && a.coop && (w0.sp > 0 || a.all_totals);
+      const int t = ring ? w0.t0 : w0.t;   // first stage of the span-total ring, or Q, dO of the walk's first tile
+      uint64_t* bar = ring ? &ring_full[0] : &qdo_full[0];
+      mbar_expect_tx(bar, C * (D + E) * 2);
+      tma_load_4d(smem, &map_q, bar, 0, t * C, 0, w0.bh);
+      tma_load_4d(smem + 2 * kBuf, &map_do, bar, 0, t * C, 0, w0.bh);
+      early_ring = ring;
+      early_q = !ring;
     }
   }
   if (warp == 2) tmem_alloc(&tmem_slot, 512);
@@ -1103,184 +1168,296 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  if (tid == 64) TRACE(0);
-  if (tid == 64) GTRACE(57);
+  if (tid == kFirstWorker) TRACE(0);
+  if (tid == kFirstWorker) GTRACE(57);
   const uint32_t t_s = tmem, t_ds = tmem + 128, t_dk = tmem + 256, t_dv = tmem + 384;
-  TileWalk w{a.items, a.nspans, a.span, a.tiles, 0, true, a.even != 0};
-  bool sums = false;
-  int sum_t0 = 0, sum_t1 = 0, my_bh = 0, my_sp = 0;
+  TileWalk<true> w{a.cut, a.even != 0};
+  // the span-total phase (see k_walk_out): from the span's start onwards, as far as the head's decay reaches
+  int sums = 0, sum_t0 = 0, my_bh = 0;
   if constexpr (FUSED) {
-    if (a.coop && w.start(blockIdx.x, gridDim.x)) {
+    if (a.coop && w.start()) {
       my_bh = w.bh;
-      my_sp = w.it - w.bh * a.nspans;
       sum_t0 = w.t0;
-      sum_t1 = w.t1;
-      sums = my_sp > 0 || a.all_totals;
+      if (w.sp > 0 || a.all_totals) sums = min(w.t1 - w.t0, reach_tiles(a.s[my_bh % a.h]));
     }
   }
-
-  if (warp == 0) {
-    if (lane == 0) {
-      bool first_qdo_issued = false;
-      if (sums) {
-        for (int t = sum_t0, g = 0; t < sum_t1; ++t, ++g) {
-          const int j = g & 1;
-          if (g >= 2) wait_or_fault(&ring_empty[j], ((g >> 1) - 1) & 1, &dead, fault, kFaultMmaWait);
-          if (!(g == 0 && early_ring)) {
-            mbar_expect_tx(&ring_full[j], C * (D + E) * 2);
-            tma_load_4d(sk[j], &map_q, &ring_full[j], 0, t * C, 0, my_bh);
-            tma_load_4d(sv[j], &map_do, &ring_full[j], 0, t * C, 0, my_bh);
-          }
-          // Q, dO of the first tile of the walk can come in during the sums, behind the first ring stages
-          if ((g == 1 || t == sum_t1 - 1) && !first_qdo_issued && w.start(blockIdx.x, gridDim.x)) {
-            mbar_expect_tx(&qdo_full, C * (D + E) * 2);
-            tma_load_4d(sq, &map_q, &qdo_full, 0, w.t * C, 0, w.bh);
-            tma_load_4d(sdo, &map_do, &qdo_full, 0, w.t * C, 0, w.bh);
-            first_qdo_issued = true;
-          }
-        }
-        wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);   // the MMAs have read every ring stage
-      }
-      int i = 0;
-      IntPair out_row{0, 0}, out_bh{0, 0};
-      for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++i) {
-        const int p = i & 1, u = i >> 1;
-        if (i >= 2) {
-          // dK and dV of tile i-2 are staged in this parity's K and V buffers
-          wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
-          tma_store_or_add_4d(&map_dk, sk[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
-          tma_store_or_add_4d(&map_dv, sv[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
-          bulk_commit();
-          bulk_wait_read<0>();
-        }
-        if (!(i == 0 && early_kv)) {
-          mbar_expect_tx(&kv_full[p], C * (D + E) * 2);
-          tma_load_4d(sk[p], &map_k, &kv_full[p], 0, w.t * C, 0, w.bh);
-          tma_load_4d(sv[p], &map_v, &kv_full[p], 0, w.t * C, 0, w.bh);
-        }
-        if (i >= 1) {   // Q, dO of tile i-1 are read: by phase B and by L
-          wait_or_fault(&b_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&l_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
-        }
-        if (i >= 1 || !first_qdo_issued) {
-          mbar_expect_tx(&qdo_full, C * (D + E) * 2);
-          tma_load_4d(sq, &map_q, &qdo_full, 0, w.t * C, 0, w.bh);
-          tma_load_4d(sdo, &map_do, &qdo_full, 0, w.t * C, 0, w.bh);
-        }
-        out_row.set(p, w.t * C);
-        out_bh.set(p, w.bh);
-      }
-      for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
-        const int p = j & 1, u = j >> 1;
-        wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
-        tma_store_or_add_4d(&map_dk, sk[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
-        tma_store_or_add_4d(&map_dv, sv[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
-        bulk_commit();
-      }
-      bulk_wait_all<0>();
+  const int row = (warp & 3) * 32 + lane;      // workers: tensor-memory lane quarter of this warp
+  const int wid = (tid - kFirstWorker) & (kWorkers - 1);   // 0..255 inside the group
+  const int half = wid >> 7;
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+  constexpr int kHalfE = E / 2;
+  // q and k enter as c * map(q), c * map(k): the map is applied to the tiles in shared memory, c is folded
+  // into factors that exist anyway
+  // (PRE = false: instantiations without any of this, for callers who bring q and k as they are)
+  const float c = PRE ? a.qk_scale : 1.f;
+  const bool elu = PRE && a.elu != 0;
+  auto span_total = [&](auto group) {
+    constexpr int grp = decltype(group)::value;
+    if (sums == 0) return;
+    const float sl2 = a.s[my_bh % a.h] * kLog2e;
+#pragma unroll 1
+    for (int g = grp; g < sums; g += 2) {
+      wait_or_fault(&ring_full[grp], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
+      const float wt = c * decay_pow(sl2, g * C + row);
+      if (elu)
+        scale_row_pieces<D / 16, true>(sq[grp], row, half * (D / 16), wt, lane);
+      else
+        scale_row_pieces<D / 16>(sq[grp], row, half * (D / 16), wt, lane);
+      fence_async_smem();
+      mbar_arrive(&ring_scaled[grp]);
     }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      if (sums) {
-        for (int t = sum_t0, g = 0; t < sum_t1; ++t, ++g) {
+    wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
+    if (tid == kFirstWorker) TRACE(59);
+    tc_fence_after_sync();
+    const int c0 = half * kHalfE + grp * 32;
+    if (row < D && grp * 32 < kHalfE) {
+      uint32_t r[32];
+      tmem_ld32(t_s + lane_base + c0, r);
+      tmem_ld_wait();
+      store_state32<D>(a.totals + (size_t)blockIdx.x * D * E, row, c0, r);
+    }
+    tc_fence_before_sync();
+    named_sync(2, 2 * kWorkers);   // every worker's part of the total is written ...
+    if (tid == kFirstWorker) {
+      __threadfence();             // ... and visible to the other CTAs before the flag is
+      st_volatile_u32(a.sync + kSyncFlags + blockIdx.x, step_s);
+    }
+    if (tid == kFirstWorker) TRACE(60);
+  };
+
+  if (warp < kFirstWorker / 32) {
+    set_regs_dec<kRegsFront>();
+    if (warp == 0) {
+      if (lane == 0) {
+        bool kv_issued = false;
+        if (sums > 0) {
+#pragma unroll 1
+          for (int g = 0; g < sums; ++g) {
+            const int j = g & 1, t = sum_t0 + g;
+            if (g >= 2) wait_or_fault(&ring_empty[j], ((g >> 1) - 1) & 1, &dead, fault, kFaultMmaWait);
+            if (!(g == 0 && early_ring)) {
+              mbar_expect_tx(&ring_full[j], C * (D + E) * 2);
+              tma_load_4d(sq[j], &map_q, &ring_full[j], 0, t * C, 0, my_bh);
+              tma_load_4d(sdo[j], &map_do, &ring_full[j], 0, t * C, 0, my_bh);
+            }
+            // K, V of the first tile of the walk can come in during the sums, behind the first ring stages
+            if ((g == 1 || g == sums - 1) && !kv_issued && w.start()) {
+              mbar_expect_tx(&kv_full, C * (D + E) * 2);
+              tma_load_4d(sk, &map_k, &kv_full, 0, w.t * C, 0, w.bh);
+              tma_load_4d(sv, &map_v, &kv_full, 0, w.t * C, 0, w.bh);
+              kv_issued = true;
+            }
+          }
+          wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);   // the MMAs have read every ring stage
+        }
+        int i = 0;
+        IntPair out_row{0, 0}, out_bh{0, 0};
+#pragma unroll 1
+        for (bool ok = w.start(); ok; ok = w.next(), ++i) {
+          const int p = i & 1, u = i >> 1;
+          if (i >= 2) {
+            // dK and dV of tile i-2 are staged in this parity's Q and dO buffers
+            wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
+            tma_store_or_add_4d(&map_dk, sq[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
+            tma_store_or_add_4d(&map_dv, sdo[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
+            bulk_commit();
+            bulk_wait_read<0>();
+          }
+          if (!(i == 0 && early_q)) {
+            mbar_expect_tx(&qdo_full[p], C * (D + E) * 2);
+            tma_load_4d(sq[p], &map_q, &qdo_full[p], 0, w.t * C, 0, w.bh);
+            tma_load_4d(sdo[p], &map_do, &qdo_full[p], 0, w.t * C, 0, w.bh);
+          }
+          if (i >= 1) {   // K, V of tile i-1 are read
+            wait_or_fault(&s_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
+            wait_or_fault(&ds_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
+            wait_or_fault(&st_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
+          }
+          if (i >= 1 || !kv_issued) {
+            mbar_expect_tx(&kv_full, C * (D + E) * 2);
+            tma_load_4d(sk, &map_k, &kv_full, 0, w.t * C, 0, w.bh);
+            tma_load_4d(sv, &map_v, &kv_full, 0, w.t * C, 0, w.bh);
+          }
+          out_row.set(p, w.t * C);
+          out_bh.set(p, w.bh);
+        }
+#pragma unroll 1
+        for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
+          const int p = j & 1, u = j >> 1;
+          wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
+          tma_store_or_add_4d(&map_dk, sq[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
+          tma_store_or_add_4d(&map_dv, sdo[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
+          bulk_commit();
+        }
+        bulk_wait_all<0>();
+      }
+    } else if (lane == 0) {
+      if (warp == 1 && sums > 0) {
+#pragma unroll 1
+        for (int g = 0; g < sums; ++g) {
           const int j = g & 1;
           wait_or_fault(&ring_scaled[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
           tc_fence_after_sync();
-          umma_gemm(t_s, Operand{smem_u32(sk[j]), C, true}, Operand{smem_u32(sv[j]), C, true}, E, C / 16, g > 0);
+          umma_gemm<true, true, E, C>(t_s, smem_u32(sq[j]), C, smem_u32(sdo[j]), C, g > 0);
           umma_commit(&ring_empty[j]);
         }
         umma_commit(&sum_done);
       }
-      int i = 0;
-      for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++i) {
-        const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
-        // phase A.  The state tile as [N = d rows] x [K = e columns] (V Dn^T) and as [K = d rows] x
-        // [N = e columns] (K Dn); T_dK, T_dV were drained by the previous epilogue, T_S by the state update
-        wait_or_fault(&kv_full[p], ph, &dead, fault, kFaultTmaWait);
-        if (PRE && a.elu) wait_or_fault(&mapped, one, &dead, fault, kFaultMmaWait);
-        wait_or_fault(&dn_ready, one, &dead, fault, kFaultMmaWait);
-        if (i >= 1) {
-          wait_or_fault(&e_free, one ^ 1, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&l_free, one ^ 1, &dead, fault, kFaultMmaWait);
+      int total = 0;
+#pragma unroll 1
+      for (bool ok = w.start(); ok; ok = w.next()) ++total;
+      if (warp == 1) {
+#pragma unroll 1
+        for (int i = 0; i < total; ++i) {
+          const int p = i & 1, one = i & 1;
+          // the state tile as [N = d rows] x [K = e columns] (V Dn^T) and as [K = d rows] x [N = e columns] (K Dn);
+          // the epilogue has drained T_dK, T_dV
+          wait_or_fault(&kv_full, one, &dead, fault, kFaultTmaWait);
+          if (elu) wait_or_fault(&mapped, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&dn_ready, one, &dead, fault, kFaultMmaWait);
+          if (i >= 1) wait_or_fault(&e_free, one ^ 1, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 1 : 999);
+          tc_fence_after_sync();
+          umma_gemm<false, false, D, E>(t_dk, smem_u32(sv), C, smem_u32(sdn), D, false);
+          umma_gemm<false, true, E, D>(t_dv, smem_u32(sk), C, smem_u32(sdn), D, false);
+          umma_commit(&st_done);
+          // the masked scores' products on top, A operands from tensor memory
+          wait_or_fault(&sm_ready, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&scaled, one, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 3 : 999);
+          tc_fence_after_sync();
+          umma_gemm_ts<true, E, 96>(t_dv, t_s, smem_u32(sdo[p]), C, true);    // += S_m^T dO
+          wait_or_fault(&dsm_ready, one, &dead, fault, kFaultMmaWait);
+          tc_fence_after_sync();
+          umma_gemm_ts<true, D, 96>(t_dk, t_ds, smem_u32(sq[p]), C, true);    // += dS_m^T Q
+          umma_commit(&b_done);
         }
-        tc_fence_after_sync();
-        umma_gemm(t_dk, Operand{smem_u32(sv[p]), C, false}, Operand{smem_u32(sdn), D, false}, D, E / 16, false);
-        umma_gemm(t_dv, Operand{smem_u32(sk[p]), C, false}, Operand{smem_u32(sdn), D, true}, E, D / 16, false);
-        wait_or_fault(&qdo_full, one, &dead, fault, kFaultTmaWait);
-        tc_fence_after_sync();
-        umma_gemm(t_s, Operand{smem_u32(sq), C, false}, Operand{smem_u32(sk[p]), C, false}, C, D / 16, false);
-        umma_gemm(t_ds, Operand{smem_u32(sdo), C, false}, Operand{smem_u32(sv[p]), C, false}, C, E / 16, false);
-        umma_commit(&a_done);
-        // L = Q_s^T dO over S's columns: the scaled copy of Q is in the state operand's buffer, S is masked
-        wait_or_fault(&ms_ready, one, &dead, fault, kFaultMmaWait);
-        tc_fence_after_sync();
-        umma_gemm(t_s, Operand{smem_u32(sdn), C, true}, Operand{smem_u32(sdo), C, true}, E, C / 16, false);
-        umma_commit(&l_done);
-        // phase B
-        wait_or_fault(&sm_ready, one, &dead, fault, kFaultMmaWait);
-        tc_fence_after_sync();
-        umma_gemm(t_dk, Operand{smem_u32(sv[p]), C, true}, Operand{smem_u32(sq), C, true}, D, C / 16, true);    // += dS_m^T Q
-        umma_gemm(t_dv, Operand{smem_u32(sk[p]), C, true}, Operand{smem_u32(sdo), C, true}, E, C / 16, true);   // += S_m^T dO
-        umma_commit(&b_done);
+      } else if (warp == 2) {
+#pragma unroll 1
+        for (int i = 0; i < total; ++i) {
+          const int p = i & 1, one = i & 1;
+          // L = Q_s^T dO in the columns that the packed scores leave free; the scaled copy of Q is in the state
+          // operand's buffer
+          wait_or_fault(&sm_ready, one, &dead, fault, kFaultMmaWait);
+          if (E > 64) wait_or_fault(&dsm_ready, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&qs_ready, one, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 2 : 999);
+          tc_fence_after_sync();
+          umma_gemm<true, true, 64, C>(t_s + 32, smem_u32(sdn), C, smem_u32(sdo[p]), C, false);
+          if constexpr (E > 64)   // columns 64..127 of dO: its second slab
+            umma_gemm<true, true, 64, C>(t_ds + 32, smem_u32(sdn), C, smem_u32(sdo[p]) + C * kSlabRowBytes, C, false);
+          umma_commit(&l_done);
+        }
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < total; ++i) {
+          const int p = i & 1, one = i & 1;
+          if (i >= 1) {   // the masked scores and L of tile i-1 have been read
+            wait_or_fault(&b_done, one ^ 1, &dead, fault, kFaultMmaWait);
+            wait_or_fault(&l_free, one ^ 1, &dead, fault, kFaultMmaWait);
+          }
+          wait_or_fault(&qdo_full[p], (i >> 1) & 1, &dead, fault, kFaultTmaWait);
+          wait_or_fault(&kv_full, one, &dead, fault, kFaultTmaWait);
+          if (elu) wait_or_fault(&mapped, one, &dead, fault, kFaultMmaWait);
+          TRACE(i < 8 ? 160 + i * 8 + 5 : 999);
+          tc_fence_after_sync();
+          umma_gemm<false, false, C, D>(t_s, smem_u32(sk), C, smem_u32(sq[p]), C, false);
+          umma_commit(&s_done);
+          umma_gemm<false, false, C, E>(t_ds, smem_u32(sv), C, smem_u32(sdo[p]), C, false);
+          umma_commit(&ds_done);
+        }
       }
     }
-  } else {
-    const int cw = warp - 2;
-    const int row = (warp & 3) * 32 + lane;
-    const int half = cw >> 2;
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    constexpr int kHalfE = E / 2;
-    float Dn[kHalfE];  // this thread's part of the suffix state: row `row`, columns [half * E/2, (half+1) * E/2)
+  } else if (warp < (kFirstWorker + kWorkers) / 32) {
+    // ---- group A
+    set_regs_dec<kRegsA>();
+    span_total(Group<0>());
     float sl2 = 0.f, lam = 1.f;
-    // q and k enter as c * map(q), c * map(k): the map is applied to the tiles in shared memory, c is folded
-    // into factors that exist anyway
-    // (PRE = false: instantiations without any of this, for callers who bring q and k as they are)
-    const float c = PRE ? a.qk_scale : 1.f;
-    const bool elu = PRE && a.elu != 0;
-    if (sums) {
-      sl2 = a.s[my_bh % a.h] * kLog2e;
-      for (int t = sum_t0, g = 0; t < sum_t1; ++t, ++g) {
-        const int j = g & 1;
-        wait_or_fault(&ring_full[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
-        const float wt = c * decay_pow(sl2, (t - sum_t0) * C + row);
-        if (elu)
-          scale_row_pieces<D / 16, true>(sk[j], row, half * (D / 16), wt, lane);
-        else
-          scale_row_pieces<D / 16>(sk[j], row, half * (D / 16), wt, lane);
-        fence_async_smem();
-        mbar_arrive(&ring_scaled[j]);
+    int i = 0;
+#pragma unroll 1
+    for (bool ok = w.start(); ok; ok = w.next(), ++i) {
+      const int p = i & 1, one = i & 1;
+      if (w.first_of_item()) {
+        sl2 = a.s[w.bh % a.h] * kLog2e;
+        lam = exp2f(-sl2);
       }
-      wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
-      if (tid == 64) TRACE(59);
-      tc_fence_after_sync();
-      if (row < D) {
-#pragma unroll
-        for (int c0 = 0; c0 < kHalfE; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(t_s + lane_base + half * kHalfE + c0, r);
-          tmem_ld_wait();
-          store_state32<D>(a.totals + (size_t)blockIdx.x * D * E, row, half * kHalfE + c0, r);
+      if (elu) {   // K of this tile through the feature map before any product reads it
+        wait_or_fault(&kv_full, one, &dead, fault, kFaultTmaWait);
+        scale_row_pieces<D / 16, true>(sk, row, half * (D / 16), 1.f, lane);
+        fence_async_smem();
+        mbar_arrive(&mapped);
+      }
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 0 : 999);
+      // S_m^T, then dS_m^T (times Q's c): one piece of code for the four blocks of 32 queries.  The second half of the
+      // queries goes from right to left, packed against the right end, so that every block is read before it is
+      // written over.
+#pragma unroll 1
+      for (int u = 0; u < 4; ++u) {
+        if ((u & 1) == 0) {
+          wait_or_fault(u == 0 ? &s_done : &ds_done, one, &dead, fault, kFaultMmaWait);
+          if (tid == kFirstWorker && u == 0) TRACE(i < 8 ? 64 + i * 6 + 1 : 999);
+          tc_fence_after_sync();
         }
+        const int blk = half == 0 ? (u & 1) : 3 - (u & 1);
+        const uint32_t t = (u < 2 ? t_s : t_ds) + lane_base;
+        uint32_t packed[16];
+        masked_pack32<true>(t + 32 * blk, row, 32 * blk, sl2, lam, packed, u < 2 ? c * c : c);
+        tmem_st16(t + (half == 0 ? 16 * blk : 96 + 16 * (blk - 2)), packed);
+        if ((u & 1) == 1) {
+          tmem_st_wait();
+          tc_fence_before_sync();
+          mbar_arrive(u == 1 ? &sm_ready : &dsm_ready);
+          if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 2 + (u >> 1) : 999);
+        }
+      }
+      // epilogue: dK and dV staged over Q and dO, which every product has read
+      wait_or_fault(&l_done, one, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&b_done, one, &dead, fault, kFaultMmaWait);
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 4 : 999);
+      tc_fence_after_sync();
+      if (elu || c != 1.f) {
+        // dk = dk' * c * map'(k), k read from the raw tensor (rows past the end of the sequence are not stored)
+        const int len = min(C, a.n - w.t * C);
+        const bool live = row < len;
+        const __nv_bfloat16* raw =
+            static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
+#pragma unroll 1
+        for (int cc = 0; cc < D / 64; ++cc) {
+          const int col0 = half * (D / 2) + cc * 32;
+          stage_row32_chain(t_dk + lane_base + col0, sq[p], row, col0, raw, c, elu && live);
+        }
+      }
+      // dV's blocks, and dK's too unless the chain rule above has staged them: one loop
+#pragma unroll 1
+      for (int u = (elu || c != 1.f) ? D / 64 : 0; u < D / 64 + E / 64; ++u) {
+        const bool dv_part = u >= D / 64;
+        const int cc = dv_part ? u - D / 64 : u;
+        const int col0 = half * ((dv_part ? E : D) / 2) + cc * 32;
+        stage_row32((dv_part ? t_dv : t_dk) + lane_base + col0, kNoAcc, 0.f, (dv_part ? sdo : sq)[p], row, col0);
       }
       tc_fence_before_sync();
-      named_sync(1, kWorkers);   // every worker's part of the total is written ...
-      if (tid == 64) {
-        __threadfence();         // ... and visible to the other CTAs before the flag is
-        st_volatile_u32(a.sync + kSyncFlags + blockIdx.x, step_s);
-      }
-      if (tid == 64) TRACE(60);
+      mbar_arrive(&e_free);
+      fence_async_smem();
+      mbar_arrive(&staged[p]);
+      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 5 : 999);
     }
+  } else {
+    // ---- group B
+    set_regs_inc<kRegsB>();
+    span_total(Group<1>());
+    float Dn[kHalfE];  // this thread's part of the suffix state: row `row`, columns [half * E/2, (half+1) * E/2)
+    float sl2 = 0.f;
     int i = 0;
-    for (bool ok = w.start(blockIdx.x, gridDim.x); ok; ok = w.next(), ++i) {
+#pragma unroll 1
+    for (bool ok = w.start(); ok; ok = w.next(), ++i) {
       const int p = i & 1, one = i & 1;
       const int len = min(C, a.n - w.t * C);
       if (__builtin_expect(w.first_of_item(), 0)) {   // once per span: kept out of the tiles' straight-line code
         sl2 = a.s[w.bh % a.h] * kLog2e;
-        lam = exp2f(-sl2);
         if constexpr (!FUSED) {
           if (row < D) load_state<kHalfE, D, false>(a.p0 + (size_t)w.it * D * E, row, half * kHalfE, Dn);
         } else {
-          const int sp_idx = w.it - w.bh * a.nspans;
+          const int sp_idx = w.sp;
           const int span_end = min(w.t1 * C, a.n);
           const size_t mine = (size_t)row * E + half * kHalfE;
           // incoming rank state, decayed from the end of the sequence to the end of the span
@@ -1296,27 +1473,33 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
 #pragma unroll
             for (int j = 0; j < kHalfE; ++j) Dn[j] = 0.f;
           }
-          // totals of the spans after this one (each decayed to its own start); one thread per flag
-          if (tid - 64 < a.nspans - 1 - sp_idx && !dead) {
-            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.nspans + sp_idx + 1 + (tid - 64), step_s, a.wait_clocks)) {
+          // totals of the spans after this one (each decayed to its own start) that still reach this one; one thread
+          // per flag
+          const int reach = reach_tiles(a.s[w.bh % a.h]);
+          int past = sp_idx + 1;
+          while (past < a.cut.nspans && w.span_t0(past) - w.t1 < reach) ++past;
+          if (wid < past - 1 - sp_idx && !dead) {
+            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + sp_idx + 1 + wid, step_s, a.wait_clocks)) {
               dead = 1;
               atomicOr(fault, kFaultFlagWait);
             }
           }
           named_sync(1, kWorkers);
-          for (int j = sp_idx + 1; j < a.nspans; ++j) {   // each total is decayed to the start of its span
+#pragma unroll 1
+          for (int j = sp_idx + 1; j < past; ++j) {   // each total is decayed to the start of its span
             if (row < D)
-              fma_state<kHalfE, D>(a.totals + (size_t)(w.bh * a.nspans + j) * D * E, row, half * kHalfE,
+              fma_state<kHalfE, D>(a.totals + (size_t)(w.bh * a.cut.nspans + j) * D * E, row, half * kHalfE,
                                    decay_pow(sl2, (w.span_t0(j) - w.t1) * C), Dn);
           }
+          if (wid == 0) TRACE(61);
           if (LINK && a.link.ranks > 0) {
             // hand-over of the rank state inside the launch.  Dn holds the local part of the border state.
             const float sn = a.s[w.bh % a.h] * (float)a.n;
-            const long long elems = (long long)(a.items / a.nspans) * D * E;
+            const long long elems = (long long)(a.cut.items / a.cut.nspans) * D * E;
             const size_t seq_off = (size_t)w.bh * D * E;
             const int n_dst = a.link.ranks - 1 - a.link.me;
             if (n_dst > 0) {
-              const int owner = w.bh * a.nspans;   // the CTA that owns the start of the sequence
+              const int owner = w.bh * a.cut.nspans;   // the CTA that owns the start of the sequence
               const bool far = n_dst > 1 && xl::reaches(sn, 1);   // the state reaches beyond the next rank
               uint32_t* ready = a.sync + kSyncFlags + kSyncSecondBank + w.bh;
               if (w.it == owner && far) {
@@ -1325,7 +1508,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
                   link_make_total<kHalfE, D>(a.totals + (size_t)owner * D * E, row, half * kHalfE,
                                              decay_pow(sl2, span_end), Dn);
                 named_sync(1, kWorkers);
-                if (tid == 64) {
+                if (wid == 0) {
                   __threadfence();
                   st_volatile_u32(ready, step_s);
                 }
@@ -1334,12 +1517,12 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
                 // the readers of the ranks after this one in the chain order (the ranks BEFORE it in the
                 // sequence) have acknowledged the slots' previous use
                 if (!dead) {
-                  bool ok = true;
-                  if (xl::needs_ack_wait(step_x) && tid - 64 < n_dst)
-                    ok = wait_flag_ge(a.link.my_acks + xl::ack_index(a.link.me + 1 + (tid - 64), 0), step_x - 2,
-                                      a.link.wait_clocks);
-                  if (far && tid == 64 + xl::kMaxRanks && w.it != owner) ok = wait_flag_eq(ready, step_s, a.wait_clocks);
-                  if (!ok) {
+                  bool ok2 = true;
+                  if (xl::needs_ack_wait(step_x) && wid < n_dst)
+                    ok2 = wait_flag_ge(a.link.my_acks + xl::ack_index(a.link.me + 1 + wid, 0), step_x - 2,
+                                       a.link.wait_clocks);
+                  if (far && wid == xl::kMaxRanks && w.it != owner) ok2 = wait_flag_eq(ready, step_s, a.wait_clocks);
+                  if (!ok2) {
                     dead = 1;
                     atomicOr(fault, kFaultRelayWait);
                   }
@@ -1348,7 +1531,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
                 if (row < D) {
                   if (far)
                     link_send_part<kHalfE, D>(a.link, step_x, elems, seq_off, row, half * kHalfE,
-                                              a.totals + (size_t)owner * D * E, sn, sp_idx, a.nspans);
+                                              a.totals + (size_t)owner * D * E, sn, sp_idx, a.cut.nspans);
                   else
                     link_send_next<kHalfE, D>(a.link, step_x, elems, seq_off, row, half * kHalfE,
                                               decay_pow(sl2, span_end), Dn, a.totals + (size_t)owner * D * E);
@@ -1363,85 +1546,51 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
             }
           }
         }
-        // the phase-A MMAs that read the operand tile of the previous item have completed (a_done was waited for)
+        // the MMAs that read the operand tile of the previous item have completed (l_done was waited for)
         if (row < D) write_state_operand<kHalfE>(sdn, D, row, half * kHalfE, Dn);
         fence_async_smem();
         mbar_arrive(&dn_ready);
       }
-      if (tid == 64) TRACE(1 + i * 6 + 0);
-      if (elu) {   // Q and K of this tile through the feature map before any product reads them
-        wait_or_fault(&kv_full[p], (i >> 1) & 1, &dead, fault, kFaultTmaWait);
-        wait_or_fault(&qdo_full, one, &dead, fault, kFaultTmaWait);
-        scale_row_pieces<D / 16, true>(sk[p], row, half * (D / 16), 1.f, lane);
-        scale_row_pieces<D / 16, true>(sq, row, half * (D / 16), 1.f, lane);
+      wait_or_fault(&qdo_full[p], (i >> 1) & 1, &dead, fault, kFaultTmaWait);
+      if (elu) {   // Q of this tile through the feature map before any product reads it
+        scale_row_pieces<D / 16, true>(sq[p], row, half * (D / 16), 1.f, lane);
         fence_async_smem();
         mbar_arrive(&mapped);
       }
-      wait_or_fault(&a_done, one, &dead, fault, kFaultMmaWait);
-      wait_or_fault(&qdo_full, one, &dead, fault, kFaultTmaWait);  // completed long ago: makes Q's bytes visible here
-      if (tid == 64) TRACE(1 + i * 6 + 1);
+      wait_or_fault(&st_done, one, &dead, fault, kFaultMmaWait);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 0 : 999);
       tc_fence_after_sync();
-      // row-scaled copy of Q over the state operand (phase A has read it), then S_m over the K tile
-      {
-        const float qd = c * decay_pow(sl2, row);
-        constexpr int kPieces = D / 16;
-        uint4 v[kPieces];
-#pragma unroll
-        for (int q = 0; q < kPieces; ++q) {
-          const int piece = half * kPieces + ((q + lane) & (kPieces - 1));
-          v[q] = *reinterpret_cast<const uint4*>(sq + (piece >> 3) * C * 128 + row * 128 + (piece & 7) * 16);
-        }
-#pragma unroll
-        for (int q = 0; q < kPieces; ++q) {
-          const int piece = half * kPieces + ((q + lane) & (kPieces - 1));
-          uint32_t* u = reinterpret_cast<uint32_t*>(&v[q]);
-#pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u[t]));
-            u[t] = pack_bf16(f.x * qd, f.y * qd);
-          }
-          *reinterpret_cast<uint4*>(sdn + (piece >> 3) * C * 128 + row * 128 + (piece & 7) * 16) = v[q];
-        }
-      }
-      // S_m over the K tile, then dS_m (times Q's c) over the V tile: one piece of code for the four blocks (the
-      // tile loop runs the faster the less code it spans)
-#pragma unroll 1
-      for (int u = 0; u < 4; ++u) {
-        const int col0 = half * 64 + (u & 1) * 32;
-        if (u == 2) {   // S_m is complete: the state update's product can go out
-          fence_async_smem();
-          tc_fence_before_sync();
-          mbar_arrive(&ms_ready);
-        }
-        masked_store32((u < 2 ? t_s : t_ds) + lane_base + col0, (u < 2 ? sk : sv)[p], row, col0, sl2, lam,
-                       u < 2 ? c * c : c);
-      }
-      if (tid == 64) TRACE(1 + i * 6 + 2);
+      // row-scaled copy of Q over the state operand (the state products have read it)
+      copy_row_pieces<D / 16>(sdn, sq[p], row, half * (D / 16), c * decay_pow(sl2, row), lane);
+      fence_async_smem();
+      mbar_arrive(&qs_ready);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 1 : 999);
+      // the two state products take their row decay in place (32 columns at a time, dV's blocks then dK's)
       const float kd = decay_pow(sl2, max(len - row, 0));
-      // the two state products take their row decay in place (32 columns at a time, dK's blocks then dV's)
 #pragma unroll 1
       for (int u = 0; u < D / 64 + E / 64; ++u) {
-        const bool dv_part = u >= D / 64;
-        const int cc = dv_part ? u - D / 64 : u;
-        scale_tmem32((dv_part ? t_dv + half * (E / 2) : t_dk + half * (D / 2)) + lane_base + cc * 32, dv_part ? kd * c : kd);
+        const bool dk_part = u >= E / 64;
+        const int cc = dk_part ? u - E / 64 : u;
+        scale_tmem32((dk_part ? t_dk + half * (D / 2) : t_dv + half * (E / 2)) + lane_base + cc * 32, dk_part ? kd : kd * c);
       }
       tmem_st_wait();
-      fence_async_smem();
       tc_fence_before_sync();
-      mbar_arrive(&sm_ready);
-      if (tid == 64) TRACE(1 + i * 6 + 3);
-      // state: Dn <- lambda^len Dn + L, while phase B runs
+      mbar_arrive(&scaled);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 2 : 999);
+      // state: Dn <- lambda^len Dn + L, this thread's half of the columns being the one in T_S or in T_dS
       wait_or_fault(&l_done, one, &dead, fault, kFaultMmaWait);
+      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 3 : 999);
       tc_fence_after_sync();
       if (row < D) {
         const float lam_len = decay_pow(sl2, len);
+        const uint32_t t_l = lane_base + 32 + (E > 64 ? (half ? t_ds : t_s) : t_s + half * 32);
 #pragma unroll
-        for (int c0 = 0; c0 < kHalfE; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(t_s + lane_base + half * kHalfE + c0, r);
+        for (int c0 = 0; c0 < kHalfE; c0 += 16) {
+          uint32_t r[16];
+          tmem_ld16(t_l + c0, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) Dn[c0 + j] = fmaf(lam_len, Dn[c0 + j], __uint_as_float(r[j]));
+          for (int j = 0; j < 16; ++j) Dn[c0 + j] = fmaf(lam_len, Dn[c0 + j], __uint_as_float(r[j]));
         }
       }
       tc_fence_before_sync();
@@ -1450,6 +1599,7 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
         if (row < D) write_state_operand<kHalfE>(sdn, D, row, half * kHalfE, Dn);
         fence_async_smem();
         mbar_arrive(&dn_ready);
+        if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 4 : 999);
       } else if constexpr (FUSED) {
         // the state after the first tile of the sequence is the outgoing rank state
         if (a.x_out != nullptr && w.t == 0 && row < D) {
@@ -1458,41 +1608,12 @@ __global__ void __launch_bounds__(320, 1) k_walk_dkv(
           for (int q = 0; q < kHalfE / 4; ++q) dst[q] = make_float4(Dn[4 * q], Dn[4 * q + 1], Dn[4 * q + 2], Dn[4 * q + 3]);
         }
       }
-      if (tid == 64) TRACE(1 + i * 6 + 4);
-      // epilogue: dK and dV staged over S_m and dS_m (both read by phase B)
-      wait_or_fault(&b_done, one, &dead, fault, kFaultMmaWait);
-      tc_fence_after_sync();
-      if (elu || c != 1.f) {
-        // dk = dk' * c * map'(k), k read from the raw tensor (rows past the end of the sequence are not stored)
-        const bool live = row < len;
-        const __nv_bfloat16* raw =
-            static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
-#pragma unroll 1
-        for (int cc = 0; cc < D / 64; ++cc) {
-          const int col0 = half * (D / 2) + cc * 32;
-          stage_row32_chain(t_dk + lane_base + col0, sk[p], row, col0, raw, c, elu && live);
-        }
-      }
-      // dV's blocks, and dK's too unless the chain rule above has staged them: one loop
-#pragma unroll 1
-      for (int u = (elu || c != 1.f) ? D / 64 : 0; u < D / 64 + E / 64; ++u) {
-        const bool dv_part = u >= D / 64;
-        const int cc = dv_part ? u - D / 64 : u;
-        const int col0 = half * ((dv_part ? E : D) / 2) + cc * 32;
-        stage_row32((dv_part ? t_dv : t_dk) + lane_base + col0, kNoAcc, 0.f, (dv_part ? sv : sk)[p], row,
-                    col0);
-      }
-      tc_fence_before_sync();
-      mbar_arrive(&e_free);
-      fence_async_smem();
-      mbar_arrive(&staged[p]);
-      if (tid == 64) TRACE(1 + i * 6 + 5);
     }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == 64) TRACE(63);
-  if (tid == 64) GTRACE(58);
+  if (tid == kFirstWorker) TRACE(63);
+  if (tid == kFirstWorker) { GTRACE(58); TRACE_VAL(54, smid()); }
   if (warp == 2) tmem_dealloc(tmem, 512);
   if constexpr (FUSED) {
     if (tid == 0 && a.coop) {
@@ -1563,8 +1684,8 @@ cudaError_t launch_span_totals(const Dims& m, const void* a, const void* bten, c
   const size_t smem = (size_t)3 * C * (D + E) * 2 + 1024;
   if ((err = opt_in_smem<k_span_totals<D, E>>(smem)) != cudaSuccess) return err;
   const int items = m.b * m.h * m.nc;
-  k_span_totals<D, E><<<grid_for(items), 320, smem, st>>>(ma, mb, s, totals, m.h, m.n, m.tiles, m.span, m.nc, items,
-                                                          reverse ? 1 : 0, fault);
+  k_span_totals<D, E><<<grid_for(items), 320, smem, st>>>(ma, mb, s, totals, m.h, m.n,
+                                                          make_span_cut(items, m.nc, m.span, m.tiles), reverse ? 1 : 0, fault);
   return launched("launch of the span-total kernel");
 }
 
@@ -1572,10 +1693,10 @@ cudaError_t launch_span_totals(const Dims& m, const void* a, const void* bten, c
 // checks), so all of them become resident as soon as whatever ran before has drained; their waits are
 // bounded all the same and report through the fault word.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_kernel(void (*kernel)(KArgs...), int grid, size_t smem, cudaStream_t st, Args... args) {
+cudaError_t launch_kernel(void (*kernel)(KArgs...), int grid, int threads, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(320);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
@@ -1596,18 +1717,18 @@ cudaError_t launch_walk_out_pre(const Dims& m, const void* x, const void* y, con
   if ((err = fault_word_address(&a.fault)) != cudaSuccess) return err;
   const size_t smem = (size_t)7 * kBuf + 1024;
   if ((err = opt_in_smem<k_walk_out<D, E, DQ, FUSED, PRE, LINK>>(smem)) != cudaSuccess) return err;
-  a.h = m.h, a.n = m.n, a.tiles = m.tiles, a.span = m.span, a.nspans = m.nc, a.items = m.b * m.h * m.nc;
+  a.h = m.h, a.n = m.n, a.cut = make_span_cut(m.b * m.h * m.nc, m.nc, m.span, m.tiles);
   a.wait_clocks = kFlagWaitClocks;
   a.qk_scale = m.qk_scale, a.elu = m.qk_map, a.raw_pitch = m.pitch_d;
   const bool waits = FUSED && (m.nc > 1 || a.link.ranks > 0);   // CTAs wait for one another: one span each, all resident
   a.coop = waits ? 1 : 0;
   if (waits) a.even = 1;
   if (a.link.ranks > 0 && a.link.me < a.link.ranks - 1) a.all_totals = 1;   // the sequence totals are sent on
-  if (waits && a.items > sm_count()) {
+  if (waits && a.cut.items > sm_count()) {
     g_failed_step = "fused walk kernel: more spans than SMs";
     return cudaErrorInvalidConfiguration;
   }
-  if ((err = launch_kernel(k_walk_out<D, E, DQ, FUSED, PRE, LINK>, grid_for(a.items), smem, st, mx, my, mz, mo, a)) !=
+  if ((err = launch_kernel(k_walk_out<D, E, DQ, FUSED, PRE, LINK>, grid_for(a.cut.items), kThreads, smem, st, mx, my, mz, mo, a)) !=
       cudaSuccess) {
     g_failed_step = "launch of a walk kernel";
     return err;
@@ -1630,18 +1751,18 @@ cudaError_t launch_walk_dkv_pre(const Dims& m, const void* q, const void* k, con
   a.raw = k;   // for the chain rule of a folded k preprocessing
   const size_t smem = (size_t)7 * kBuf + 1024;
   if ((err = opt_in_smem<k_walk_dkv<D, E, FUSED, PRE, LINK>>(smem)) != cudaSuccess) return err;
-  a.h = m.h, a.n = m.n, a.tiles = m.tiles, a.span = m.span, a.nspans = m.nc, a.items = m.b * m.h * m.nc;
+  a.h = m.h, a.n = m.n, a.cut = make_span_cut(m.b * m.h * m.nc, m.nc, m.span, m.tiles);
   a.wait_clocks = kFlagWaitClocks;
   a.qk_scale = m.qk_scale, a.elu = m.qk_map, a.raw_pitch = m.pitch_d;
   const bool waits = FUSED && (m.nc > 1 || a.link.ranks > 0);
   a.coop = waits ? 1 : 0;
   if (waits) a.even = 1;
   if (a.link.ranks > 0 && a.link.me < a.link.ranks - 1) a.all_totals = 1;
-  if (waits && a.items > sm_count()) {
+  if (waits && a.cut.items > sm_count()) {
     g_failed_step = "fused walk kernel: more spans than SMs";
     return cudaErrorInvalidConfiguration;
   }
-  if ((err = launch_kernel(k_walk_dkv<D, E, FUSED, PRE, LINK>, grid_for(a.items), smem, st, mq, mk, mv, mdo, mdk, mdv, a)) !=
+  if ((err = launch_kernel(k_walk_dkv<D, E, FUSED, PRE, LINK>, grid_for(a.cut.items), kThreads, smem, st, mq, mk, mv, mdo, mdk, mdv, a)) !=
       cudaSuccess) {
     g_failed_step = "launch of the dk/dv walk kernel";
     return err;
@@ -1783,7 +1904,7 @@ cudaError_t walk_bwd_dkv_fused(const Dims& m, const void* q, const void* k, cons
 
 #ifdef LASP_TRACE
 extern "C" __attribute__((visibility("default"))) int lasp_b200_debug_trace(long long* host) {
-  return (int)cudaMemcpyFromSymbol(host, g_trace, sizeof(long long) * 160 * 64);
+  return (int)cudaMemcpyFromSymbol(host, g_trace, sizeof(long long) * 160 * kTraceSlots);
 }
 #endif
 
