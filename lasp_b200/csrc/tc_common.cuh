@@ -48,13 +48,49 @@ __device__ __forceinline__ int reach_tiles(float s) {
   return s > 0.f && r < 1e6f ? (int)r + 1 : 1 << 20;
 }
 
+// Arithmetic on pairs: one instruction for two fp32 values (packed operations of this architecture), and a product of
+// bf16 pairs with an fp32 factor f in two instead of the five of unpacking, multiplying and packing again:
+// f = hi + lo in bf16, x f = fma(x, hi, x lo), rounded once but for the 2^-18 that x lo loses.
+struct F2 {
+  float x, y;
+};
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+  F2 d;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 d, a, b;\n\t"
+      "mov.b64 {%0, %1}, d;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 d;
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ F2 pair(uint32_t a, uint32_t b) { return {__uint_as_float(a), __uint_as_float(b)}; }
+struct SplitFactor {
+  __nv_bfloat162 hi, lo;
+};
+__device__ __forceinline__ SplitFactor split_factor(float f) {
+  const __nv_bfloat16 h = __float2bfloat16_rn(f);
+  return {__bfloat162bfloat162(h), __float2bfloat162_rn(f - __bfloat162float(h))};
+}
+__device__ __forceinline__ uint32_t scale_bf16x2(uint32_t u, const SplitFactor& f) {
+  const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(&u);
+  const __nv_bfloat162 r = __hfma2(x, f.hi, __hmul2(x, f.lo));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+
 // acc (32 columns) *= f, in tensor memory
 __device__ __forceinline__ void scale_tmem32(uint32_t taddr, float f) {
   uint32_t r[32];
   tmem_ld32(taddr, r);
   tmem_ld_wait();
 #pragma unroll
-  for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
+  for (int j = 0; j < 32; j += 2) {
+    const F2 v = mul2(pair(r[j], r[j + 1]), {f, f});
+    r[j] = __float_as_uint(v.x), r[j + 1] = __float_as_uint(v.y);
+  }
   tmem_st32(taddr, r);
 }
 
@@ -158,7 +194,21 @@ __device__ __forceinline__ void masked_pack32(uint32_t src, int row, int col0, f
     f[g] = pre * decay_pow(sl2, TRANSPOSED ? start - row : row - start);
   }
   tmem_ld_wait();
-  const bool all = TRANSPOSED ? (col0 >= row0 + 31) : (col0 + 31 <= row0);
+  if (TRANSPOSED ? (col0 >= row0 + 31) : (col0 + 31 <= row0)) {   // the whole block is below the diagonal
+    const F2 step = {lam * lam, lam * lam};   // a pair of columns further from it
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      F2 fac = TRANSPOSED ? F2{f[g], f[g] * lam} : F2{f[g] * lam, f[g]};   // of the group's nearest pair
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = TRANSPOSED ? jj : 3 - jj;
+        const F2 m = mul2(pair(r[8 * g + 2 * j], r[8 * g + 2 * j + 1]), fac);
+        out[4 * g + j] = pack_bf16(m.x, m.y);
+        if (jj < 3) fac = mul2(fac, step);
+      }
+    }
+    return;
+  }
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     float m[8];
@@ -166,7 +216,7 @@ __device__ __forceinline__ void masked_pack32(uint32_t src, int row, int col0, f
     for (int jj = 0; jj < 8; ++jj) {
       const int j = TRANSPOSED ? jj : 7 - jj;           // away from the diagonal
       const int col = col0 + 8 * g + j;
-      const bool live = all || (TRANSPOSED ? col >= row : col <= row);
+      const bool live = TRANSPOSED ? col >= row : col <= row;
       m[j] = live ? __uint_as_float(r[8 * g + j]) * f[g] : 0.f;
       f[g] = live ? f[g] * lam : f[g];
     }
@@ -203,6 +253,7 @@ __device__ __forceinline__ float2 elu1_slope_bf16x2(uint32_t u) {
 template <int CHUNKS, bool MAP = false>
 __device__ __forceinline__ void scale_row_pieces(uint8_t* tile, int row, int first, float w, int lane) {
   static_assert((CHUNKS & (CHUNKS - 1)) == 0, "a power of two");
+  const SplitFactor f = split_factor(w);
   uint4 v[CHUNKS];
   uint4* p[CHUNKS];
 #pragma unroll
@@ -217,10 +268,7 @@ __device__ __forceinline__ void scale_row_pieces(uint8_t* tile, int row, int fir
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       if (MAP) u[t] = elu1_bf16x2(u[t]);
-      if (!MAP || w != 1.f) {
-        const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u[t]));
-        u[t] = pack_bf16(f.x * w, f.y * w);
-      }
+      if (!MAP || w != 1.f) u[t] = scale_bf16x2(u[t], f);
     }
     *p[q] = v[q];
   }
@@ -229,6 +277,7 @@ __device__ __forceinline__ void scale_row_pieces(uint8_t* tile, int row, int fir
 // dst row = w * src row, the same pieces of two tiles of C rows
 template <int CHUNKS>
 __device__ __forceinline__ void copy_row_pieces(uint8_t* dst, const uint8_t* src, int row, int first, float w, int lane) {
+  const SplitFactor f = split_factor(w);
   uint4 v[CHUNKS];
 #pragma unroll
   for (int q = 0; q < CHUNKS; ++q) {
@@ -241,8 +290,7 @@ __device__ __forceinline__ void copy_row_pieces(uint8_t* dst, const uint8_t* src
     uint32_t* u = reinterpret_cast<uint32_t*>(&v[q]);
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      const float2 f = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u[t]));
-      u[t] = pack_bf16(f.x * w, f.y * w);
+      u[t] = scale_bf16x2(u[t], f);
     }
     *reinterpret_cast<uint4*>(dst + (piece >> 3) * C * 128 + row * 128 + (piece & 7) * 16) = v[q];
   }

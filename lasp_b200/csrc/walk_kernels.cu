@@ -1013,7 +1013,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           tmem_ld16(t_l + lane_base + half * kHalfE + c0, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) P[c0 + j] = fmaf(lam_c, P[c0 + j], __uint_as_float(r[j]));
+          for (int j = 0; j < 16; j += 2) {
+            const F2 v = fma2({lam_c, lam_c}, {P[c0 + j], P[c0 + j + 1]}, pair(r[j], r[j + 1]));
+            P[c0 + j] = v.x, P[c0 + j + 1] = v.y;
+          }
         }
       }
       tc_fence_before_sync();
@@ -1590,7 +1593,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           tmem_ld16(t_l + c0, r);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) Dn[c0 + j] = fmaf(lam_len, Dn[c0 + j], __uint_as_float(r[j]));
+          for (int j = 0; j < 16; j += 2) {
+            const F2 v = fma2({lam_len, lam_len}, {Dn[c0 + j], Dn[c0 + j + 1]}, pair(r[j], r[j + 1]));
+            Dn[c0 + j] = v.x, Dn[c0 + j + 1] = v.y;
+          }
         }
       }
       tc_fence_before_sync();
