@@ -67,22 +67,15 @@ template <> __device__ __forceinline__ void to_floats<__nv_bfloat16>(const Raw<_
   for (int j = 0; j < 4; ++j) x[2 * j] = __uint_as_float(u[j] << 16), x[2 * j + 1] = __uint_as_float(u[j] & 0xFFFF0000u);
 }
 
-// x0, x1 -> N bf16 pairs whose sum is the pair (N = 3: exactly; the last term of N = 2 is rounded).  Rounding to
-// bf16 by integer arithmetic: half of a unit in the last place added, the rest cut off (the conversion
-// instruction runs at a fraction of the rate, and the remainder x - hi is exact either way).
+// x0, x1 -> N bf16 pairs whose sum is the pair (N = 3: exactly; the last term of N = 2 is rounded): round, take the
+// remainder, which is exact, and so on - nine instructions for three terms of a pair
 template <int N>
 __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t (&t)[N]) {
+  F2 x = {x0, x1};
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    if (i == N - 1 && N < 3) {
-      t[i] = pack_bf16(x0, x1);
-    } else if (i == N - 1) {
-      t[i] = __byte_perm(__float_as_uint(x0), __float_as_uint(x1), 0x7632);
-    } else {
-      const uint32_t h0 = (__float_as_uint(x0) + 0x8000u) & 0xFFFF0000u, h1 = (__float_as_uint(x1) + 0x8000u) & 0xFFFF0000u;
-      t[i] = __byte_perm(h0, h1, 0x7632);
-      x0 -= __uint_as_float(h0), x1 -= __uint_as_float(h1);
-    }
+    t[i] = pack_bf16(x.x, x.y);
+    if (i + 1 < N) x = fma2({__uint_as_float(t[i] << 16), __uint_as_float(t[i] & 0xFFFF0000u)}, {-1.f, -1.f}, x);
   }
 }
 
