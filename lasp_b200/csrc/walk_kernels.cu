@@ -829,21 +829,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       mbar_arrive(&sm_ready[p]);
       if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 2 : 999);
       if (elu && i + 1 < total) map_tile(i + 1, grp);   // the next tile's S can then go out under this tile's work
+      // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
+      const bool chain = PRE && DQ && (elu || c != 1.f);
+      const bool live = row < a.n - w.t * C;
+      const __nv_bfloat16* raw = nullptr;
+      uint4 raw_x[4];
+      if (PRE && DQ && elu) {
+        raw = static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
+        raw_row32(raw_x, raw, half * (WZ / 2));
+      }
       // epilogue: OUT staged in Z's buffer, once L and O1 have read it
       wait_or_fault(&l_full[p], ph, &dead, fault, kFaultMmaWait);
       wait_or_fault(&o_full[p], ph, &dead, fault, kFaultMmaWait);
       if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 3 : 999);
       tc_fence_after_sync();
-      if (DQ && (elu || c != 1.f)) {
-        // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
-        const int len = min(C, a.n - w.t * C);     // tokens really in the tile
-        const bool live = row < len;
-        const __nv_bfloat16* raw =
-            static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
+      if (chain) {
 #pragma unroll 1
         for (int cc = 0; cc < WZ / 64; ++cc) {
           const int col0 = half * (WZ / 2) + cc * 32;
-          stage_row32_chain(t_o + lane_base + col0, sz[p], row, col0, raw, c, elu && live);
+          stage_row32_chain(t_o + lane_base + col0, sz[p], row, col0, raw_x, c, elu && live);
+          if (WZ > 64 && cc == 0 && elu) raw_row32(raw_x, raw, col0 + 32);
         }
       } else {
 #pragma unroll 1
@@ -1413,21 +1418,25 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 2 + (u >> 1) : 999);
         }
       }
+      // dk = dk' * c * map'(k), k read from the raw tensor (rows past the end of the sequence are not stored)
+      const bool live = row < a.n - w.t * C;
+      const __nv_bfloat16* raw = nullptr;
+      uint4 raw_x[4];
+      if (PRE && elu) {
+        raw = static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
+        raw_row32(raw_x, raw, half * (D / 2));
+      }
       // epilogue: dK and dV staged over Q and dO, which every product has read
       wait_or_fault(&l_done, one, &dead, fault, kFaultMmaWait);
       wait_or_fault(&b_done, one, &dead, fault, kFaultMmaWait);
       if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 4 : 999);
       tc_fence_after_sync();
-      if (elu || c != 1.f) {
-        // dk = dk' * c * map'(k), k read from the raw tensor (rows past the end of the sequence are not stored)
-        const int len = min(C, a.n - w.t * C);
-        const bool live = row < len;
-        const __nv_bfloat16* raw =
-            static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
+      if (PRE && (elu || c != 1.f)) {
 #pragma unroll 1
         for (int cc = 0; cc < D / 64; ++cc) {
           const int col0 = half * (D / 2) + cc * 32;
-          stage_row32_chain(t_dk + lane_base + col0, sq[p], row, col0, raw, c, elu && live);
+          stage_row32_chain(t_dk + lane_base + col0, sq[p], row, col0, raw_x, c, elu && live);
+          if (D > 64 && cc == 0 && elu) raw_row32(raw_x, raw, col0 + 32);
         }
       }
       // dV's blocks, and dK's too unless the chain rule above has staged them: one loop
