@@ -881,7 +881,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
     int i = 0;
 #pragma unroll 1
     for (bool ok = w.start(); ok; ok = w.next(), ++i) {
-      const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
+      const int p = i & 1, ph = (i >> 1) & 1;
       const int len = min(C, a.n - w.t * C);     // tokens really in the tile
       if (w.first_of_item()) sl2 = a.s[w.bh % a.h] * kLog2e;
       wait_or_fault(&s_full[p], ph, &dead, fault, kFaultMmaWait);   // S has read Y
