@@ -55,39 +55,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// non-blocking probe of a phase (try_wait may suspend the thread for a while; this never does)
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 // Waits give up after ~1e9 clocks (about half a second), so that a lost arrival becomes a reported fault instead of a
 // hung GPU.
 constexpr uint32_t kWaitClocks = 1000000000u;
 
 // ---------------------------------------------------------------------------
-// TMA: 3-D tiled load global -> shared, completion counted on an mbarrier
+// TMA: tiled copies, loads counted on an mbarrier
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
-                                            int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-// 3-D tiled store shared -> global (bulk async group of the issuing thread)
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* smem_src, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map),
-               "r"(smem_u32(smem_src)), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
-}
-// 4-D forms: coordinates {element, token, 64-column slab, sequence}.  Rows past the end of a sequence read
+// Coordinates {element, token, 64-column slab, sequence}.  Rows past the end of a sequence read
 // as zero and are not written, so a ragged last tile needs no special case.
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1,
                                             int c2, int c3) {
@@ -294,7 +269,7 @@ __device__ __forceinline__ void umma_gemm_ts(uint32_t d_tmem, uint32_t a_tmem, u
 }
 
 // ---------------------------------------------------------------------------
-// host: tensor map of a row-major bf16 matrix [rows x width], box = {64, box_rows, width/64}
+// host: tensor maps
 // ---------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -316,22 +291,6 @@ inline EncodeTiledFn encode_tiled_fn() {
 inline int& last_encode_result() {
   static thread_local int r = 0;
   return r;
-}
-
-inline cudaError_t make_tile_map(CUtensorMap* map, const void* base, uint64_t rows, uint32_t width,
-                                 uint32_t box_rows) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return cudaErrorNotSupported;
-  if (width % 64 || box_rows > 256 || rows == 0) return cudaErrorInvalidValue;
-  const cuuint64_t dims[3] = {64, rows, width / 64};
-  const cuuint64_t strides[2] = {(cuuint64_t)width * 2, 128};  // bytes, for dims 1 and 2
-  const cuuint32_t box[3] = {64, box_rows, width / 64};
-  const cuuint32_t elem[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) last_encode_result() = (int)r;
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 // tensor map of `seqs` row-major bf16 matrices [n x width] lying one after the other,

@@ -12,7 +12,6 @@ using namespace sm100;
 
 constexpr int C = kTensorTile;  // 128 tokens per tile
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr uint32_t kNoAcc = 0xFFFFFFFFu;
 
 // Bounded wait that records a fault once and lets later waits of the CTA give up at once.  There are some thirty of
 // these in a walk kernel: the code that a wait normally runs is one probe, and 32-bit clocks keep the rest short.
@@ -94,21 +93,11 @@ __device__ __forceinline__ void scale_tmem32(uint32_t taddr, float f) {
   tmem_st32(taddr, r);
 }
 
-// tile[row][col0 .. col0+31] = bf16(acc1 + f * acc2) into a swizzled staging tile of C rows
-// (acc2 skipped when taddr2 == kNoAcc); a TMA store then moves the tile out
-__device__ __forceinline__ void stage_row32(uint32_t taddr1, uint32_t taddr2, float f, uint8_t* tile, int row,
-                                            int col0) {
+// tile[row][col0 .. col0+31] = bf16(acc) into a swizzled staging tile of C rows; a TMA store then moves the tile out
+__device__ __forceinline__ void stage_row32(uint32_t taddr, uint8_t* tile, int row, int col0) {
   uint32_t a[32];
-  tmem_ld32(taddr1, a);
-  if (taddr2 != kNoAcc) {
-    uint32_t b[32];
-    tmem_ld32(taddr2, b);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(fmaf(f, __uint_as_float(b[j]), __uint_as_float(a[j])));
-  } else {
-    tmem_ld_wait();
-  }
+  tmem_ld32(taddr, a);
+  tmem_ld_wait();
 #pragma unroll
   for (int j = 0; j < 32; j += 8) {
     uint4 v = make_uint4(pack_bf16(__uint_as_float(a[j]), __uint_as_float(a[j + 1])),
@@ -119,59 +108,11 @@ __device__ __forceinline__ void stage_row32(uint32_t taddr1, uint32_t taddr2, fl
   }
 }
 
-// Tensor-memory accumulator (32 columns at `taddr`, this thread's lane = row) ->
-// decay-masked bf16 in a K-major swizzled tile:
-//   out[row][col] = [row >= col] lambda^(row-col) acc[col].
-// Per group of eight columns the factor is built from the group's right-most unmasked column
-// leftwards by repeated multiplication with lambda (short independent chains), so it can only
-// underflow towards the far columns.  The 32 rows of a warp are `row0 .. row0+31`: groups wholly
-// below the diagonal for every row of the warp need no comparisons, groups wholly above it are zero.
+// Decay mask.  32 fp32 accumulator columns at `src` (columns col0 .. col0+31 of a score tile, this thread's lane = row)
+// become 16 columns of masked bf16 pairs, which the caller leaves in tensor memory as the A operand of the next MMA.
+// Per group of eight columns the factor is built from the group's live column nearest the diagonal away from it by
+// repeated multiplication with lambda (short independent chains), so it can only underflow towards the far columns.
 // `pre` multiplies every element (the folded q,k scale).
-__device__ __forceinline__ void masked_store32(uint32_t taddr, uint8_t* tile, int row, int col0, float sl2,
-                                               float lam, float pre = 1.f) {
-  const int row0 = row & ~31;
-  if (col0 > row0 + 31) {   // the whole block is above the diagonal (same for every lane of the warp)
-#pragma unroll
-    for (int g = 0; g < 4; ++g)
-      *reinterpret_cast<uint4*>(tile + tile_offset(row, col0 + 8 * g, C)) = make_uint4(0u, 0u, 0u, 0u);
-    return;
-  }
-  uint32_t r[32];
-  tmem_ld32(taddr, r);
-  float f[4];
-#pragma unroll
-  for (int g = 0; g < 4; ++g) f[g] = pre * decay_pow(sl2, row - min(row, col0 + 8 * g + 7));
-  tmem_ld_wait();
-  if (col0 + 31 <= row0) {  // the whole block is below the diagonal
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      float m[8];
-#pragma unroll
-      for (int j = 7; j >= 0; --j) {
-        m[j] = __uint_as_float(r[8 * g + j]) * f[g];
-        f[g] *= lam;
-      }
-      *reinterpret_cast<uint4*>(tile + tile_offset(row, col0 + 8 * g, C)) =
-          make_uint4(pack_bf16(m[0], m[1]), pack_bf16(m[2], m[3]), pack_bf16(m[4], m[5]), pack_bf16(m[6], m[7]));
-    }
-    return;
-  }
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    float m[8];
-#pragma unroll
-    for (int j = 7; j >= 0; --j) {
-      const bool live = (col0 + 8 * g + j) <= row;
-      m[j] = live ? __uint_as_float(r[8 * g + j]) * f[g] : 0.f;
-      f[g] = live ? f[g] * lam : f[g];
-    }
-    *reinterpret_cast<uint4*>(tile + tile_offset(row, col0 + 8 * g, C)) =
-        make_uint4(pack_bf16(m[0], m[1]), pack_bf16(m[2], m[3]), pack_bf16(m[4], m[5]), pack_bf16(m[6], m[7]));
-  }
-}
-
-// The same mask, but the result stays in tensor memory as the A operand of the next MMA: 32 fp32
-// columns at `src` (columns col0 .. col0+31 of the score tile) become 16 columns of bf16 pairs at `dst`.
 // TRANSPOSED = false: lane = query row r, column = key c:  [r >= c] lambda^(r-c)
 // TRANSPOSED = true : lane = key c, column = query row r:  [r >= c] lambda^(r-c)   (the tile is S^T)
 template <bool TRANSPOSED>

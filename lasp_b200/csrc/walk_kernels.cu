@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
         for (int cc = 0; cc < WZ / 64; ++cc) {
           const int col0 = half * (WZ / 2) + cc * 32;
-          stage_row32(t_o + lane_base + col0, kNoAcc, 0.f, sz[p], row, col0);
+          stage_row32(t_o + lane_base + col0, sz[p], row, col0);
         }
       }
       tc_fence_before_sync();
@@ -1445,7 +1445,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         const bool dv_part = u >= D / 64;
         const int cc = dv_part ? u - D / 64 : u;
         const int col0 = half * ((dv_part ? E : D) / 2) + cc * 32;
-        stage_row32((dv_part ? t_dv : t_dk) + lane_base + col0, kNoAcc, 0.f, (dv_part ? sdo : sq)[p], row, col0);
+        stage_row32((dv_part ? t_dv : t_dk) + lane_base + col0, (dv_part ? sdo : sq)[p], row, col0);
       }
       tc_fence_before_sync();
       mbar_arrive(&e_free);
