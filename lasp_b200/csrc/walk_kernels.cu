@@ -413,6 +413,33 @@ __device__ __forceinline__ bool wait_flag_ge(const uint32_t* flag, uint32_t want
   return true;
 }
 
+// The span-total phase streams its tiles through a ring over tile buffers that the walk is not using yet: three stages of
+// 64 KB (128-wide heads) or four of 48 KB over all six, or four of 32 KB (64-wide heads) over four, whose first is
+// BASE, so that the walk's first loads into the other two can come in meanwhile.  With two stages a tile took a load's
+// latency and a half: 131072 tokens, 16 heads, forward 414 -> 404 us; 4 x 16 x 4096 tokens, 64-wide, folded
+// preprocessing, 86 -> 75 us.
+// Where the number of stages is even the worker groups take the tiles in turn; where it is odd each takes half of every
+// tile, because a group has to see every phase of a barrier that it waits for.
+template <int D, int E, int BASE>
+struct Ring {
+  static constexpr int kStage = C * (D + E) * 2;
+  static constexpr bool kNarrow = D + E == 128;   // over four buffers
+  static constexpr int kStages = (kNarrow ? 4 : 6) * kBuf / kStage;
+  static constexpr bool kInTurn = kStages % 2 == 0;
+  uint8_t* smem;
+  __device__ __forceinline__ uint8_t* a(int j) const { return smem + (kNarrow ? BASE : 0) * kBuf + j * kStage; }
+  __device__ __forceinline__ uint8_t* b(int j) const { return a(j) + C * D * 2; }
+  // a group's share of the row scaling of stage j
+  template <int GRP, bool MAP>
+  __device__ __forceinline__ void scale(int j, int row, int half, float w, int lane) const {
+    if constexpr (kInTurn)
+      scale_row_pieces<D / 16, MAP>(a(j), row, half * (D / 16), w, lane);
+    else
+      scale_row_pieces<D / 32, MAP>(a(j), row, (2 * half + GRP) * (D / 32), w, lane);
+  }
+};
+constexpr int kMaxRing = 4;
+
 struct WalkArgs {
   const float* s;
   const float* p0;     // not fused: fp32 state of every span at its border, [items][D][E] (from the scan)
@@ -478,7 +505,7 @@ __device__ __forceinline__ void write_state_operand(uint8_t* tile, int rows, int
 // FUSED = false: the state of every span at its border comes from the scan (a.p0).
 // FUSED = true : one launch does everything.  With more than one span per sequence every CTA has
 //   exactly one span (a cooperative launch, all CTAs resident).  It first sums its own span,
-//   T = sum_c lambda^(span end - c) k_c v_c^T, streaming K and V once through the Y and Z buffers, writes
+//   T = sum_c lambda^(span end - c) k_c v_c^T, streaming K and V once through a ring of stages, writes
 //   T to global memory and raises a flag; then it adds up the totals of the spans before it (and the
 //   incoming rank state) with their decays - that is its border state - and walks.  The last span of a sequence
 //   needs no total unless a.all_totals; the outgoing rank state is the state after the last tile of the last span.
@@ -501,10 +528,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
   const BufPair sy{smem + 2 * kBuf};
   const BufPair sz{smem + 4 * kBuf};
   uint8_t* sp = smem + 6 * kBuf;
+  using R = Ring<WX, WZ, 2>;
+  const R ring{smem};
   __shared__ uint64_t x_full[2], y_full[2], z_full[2], s_full[2], sm_ready[2], o_full[2], o2_full[2], l_full[2], staged[2];
   __shared__ uint64_t p_ready, l_free, o_free, ys_ready, o2s_ready;
   __shared__ uint64_t mapped[2];   // with a feature map: the workers have mapped the tile's X, Y (dQ: Z) in place
-  __shared__ uint64_t ring_full[2], ring_scaled[2], ring_empty[2], sum_done;   // the span-total phase
+  __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x, even_s;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -533,9 +562,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       mbar_init(&l_full[p], 1);
       mbar_init(&staged[p], kWorkers);
       mbar_init(&mapped[p], 2 * kWorkers);
-      mbar_init(&ring_full[p], 1);
-      mbar_init(&ring_scaled[p], kWorkers);
-      mbar_init(&ring_empty[p], 1);
+    }
+    if constexpr (FUSED) {
+      for (int j = 0; j < R::kStages; ++j) {
+        mbar_init(&ring_full[j], 1);
+        mbar_init(&ring_scaled[j], (R::kInTurn ? 1 : 2) * kWorkers / 32);
+        mbar_init(&ring_empty[j], 1);
+      }
     }
     mbar_init(&p_ready, kWorkers);
     mbar_init(&l_free, kWorkers);
@@ -558,8 +591,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       const int sp0 = w0.sp;
       if (FUSED && a.coop && (sp0 < a.cut.nspans - 1 || a.all_totals)) {   // first stage of the span-total ring
         mbar_expect_tx(&ring_full[0], C * (WX + WZ) * 2);
-        tma_load_4d(smem + 2 * kBuf, &map_y, &ring_full[0], 0, (w0.t1 - 1) * C, 0, w0.bh);
-        tma_load_4d(smem + 4 * kBuf, &map_z, &ring_full[0], 0, (w0.t1 - 1) * C, 0, w0.bh);
+        tma_load_4d(ring.a(0), &map_y, &ring_full[0], 0, (w0.t1 - 1) * C, 0, w0.bh);
+        tma_load_4d(ring.b(0), &map_z, &ring_full[0], 0, (w0.t1 - 1) * C, 0, w0.bh);
         early_ring = true;
       } else {                                                          // X of the first tile of the walk
         mbar_expect_tx(&x_full[0], C * WX * 2);
@@ -620,16 +653,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
     const float sl2 = a.s[my_bh % a.h] * kLog2e;
     const int span_end = min(sum_t1 * C, a.n);
 #pragma unroll 1
-    for (int g = grp; g < sums; g += 2) {
-      const int j = g & 1, t = sum_t1 - 1 - g;
-      wait_or_fault(&ring_full[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
-      const float wt = c * decay_pow(sl2, max(span_end - (t * C + row), 0));
+    for (int g = R::kInTurn ? grp : 0; g < sums; g += R::kInTurn ? 2 : 1) {
+      const int j = g % R::kStages;
+      wait_or_fault(&ring_full[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
+      const float wt = c * decay_pow(sl2, max(span_end - ((sum_t1 - 1 - g) * C + row), 0));
       if (elu)
-        scale_row_pieces<WX / 16, true>(sy[j], row, half * (WX / 16), wt, lane);
+        ring.template scale<grp, true>(j, row, half, wt, lane);
       else
-        scale_row_pieces<WX / 16>(sy[j], row, half * (WX / 16), wt, lane);
+        ring.template scale<grp, false>(j, row, half, wt, lane);
       fence_async_smem();
-      mbar_arrive(&ring_scaled[j]);
+      warp_arrive(&ring_scaled[j]);
     }
     wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
     if (tid == kFirstWorker) TRACE(59);
@@ -658,14 +691,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         if (sums > 0) {
 #pragma unroll 1
           for (int g = 0; g < sums; ++g) {
-            const int j = g & 1, t = sum_t1 - 1 - g;
-            if (g >= 2) wait_or_fault(&ring_empty[j], ((g >> 1) - 1) & 1, &dead, fault, kFaultMmaWait);
+            const int j = g % R::kStages, t = sum_t1 - 1 - g;
+            if (g >= R::kStages) wait_or_fault(&ring_empty[j], (g / R::kStages - 1) & 1, &dead, fault, kFaultMmaWait);
             if (!(g == 0 && early_ring)) {
-              mbar_expect_tx(&ring_full[j], C * (WX + WZ) * 2);
-              tma_load_4d(sy[j], &map_y, &ring_full[j], 0, t * C, 0, my_bh);
-              tma_load_4d(sz[j], &map_z, &ring_full[j], 0, t * C, 0, my_bh);
+              mbar_expect_tx(&ring_full[j], R::kStage);
+              tma_load_4d(ring.a(j), &map_y, &ring_full[j], 0, t * C, 0, my_bh);
+              tma_load_4d(ring.b(j), &map_z, &ring_full[j], 0, t * C, 0, my_bh);
             }
-            if (g == 1 || g == sums - 1) {
+            if (R::kNarrow && (g == 1 || g == sums - 1)) {
               // X of the first two tiles of the walk can come in during the sums - behind the first ring
               // stages, which every CTA of the launch asks for at the same moment and the sums wait for
 #pragma unroll 1
@@ -724,10 +757,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       if (warp == 1 && sums > 0) {
 #pragma unroll 1
         for (int g = 0; g < sums; ++g) {
-          const int j = g & 1;
-          wait_or_fault(&ring_scaled[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
+          const int j = g % R::kStages;
+          wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
           tc_fence_after_sync();
-          umma_gemm<true, true, E, C>(t_l, smem_u32(sy[j]), C, smem_u32(sz[j]), C, g > 0);
+          umma_gemm<true, true, E, C>(t_l, smem_u32(ring.a(j)), C, smem_u32(ring.b(j)), C, g > 0);
           umma_commit(&ring_empty[j]);
         }
         umma_commit(&sum_done);
@@ -1109,10 +1142,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   uint8_t* sk = smem + 4 * kBuf;
   uint8_t* sv = smem + 5 * kBuf;
   uint8_t* sdn = smem + 6 * kBuf;
+  using R = Ring<D, E, 0>;
+  const R ring_buf{smem};
   __shared__ uint64_t qdo_full[2], staged[2];
   __shared__ uint64_t kv_full, dn_ready, st_done, s_done, ds_done, sm_ready, dsm_ready, qs_ready, scaled, l_done, l_free, b_done, e_free;
   __shared__ uint64_t mapped;   // with a feature map: the workers have mapped the tile's Q and K in place
-  __shared__ uint64_t ring_full[2], ring_scaled[2], ring_empty[2], sum_done;   // the span-total phase
+  __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x;
   __shared__ int dead;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1129,9 +1164,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     for (int p = 0; p < 2; ++p) {
       mbar_init(&qdo_full[p], 1);
       mbar_init(&staged[p], kWorkers);
-      mbar_init(&ring_full[p], 1);
-      mbar_init(&ring_scaled[p], kWorkers);
-      mbar_init(&ring_empty[p], 1);
+    }
+    if constexpr (FUSED) {
+      for (int j = 0; j < R::kStages; ++j) {
+        mbar_init(&ring_full[j], 1);
+        mbar_init(&ring_scaled[j], (R::kInTurn ? 1 : 2) * kWorkers / 32);
+        mbar_init(&ring_empty[j], 1);
+      }
     }
     mbar_init(&mapped, 2 * kWorkers);
     mbar_init(&kv_full, 1);
@@ -1165,8 +1204,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       const int t = ring ? w0.t0 : w0.t;   // first stage of the span-total ring, or Q, dO of the walk's first tile
       uint64_t* bar = ring ? &ring_full[0] : &qdo_full[0];
       mbar_expect_tx(bar, C * (D + E) * 2);
-      tma_load_4d(smem, &map_q, bar, 0, t * C, 0, w0.bh);
-      tma_load_4d(smem + 2 * kBuf, &map_do, bar, 0, t * C, 0, w0.bh);
+      tma_load_4d(sq[0], &map_q, bar, 0, t * C, 0, w0.bh);   // (where the first ring stage begins too)
+      tma_load_4d(ring ? ring_buf.b(0) : sdo[0], &map_do, bar, 0, t * C, 0, w0.bh);
       early_ring = ring;
       early_q = !ring;
     }
@@ -1204,15 +1243,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     if (sums == 0) return;
     const float sl2 = a.s[my_bh % a.h] * kLog2e;
 #pragma unroll 1
-    for (int g = grp; g < sums; g += 2) {
-      wait_or_fault(&ring_full[grp], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
+    for (int g = R::kInTurn ? grp : 0; g < sums; g += R::kInTurn ? 2 : 1) {
+      const int j = g % R::kStages;
+      wait_or_fault(&ring_full[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
       const float wt = c * decay_pow(sl2, g * C + row);
       if (elu)
-        scale_row_pieces<D / 16, true>(sq[grp], row, half * (D / 16), wt, lane);
+        ring_buf.template scale<grp, true>(j, row, half, wt, lane);
       else
-        scale_row_pieces<D / 16>(sq[grp], row, half * (D / 16), wt, lane);
+        ring_buf.template scale<grp, false>(j, row, half, wt, lane);
       fence_async_smem();
-      mbar_arrive(&ring_scaled[grp]);
+      warp_arrive(&ring_scaled[j]);
     }
     wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
     if (tid == kFirstWorker) TRACE(59);
@@ -1241,15 +1281,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         if (sums > 0) {
 #pragma unroll 1
           for (int g = 0; g < sums; ++g) {
-            const int j = g & 1, t = sum_t0 + g;
-            if (g >= 2) wait_or_fault(&ring_empty[j], ((g >> 1) - 1) & 1, &dead, fault, kFaultMmaWait);
+            const int j = g % R::kStages, t = sum_t0 + g;
+            if (g >= R::kStages) wait_or_fault(&ring_empty[j], (g / R::kStages - 1) & 1, &dead, fault, kFaultMmaWait);
             if (!(g == 0 && early_ring)) {
-              mbar_expect_tx(&ring_full[j], C * (D + E) * 2);
-              tma_load_4d(sq[j], &map_q, &ring_full[j], 0, t * C, 0, my_bh);
-              tma_load_4d(sdo[j], &map_do, &ring_full[j], 0, t * C, 0, my_bh);
+              mbar_expect_tx(&ring_full[j], R::kStage);
+              tma_load_4d(ring_buf.a(j), &map_q, &ring_full[j], 0, t * C, 0, my_bh);
+              tma_load_4d(ring_buf.b(j), &map_do, &ring_full[j], 0, t * C, 0, my_bh);
             }
             // K, V of the first tile of the walk can come in during the sums, behind the first ring stages
-            if ((g == 1 || g == sums - 1) && !kv_issued && w.start()) {
+            if (R::kNarrow && (g == 1 || g == sums - 1) && !kv_issued && w.start()) {
               mbar_expect_tx(&kv_full, C * (D + E) * 2);
               tma_load_4d(sk, &map_k, &kv_full, 0, w.t * C, 0, w.bh);
               tma_load_4d(sv, &map_v, &kv_full, 0, w.t * C, 0, w.bh);
@@ -1303,10 +1343,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       if (warp == 1 && sums > 0) {
 #pragma unroll 1
         for (int g = 0; g < sums; ++g) {
-          const int j = g & 1;
-          wait_or_fault(&ring_scaled[j], (g >> 1) & 1, &dead, fault, kFaultTmaWait);
+          const int j = g % R::kStages;
+          wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
           tc_fence_after_sync();
-          umma_gemm<true, true, E, C>(t_s, smem_u32(sq[j]), C, smem_u32(sdo[j]), C, g > 0);
+          umma_gemm<true, true, E, C>(t_s, smem_u32(ring_buf.a(j)), C, smem_u32(ring_buf.b(j)), C, g > 0);
           umma_commit(&ring_empty[j]);
         }
         umma_commit(&sum_done);
