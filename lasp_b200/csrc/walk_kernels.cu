@@ -37,7 +37,9 @@ __device__ __forceinline__ long long gtime() { long long t; asm volatile("mov.u6
 #define GTRACE(slot) do { if (blockIdx.x < 160) g_trace[blockIdx.x * kTraceSlots + (slot)] = gtime(); } while (0)
 #define TRACE_VAL(slot, v) do { if (blockIdx.x < 160) g_trace[blockIdx.x * kTraceSlots + (slot)] = (v); } while (0)
 __device__ __forceinline__ uint32_t smid() { uint32_t v; asm volatile("mov.u32 %0, %%smid;" : "=r"(v)); return v; }
+#define TRACE_TILE(base, stride, i, k) do { if ((i) < 8) TRACE((base) + (i) * (stride) + (k)); } while (0)   // first tiles
 #else
+#define TRACE_TILE(base, stride, i, k) do {} while (0)
 #define TRACE_VAL(slot, v) do {} while (0)
 #define TRACE(slot) do {} while (0)
 #define GTRACE(slot) do {} while (0)
@@ -777,7 +779,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (i >= 1) wait_or_fault(&o_free, one ^ 1, &dead, fault, kFaultMmaWait);
           wait_or_fault(&x_full[p], ph, &dead, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 0 : 999);
+          TRACE_TILE(160, 8, i, 0);
           tc_fence_after_sync();
           if constexpr (!DQ)  // X P: the state tile as [K = d rows] x [N = e columns]
             umma_gemm<false, true, E, D>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false);
@@ -789,7 +791,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           wait_or_fault(&z_full[p], ph, &dead, fault, kFaultTmaWait);
           if (map_z) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
           wait_or_fault(&o2s_ready, one, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 3 : 999);
+          TRACE_TILE(160, 8, i, 3);
           tc_fence_after_sync();
           umma_gemm_ts<true, WZ, 64>(t_o, t_s[p], smem_u32(sz[p]), C, true);
           umma_commit(&o_full[p]);
@@ -802,7 +804,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (map_z) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&l_free, one ^ 1, &dead, fault, kFaultMmaWait);   // the state update has read the previous L
           wait_or_fault(&ys_ready, one, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 1 : 999);
+          TRACE_TILE(160, 8, i, 1);
           tc_fence_after_sync();
           if constexpr (!DQ)
             umma_gemm<true, true, E, C>(t_l, smem_u32(sy[p]), C, smem_u32(sz[p]), C, false);
@@ -818,7 +820,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           wait_or_fault(&x_full[p], ph, &dead, fault, kFaultTmaWait);
           wait_or_fault(&y_full[p], ph, &dead, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 2 : 999);
+          TRACE_TILE(160, 8, i, 2);
           tc_fence_after_sync();
           umma_gemm<false, false, C, WX>(t_s[p], smem_u32(sx[p]), C, smem_u32(sy[p]), C, false);
           umma_commit(&s_full[p]);
@@ -846,9 +848,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         sl2 = a.s[w.bh % a.h] * kLog2e;
         lam = exp2f(-sl2);
       }
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 0 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 0);
       wait_or_fault(&s_full[p], ph, &dead, fault, kFaultMmaWait);
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 1 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 1);
       tc_fence_after_sync();
       // masked scores, packed to bf16 in place: they are the A operand of O1 straight from tensor memory
 #pragma unroll 1
@@ -860,7 +862,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&sm_ready[p]);
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 2 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 2);
       if (elu && i + 1 < total) map_tile(i + 1, grp);   // the next tile's S can then go out under this tile's work
       // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
       const bool chain = PRE && DQ && (elu || c != 1.f);
@@ -874,7 +876,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       // epilogue: OUT staged in Z's buffer, once L and O1 have read it
       wait_or_fault(&l_full[p], ph, &dead, fault, kFaultMmaWait);
       wait_or_fault(&o_full[p], ph, &dead, fault, kFaultMmaWait);
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 3 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 3);
       tc_fence_after_sync();
       if (chain) {
 #pragma unroll 1
@@ -892,10 +894,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       }
       tc_fence_before_sync();
       mbar_arrive(&o_free);
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 4 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 4);
       fence_async_smem();
       mbar_arrive(&staged[p]);
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 5 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 5);
     }
   } else {
     set_regs_inc<kRegsB>();
@@ -918,12 +920,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       const int len = min(C, a.n - w.t * C);     // tokens really in the tile
       if (w.first_of_item()) sl2 = a.s[w.bh % a.h] * kLog2e;
       wait_or_fault(&s_full[p], ph, &dead, fault, kFaultMmaWait);   // S has read Y
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 0 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 0);
       wait_or_fault(&y_full[p], ph, &dead, fault, kFaultTmaWait);   // completed long ago: makes Y's bytes visible here
       scale_row_pieces<WX / 16>(sy[p], row, half * (WX / 16), c * decay_pow(sl2, max(len - row, 0)), lane);
       fence_async_smem();
       mbar_arrive(&ys_ready);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 1 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 1);
       if (elu && i + 1 < total) map_tile(i + 1, grp);
       if (__builtin_expect(w.first_of_item(), 0)) {   // once per span: kept out of the tiles' straight-line code
         // the state at the span border; the O2 MMA that read the operand tile of the previous item has completed
@@ -1028,7 +1030,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       }
       // O2's rows take their decay lambda^row in tensor memory; O1 then accumulates on top
       wait_or_fault(&o2_full[p], ph, &dead, fault, kFaultMmaWait);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 2 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 2);
       tc_fence_after_sync();
       {
         const float qd = c_o2 * decay_pow(sl2, row);
@@ -1038,10 +1040,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&o2s_ready);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 3 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 3);
       // state: P <- lambda^len P + L
       wait_or_fault(&l_full[p], ph, &dead, fault, kFaultMmaWait);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 4 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 4);
       tc_fence_after_sync();
       if (row < D) {
         const float lam_c = decay_pow(sl2, len);
@@ -1059,7 +1061,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       }
       tc_fence_before_sync();
       mbar_arrive(&l_free);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 5 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 5);
       if (!w.last_of_item()) {
         if (row < D) write_state_operand<kHalfE>(sp, D, row, half * kHalfE, P);
         fence_async_smem();
@@ -1364,7 +1366,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           if (elu) wait_or_fault(&mapped, one, &dead, fault, kFaultMmaWait);
           wait_or_fault(&dn_ready, one, &dead, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&e_free, one ^ 1, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 1 : 999);
+          TRACE_TILE(160, 8, i, 1);
           tc_fence_after_sync();
           umma_gemm<false, false, D, E>(t_dk, smem_u32(sv), C, smem_u32(sdn), D, false);
           umma_gemm<false, true, E, D>(t_dv, smem_u32(sk), C, smem_u32(sdn), D, false);
@@ -1372,7 +1374,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           // the masked scores' products on top, A operands from tensor memory
           wait_or_fault(&sm_ready, one, &dead, fault, kFaultMmaWait);
           wait_or_fault(&scaled, one, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 3 : 999);
+          TRACE_TILE(160, 8, i, 3);
           tc_fence_after_sync();
           umma_gemm_ts<true, E, 96>(t_dv, t_s, smem_u32(sdo[p]), C, true);    // += S_m^T dO
           wait_or_fault(&dsm_ready, one, &dead, fault, kFaultMmaWait);
@@ -1389,7 +1391,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&sm_ready, one, &dead, fault, kFaultMmaWait);
           if (E > 64) wait_or_fault(&dsm_ready, one, &dead, fault, kFaultMmaWait);
           wait_or_fault(&qs_ready, one, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 2 : 999);
+          TRACE_TILE(160, 8, i, 2);
           tc_fence_after_sync();
           umma_gemm<true, true, 64, C>(t_s + 32, smem_u32(sdn), C, smem_u32(sdo[p]), C, false);
           if constexpr (E > 64)   // columns 64..127 of dO: its second slab
@@ -1407,7 +1409,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&qdo_full[p], (i >> 1) & 1, &dead, fault, kFaultTmaWait);
           wait_or_fault(&kv_full, one, &dead, fault, kFaultTmaWait);
           if (elu) wait_or_fault(&mapped, one, &dead, fault, kFaultMmaWait);
-          TRACE(i < 8 ? 160 + i * 8 + 5 : 999);
+          TRACE_TILE(160, 8, i, 5);
           tc_fence_after_sync();
           umma_gemm<false, false, C, D>(t_s, smem_u32(sk), C, smem_u32(sq[p]), C, false);
           umma_commit(&s_done);
@@ -1435,7 +1437,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         fence_async_smem();
         mbar_arrive(&mapped);
       }
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 0 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 0);
       // S_m^T, then dS_m^T (times Q's c): one piece of code for the four blocks of 32 queries.  The second half of the
       // queries goes from right to left, packed against the right end, so that every block is read before it is
       // written over.
@@ -1443,7 +1445,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       for (int u = 0; u < 4; ++u) {
         if ((u & 1) == 0) {
           wait_or_fault(u == 0 ? &s_done : &ds_done, one, &dead, fault, kFaultMmaWait);
-          if (tid == kFirstWorker && u == 0) TRACE(i < 8 ? 64 + i * 6 + 1 : 999);
+          if (tid == kFirstWorker && u == 0) TRACE_TILE(64, 6, i, 1);
           tc_fence_after_sync();
         }
         const int blk = half == 0 ? (u & 1) : 3 - (u & 1);
@@ -1469,7 +1471,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       // epilogue: dK and dV staged over Q and dO, which every product has read
       wait_or_fault(&l_done, one, &dead, fault, kFaultMmaWait);
       wait_or_fault(&b_done, one, &dead, fault, kFaultMmaWait);
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 4 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 4);
       tc_fence_after_sync();
       if (PRE && (elu || c != 1.f)) {
 #pragma unroll 1
@@ -1491,7 +1493,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       mbar_arrive(&e_free);
       fence_async_smem();
       mbar_arrive(&staged[p]);
-      if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 5 : 999);
+      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 5);
     }
   } else {
     // ---- group B
@@ -1610,13 +1612,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         mbar_arrive(&mapped);
       }
       wait_or_fault(&st_done, one, &dead, fault, kFaultMmaWait);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 0 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 0);
       tc_fence_after_sync();
       // row-scaled copy of Q over the state operand (the state products have read it)
       copy_row_pieces<D / 16>(sdn, sq[p], row, half * (D / 16), c * decay_pow(sl2, row), lane);
       fence_async_smem();
       mbar_arrive(&qs_ready);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 1 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 1);
       // the two state products take their row decay in place (32 columns at a time, dV's blocks then dK's)
       const float kd = decay_pow(sl2, max(len - row, 0));
 #pragma unroll 1
@@ -1628,10 +1630,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&scaled);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 2 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 2);
       // state: Dn <- lambda^len Dn + L, this thread's half of the columns being the one in T_S or in T_dS
       wait_or_fault(&l_done, one, &dead, fault, kFaultMmaWait);
-      if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 3 : 999);
+      if (wid == 0) TRACE_TILE(112, 6, i, 3);
       tc_fence_after_sync();
       if (row < D) {
         const float lam_len = decay_pow(sl2, len);
@@ -1654,7 +1656,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         if (row < D) write_state_operand<kHalfE>(sdn, D, row, half * kHalfE, Dn);
         fence_async_smem();
         mbar_arrive(&dn_ready);
-        if (wid == 0) TRACE(i < 8 ? 112 + i * 6 + 4 : 999);
+        if (wid == 0) TRACE_TILE(112, 6, i, 4);
       } else if constexpr (FUSED) {
         // the state after the first tile of the sequence is the outgoing rank state
         if (a.x_out != nullptr && w.t == 0 && row < D) {
