@@ -282,7 +282,7 @@ class SequenceParallelAttention(torch.autograd.Function):
 def _check_state_buffers(q, v, KV, DKV):
     shape = (q.shape[0], q.shape[1], q.shape[3], v.shape[3])
     for name, buf in (("KV", KV), ("DKV", DKV)):
-        if tuple(buf.shape) != shape or buf.dtype != torch.float32 or not buf.is_contiguous():
+        if buf.shape != shape or buf.dtype != torch.float32 or not buf.is_contiguous():
             raise ValueError(f"{name} must be a contiguous float32 tensor of shape {shape}")
 
 
@@ -293,20 +293,22 @@ def _alone(q) -> bool:
     return q.is_cuda and get_sequence_parallel_world_size() == 1
 
 
+def _on_its_own(q, k, v, s, KV, DKV, qk_scale=1.0, feature_map=None):
+    if q.dim() == 4 and v.dim() == 4:     # (the operator itself checks q, k, v and s, in native code)
+        _check_state_buffers(q, v, KV, DKV)
+    return lightning(q, k, v, s, qk_scale, feature_map)
+
+
 def sequence_parallel_slice(q, k, v, s, KV, DKV, overlap: bool):
     """The autograd function itself (head dimensions of one slice at most)."""
     if q.dim() == 4 and v.dim() == 4 and max(q.shape[-1], v.shape[-1]) <= MAX_HEAD_SLICE and _alone(q):
-        _check_shapes(q, k, v, s)
-        _check_state_buffers(q, v, KV, DKV)
-        return lightning(q, k, v, s)
+        return _on_its_own(q, k, v, s, KV, DKV)
     return SequenceParallelAttention.apply(q, k, v, s, KV, DKV, overlap)
 
 
 def sequence_parallel(q, k, v, s, KV, DKV, overlap: bool):
     if _alone(q):
-        _check_shapes(q, k, v, s)
-        _check_state_buffers(q, v, KV, DKV)
-        return lightning(q, k, v, s)
+        return _on_its_own(q, k, v, s, KV, DKV)
     return sliced_apply(lambda qs, ks, vs, kv, dkv: SequenceParallelAttention.apply(qs, ks, vs, s, kv, dkv, overlap),
                         q, k, v, (KV, DKV))
 
@@ -330,9 +332,7 @@ def sequence_parallel_fused(q, k, v, s, KV, DKV, qk_scale: float = 1.0, feature_
     rank's launches are the fused ones that hand the state over themselves; torch operations otherwise."""
     qs, vs = _slice_like(q, v)
     if _alone(q):
-        _check_shapes(q, k, v, s)
-        _check_state_buffers(q, v, KV, DKV)
-        return lightning(q, k, v, s, qk_scale, feature_map)
+        return _on_its_own(q, k, v, s, KV, DKV, qk_scale, feature_map)
     in_kernel = (qk_scale != 1.0 or feature_map is not None) and kernels_preprocess(qs, vs, qk_scale, feature_map)
     if in_kernel and get_sequence_parallel_world_size() > 1:
         b, h, n, d = qs.shape

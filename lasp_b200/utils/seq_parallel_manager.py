@@ -120,7 +120,8 @@ def set_sequence_parallel_world_size(world_size) -> None:
 def get_sequence_parallel_world_size() -> int:
     if _G.sp_world_override is not None:
         return _G.sp_world_override
-    return dist.get_world_size(group=get_sequence_parallel_group())
+    get_sequence_parallel_group()      # (asserts that there is one)
+    return len(_G.sp_ranks)            # its size, without the lookups of torch.distributed on every call
 
 
 def set_sequence_parallel_rank(rank) -> None:
