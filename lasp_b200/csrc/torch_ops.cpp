@@ -130,6 +130,8 @@ Shape check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
                       kSlice, ": cut in ", kSlice, "-wide slices)");
   TORCH_CHECK_VALUE(q.size(0) * q.size(1) <= 65535, "batch x heads = ", q.size(0) * q.size(1), " exceeds 65535");
   lasp_dtype_of(q.scalar_type());
+  // (a width of zero is a multiple of 16: it would leave no slice to run and the output as it was allocated)
+  if (q.size(3) == 0 || v.size(3) == 0) check_status("lasp_b200_resolve_path", LASP_ERR_SHAPE);
   for (const Tensor* t : {&q, &k, &v})
     TORCH_CHECK(t->is_cuda(), "lasp_b200 runs on CUDA tensors only (there is no CPU fallback); got a tensor on ", t->device());
   return {q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
