@@ -132,6 +132,9 @@ Shape check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
   lasp_dtype_of(q.scalar_type());
   // (a width of zero is a multiple of 16: it would leave no slice to run and the output as it was allocated)
   if (q.size(3) == 0 || v.size(3) == 0) check_status("lasp_b200_resolve_path", LASP_ERR_SHAPE);
+  // (a call without gradients does not pass through the autograd function, which would refuse a tangent)
+  for (const Tensor* t : {&q, &k, &v, &s})
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->_fw_grad(0).defined(), "lasp_b200 has no forward-mode derivative");
   for (const Tensor* t : {&q, &k, &v})
     TORCH_CHECK(t->is_cuda(), "lasp_b200 runs on CUDA tensors only (there is no CPU fallback); got a tensor on ", t->device());
   return {q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
