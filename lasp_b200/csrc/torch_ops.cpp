@@ -16,6 +16,8 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/library.h>
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -280,6 +282,22 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const Tensor& ed, double scale, i
   return run_forward(q, k, v, s, m, scale, map, false)[0];
 }
 
+// The operator as a node of a traced graph: torch.jit.trace records what goes through the dispatcher, and the launches do
+// not (it would keep the allocation of o alone).  Calls outside a trace spare themselves the dispatcher.
+Tensor attention_op(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s, double scale, int64_t map) {
+  return attention(q, k, v, s, scale, map);
+}
+TORCH_LIBRARY(lasp_b200, m) {
+  m.def("attention(Tensor q, Tensor k, Tensor v, Tensor s, float qk_scale, int map) -> Tensor");
+  m.impl("attention", c10::DispatchKey::CompositeImplicitAutograd, TORCH_FN(attention_op));
+}
+Tensor traced_attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s, double scale, int64_t map) {
+  static const auto op = c10::Dispatcher::singleton()
+                             .findSchemaOrThrow("lasp_b200::attention", "")
+                             .typed<Tensor(const Tensor&, const Tensor&, const Tensor&, const Tensor&, double, int64_t)>();
+  return op.call(q, k, v, s, scale, map);
+}
+
 // attention(q, k, v, s, qk_scale, map) -> o
 PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
@@ -294,7 +312,7 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   Tensor o;
   {
     pybind11::gil_scoped_release no_gil;
-    o = attention(q, k, v, s, scale, map);
+    o = torch::jit::tracer::isTracing() ? traced_attention(q, k, v, s, scale, map) : attention(q, k, v, s, scale, map);
   }
   return THPVariable_Wrap(std::move(o));
   END_HANDLE_TH_ERRORS
