@@ -273,11 +273,12 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const Tensor& ed, double scale, i
     lasp_problem p = problem_of(m, std::min(m.d, kSlice), std::min(m.e, kSlice), lasp_dtype_of(q.scalar_type()), scale, map, false);
     if (!resolve(p)) q = preprocess(q, scale, map), k = preprocess(k, scale, map), scale = 1.0, map = 0;
   }
-  Tensor s = ed.detach().reshape({-1});
+  Tensor s = ed.reshape({-1});
   if (s.device() != q.device() || s.scalar_type() != at::kFloat) s = s.to(q.device(), at::kFloat);
   s = s.contiguous();
   q = q.contiguous(), k = k.contiguous(), v = v.contiguous();
-  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
+  // (the decay rates get no gradient, but a result that depends on them through a graph says so)
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || s.requires_grad()))
     return Lightning::apply(q, k, v, s, scale, map);
   return run_forward(q, k, v, s, m, scale, map, false)[0];
 }

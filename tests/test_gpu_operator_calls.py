@@ -33,3 +33,20 @@ def test_a_traced_function_computes(grad, fused, tmp_path):
         assert torch.equal(got, want)
         if grad:
             assert torch.equal(*(torch.autograd.grad(o, q, torch.ones_like(o))[0] for o in (got, want)))
+
+
+def test_decay_rates_that_require_grad():
+    """They are part of the graph (o requires grad on their account alone) and get no gradient."""
+    from lasp_b200 import lightning_attn
+    q, k, v = _inputs(3)
+    s = torch.full((2, 1, 1), 0.01, device=DEV, requires_grad=True)
+    o = lightning_attn(q, k, v, s * 1.0)
+    assert o.requires_grad
+    o.sum().backward()
+    assert s.grad is None and q.grad is None
+    q.requires_grad_(True)
+    with_s = torch.autograd.grad(lightning_attn(q, k, v, s), (q, s), torch.ones_like(o), allow_unused=True)
+    without = torch.autograd.grad(lightning_attn(q, k, v, s.detach()), q, torch.ones_like(o))[0]
+    assert with_s[1] is None and torch.equal(with_s[0], without)
+    with torch.no_grad():
+        assert not lightning_attn(q, k, v, s).requires_grad
