@@ -227,10 +227,19 @@ class Lightning : public torch::autograd::Function<Lightning> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list saved = ctx->get_saved_variables();
-    const Tensor &q = saved[0], &k = saved[1], &v = saved[2], &s = saved[3];
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
-    const Tensor d_o = grads[0].contiguous();
+    // What was saved may have been through a saved-tensor hook (offloading, compression): it can come back with other
+    // strides, or not as what it was.
+    const Tensor q = saved[0].contiguous(), k = saved[1].contiguous(), v = saved[2].contiguous(), d_o = grads[0].contiguous();
+    TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda() && d_o.is_cuda(), "lasp_b200: a saved tensor is not on a GPU any more");
+    TORCH_CHECK_TYPE(q.scalar_type() == d_o.scalar_type() && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
+                     "lasp_b200: a saved tensor has changed its dtype");
+    Tensor s = saved[3];
+    if (s.device() != q.device() || s.scalar_type() != at::kFloat) s = s.to(q.device(), at::kFloat);
+    s = s.contiguous();
     const Shape m{q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
+    TORCH_CHECK_VALUE(k.sizes() == q.sizes() && v.sizes() == d_o.sizes() && v.sizes().slice(0, 3) == q.sizes().slice(0, 3) && s.numel() == m.h,
+                      "lasp_b200: a saved tensor has changed its shape");
     const c10::cuda::CUDAGuard guard(q.device());
     const auto stream = at::cuda::getCurrentCUDAStream();
     Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options()), dv = at::empty(v.sizes(), v.options());
@@ -240,7 +249,9 @@ class Lightning : public torch::autograd::Function<Lightning> {
                                                 ctx->saved_data["map"].toInt());
     for (size_t i = 0; i < pairs.size(); ++i) {
       const Pair& p = pairs[i];
-      const Tensor& fwd_ws = saved[4 + i];
+      const Tensor fwd_ws = saved[4 + i].contiguous();
+      TORCH_CHECK(fwd_ws.is_cuda() && fwd_ws.scalar_type() == at::kByte && (size_t)fwd_ws.numel() >= p.ws_bytes,
+                  "lasp_b200: the states saved by the forward pass did not come back as the bytes that they are");
       if (!ws.defined() || (size_t)ws.numel() < p.ws_bytes)
         ws = at::empty({(int64_t)p.ws_bytes}, q.options().dtype(at::kByte));
       lasp_bwd_args a = {};

@@ -50,3 +50,38 @@ def test_decay_rates_that_require_grad():
     assert with_s[1] is None and torch.equal(with_s[0], without)
     with torch.no_grad():
         assert not lightning_attn(q, k, v, s).requires_grad
+
+
+def _gradients_through(pack, unpack, n=200):
+    from lasp_b200 import lightning_attn
+    q, k, v = (t.requires_grad_(True) for t in _inputs(4, n))
+    s = torch.full((2, 1, 1), 0.01, device=DEV)
+    plain = torch.autograd.grad(lightning_attn(q, k, v, s), (q, k, v), torch.ones_like(v))
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        o = lightning_attn(q, k, v, s)
+    return plain, torch.autograd.grad(o, (q, k, v), torch.ones_like(v))
+
+
+@pytest.mark.parametrize("n", [100, 200])
+def test_saved_tensors_may_come_back_laid_out_differently(n):
+    """A hook that transposes, offloads or changes the type of the decay rates: same gradients."""
+    def back(t):
+        if t.dim() == 4:
+            return t.transpose(2, 3).contiguous().transpose(2, 3)      # the values in another order in memory
+        return t.double().cpu() if t.dtype == torch.float32 else t
+    for pack, unpack in ((lambda t: t, back), (lambda t: t.cpu(), lambda t: t.to(DEV))):
+        plain, got = _gradients_through(pack, unpack, n)
+        for a, b in zip(plain, got):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("change", [lambda t: t.half(), lambda t: t.cpu(), lambda t: t[..., :32], lambda t: t[:, :, 1:]])
+def test_saved_tensors_that_are_not_what_they_were_are_refused(change):
+    """... and one that changes what it was given is told so, before anything is launched."""
+    for kind in (4, 1):                                                 # q, k, v; the states kept by the forward pass
+        def back(t):
+            if t.dim() != kind or (kind == 1 and t.dtype != torch.uint8):
+                return t
+            return change(t.view(1, 1, 1, -1) if kind == 1 else t)
+        with pytest.raises((RuntimeError, TypeError, ValueError), match="saved"):
+            _gradients_through(lambda t: t, back)
