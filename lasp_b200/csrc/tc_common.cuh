@@ -4,6 +4,7 @@
 #pragma once
 #include "common.cuh"
 #include "sm100.cuh"
+#include "span_cut.h"
 
 namespace lasp {
 namespace tc {
@@ -269,40 +270,19 @@ __device__ __forceinline__ void stage_row32_chain(uint32_t taddr, uint8_t* tile,
   }
 }
 
-// How the sequences of a launch are cut into spans of tiles; `base`, `extra` and `magic` are what the kernels would
-// otherwise divide for at every item (three integer divisions, inlined wherever a role steps through its tiles, were a
-// third of a walk kernel's code).
-struct SpanCut {
-  int items, nspans, span, tiles;
-  int base, extra;   // tiles / nspans and the remainder
-  uint32_t magic;    // it / nspans = (it * magic) >> 32 with 64-bit arithmetic while items * nspans < 2^32
-};
-inline SpanCut make_span_cut(int items, int nspans, int span, int tiles) {
-  return {items, nspans, span, tiles, tiles / nspans, tiles % nspans, nspans > 1 ? (uint32_t)(0x100000000ull / nspans) + 1 : 0};
-}
-
-// The work of a persistent CTA: items blockIdx.x, blockIdx.x + gridDim.x, ...; an item is one span of
-// consecutive tiles of one (batch, head) sequence, walked first to last tile or last to first.
-// Spans: `span` tiles each, the last one of a sequence whatever is left (even = false), or - for a
-// kernel whose CTAs wait for one another - the tiles shared out evenly, spans differing by one tile at
-// most, with the longer spans where the walk starts: there nobody has to wait for anybody's total, and the
-// spans with the longest look-back get the fewest tiles (even = true).
+// The work of a persistent CTA (span_cut.h): items blockIdx.x, + gridDim.x, ..., walked first to last tile or last to
+// first.
 template <bool BACKWARDS>
 struct TileWalk {
   const SpanCut& c;
   bool even;
   int it, bh, sp, t, t0, t1;  // current item, its sequence and span, current tile, the item's tile range [t0, t1)
 
-  // first tile of span sp (sp = nspans: one past the last tile)
-  __device__ __forceinline__ int span_t0(int s) const {
-    if (!even) return min(s * c.span, c.tiles);
-    // `extra` spans have base + 1 tiles
-    return s * c.base + (BACKWARDS ? max(0, s - (c.nspans - c.extra)) : min(s, c.extra));
-  }
+  __device__ __forceinline__ int span_t0(int s) const { return span_first_tile<BACKWARDS>(c, even, s); }
   __device__ __forceinline__ bool load() {
     if (it >= c.items) return false;
-    bh = c.nspans == 1 ? it : (int)(((uint64_t)(uint32_t)it * c.magic) >> 32);
-    sp = it - bh * c.nspans;
+    bh = sequence_of_item(c, it);
+    sp = span_of_place<BACKWARDS>(c, even, it - bh * c.nspans);
     t0 = span_t0(sp);
     t1 = span_t0(sp + 1);
     t = BACKWARDS ? t1 - 1 : t0;

@@ -1230,6 +1230,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       if (w.sp > 0 || a.all_totals) sums = min(w.t1 - w.t0, reach_tiles(a.s[my_bh % a.h]));
     }
   }
+  // this CTA's span among all spans (the places of a sequence count down, see span_of_place), not kept in a register
+  const auto my_item = [&] { return (2 * my_bh + 1) * a.cut.nspans - 1 - (int)blockIdx.x; };
   const int row = (warp & 3) * 32 + lane;      // workers: tensor-memory lane quarter of this warp
   const int wid = (tid - kFirstWorker) & (kWorkers - 1);   // 0..255 inside the group
   const int half = wid >> 7;
@@ -1264,13 +1266,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       uint32_t r[32];
       tmem_ld32(t_s + lane_base + c0, r);
       tmem_ld_wait();
-      store_state32<D>(a.totals + (size_t)blockIdx.x * D * E, row, c0, r);
+      store_state32<D>(a.totals + (size_t)my_item() * D * E, row, c0, r);
     }
     tc_fence_before_sync();
     named_sync(2, 2 * kWorkers);   // every worker's part of the total is written ...
     if (tid == kFirstWorker) {
       __threadfence();             // ... and visible to the other CTAs before the flag is
-      st_volatile_u32(a.sync + kSyncFlags + blockIdx.x, step_s);
+      st_volatile_u32(a.sync + kSyncFlags + my_item(), step_s);
     }
     if (tid == kFirstWorker) TRACE(60);
   };
@@ -1556,7 +1558,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
               const int owner = w.bh * a.cut.nspans;   // the CTA that owns the start of the sequence
               const bool far = n_dst > 1 && xl::reaches(sn, 1);   // the state reaches beyond the next rank
               uint32_t* ready = a.sync + kSyncFlags + kSyncSecondBank + w.bh;
-              if (w.it == owner && far) {
+              if (sp_idx == 0 && far) {
                 // the sequence's total, lambda^(span end) Dn + T, where the other CTAs of the sequence find it
                 if (row < D)
                   link_make_total<kHalfE, D>(a.totals + (size_t)owner * D * E, row, half * kHalfE,
@@ -1567,7 +1569,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
                   st_volatile_u32(ready, step_s);
                 }
               }
-              if (far || w.it == owner) {
+              if (far || sp_idx == 0) {
                 // the readers of the ranks after this one in the chain order (the ranks BEFORE it in the
                 // sequence) have acknowledged the slots' previous use
                 if (!dead) {
@@ -1575,7 +1577,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
                   if (xl::needs_ack_wait(step_x) && wid < n_dst)
                     ok2 = wait_flag_ge(a.link.my_acks + xl::ack_index(a.link.me + 1 + wid, 0), step_x - 2,
                                        a.link.wait_clocks);
-                  if (far && wid == xl::kMaxRanks && w.it != owner) ok2 = wait_flag_eq(ready, step_s, a.wait_clocks);
+                  if (far && wid == xl::kMaxRanks && sp_idx != 0) ok2 = wait_flag_eq(ready, step_s, a.wait_clocks);
                   if (!ok2) {
                     dead = 1;
                     atomicOr(fault, kFaultRelayWait);
