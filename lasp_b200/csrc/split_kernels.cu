@@ -233,13 +233,13 @@ __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t done;
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead;
+  __shared__ Health<false> cta;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dp = padded(g.d), ep = padded(g.e);
   uint8_t* sa = align1024(smem_raw);
   uint8_t* sb = sa + TT::mid * C * dp * 2;   // (with dp = 64 the M = 128 MMA reads on from A into B: valid memory)
   if (tid == 0) {
-    dead = 0;
+    cta.word = 0;
     mbar_init(&done, 1);
     fence_mbar_init();
   }
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
     int next = task + gridDim.x;
     while (next < g.tasks && skipped(next)) next += gridDim.x;
     if (next < g.tasks) fetch(next);
-    wait_or_fault(&done, it & 1, &dead, g.fault, kFaultMmaWait);
+    wait_or_fault(&done, it & 1, &cta, g.fault, kFaultMmaWait);
     tc_fence_after_sync();
     float4* out = reinterpret_cast<float4*>(g.states + (size_t)task * g.d * g.e);
     const int per = ep / 4;   // columns of this warp's group
@@ -379,14 +379,14 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t s_done, o2_done, o1_done;
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead;
+  __shared__ Health<false> cta;
   __shared__ float decay[C + 1];   // lambda^0 .. lambda^128 of the task's head
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dp = padded(g.d), ep = padded(g.e);
   uint8_t* set_a = align1024(smem_raw);
   uint8_t* set_b = set_a + g.set_bytes;
   if (tid == 0) {
-    dead = 0;
+    cta.word = 0;
     mbar_init(&s_done, 1);
     mbar_init(&o2_done, 1);
     mbar_init(&o1_done, 1);
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
       if (k.has_state) {
         Raw<float> rp[kPieces];
         load_state(rp, k.r->state + ((size_t)k.bh * g.nc + k.chunk) * g.d * g.e, g.d, g.e, dp, ep, tid);
-        wait_or_fault(&s_done, it & 1, &dead, g.fault, kFaultMmaWait);
+        wait_or_fault(&s_done, it & 1, &cta, g.fault, kFaultMmaWait);
         store_state_terms<TT::mid>(set_b, rp, dp, ep, tid);
         fence_async_smem();
         tc_fence_before_sync();
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
           umma_commit(&o2_done);
         }
       } else {
-        wait_or_fault(&s_done, it & 1, &dead, g.fault, kFaultMmaWait);
+        wait_or_fault(&s_done, it & 1, &cta, g.fault, kFaultMmaWait);
       }
       // ---- the masked scores' terms, Z's terms over X, O1 = S_m Z
       {
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
           if constexpr (TT::mid == 3) tmem_st16(t_lo + lane_base + 16 * group, lo);
           tmem_st_wait();
         }
-        if (k.has_state) wait_or_fault(&o2_done, o2_uses & 1, &dead, g.fault, kFaultMmaWait);   // O2 has read X
+        if (k.has_state) wait_or_fault(&o2_done, o2_uses & 1, &cta, g.fault, kFaultMmaWait);   // O2 has read X
         store_tile<T, TT::in, false>(set_a, rz, wz, tid, NoWeight());
       }
       fence_async_smem();
@@ -527,14 +527,14 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
         load_xy(rx, kn.r->x, kn);
         if (tid <= C) decay[tid] = expf(-kn.sh * (float)tid);   // this task's masks are done (barrier above)
         store_tile<T, TT::in, false>(set_b, ry, padded(kn.r->wx), tid, NoWeight());   // O2 has read P
-        wait_or_fault(&o1_done, it & 1, &dead, g.fault, kFaultMmaWait);
+        wait_or_fault(&o1_done, it & 1, &cta, g.fault, kFaultMmaWait);
         store_tile<T, TT::in, false>(set_a, rx, padded(kn.r->wx), tid, NoWeight());
         fence_async_smem();
         tc_fence_before_sync();
         __syncthreads();
         if (tid == 0) issue_s(kn);
       } else {
-        wait_or_fault(&o1_done, it & 1, &dead, g.fault, kFaultMmaWait);
+        wait_or_fault(&o1_done, it & 1, &cta, g.fault, kFaultMmaWait);
       }
       // ---- epilogue, under the next scores
       tc_fence_after_sync();

@@ -14,16 +14,30 @@ using namespace sm100;
 constexpr int C = kTensorTile;  // 128 tokens per tile
 constexpr float kLog2e = 1.4426950408889634f;
 
+// Whether a wait of the CTA has run out (in shared memory).  With a link (LINK) some of its warps may also be waiting for
+// another rank, for as long as the hand-over's own limit says; the time of the other warps' waits stands still meanwhile.
+template <bool LINK>
+struct Health {
+  enum { kWell = 0, kGaveUp = 1, kAwaitsPeer = 2 };
+  int word;
+  __device__ __forceinline__ bool gave_up() const { return *const_cast<const volatile int*>(&word) == kGaveUp; }
+  __device__ __forceinline__ void give_up() { *const_cast<volatile int*>(&word) = kGaveUp; }
+  __device__ __forceinline__ void peer_wait_begins() { atomicCAS(&word, kWell, kAwaitsPeer); }
+  __device__ __forceinline__ void peer_wait_ends() { atomicCAS(&word, kAwaitsPeer, kWell); }
+};
+
 // Bounded wait that records a fault once and lets later waits of the CTA give up at once.  There are some thirty of
 // these in a walk kernel: the code that a wait normally runs is one probe, and 32-bit clocks keep the rest short.
-__device__ __forceinline__ void wait_or_fault(uint64_t* bar, uint32_t parity, volatile int* dead, int32_t* fault,
-                                              int32_t code) {
+template <bool LINK>
+__device__ __forceinline__ void wait_or_fault(uint64_t* bar, uint32_t parity, Health<LINK>* cta, int32_t* fault, int32_t code) {
   if (mbar_try_wait(bar, parity)) return;
-  const uint32_t t0 = clock();
+  uint32_t t0 = clock();
   while (!mbar_try_wait(bar, parity)) {
-    if (*dead) return;
+    const int state = *const_cast<const volatile int*>(&cta->word);
+    if (state == Health<LINK>::kGaveUp) return;
+    if (LINK && state == Health<LINK>::kAwaitsPeer) t0 = clock();
     if ((uint32_t)clock() - t0 > kWaitClocks) {
-      *dead = 1;
+      cta->give_up();
       atomicOr(fault, code);
       return;
     }

@@ -142,10 +142,10 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
   // per stage: A then B (with D = 64 the M = 128 MMA reads on from A into B, which is valid memory)
   __shared__ uint64_t full[kStages], scaled[kStages], empty[kStages], acc_full[2], acc_free[2];
   __shared__ uint32_t tmem_slot;
-  __shared__ int dead;
+  __shared__ Health<false> cta;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    dead = 0;
+    cta.word = 0;
     for (int j = 0; j < kStages; ++j) {
       mbar_init(&full[j], 1);
       mbar_init(&scaled[j], 128);
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
       int g = 0;
       for (bool ok = w.start(); ok; ok = w.next(), ++g) {
         const int j = g % kStages, use = g / kStages;
-        if (use >= 1) wait_or_fault(&empty[j], (use - 1) & 1, &dead, fault, kFaultMmaWait);
+        if (use >= 1) wait_or_fault(&empty[j], (use - 1) & 1, &cta, fault, kFaultMmaWait);
         uint8_t* sa = smem + j * (kA + kB);
         mbar_expect_tx(&full[j], kA + kB);
         tma_load_4d(sa, &map_a, &full[j], 0, w.t * C, 0, w.bh);
@@ -185,9 +185,9 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
         const int j = g % kStages, use = g / kStages;
         if (w.first_of_item()) {
           ++li;
-          if (li >= 2) wait_or_fault(&acc_free[li & 1], ((li >> 1) - 1) & 1, &dead, fault, kFaultMmaWait);
+          if (li >= 2) wait_or_fault(&acc_free[li & 1], ((li >> 1) - 1) & 1, &cta, fault, kFaultMmaWait);
         }
-        wait_or_fault(&scaled[j], use & 1, &dead, fault, kFaultTmaWait);
+        wait_or_fault(&scaled[j], use & 1, &cta, fault, kFaultTmaWait);
         tc_fence_after_sync();
         uint8_t* sa = smem + j * (kA + kB);
         umma_gemm<true, true, E, C>(tmem + 128 * (li & 1), smem_u32(sa), C, smem_u32(sa + kA), C, !w.first_of_item());
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
       const int pos = w.t * C + row;
       const int dist = reverse ? pos - w.t0 * C : min(w.t1 * C, n) - pos;
       const float wt = decay_pow(sl2, max(dist, 0));  // rows past the end of the sequence are zero anyway
-      wait_or_fault(&full[j], use & 1, &dead, fault, kFaultTmaWait);
+      wait_or_fault(&full[j], use & 1, &cta, fault, kFaultTmaWait);
       scale_row_pieces<D / 8>(smem + j * (kA + kB), row, 0, wt, lane);
       fence_async_smem();
       mbar_arrive(&scaled[j]);
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
     for (bool ok = w.start(); ok; ok = w.next()) {
       if (!w.last_of_item()) continue;
       ++li;
-      wait_or_fault(&acc_full[li & 1], (li >> 1) & 1, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&acc_full[li & 1], (li >> 1) & 1, &cta, fault, kFaultMmaWait);
       tc_fence_after_sync();
       if (row < D) {
 #pragma unroll
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
   __shared__ uint64_t mapped[2];   // with a feature map: the workers have mapped the tile's X, Y (dQ: Z) in place
   __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x, even_s;
-  __shared__ int dead;
+  __shared__ Health<LINK> cta;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int32_t* fault = a.fault;
   // Thread 0 is also the producer: it asks for its first tiles before the CTA-wide barrier below, so that their
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
   bool early_ring = false;
   int early_x = 0;
   if (tid == 0) {
-    dead = 0;
+    cta.word = 0;
     // the words this launch reads from global memory, all in flight while the barriers are set up
     const uint32_t ev = a.even_word != nullptr ? ld_volatile_u32(a.even_word) : (uint32_t)a.even;
     uint32_t ss = 0, sx_ = 0;
@@ -639,10 +639,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
     constexpr int grp = decltype(group)::value;
     const int q = j & 1, uq = (j >> 1) & 1;
     if constexpr (!DQ) {
-      wait_or_fault(grp ? &y_full[q] : &x_full[q], uq, &dead, fault, kFaultTmaWait);
+      wait_or_fault(grp ? &y_full[q] : &x_full[q], uq, &cta, fault, kFaultTmaWait);
       scale_row_pieces<WX / 16, true>(grp ? sy[q] : sx[q], row, half * (WX / 16), 1.f, lane);
     } else {
-      wait_or_fault(&z_full[q], uq, &dead, fault, kFaultTmaWait);
+      wait_or_fault(&z_full[q], uq, &cta, fault, kFaultTmaWait);
       scale_row_pieces<WZ / 32, true>(sz[q], row, (2 * half + grp) * (WZ / 32), 1.f, lane);
     }
     fence_async_smem();
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
     for (int g = R::kInTurn ? grp : 0; g < sums; g += R::kInTurn ? 2 : 1) {
       const int j = g % R::kStages;
-      wait_or_fault(&ring_full[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
+      wait_or_fault(&ring_full[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
       const float wt = c * decay_pow(sl2, max(span_end - ((sum_t1 - 1 - g) * C + row), 0));
       if (elu)
         ring.template scale<grp, true>(j, row, half, wt, lane);
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       fence_async_smem();
       warp_arrive(&ring_scaled[j]);
     }
-    wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
+    wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);
     if (tid == kFirstWorker) TRACE(59);
     tc_fence_after_sync();
     const int c0 = half * kHalfE + grp * 32;
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
           for (int g = 0; g < sums; ++g) {
             const int j = g % R::kStages, t = sum_t1 - 1 - g;
-            if (g >= R::kStages) wait_or_fault(&ring_empty[j], (g / R::kStages - 1) & 1, &dead, fault, kFaultMmaWait);
+            if (g >= R::kStages) wait_or_fault(&ring_empty[j], (g / R::kStages - 1) & 1, &cta, fault, kFaultMmaWait);
             if (!(g == 0 && early_ring)) {
               mbar_expect_tx(&ring_full[j], R::kStage);
               tma_load_4d(ring.a(j), &map_y, &ring_full[j], 0, t * C, 0, my_bh);
@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
               }
             }
           }
-          wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);   // the MMAs have read every ring stage
+          wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);   // the MMAs have read every ring stage
         }
         int i = 0;
         IntPair out_row{0, 0}, out_bh{0, 0};
@@ -719,18 +719,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           const int p = i & 1, u = i >> 1;
           if (i >= x_issued) {
             if (i >= 2) {   // S, O2 of tile i-2 read X
-              wait_or_fault(&s_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
-              wait_or_fault(&o2_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
+              wait_or_fault(&s_full[p], (u - 1) & 1, &cta, fault, kFaultMmaWait);
+              wait_or_fault(&o2_full[p], (u - 1) & 1, &cta, fault, kFaultMmaWait);
             }
             mbar_expect_tx(&x_full[p], C * WX * 2);
             tma_load_4d(sx[p], &map_x, &x_full[p], 0, w.t * C, 0, w.bh);
           }
-          if (i >= 2) wait_or_fault(&l_full[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);   // S, L of tile i-2 read Y
+          if (i >= 2) wait_or_fault(&l_full[p], (u - 1) & 1, &cta, fault, kFaultMmaWait);   // S, L of tile i-2 read Y
           mbar_expect_tx(&y_full[p], C * WX * 2);
           tma_load_4d(sy[p], &map_y, &y_full[p], 0, w.t * C, 0, w.bh);
           if (i >= 2) {
             // the output of tile i-2 is staged in Z's buffer: store it, then reuse the buffer
-            wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
+            wait_or_fault(&staged[p], (u - 1) & 1, &cta, fault, kFaultMmaWait);
             tma_store_or_add_4d(&map_out, sz[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
             bulk_commit();
             bulk_wait_read<0>();
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
         for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
           const int p = j & 1, u = j >> 1;
-          wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&staged[p], u & 1, &cta, fault, kFaultMmaWait);
           tma_store_or_add_4d(&map_out, sz[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
           bulk_commit();
         }
@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
         for (int g = 0; g < sums; ++g) {
           const int j = g % R::kStages;
-          wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
+          wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
           tc_fence_after_sync();
           umma_gemm<true, true, E, C>(t_l, smem_u32(ring.a(j)), C, smem_u32(ring.b(j)), C, g > 0);
           umma_commit(&ring_empty[j]);
@@ -775,10 +775,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         for (int i = 0; i < total; ++i) {
           const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
           // the state operand of this tile is written, the epilogue has drained O
-          wait_or_fault(&p_ready, one, &dead, fault, kFaultMmaWait);
-          if (i >= 1) wait_or_fault(&o_free, one ^ 1, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&x_full[p], ph, &dead, fault, kFaultTmaWait);
-          if (map_xy) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&p_ready, one, &cta, fault, kFaultMmaWait);
+          if (i >= 1) wait_or_fault(&o_free, one ^ 1, &cta, fault, kFaultMmaWait);
+          wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
+          if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 0);
           tc_fence_after_sync();
           if constexpr (!DQ)  // X P: the state tile as [K = d rows] x [N = e columns]
@@ -787,10 +787,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
             umma_gemm<false, false, D, E>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false);
           umma_commit(&o2_full[p]);
           // the masked scores are read from tensor memory
-          wait_or_fault(&sm_ready[p], ph, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&z_full[p], ph, &dead, fault, kFaultTmaWait);
-          if (map_z) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&o2s_ready, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&sm_ready[p], ph, &cta, fault, kFaultMmaWait);
+          wait_or_fault(&z_full[p], ph, &cta, fault, kFaultTmaWait);
+          if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
+          wait_or_fault(&o2s_ready, one, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 3);
           tc_fence_after_sync();
           umma_gemm_ts<true, WZ, 64>(t_o, t_s[p], smem_u32(sz[p]), C, true);
@@ -800,10 +800,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
         for (int i = 0; i < total; ++i) {
           const int p = i & 1, ph = (i >> 1) & 1, one = i & 1;
-          wait_or_fault(&z_full[p], ph, &dead, fault, kFaultTmaWait);
-          if (map_z) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
-          if (i >= 1) wait_or_fault(&l_free, one ^ 1, &dead, fault, kFaultMmaWait);   // the state update has read the previous L
-          wait_or_fault(&ys_ready, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&z_full[p], ph, &cta, fault, kFaultTmaWait);
+          if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
+          if (i >= 1) wait_or_fault(&l_free, one ^ 1, &cta, fault, kFaultMmaWait);   // the state update has read the previous L
+          wait_or_fault(&ys_ready, one, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 1);
           tc_fence_after_sync();
           if constexpr (!DQ)
@@ -816,10 +816,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
         for (int i = 0; i < total; ++i) {
           const int p = i & 1, ph = (i >> 1) & 1;
-          if (i >= 2) wait_or_fault(&o_full[p], ph ^ 1, &dead, fault, kFaultMmaWait);   // O1 of tile i-2 has read S_m
-          wait_or_fault(&x_full[p], ph, &dead, fault, kFaultTmaWait);
-          wait_or_fault(&y_full[p], ph, &dead, fault, kFaultTmaWait);
-          if (map_xy) wait_or_fault(&mapped[p], ph, &dead, fault, kFaultMmaWait);
+          if (i >= 2) wait_or_fault(&o_full[p], ph ^ 1, &cta, fault, kFaultMmaWait);   // O1 of tile i-2 has read S_m
+          wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
+          wait_or_fault(&y_full[p], ph, &cta, fault, kFaultTmaWait);
+          if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 2);
           tc_fence_after_sync();
           umma_gemm<false, false, C, WX>(t_s[p], smem_u32(sx[p]), C, smem_u32(sy[p]), C, false);
@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         lam = exp2f(-sl2);
       }
       if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 0);
-      wait_or_fault(&s_full[p], ph, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&s_full[p], ph, &cta, fault, kFaultMmaWait);
       if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 1);
       tc_fence_after_sync();
       // masked scores, packed to bf16 in place: they are the A operand of O1 straight from tensor memory
@@ -874,8 +874,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         raw_row32(raw_x, raw, half * (WZ / 2));
       }
       // epilogue: OUT staged in Z's buffer, once L and O1 have read it
-      wait_or_fault(&l_full[p], ph, &dead, fault, kFaultMmaWait);
-      wait_or_fault(&o_full[p], ph, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&l_full[p], ph, &cta, fault, kFaultMmaWait);
+      wait_or_fault(&o_full[p], ph, &cta, fault, kFaultMmaWait);
       if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 3);
       tc_fence_after_sync();
       if (chain) {
@@ -919,9 +919,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       const int p = i & 1, ph = (i >> 1) & 1;
       const int len = min(C, a.n - w.t * C);     // tokens really in the tile
       if (w.first_of_item()) sl2 = a.s[w.bh % a.h] * kLog2e;
-      wait_or_fault(&s_full[p], ph, &dead, fault, kFaultMmaWait);   // S has read Y
+      wait_or_fault(&s_full[p], ph, &cta, fault, kFaultMmaWait);   // S has read Y
       if (wid == 0) TRACE_TILE(112, 6, i, 0);
-      wait_or_fault(&y_full[p], ph, &dead, fault, kFaultTmaWait);   // completed long ago: makes Y's bytes visible here
+      wait_or_fault(&y_full[p], ph, &cta, fault, kFaultTmaWait);   // completed long ago: makes Y's bytes visible here
       scale_row_pieces<WX / 16>(sy[p], row, half * (WX / 16), c * decay_pow(sl2, max(len - row, 0)), lane);
       fence_async_smem();
       mbar_arrive(&ys_ready);
@@ -952,9 +952,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           const int reach = reach_tiles(a.s[w.bh % a.h]);
           int first = sp_idx;
           while (first > 0 && w.t0 - w.span_t0(first) < reach) --first;
-          if (wid < sp_idx && wid >= first && !dead) {
+          if (wid < sp_idx && wid >= first && !cta.gave_up()) {
             if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + wid, step_s, a.wait_clocks)) {
-              dead = 1;
+              cta.give_up();
               atomicOr(fault, kFaultFlagWait);
             }
           }
@@ -968,6 +968,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (wid == 0) TRACE(61);
           if (LINK && a.link.ranks > 0) {
             // hand-over of the rank state inside the launch.  P holds the local part of the border state.
+            // The waits for peers below may take longer than any other (a.link.wait_clocks).
+            if (wid == 0) cta.peer_wait_begins();
             const float sn = a.s[w.bh % a.h] * (float)a.n;
             const long long elems = (long long)(a.cut.items / a.cut.nspans) * D * E;
             const size_t seq_off = (size_t)w.bh * D * E;
@@ -989,14 +991,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
               }
               if (far || w.it == owner) {
                 // the readers of the ranks after this one have acknowledged the slots' previous use
-                if (!dead) {
+                if (!cta.gave_up()) {
                   bool ok2 = true;
                   if (xl::needs_ack_wait(step_x) && wid < n_dst)
                     ok2 = wait_flag_ge(a.link.my_acks + xl::ack_index(a.link.me + 1 + wid, 0), step_x - 2,
                                        a.link.wait_clocks);
-                  if (far && wid == xl::kMaxRanks && w.it != owner) ok2 = wait_flag_eq(ready, step_s, a.wait_clocks);
+                  if (far && wid == xl::kMaxRanks && w.it != owner) ok2 = wait_flag_eq(ready, step_s, a.link.wait_clocks);
                   if (!ok2) {
-                    dead = 1;
+                    cta.give_up();
                     atomicOr(fault, kFaultRelayWait);
                   }
                 }
@@ -1019,6 +1021,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
                 atomicOr(fault, kFaultRelayWait);
             }
             if (wid == 0) TRACE(55);
+            named_sync(1, kWorkers);
+            if (wid == 0) cta.peer_wait_ends();
           }
         }
         if (row < D) write_state_operand<kHalfE>(sp, D, row, half * kHalfE, P);
@@ -1029,7 +1033,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         }
       }
       // O2's rows take their decay lambda^row in tensor memory; O1 then accumulates on top
-      wait_or_fault(&o2_full[p], ph, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&o2_full[p], ph, &cta, fault, kFaultMmaWait);
       if (wid == 0) TRACE_TILE(112, 6, i, 2);
       tc_fence_after_sync();
       {
@@ -1042,7 +1046,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       mbar_arrive(&o2s_ready);
       if (wid == 0) TRACE_TILE(112, 6, i, 3);
       // state: P <- lambda^len P + L
-      wait_or_fault(&l_full[p], ph, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&l_full[p], ph, &cta, fault, kFaultMmaWait);
       if (wid == 0) TRACE_TILE(112, 6, i, 4);
       tc_fence_after_sync();
       if (row < D) {
@@ -1151,13 +1155,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   __shared__ uint64_t mapped;   // with a feature map: the workers have mapped the tile's Q and K in place
   __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x;
-  __shared__ int dead;
+  __shared__ Health<LINK> cta;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int32_t* fault = a.fault;
   // thread 0 is also the producer: its first loads go out before the CTA-wide barrier (see k_walk_out)
   bool early_ring = false, early_q = false;
   if (tid == 0) {
-    dead = 0;
+    cta.word = 0;
     uint32_t ss = 0, sx_ = 0;   // in flight while the barriers are set up
     if constexpr (FUSED) {
       if (a.coop) ss = ld_volatile_u32(a.sync);
@@ -1249,7 +1253,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
 #pragma unroll 1
     for (int g = R::kInTurn ? grp : 0; g < sums; g += R::kInTurn ? 2 : 1) {
       const int j = g % R::kStages;
-      wait_or_fault(&ring_full[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
+      wait_or_fault(&ring_full[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
       const float wt = c * decay_pow(sl2, g * C + row);
       if (elu)
         ring_buf.template scale<grp, true>(j, row, half, wt, lane);
@@ -1258,7 +1262,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       fence_async_smem();
       warp_arrive(&ring_scaled[j]);
     }
-    wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);
+    wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);
     if (tid == kFirstWorker) TRACE(59);
     tc_fence_after_sync();
     const int c0 = half * kHalfE + grp * 32;
@@ -1286,7 +1290,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
 #pragma unroll 1
           for (int g = 0; g < sums; ++g) {
             const int j = g % R::kStages, t = sum_t0 + g;
-            if (g >= R::kStages) wait_or_fault(&ring_empty[j], (g / R::kStages - 1) & 1, &dead, fault, kFaultMmaWait);
+            if (g >= R::kStages) wait_or_fault(&ring_empty[j], (g / R::kStages - 1) & 1, &cta, fault, kFaultMmaWait);
             if (!(g == 0 && early_ring)) {
               mbar_expect_tx(&ring_full[j], R::kStage);
               tma_load_4d(ring_buf.a(j), &map_q, &ring_full[j], 0, t * C, 0, my_bh);
@@ -1300,7 +1304,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
               kv_issued = true;
             }
           }
-          wait_or_fault(&sum_done, 0, &dead, fault, kFaultMmaWait);   // the MMAs have read every ring stage
+          wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);   // the MMAs have read every ring stage
         }
         int i = 0;
         IntPair out_row{0, 0}, out_bh{0, 0};
@@ -1309,7 +1313,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           const int p = i & 1, u = i >> 1;
           if (i >= 2) {
             // dK and dV of tile i-2 are staged in this parity's Q and dO buffers
-            wait_or_fault(&staged[p], (u - 1) & 1, &dead, fault, kFaultMmaWait);
+            wait_or_fault(&staged[p], (u - 1) & 1, &cta, fault, kFaultMmaWait);
             tma_store_or_add_4d(&map_dk, sq[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
             tma_store_or_add_4d(&map_dv, sdo[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
             bulk_commit();
@@ -1321,9 +1325,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
             tma_load_4d(sdo[p], &map_do, &qdo_full[p], 0, w.t * C, 0, w.bh);
           }
           if (i >= 1) {   // K, V of tile i-1 are read
-            wait_or_fault(&s_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
-            wait_or_fault(&ds_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
-            wait_or_fault(&st_done, (i - 1) & 1, &dead, fault, kFaultMmaWait);
+            wait_or_fault(&s_done, (i - 1) & 1, &cta, fault, kFaultMmaWait);
+            wait_or_fault(&ds_done, (i - 1) & 1, &cta, fault, kFaultMmaWait);
+            wait_or_fault(&st_done, (i - 1) & 1, &cta, fault, kFaultMmaWait);
           }
           if (i >= 1 || !kv_issued) {
             mbar_expect_tx(&kv_full, C * (D + E) * 2);
@@ -1336,7 +1340,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
 #pragma unroll 1
         for (int j = (i >= 2 ? i - 2 : 0); j < i; ++j) {   // the last two tiles
           const int p = j & 1, u = j >> 1;
-          wait_or_fault(&staged[p], u & 1, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&staged[p], u & 1, &cta, fault, kFaultMmaWait);
           tma_store_or_add_4d(&map_dk, sq[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out);
           tma_store_or_add_4d(&map_dv, sdo[p], 0, out_row.get(p), 0, out_bh.get(p), a.add_out2);
           bulk_commit();
@@ -1348,7 +1352,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
 #pragma unroll 1
         for (int g = 0; g < sums; ++g) {
           const int j = g % R::kStages;
-          wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &dead, fault, kFaultTmaWait);
+          wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
           tc_fence_after_sync();
           umma_gemm<true, true, E, C>(t_s, smem_u32(ring_buf.a(j)), C, smem_u32(ring_buf.b(j)), C, g > 0);
           umma_commit(&ring_empty[j]);
@@ -1364,22 +1368,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           const int p = i & 1, one = i & 1;
           // the state tile as [N = d rows] x [K = e columns] (V Dn^T) and as [K = d rows] x [N = e columns] (K Dn);
           // the epilogue has drained T_dK, T_dV
-          wait_or_fault(&kv_full, one, &dead, fault, kFaultTmaWait);
-          if (elu) wait_or_fault(&mapped, one, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&dn_ready, one, &dead, fault, kFaultMmaWait);
-          if (i >= 1) wait_or_fault(&e_free, one ^ 1, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&kv_full, one, &cta, fault, kFaultTmaWait);
+          if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
+          wait_or_fault(&dn_ready, one, &cta, fault, kFaultMmaWait);
+          if (i >= 1) wait_or_fault(&e_free, one ^ 1, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 1);
           tc_fence_after_sync();
           umma_gemm<false, false, D, E>(t_dk, smem_u32(sv), C, smem_u32(sdn), D, false);
           umma_gemm<false, true, E, D>(t_dv, smem_u32(sk), C, smem_u32(sdn), D, false);
           umma_commit(&st_done);
           // the masked scores' products on top, A operands from tensor memory
-          wait_or_fault(&sm_ready, one, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&scaled, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
+          wait_or_fault(&scaled, one, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 3);
           tc_fence_after_sync();
           umma_gemm_ts<true, E, 96>(t_dv, t_s, smem_u32(sdo[p]), C, true);    // += S_m^T dO
-          wait_or_fault(&dsm_ready, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
           tc_fence_after_sync();
           umma_gemm_ts<true, D, 96>(t_dk, t_ds, smem_u32(sq[p]), C, true);    // += dS_m^T Q
           umma_commit(&b_done);
@@ -1390,9 +1394,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           const int p = i & 1, one = i & 1;
           // L = Q_s^T dO in the columns that the packed scores leave free; the scaled copy of Q is in the state
           // operand's buffer
-          wait_or_fault(&sm_ready, one, &dead, fault, kFaultMmaWait);
-          if (E > 64) wait_or_fault(&dsm_ready, one, &dead, fault, kFaultMmaWait);
-          wait_or_fault(&qs_ready, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
+          if (E > 64) wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
+          wait_or_fault(&qs_ready, one, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 2);
           tc_fence_after_sync();
           umma_gemm<true, true, 64, C>(t_s + 32, smem_u32(sdn), C, smem_u32(sdo[p]), C, false);
@@ -1405,12 +1409,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         for (int i = 0; i < total; ++i) {
           const int p = i & 1, one = i & 1;
           if (i >= 1) {   // the masked scores and L of tile i-1 have been read
-            wait_or_fault(&b_done, one ^ 1, &dead, fault, kFaultMmaWait);
-            wait_or_fault(&l_free, one ^ 1, &dead, fault, kFaultMmaWait);
+            wait_or_fault(&b_done, one ^ 1, &cta, fault, kFaultMmaWait);
+            wait_or_fault(&l_free, one ^ 1, &cta, fault, kFaultMmaWait);
           }
-          wait_or_fault(&qdo_full[p], (i >> 1) & 1, &dead, fault, kFaultTmaWait);
-          wait_or_fault(&kv_full, one, &dead, fault, kFaultTmaWait);
-          if (elu) wait_or_fault(&mapped, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(&qdo_full[p], (i >> 1) & 1, &cta, fault, kFaultTmaWait);
+          wait_or_fault(&kv_full, one, &cta, fault, kFaultTmaWait);
+          if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
           TRACE_TILE(160, 8, i, 5);
           tc_fence_after_sync();
           umma_gemm<false, false, C, D>(t_s, smem_u32(sk), C, smem_u32(sq[p]), C, false);
@@ -1434,7 +1438,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         lam = exp2f(-sl2);
       }
       if (elu) {   // K of this tile through the feature map before any product reads it
-        wait_or_fault(&kv_full, one, &dead, fault, kFaultTmaWait);
+        wait_or_fault(&kv_full, one, &cta, fault, kFaultTmaWait);
         scale_row_pieces<D / 16, true>(sk, row, half * (D / 16), 1.f, lane);
         fence_async_smem();
         mbar_arrive(&mapped);
@@ -1446,7 +1450,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
 #pragma unroll 1
       for (int u = 0; u < 4; ++u) {
         if ((u & 1) == 0) {
-          wait_or_fault(u == 0 ? &s_done : &ds_done, one, &dead, fault, kFaultMmaWait);
+          wait_or_fault(u == 0 ? &s_done : &ds_done, one, &cta, fault, kFaultMmaWait);
           if (tid == kFirstWorker && u == 0) TRACE_TILE(64, 6, i, 1);
           tc_fence_after_sync();
         }
@@ -1471,8 +1475,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         raw_row32(raw_x, raw, half * (D / 2));
       }
       // epilogue: dK and dV staged over Q and dO, which every product has read
-      wait_or_fault(&l_done, one, &dead, fault, kFaultMmaWait);
-      wait_or_fault(&b_done, one, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&l_done, one, &cta, fault, kFaultMmaWait);
+      wait_or_fault(&b_done, one, &cta, fault, kFaultMmaWait);
       if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 4);
       tc_fence_after_sync();
       if (PRE && (elu || c != 1.f)) {
@@ -1534,9 +1538,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           const int reach = reach_tiles(a.s[w.bh % a.h]);
           int past = sp_idx + 1;
           while (past < a.cut.nspans && w.span_t0(past) - w.t1 < reach) ++past;
-          if (wid < past - 1 - sp_idx && !dead) {
+          if (wid < past - 1 - sp_idx && !cta.gave_up()) {
             if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + sp_idx + 1 + wid, step_s, a.wait_clocks)) {
-              dead = 1;
+              cta.give_up();
               atomicOr(fault, kFaultFlagWait);
             }
           }
@@ -1550,6 +1554,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           if (wid == 0) TRACE(61);
           if (LINK && a.link.ranks > 0) {
             // hand-over of the rank state inside the launch.  Dn holds the local part of the border state.
+            // The waits for peers below may take longer than any other (a.link.wait_clocks).
+            if (wid == 0) cta.peer_wait_begins();
             const float sn = a.s[w.bh % a.h] * (float)a.n;
             const long long elems = (long long)(a.cut.items / a.cut.nspans) * D * E;
             const size_t seq_off = (size_t)w.bh * D * E;
@@ -1572,14 +1578,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
               if (far || sp_idx == 0) {
                 // the readers of the ranks after this one in the chain order (the ranks BEFORE it in the
                 // sequence) have acknowledged the slots' previous use
-                if (!dead) {
+                if (!cta.gave_up()) {
                   bool ok2 = true;
                   if (xl::needs_ack_wait(step_x) && wid < n_dst)
                     ok2 = wait_flag_ge(a.link.my_acks + xl::ack_index(a.link.me + 1 + wid, 0), step_x - 2,
                                        a.link.wait_clocks);
-                  if (far && wid == xl::kMaxRanks && sp_idx != 0) ok2 = wait_flag_eq(ready, step_s, a.wait_clocks);
+                  if (far && wid == xl::kMaxRanks && sp_idx != 0) ok2 = wait_flag_eq(ready, step_s, a.link.wait_clocks);
                   if (!ok2) {
-                    dead = 1;
+                    cta.give_up();
                     atomicOr(fault, kFaultRelayWait);
                   }
                 }
@@ -1600,6 +1606,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
                                            decay_pow(sl2, a.n - span_end), Dn, sn))
                 atomicOr(fault, kFaultRelayWait);
             }
+            named_sync(1, kWorkers);
+            if (wid == 0) cta.peer_wait_ends();
           }
         }
         // the MMAs that read the operand tile of the previous item have completed (l_done was waited for)
@@ -1607,13 +1615,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         fence_async_smem();
         mbar_arrive(&dn_ready);
       }
-      wait_or_fault(&qdo_full[p], (i >> 1) & 1, &dead, fault, kFaultTmaWait);
+      wait_or_fault(&qdo_full[p], (i >> 1) & 1, &cta, fault, kFaultTmaWait);
       if (elu) {   // Q of this tile through the feature map before any product reads it
         scale_row_pieces<D / 16, true>(sq[p], row, half * (D / 16), 1.f, lane);
         fence_async_smem();
         mbar_arrive(&mapped);
       }
-      wait_or_fault(&st_done, one, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&st_done, one, &cta, fault, kFaultMmaWait);
       if (wid == 0) TRACE_TILE(112, 6, i, 0);
       tc_fence_after_sync();
       // row-scaled copy of Q over the state operand (the state products have read it)
@@ -1634,7 +1642,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       mbar_arrive(&scaled);
       if (wid == 0) TRACE_TILE(112, 6, i, 2);
       // state: Dn <- lambda^len Dn + L, this thread's half of the columns being the one in T_S or in T_dS
-      wait_or_fault(&l_done, one, &dead, fault, kFaultMmaWait);
+      wait_or_fault(&l_done, one, &cta, fault, kFaultMmaWait);
       if (wid == 0) TRACE_TILE(112, 6, i, 3);
       tc_fence_after_sync();
       if (row < D) {
