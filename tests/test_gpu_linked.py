@@ -130,6 +130,31 @@ class Problem:
         return bw
 
 
+SLOPES = [0.0, 0.002, 0.02, 1.5]        # reach every rank, every rank, the next one or two, the next rank only
+
+
+@pytest.mark.parametrize("ranks,pos", [(2, 0), (2, 1), (4, 0), (4, 1), (4, 2), (4, 3)])
+@pytest.mark.parametrize("d,e,n", [(128, 128, 1000), (128, 64, 2048), (64, 128, 700), (64, 64, 3001)])
+@pytest.mark.parametrize("scale,fmap", [(1.0, None), (0.125, "elu1")])
+def test_a_rank_of_a_group(ranks, pos, d, e, n, scale, fmap):
+    from lasp_b200 import engine
+    p = Problem(ranks, pos, 2, n, d, e, SLOPES, scale, fmap)
+    o, total, dq, dk, dv, dtotal = p.expected()
+    for step in (1, 6):                                # the first hand-over, and one whose slots have been used before
+        fr = Rank(ranks, pos, p.shape, step)
+        p.fill(fr)
+        fw = p.forward(fr)
+        br = Rank(ranks, ranks - 1 - pos, p.shape, step)
+        p.fill(br)
+        bw = p.backward(br, fw)
+        torch.cuda.synchronize()
+        assert engine.read_status() == 0
+        for got, want, key in ((fw.o, o, "o"), (bw.dq, dq, "dq"), (bw.dk, dk, "dk"), (bw.dv, dv, "dv")):
+            assert O.max_rel_err(got.float(), want) < 2e-2, (key, step)
+        fr.check_sent(total, p.reach)
+        br.check_sent(dtotal, p.reach)
+
+
 def test_a_late_peer_is_waited_for():
     """The words of the rank before arrive more than half a second - the limit of every other wait of the kernels - after
     the launch: same results, no fault."""
