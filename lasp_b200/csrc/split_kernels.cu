@@ -2,7 +2,9 @@
 // 64 and 128, sequences shorter than a tile), on the tensor cores without giving up fp32 arithmetic.
 //
 // An fp32 number is the exact sum of three bf16 numbers (24 bits = 8 + 8 + 8), an fp16 number of two, so a product
-// of fp32 matrices is a sum of products of bf16 matrices accumulated in fp32.  Of the nine products of two
+// of fp32 matrices is a sum of products of bf16 matrices accumulated in fp32.  (From 2^-110 on: of smaller numbers the
+// last term falls below bf16's smallest, 2^-133, which is then the absolute error.  Not from bf16's largest, 3.39e38, on:
+// see "outside the terms' range" below.)  Of the nine products of two
 // three-term operands the six with i + j <= 2 are kept: what is left out is below 2^-24 of a factor, the rounding of
 // an fp32 product (the method of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype
 // for higher-precision computations", 2019).  Small products go first, so that the few additions at full magnitude
@@ -213,6 +215,26 @@ __device__ __forceinline__ void issue_terms_ts(uint32_t d_tmem, uint32_t t_s, ui
 }
 
 // ---------------------------------------------------------------------------
+// Outside the terms' range.  Infinities, and finite values above bf16's largest, have an infinite first term and a
+// remainder that is NaN or infinite too, so that wherever one of them - an input, a state, a score - takes part, the
+// products of terms give no finite number.  Results that are not finite are computed again in plain fp32 arithmetic from
+// the tensors: infinities, large numbers and NaN come out as they do there, and reach the tokens that they do there.
+// The kernels look at every 16 results at once and come back to those that need it where few registers are live: after
+// all of a CTA's tasks, or, where results are added to what a tensor holds, at the end of the task.  (Calls inside the
+// epilogue's loop cost fp32 outputs 5 to 12 % by the registers that they take; this way 1.8 %, fp16 nothing, bf16 1 %.)
+// ---------------------------------------------------------------------------
+// (by their sum: eight packed additions; one that overflows costs a look at results that are finite)
+__device__ __forceinline__ bool all_finite(const uint32_t (&r)[16]) {
+  F2 z = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 16; j += 2) z = fma2(pair(r[j], r[j + 1]), {1.f, 1.f}, z);
+  return isfinite(z.x + z.y);
+}
+__device__ __forceinline__ float to_float(float x) { return x; }
+__device__ __forceinline__ float to_float(__half x) { return __half2float(x); }
+__device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
+
+// ---------------------------------------------------------------------------
 // chunk states: T[i][j] = sum_c w_c A[c][i] B[c][j], in lane order
 //   forward : A = K, B = V,  w_c = lambda^(len-c);   backward: A = Q, B = dO, w_c = lambda^c
 // A task per chunk, persistent CTAs; the next chunk's rows are on their way while the products of this one run.
@@ -227,6 +249,28 @@ struct StateArgs {
   int32_t* fault;
 };
 
+// The elements of a task's state that are not finite, again
+template <typename T>
+__device__ __forceinline__ void plain_state(const StateArgs& g, int task) {
+  const int bh = task / g.nc, chunk = task - bh * g.nc, len = min(C, g.n - chunk * C);
+  const size_t tok = (size_t)bh * g.n + (size_t)chunk * C;
+  const T *a = static_cast<const T*>(g.a) + tok * g.pitch_a, *b = static_cast<const T*>(g.b) + tok * g.pitch_b;
+  const float sh = g.s[bh % g.h];
+  float4* state = reinterpret_cast<float4*>(g.states + (size_t)task * g.d * g.e);
+  for (int p = threadIdx.x; p < g.d * g.e / 4; p += NT) {   // four columns of a row, in lane order
+    const int row = p % g.d, col = p / g.d * 4;
+    const float4 old = state[p];
+    if (isfinite(old.x + old.y + old.z + old.w)) continue;
+    float y[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c = 0; c < len && !(isnan(y[0]) && isnan(y[1]) && isnan(y[2]) && isnan(y[3])); ++c) {
+      const float x = to_float(a[(size_t)c * g.pitch_a + row]) * expf(-sh * (float)(g.backward ? c : len - c));
+      for (int j = 0; j < 4; ++j) y[j] = fmaf(x, to_float(b[(size_t)c * g.pitch_b + col + j]), y[j]);
+    }
+    state[p] = make_float4(isfinite(old.x) ? old.x : y[0], isfinite(old.y) ? old.y : y[1], isfinite(old.z) ? old.z : y[2],
+                           isfinite(old.w) ? old.w : y[3]);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
   using TT = Terms<T>;
@@ -234,12 +278,13 @@ __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
   __shared__ uint64_t done;
   __shared__ uint32_t tmem_slot;
   __shared__ Health<false> cta;
+  __shared__ int look_again;   // a state with an element that is not finite has been written
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dp = padded(g.d), ep = padded(g.e);
   uint8_t* sa = align1024(smem_raw);
   uint8_t* sb = sa + TT::mid * C * dp * 2;   // (with dp = 64 the M = 128 MMA reads on from A into B: valid memory)
   if (tid == 0) {
-    cta.word = 0;
+    cta.word = look_again = 0;
     mbar_init(&done, 1);
     fence_mbar_init();
   }
@@ -292,6 +337,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
       tmem_ld16(tmem + lane_base + c0, r);
       tmem_ld_wait();
       if (row_l < g.d && c0 < g.e) {
+        if (!all_finite(r)) look_again = 1;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           out[(size_t)(c0 / 4 + q) * g.d + row_l] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
@@ -303,6 +349,10 @@ __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 128);
+  if (look_again) {   // (after the loop, whose registers hold the next chunk's rows)
+    for (int u = blockIdx.x; u < g.tasks; u += gridDim.x)
+      if (u % g.nc != g.skip) plain_state<T>(g, u);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -373,20 +423,88 @@ __device__ __forceinline__ void put16(T* p, const float (&x)[16], bool add) {
   }
 }
 
+// Blocks of 16 columns of row `row` of a task's output from column `col` on, those whose bit is set
 template <typename T>
+__device__ __noinline__ void plain_out(const OutArgs* g, int t, int row, int col, uint32_t blocks) {
+  const OutRole& r = g->role[t % g->roles];
+  const int u = t / g->roles, bh = u / g->nc, chunk = u - bh * g->nc, len = min(C, g->n - chunk * C);
+  const size_t tok = (size_t)bh * g->n + (size_t)chunk * C;
+  const T *x = static_cast<const T*>(r.x) + (tok + row) * r.pitch_x, *y = static_cast<const T*>(r.y) + tok * r.pitch_x;
+  const float sh = g->s[bh % g->h];
+  for (; blocks != 0; blocks >>= 1, col += 16) {
+    if ((blocks & 1) == 0) continue;
+    const T* z = static_cast<const T*>(r.z) + tok * r.pitch_z + col;
+    float sum[16], inter[16];
+    for (int j = 0; j < 16; ++j) sum[j] = inter[j] = 0.f;
+    bool settled = false;   // all NaN: so they stay
+    for (int c = r.rev ? row : 0; !settled && (r.rev ? c < len : c <= row); ++c) {   // the tokens that the mask lets through
+      float dot = 0.f;
+      for (int i = 0; i < r.wx; i += 8) {
+        Raw<T> rx, ry;
+        load_piece<T>(rx, x + i), load_piece<T>(ry, y + (size_t)c * r.pitch_x + i);
+        float fx[8], fy[8];
+        to_floats<T>(rx, fx), to_floats<T>(ry, fy);
+        for (int j = 0; j < 8; ++j) dot = fmaf(fx[j], fy[j], dot);
+      }
+      dot *= expf(-sh * (float)(r.rev ? c - row : row - c));
+      settled = true;
+      for (int h = 0; h < 16; h += 8) {
+        Raw<T> rz;
+        load_piece<T>(rz, z + (size_t)c * r.pitch_z + h);
+        float fz[8];
+        to_floats<T>(rz, fz);
+        for (int j = 0; j < 8; ++j) {
+          sum[h + j] = fmaf(dot, fz[j], sum[h + j]);
+          settled = settled && isnan(sum[h + j]);
+        }
+      }
+    }
+    if (!settled && r.state != nullptr && chunk != r.zero_chunk) {
+      const float* p = r.state + ((size_t)bh * g->nc + chunk) * g->d * g->e;   // lane order (common.cuh)
+      for (int i = 0; i < r.wx; ++i) {
+        for (int j = 0; j < 16; ++j) {
+          const int pr = r.transposed ? col + j : i, pc = r.transposed ? i : col + j;
+          inter[j] = fmaf(to_float(x[i]), p[((size_t)(pc / 4) * g->d + pr) * 4 + pc % 4], inter[j]);
+        }
+      }
+      const float w_row = expf(-sh * (float)(r.rev ? len - row : row));
+      for (int j = 0; j < 16; ++j) sum[j] = fmaf(w_row, inter[j], sum[j]);
+    }
+    put16(static_cast<T*>(r.out) + (tok + row) * r.pitch_z + col, sum, r.add != 0);
+  }
+}
+
+// ... of a whole task, the blocks of its output that hold such a result
+template <typename T>
+__device__ __noinline__ void plain_out_where_needed(const OutArgs* g, int t) {
+  const OutRole& r = g->role[t % g->roles];
+  const int u = t / g->roles, bh = u / g->nc, chunk = u - bh * g->nc, len = min(C, g->n - chunk * C);
+  const size_t tok = (size_t)bh * g->n + (size_t)chunk * C;
+  for (int p = threadIdx.x; p < C * (r.wz / 16); p += NT) {
+    const int row = p % C, col = p / C * 16;
+    if (row >= len) continue;
+    const T* out = static_cast<const T*>(r.out) + (tok + row) * r.pitch_z + col;
+    bool finite = true;
+    for (int j = 0; j < 16; ++j) finite = finite && isfinite(to_float(out[j]));
+    if (!finite) plain_out<T>(g, t, row, col, 1u);
+  }
+}
+
+template <typename T, bool ADD>
 __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ OutArgs g) {
   using TT = Terms<T>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t s_done, o2_done, o1_done;
   __shared__ uint32_t tmem_slot;
   __shared__ Health<false> cta;
+  __shared__ int look_again;   // a result that is not finite has been written
   __shared__ float decay[C + 1];   // lambda^0 .. lambda^128 of the task's head
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dp = padded(g.d), ep = padded(g.e);
   uint8_t* set_a = align1024(smem_raw);
   uint8_t* set_b = set_a + g.set_bytes;
   if (tid == 0) {
-    cta.word = 0;
+    cta.word = look_again = 0;
     mbar_init(&s_done, 1);
     mbar_init(&o2_done, 1);
     mbar_init(&o1_done, 1);
@@ -541,6 +659,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
       {
         const int per = wz / 4;
         T* out = static_cast<T*>(k.r->out) + (k.tok + row_l) * k.r->pitch_z;
+        uint32_t again = 0;   // blocks of 16 columns with a result that is not finite
 #pragma unroll 1
         for (int c0 = group * per; c0 < (group + 1) * per; c0 += 16) {
           uint32_t a1[16], a2[16];
@@ -550,10 +669,23 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
           if (row_l < k.len && c0 < k.r->wz) {
             float x[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
+            for (int j = 0; j < 16; ++j) {
               x[j] = k.has_state ? fmaf(w_row, __uint_as_float(a2[j]), __uint_as_float(a1[j])) : __uint_as_float(a1[j]);
-            put16(out + c0, x, k.r->add != 0);
+              a1[j] = __float_as_uint(x[j]);
+            }
+            if constexpr (ADD) {
+              if (all_finite(a1))
+                put16(out + c0, x, k.r->add != 0);
+              else
+                again |= 1u << ((c0 - group * per) / 16);
+            } else {
+              if (!all_finite(a1)) look_again = 1;
+              put16(out + c0, x, false);
+            }
           }
+        }
+        if constexpr (ADD) {
+          if (again) plain_out<T>(&g, t, row_l, group * per, again);   // (here few registers are live)
         }
       }
       o2_uses += k.has_state ? 1 : 0;
@@ -565,6 +697,10 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, 512);
+  if constexpr (!ADD) {
+    if (look_again)   // (after the loop, whose registers are all taken)
+      for (int u = blockIdx.x; u < g.tasks; u += gridDim.x) plain_out_where_needed<T>(&g, u);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -602,16 +738,16 @@ cudaError_t launch_states(const Dims& m, const StateArgs& g, cudaStream_t st) {
   return err;
 }
 
-template <typename T>
+template <typename T, bool ADD>
 cudaError_t launch_out(const Dims& m, OutArgs& g, cudaStream_t st) {
   const int dp = host_padded(m.d), ep = host_padded(m.e), widest = dp > ep ? dp : ep;
   g.set_bytes = (uint32_t)(Terms<T>::in * C * widest * 2);
   const size_t state = (size_t)Terms<T>::mid * dp * ep * 2;
   const size_t smem = g.set_bytes + (state > g.set_bytes ? state : g.set_bytes) + 1024;
-  cudaError_t err = opt_in_smem<k_split_out<T>>(kMaxSmem);
+  cudaError_t err = opt_in_smem<k_split_out<T, ADD>>(kMaxSmem);
   if (err != cudaSuccess) return err;
   const int grid = g.tasks < sm_count() ? g.tasks : sm_count();
-  k_split_out<T><<<grid, NT, smem, st>>>(g);
+  k_split_out<T, ADD><<<grid, NT, smem, st>>>(g);
   err = cudaGetLastError();
   if (err != cudaSuccess) g_failed_step = "launch of the output kernel";
   return err;
@@ -649,7 +785,7 @@ cudaError_t split_fwd_output(const Dims& m, const void* q, const void* k, const 
   g.s = s, g.h = m.h, g.n = m.n, g.nc = m.nc, g.d = m.d, g.e = m.e, g.tasks = m.b * m.h * m.nc;
   const cudaError_t err = fault_word_address(&g.fault);
   if (err != cudaSuccess) return err;
-  return by_dtype(m.dtype, [&](auto t) { return launch_out<decltype(t)>(m, g, st); });
+  return by_dtype(m.dtype, [&](auto t) { return g.role[0].add || g.role[1].add || g.role[2].add ? launch_out<decltype(t), true>(m, g, st) : launch_out<decltype(t), false>(m, g, st); });
 }
 
 cudaError_t split_bwd_grads(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, const float* s,
@@ -665,7 +801,7 @@ cudaError_t split_bwd_grads(const Dims& m, const void* q, const void* k, const v
   g.s = s, g.h = m.h, g.n = m.n, g.nc = m.nc, g.d = m.d, g.e = m.e, g.tasks = 3 * m.b * m.h * m.nc;
   const cudaError_t err = fault_word_address(&g.fault);
   if (err != cudaSuccess) return err;
-  return by_dtype(m.dtype, [&](auto t) { return launch_out<decltype(t)>(m, g, st); });
+  return by_dtype(m.dtype, [&](auto t) { return g.role[0].add || g.role[1].add || g.role[2].add ? launch_out<decltype(t), true>(m, g, st) : launch_out<decltype(t), false>(m, g, st); });
 }
 
 }  // namespace lasp
