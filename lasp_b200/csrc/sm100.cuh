@@ -189,7 +189,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
-// tcgen05.mma (bf16 x bf16 -> fp32, M = 128, one CTA)
+// tcgen05.mma (bf16 x bf16 or fp16 x fp16 -> fp32, M = 128, one CTA)
 // ---------------------------------------------------------------------------
 // shared-memory matrix descriptor, 128-byte swizzle.  lbo/sbo in bytes:
 //   K-major : sbo = stride between 8-row groups (1024); lbo unused (16)
@@ -202,9 +202,9 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr, uint32_t lbo, 
   d |= (uint64_t)2 << 61;  // 128-byte swizzle
   return d;
 }
-// instruction descriptor: fp32 accumulate, bf16 A and B, dense
-__host__ __device__ constexpr uint32_t umma_idesc(uint32_t m, uint32_t n, bool a_mn_major, bool b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
+// instruction descriptor: fp32 accumulate, A and B both bf16 or both fp16, dense
+__host__ __device__ constexpr uint32_t umma_idesc(uint32_t m, uint32_t n, bool a_mn_major, bool b_mn_major, bool fp16 = false) {
+  return (1u << 4) | (fp16 ? 0u : (1u << 7) | (1u << 10)) | ((a_mn_major ? 1u : 0u) << 15) | ((b_mn_major ? 1u : 0u) << 16) |
          ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 // One MMA of shape M x N x 16; accumulate = 0 overwrites the accumulator.  A descriptor is passed as its two words: the

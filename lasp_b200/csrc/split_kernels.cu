@@ -4,12 +4,14 @@
 // An fp32 number is the exact sum of three bf16 numbers (24 bits = 8 + 8 + 8), an fp16 number of two, so a product
 // of fp32 matrices is a sum of products of bf16 matrices accumulated in fp32.  (From 2^-110 on: of smaller numbers the
 // last term falls below bf16's smallest, 2^-133, which is then the absolute error.  Not from bf16's largest, 3.39e38, on:
-// see "outside the terms' range" below.)  Of the nine products of two
-// three-term operands the six with i + j <= 2 are kept: what is left out is below 2^-24 of a factor, the rounding of
-// an fp32 product (the method of Henry, Tang and Heinecke, "Leveraging the bfloat16 artificial intelligence datatype
-// for higher-precision computations", 2019).  Small products go first, so that the few additions at full magnitude
-// come last.  Operands in 16-bit types need fewer terms: the inputs are exact in two (fp16) or one (bf16), the
-// quantities computed on the way - masked scores, states, decayed rows - carry 17 bits there and 24 bits for fp32.
+// see "outside the terms' range" below.)  Of the nine products of two three-term operands the six with i + j <= 2 are
+// kept: what is left out is below 2^-24 of a factor, the rounding of an fp32 product (the method of Henry, Tang and
+// Heinecke, "Leveraging the bfloat16 artificial intelligence datatype for higher-precision computations", 2019).  Small products go first, so that the few additions at full magnitude
+// come last.  Inputs in 16-bit types need fewer terms: they are exact in two (fp16) or one (bf16), and the scores, whose
+// operands are both inputs, come from fp16 tiles as they are, one exact product.  What is computed on the way - masked
+// scores, states, decayed rows - has three terms, 24 bits, for all types.  (With two there, 17 bits, and the scores from
+// two terms of fp16 operands, a tenth faster, the rank states of fp16 and bf16 tensors were 3.7e-6 and 2.4e-6 off instead
+// of 1.5e-7, and the rounded fp16 results' error against fp64 was larger by 3e-4 of itself.)
 //
 // Sequences are cut into 128-token chunks (the last one ragged), everything in parallel over chunks:
 //   k_split_states  T = sum_c w_c a_c b_c^T of every chunk                       (a,b = k,v or q,do)
@@ -20,8 +22,10 @@
 // the scores once per result costs one product in nine and makes every chunk three independent tasks.
 //
 // One B200, b=2, h=12, n=2048, forward / backward, before (a CTA of 256 FFMA threads per 64-token chunk) and now:
-// fp32 d=e=128 730 / 1421 -> 86 / 167 us, fp16 d=128, e=64 365 / 869 -> 45 / 84 us, bf16 d=e=96 363 / 920 -> 42 / 79 us;
-// the relative error of fp32 results against fp64 stays at 2e-7.
+// fp32 d=e=128 730 / 1421 -> 82 / 154 us, fp16 d=128, e=64 365 / 869 -> 48 / 86 us, bf16 d=e=96 363 / 920 -> 44 / 79 us;
+// the relative error against fp64 is no larger than theirs: fp32 results 2e-7, fp16 results and states of all types the same.
+#include <type_traits>
+
 #include "tc_common.cuh"
 
 namespace lasp {
@@ -35,8 +39,8 @@ constexpr int kPieces = 4;        // 8-element pieces of a 128 x 128 tile per th
 // terms of the inputs and of intermediate quantities, and the largest i + j of a product that is kept
 template <typename T> struct Terms;
 template <> struct Terms<float> { static constexpr int in = 3, mid = 3, cut = 2; };
-template <> struct Terms<__half> { static constexpr int in = 2, mid = 2, cut = 1; };
-template <> struct Terms<__nv_bfloat16> { static constexpr int in = 1, mid = 2, cut = 1; };
+template <> struct Terms<__half> { static constexpr int in = 2, mid = 3, cut = 2; };
+template <> struct Terms<__nv_bfloat16> { static constexpr int in = 1, mid = 3, cut = 2; };
 
 // eight elements of a row as they come from global memory
 template <typename T> struct Raw { uint4 v; };
@@ -131,6 +135,17 @@ __device__ __forceinline__ void store_tile(uint8_t* tiles, const Raw<T> (&r)[kPi
   }
 }
 struct NoWeight {};
+// ... as it is, a 16-bit type
+template <typename T>
+__device__ __forceinline__ void store_raw(uint8_t* tile, const Raw<T> (&r)[kPieces], int wp, int tid) {
+  const int sh = wp == 128 ? 4 : 3;
+#pragma unroll
+  for (int i = 0; i < kPieces; ++i) {
+    const int p = tid + NT * i, row = p >> sh, col = (p & ((1 << sh) - 1)) * 8;
+    if (row >= C) break;
+    *reinterpret_cast<uint4*>(tile + tile_offset(row, col, C)) = r[i].v;
+  }
+}
 
 // a d x e state in lane order (common.cuh), padded to dp x ep: piece p is row p mod dp, columns 8 (p / dp) on
 __device__ __forceinline__ void load_state(Raw<float> (&r)[kPieces], const float* state, int d, int e, int dp, int ep, int tid) {
@@ -165,9 +180,9 @@ struct TermOperand {
   __device__ __forceinline__ SmemDesc desc(int term) const { return operand_desc(addr + term * stride, rows, mn_major); }
 };
 // D[128 x n] = A B: every kept product of terms, the smallest first; issued by one thread
-template <int NA, int NB, int CUT>
+template <int NA, int NB, int CUT, bool FP16 = false>
 __device__ __forceinline__ void issue_terms(uint32_t d_tmem, const TermOperand& a, const TermOperand& b, uint32_t n, int ksteps) {
-  const uint32_t idesc = umma_idesc(128, n, a.mn_major, b.mn_major);
+  const uint32_t idesc = umma_idesc(128, n, a.mn_major, b.mn_major, FP16);
   uint32_t acc = 0;
 #pragma unroll
   for (int sum = CUT; sum >= 0; --sum) {
@@ -359,7 +374,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
 // outputs: OUT = (X Y^T . M) Z + diag(w) X op(P)
 //   rev = 0: M_ij = lambda^(i-j) [i >= j], w_i = lambda^i;   rev = 1: M_ij = lambda^(j-i) [j >= i], w_i = lambda^(len-i)
 // Tensor memory: S (terms 0 and 1 of the masked scores over S itself), its term 2, the two products.  Shared memory:
-// two sets of term tiles, X then Z in the first, Y then P in the second.  A task's steps, each product running
+// two sets of term tiles, X then Z in the first, Y (fp16: Y and X as they are) then P in the second.  A task's steps, each product running
 // under the next step's work (the loads of a step are issued one step earlier):
 //   S = X Y^T | P's terms | O2 = X P | mask, split S; Z's terms | O1 = S_m Z | next task's Y, X terms | next S | epilogue
 // ---------------------------------------------------------------------------
@@ -542,11 +557,25 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
   const auto load_xy = [&](Raw<T> (&dst)[kPieces], const void* p, const Task& k) {
     load_tile<T>(dst, static_cast<const T*>(p) + k.tok * k.r->pitch_x, k.r->pitch_x, k.len, k.r->wx, padded(k.r->wx), tid);
   };
+  // the scores' operands: Y and, for fp16, X as they are in the second set, X's terms in the first
+  constexpr bool kRawScores = std::is_same<T, __half>::value;
+  const auto store_y = [&](const Raw<T> (&ry)[kPieces], const Raw<T> (&rx)[kPieces], int wx) {
+    if constexpr (kRawScores) {
+      store_raw<T>(set_b, ry, wx, tid);
+      store_raw<T>(set_b + C * wx * 2, rx, wx, tid);
+    } else {
+      store_tile<T, TT::in, false>(set_b, ry, wx, tid, NoWeight());
+    }
+  };
   const auto issue_s = [&](const Task& k) {
     const int wx = padded(k.r->wx);
     tc_fence_after_sync();
-    issue_terms<TT::in, TT::in, TT::cut>(t_s, TermOperand{addr_a, (uint32_t)(C * wx * 2), C, false},
-                                         TermOperand{addr_b, (uint32_t)(C * wx * 2), C, false}, C, wx / 16);
+    if constexpr (kRawScores)
+      issue_terms<1, 1, 0, true>(t_s, TermOperand{addr_b + (uint32_t)(C * wx * 2), 0, C, false}, TermOperand{addr_b, 0, C, false}, C,
+                                 wx / 16);
+    else
+      issue_terms<TT::in, TT::in, TT::cut>(t_s, TermOperand{addr_a, (uint32_t)(C * wx * 2), C, false},
+                                           TermOperand{addr_b, (uint32_t)(C * wx * 2), C, false}, C, wx / 16);
     umma_commit(&s_done);
   };
 
@@ -558,7 +587,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
       load_xy(rx, k.r->x, k);
       load_xy(ry, k.r->y, k);
       if (tid <= C) decay[tid] = expf(-k.sh * (float)tid);
-      store_tile<T, TT::in, false>(set_b, ry, padded(k.r->wx), tid, NoWeight());
+      store_y(ry, rx, padded(k.r->wx));
       store_tile<T, TT::in, false>(set_a, rx, padded(k.r->wx), tid, NoWeight());
     }
     fence_async_smem();
@@ -644,7 +673,7 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
         load_xy(ry, kn.r->y, kn);
         load_xy(rx, kn.r->x, kn);
         if (tid <= C) decay[tid] = expf(-kn.sh * (float)tid);   // this task's masks are done (barrier above)
-        store_tile<T, TT::in, false>(set_b, ry, padded(kn.r->wx), tid, NoWeight());   // O2 has read P
+        store_y(ry, rx, padded(kn.r->wx));   // O2 has read P
         wait_or_fault(&o1_done, it & 1, &cta, g.fault, kFaultMmaWait);
         store_tile<T, TT::in, false>(set_a, rx, padded(kn.r->wx), tid, NoWeight());
         fence_async_smem();
