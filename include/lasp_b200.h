@@ -134,7 +134,8 @@ LASP_B200_API const char* lasp_b200_last_cuda_error(void);
  * negative status when the problem is invalid (lasp_forward's shape asserts,
  * lasp/lasp_fuse_parallel.py:1080-1085, made explicit). */
 LASP_B200_API int lasp_b200_resolve_path(const lasp_problem* p);
-/* tokens per chunk state for the resolved path */
+/* Tokens per span of the tensor path (lasp_b200_linked_ok and the workspace go by it); on the full-precision path the
+ * reference's block size, 64, in which the workspace is sized (its kernels keep a state per 128 tokens). */
 LASP_B200_API int lasp_b200_chunk_tokens(const lasp_problem* p);
 LASP_B200_API size_t lasp_b200_fwd_workspace_bytes(const lasp_problem* p);
 LASP_B200_API size_t lasp_b200_bwd_workspace_bytes(const lasp_problem* p);

@@ -47,8 +47,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
                      "-I", CSRC]
     if verbose:
         common += ["-Xptxas", "-v"]
-    if os.environ.get("LASP_TRACE") == "1":
-        common += ["-DLASP_TRACE"]
     procs = []
     for src in SOURCES:
         path = os.path.join(CSRC, src)

@@ -304,7 +304,10 @@ int lasp_b200_forward_opt(const lasp_problem* p, const lasp_fwd_args* a, const l
   if ((st = check_options(opt, a->kv_in || a->kv_out)) != LASP_OK) return st;
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
   // Without a backward pass to leave states for, sequences of two tiles are walked in one go: handing a total from CTA
-  // to CTA takes longer than a second tile (9.2 us against 8.0 for 8 heads of 256 tokens, 64-wide; three tiles: even).
+  // to CTA takes longer than a second tile, at every width and number of heads that would be cut in two (up to half as
+  // many as SMs).  256 tokens, in one go against in two spans: 64-wide 1 / 8 / 74 heads 8.0 / 8.0 / 8.9 against 9.1 / 9.2 /
+  // 10.7 us, 128-wide 9.7 / 9.8 / 11.7 against 10.9 / 11.6 / 14.7, 128/64 8.4 / 8.5 / 9.4 against 9.3 / 10.1 / 12.6; 129
+  // tokens alike.  Three tiles: even.
   if (m.walk && !opt->keep_states && m.tiles <= 2 && fusable(m)) m.span = m.tiles, m.nc = 1;
   if (fusable(m))
     return cuda_fail(lasp::walk_fwd_fused(m, a->q, a->k, a->v, a->s, a->kv_in, a->kv_out,

@@ -24,8 +24,9 @@ namespace lasp {
 //                      [4096 + S*4, + S*4)  prefix states: fp32 states at the span borders
 // The running prefix inside the scan is always fp32.
 constexpr int kTensorTile = 128;  // one tcgen05 M=128 tile
-constexpr int kAbiChunk = 64;     // the reference's block size: what the C ABI reports and sizes the full-precision
-                                  // path's workspace by (its chunks are two of these)
+constexpr int kAbiChunk = 64;     // the reference's block size: the unit in which the C ABI states the chunks of the
+                                  // full-precision path and sizes its workspace.  The kernels' chunks are two of these,
+                                  // so they use half of it; the sizes are part of the interface and stay.
 
 struct Dims {
   int b, h, n, d, e;
@@ -90,6 +91,23 @@ cudaError_t fault_word_address(int32_t** out);
 
 // name of the host-side step that produced the last cudaError_t (for error text)
 extern thread_local const char* g_failed_step;
+
+// Lets a kernel ask for up to `bytes` (the most that it ever takes) of dynamic shared memory; once per kernel and device,
+// the attribute call costs the host about as much as a launch.
+template <auto fn>
+cudaError_t opt_in_smem(size_t bytes) {
+  static bool done[64] = {};
+  int dev = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err == cudaSuccess && dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
+  if (err == cudaSuccess)
+    err = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (err != cudaSuccess)
+    g_failed_step = "cudaFuncSetAttribute(max dynamic shared memory)";
+  else if (dev >= 0 && dev < 64)
+    done[dev] = true;
+  return err;
+}
 
 // ---- launchers implemented in the .cu files (return cudaError_t) -----------
 // Full-precision path (split_kernels.cu).  `alone`: no rank state comes in or goes out, so the states at the

@@ -737,21 +737,6 @@ __global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ Out
 // ---------------------------------------------------------------------------
 int host_padded(int w) { return w <= 64 ? 64 : 128; }
 
-template <auto fn>
-cudaError_t opt_in_smem(size_t bytes) {   // the largest the kernel ever asks for, once per device
-  static bool done[64] = {};
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err == cudaSuccess && dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err != cudaSuccess)
-    g_failed_step = "cudaFuncSetAttribute(max dynamic shared memory)";
-  else if (dev >= 0 && dev < 64)
-    done[dev] = true;
-  return err;
-}
-
 constexpr size_t kMaxSmem = 6 * 32768 + 1024;
 
 template <typename T>

@@ -29,22 +29,6 @@ namespace {
 
 using namespace tc;
 
-#ifdef LASP_TRACE
-constexpr int kTraceSlots = 256;
-__device__ long long g_trace[160 * kTraceSlots];
-#define TRACE(slot) do { if (blockIdx.x < 160 && (slot) < kTraceSlots) g_trace[blockIdx.x * kTraceSlots + (slot)] = clock64(); } while (0)
-__device__ __forceinline__ long long gtime() { long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; }
-#define GTRACE(slot) do { if (blockIdx.x < 160) g_trace[blockIdx.x * kTraceSlots + (slot)] = gtime(); } while (0)
-#define TRACE_VAL(slot, v) do { if (blockIdx.x < 160) g_trace[blockIdx.x * kTraceSlots + (slot)] = (v); } while (0)
-__device__ __forceinline__ uint32_t smid() { uint32_t v; asm volatile("mov.u32 %0, %%smid;" : "=r"(v)); return v; }
-#define TRACE_TILE(base, stride, i, k) do { if ((i) < 8) TRACE((base) + (i) * (stride) + (k)); } while (0)   // first tiles
-#else
-#define TRACE_TILE(base, stride, i, k) do {} while (0)
-#define TRACE_VAL(slot, v) do {} while (0)
-#define TRACE(slot) do {} while (0)
-#define GTRACE(slot) do {} while (0)
-#endif
-
 constexpr int kBuf = 32768;       // one shared-memory buffer: a 128 x 128 bf16 tile
 
 // Two buffers of a double-buffered tile / two accumulators, addressed by arithmetic: an array of two pointers
@@ -506,7 +490,7 @@ __device__ __forceinline__ void write_state_operand(uint8_t* tile, int rows, int
 //
 // FUSED = false: the state of every span at its border comes from the scan (a.p0).
 // FUSED = true : one launch does everything.  With more than one span per sequence every CTA has
-//   exactly one span (a cooperative launch, all CTAs resident).  It first sums its own span,
+//   exactly one span (one CTA per SM at most; each waits for lower block indexes only).  It first sums its own span,
 //   T = sum_c lambda^(span end - c) k_c v_c^T, streaming K and V once through a ring of stages, writes
 //   T to global memory and raises a flag; then it adds up the totals of the spans before it (and the
 //   incoming rank state) with their decays - that is its border state - and walks.  The last span of a sequence
@@ -521,7 +505,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
                                                      const __grid_constant__ CUtensorMap map_out,
                                                      const __grid_constant__ WalkArgs a) {
   static_assert(!(DQ && FUSED), "dQ walks over states the forward pass kept");
-  if (threadIdx.x == 0) GTRACE(56);
   constexpr int WX = DQ ? E : D;  // width of X and Y
   constexpr int WZ = DQ ? D : E;  // width of Z and OUT
   extern __shared__ uint8_t smem_raw[];
@@ -608,8 +591,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  if (tid == kFirstWorker) TRACE(0);
-  if (tid == kFirstWorker) GTRACE(57);
   const TmemPair t_s{tmem};
   const uint32_t t_o = tmem + 256, t_l = tmem + 384;
   TileWalk<false> w{a.cut, even_s != 0};
@@ -667,7 +648,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       warp_arrive(&ring_scaled[j]);
     }
     wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);
-    if (tid == kFirstWorker) TRACE(59);
     tc_fence_after_sync();
     const int c0 = half * kHalfE + grp * 32;
     if (row < D && grp * 32 < kHalfE) {
@@ -682,7 +662,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       __threadfence();             // ... and visible to the other CTAs before the flag is
       st_volatile_u32(a.sync + kSyncFlags + blockIdx.x, step_s);
     }
-    if (tid == kFirstWorker) TRACE(60);
   };
   // The three kinds of warps part for good here: each branch sets its registers and is compiled for them.
   if (warp < kFirstWorker / 32) {
@@ -779,7 +758,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (i >= 1) wait_or_fault(&o_free, one ^ 1, &cta, fault, kFaultMmaWait);
           wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 0);
           tc_fence_after_sync();
           if constexpr (!DQ)  // X P: the state tile as [K = d rows] x [N = e columns]
             umma_gemm<false, true, E, D>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false);
@@ -791,7 +769,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           wait_or_fault(&z_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           wait_or_fault(&o2s_ready, one, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 3);
           tc_fence_after_sync();
           umma_gemm_ts<true, WZ, 64>(t_o, t_s[p], smem_u32(sz[p]), C, true);
           umma_commit(&o_full[p]);
@@ -804,7 +781,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&l_free, one ^ 1, &cta, fault, kFaultMmaWait);   // the state update has read the previous L
           wait_or_fault(&ys_ready, one, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 1);
           tc_fence_after_sync();
           if constexpr (!DQ)
             umma_gemm<true, true, E, C>(t_l, smem_u32(sy[p]), C, smem_u32(sz[p]), C, false);
@@ -820,7 +796,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
           wait_or_fault(&y_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 2);
           tc_fence_after_sync();
           umma_gemm<false, false, C, WX>(t_s[p], smem_u32(sx[p]), C, smem_u32(sy[p]), C, false);
           umma_commit(&s_full[p]);
@@ -848,9 +823,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         sl2 = a.s[w.bh % a.h] * kLog2e;
         lam = exp2f(-sl2);
       }
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 0);
       wait_or_fault(&s_full[p], ph, &cta, fault, kFaultMmaWait);
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 1);
       tc_fence_after_sync();
       // masked scores, packed to bf16 in place: they are the A operand of O1 straight from tensor memory
 #pragma unroll 1
@@ -862,7 +835,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&sm_ready[p]);
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 2);
       if (elu && i + 1 < total) map_tile(i + 1, grp);   // the next tile's S can then go out under this tile's work
       // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
       const bool chain = PRE && DQ && (elu || c != 1.f);
@@ -876,7 +848,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       // epilogue: OUT staged in Z's buffer, once L and O1 have read it
       wait_or_fault(&l_full[p], ph, &cta, fault, kFaultMmaWait);
       wait_or_fault(&o_full[p], ph, &cta, fault, kFaultMmaWait);
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 3);
       tc_fence_after_sync();
       if (chain) {
 #pragma unroll 1
@@ -894,10 +865,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       }
       tc_fence_before_sync();
       mbar_arrive(&o_free);
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 4);
       fence_async_smem();
       mbar_arrive(&staged[p]);
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 5);
     }
   } else {
     set_regs_inc<kRegsB>();
@@ -920,12 +889,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       const int len = min(C, a.n - w.t * C);     // tokens really in the tile
       if (w.first_of_item()) sl2 = a.s[w.bh % a.h] * kLog2e;
       wait_or_fault(&s_full[p], ph, &cta, fault, kFaultMmaWait);   // S has read Y
-      if (wid == 0) TRACE_TILE(112, 6, i, 0);
       wait_or_fault(&y_full[p], ph, &cta, fault, kFaultTmaWait);   // completed long ago: makes Y's bytes visible here
       scale_row_pieces<WX / 16>(sy[p], row, half * (WX / 16), c * decay_pow(sl2, max(len - row, 0)), lane);
       fence_async_smem();
       mbar_arrive(&ys_ready);
-      if (wid == 0) TRACE_TILE(112, 6, i, 1);
       if (elu && i + 1 < total) map_tile(i + 1, grp);
       if (__builtin_expect(w.first_of_item(), 0)) {   // once per span: kept out of the tiles' straight-line code
         // the state at the span border; the O2 MMA that read the operand tile of the previous item has completed
@@ -965,7 +932,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
               fma_state<kHalfE, D>(a.totals + (size_t)(w.bh * a.cut.nspans + j) * D * E, row, half * kHalfE,
                                    decay_pow(sl2, (w.t0 - w.span_t0(j + 1)) * C), P);
           }
-          if (wid == 0) TRACE(61);
           if (LINK && a.link.ranks > 0) {
             // hand-over of the rank state inside the launch.  P holds the local part of the border state.
             // The waits for peers below may take longer than any other (a.link.wait_clocks).
@@ -1013,14 +979,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
                 }
               }
             }
-            if (wid == 0) TRACE(62);
             if (a.link.me > 0 && row < D) {
               // what the ranks before this one sent, decayed from the first token of the sequence to the span
               if (!link_receive<kHalfE, D>(a.link, step_x, elems, seq_off, row, half * kHalfE,
                                            decay_pow(sl2, w.t0 * C), P, sn))
                 atomicOr(fault, kFaultRelayWait);
             }
-            if (wid == 0) TRACE(55);
             named_sync(1, kWorkers);
             if (wid == 0) cta.peer_wait_ends();
           }
@@ -1034,7 +998,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       }
       // O2's rows take their decay lambda^row in tensor memory; O1 then accumulates on top
       wait_or_fault(&o2_full[p], ph, &cta, fault, kFaultMmaWait);
-      if (wid == 0) TRACE_TILE(112, 6, i, 2);
       tc_fence_after_sync();
       {
         const float qd = c_o2 * decay_pow(sl2, row);
@@ -1044,10 +1007,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&o2s_ready);
-      if (wid == 0) TRACE_TILE(112, 6, i, 3);
       // state: P <- lambda^len P + L
       wait_or_fault(&l_full[p], ph, &cta, fault, kFaultMmaWait);
-      if (wid == 0) TRACE_TILE(112, 6, i, 4);
       tc_fence_after_sync();
       if (row < D) {
         const float lam_c = decay_pow(sl2, len);
@@ -1065,7 +1026,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       }
       tc_fence_before_sync();
       mbar_arrive(&l_free);
-      if (wid == 0) TRACE_TILE(112, 6, i, 5);
       if (!w.last_of_item()) {
         if (row < D) write_state_operand<kHalfE>(sp, D, row, half * kHalfE, P);
         fence_async_smem();
@@ -1082,8 +1042,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == kFirstWorker) TRACE(63);
-  if (tid == kFirstWorker) { GTRACE(58); TRACE_VAL(54, smid()); }
   if (warp == 2) tmem_dealloc(tmem, 512);
   if constexpr (!DQ) {   // how this pass cut the sequences, for the dQ walk over the border states it leaves
     if (tid == 0 && blockIdx.x == 0 && a.sync != nullptr) st_volatile_u32(a.sync + kSyncEven, even_s);
@@ -1140,7 +1098,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
     const __grid_constant__ CUtensorMap map_dk, const __grid_constant__ CUtensorMap map_dv,
     const __grid_constant__ WalkArgs a) {
-  if (threadIdx.x == 0) GTRACE(56);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   const BufPair sq{smem};
@@ -1221,8 +1178,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  if (tid == kFirstWorker) TRACE(0);
-  if (tid == kFirstWorker) GTRACE(57);
   const uint32_t t_s = tmem, t_ds = tmem + 128, t_dk = tmem + 256, t_dv = tmem + 384;
   TileWalk<true> w{a.cut, a.even != 0};
   // the span-total phase (see k_walk_out): from the span's start onwards, as far as the head's decay reaches
@@ -1263,7 +1218,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       warp_arrive(&ring_scaled[j]);
     }
     wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);
-    if (tid == kFirstWorker) TRACE(59);
     tc_fence_after_sync();
     const int c0 = half * kHalfE + grp * 32;
     if (row < D && grp * 32 < kHalfE) {
@@ -1278,7 +1232,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       __threadfence();             // ... and visible to the other CTAs before the flag is
       st_volatile_u32(a.sync + kSyncFlags + my_item(), step_s);
     }
-    if (tid == kFirstWorker) TRACE(60);
   };
 
   if (warp < kFirstWorker / 32) {
@@ -1372,7 +1325,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&dn_ready, one, &cta, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&e_free, one ^ 1, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 1);
           tc_fence_after_sync();
           umma_gemm<false, false, D, E>(t_dk, smem_u32(sv), C, smem_u32(sdn), D, false);
           umma_gemm<false, true, E, D>(t_dv, smem_u32(sk), C, smem_u32(sdn), D, false);
@@ -1380,7 +1332,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           // the masked scores' products on top, A operands from tensor memory
           wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&scaled, one, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 3);
           tc_fence_after_sync();
           umma_gemm_ts<true, E, 96>(t_dv, t_s, smem_u32(sdo[p]), C, true);    // += S_m^T dO
           wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
@@ -1397,7 +1348,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
           if (E > 64) wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&qs_ready, one, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 2);
           tc_fence_after_sync();
           umma_gemm<true, true, 64, C>(t_s + 32, smem_u32(sdn), C, smem_u32(sdo[p]), C, false);
           if constexpr (E > 64)   // columns 64..127 of dO: its second slab
@@ -1415,7 +1365,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&qdo_full[p], (i >> 1) & 1, &cta, fault, kFaultTmaWait);
           wait_or_fault(&kv_full, one, &cta, fault, kFaultTmaWait);
           if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
-          TRACE_TILE(160, 8, i, 5);
           tc_fence_after_sync();
           umma_gemm<false, false, C, D>(t_s, smem_u32(sk), C, smem_u32(sq[p]), C, false);
           umma_commit(&s_done);
@@ -1443,7 +1392,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         fence_async_smem();
         mbar_arrive(&mapped);
       }
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 0);
       // S_m^T, then dS_m^T (times Q's c): one piece of code for the four blocks of 32 queries.  The second half of the
       // queries goes from right to left, packed against the right end, so that every block is read before it is
       // written over.
@@ -1451,7 +1399,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       for (int u = 0; u < 4; ++u) {
         if ((u & 1) == 0) {
           wait_or_fault(u == 0 ? &s_done : &ds_done, one, &cta, fault, kFaultMmaWait);
-          if (tid == kFirstWorker && u == 0) TRACE_TILE(64, 6, i, 1);
           tc_fence_after_sync();
         }
         const int blk = half == 0 ? (u & 1) : 3 - (u & 1);
@@ -1463,7 +1410,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           tmem_st_wait();
           tc_fence_before_sync();
           mbar_arrive(u == 1 ? &sm_ready : &dsm_ready);
-          if (tid == kFirstWorker) TRACE(i < 8 ? 64 + i * 6 + 2 + (u >> 1) : 999);
         }
       }
       // dk = dk' * c * map'(k), k read from the raw tensor (rows past the end of the sequence are not stored)
@@ -1477,7 +1423,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       // epilogue: dK and dV staged over Q and dO, which every product has read
       wait_or_fault(&l_done, one, &cta, fault, kFaultMmaWait);
       wait_or_fault(&b_done, one, &cta, fault, kFaultMmaWait);
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 4);
       tc_fence_after_sync();
       if (PRE && (elu || c != 1.f)) {
 #pragma unroll 1
@@ -1499,7 +1444,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       mbar_arrive(&e_free);
       fence_async_smem();
       mbar_arrive(&staged[p]);
-      if (tid == kFirstWorker) TRACE_TILE(64, 6, i, 5);
     }
   } else {
     // ---- group B
@@ -1551,7 +1495,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
               fma_state<kHalfE, D>(a.totals + (size_t)(w.bh * a.cut.nspans + j) * D * E, row, half * kHalfE,
                                    decay_pow(sl2, (w.span_t0(j) - w.t1) * C), Dn);
           }
-          if (wid == 0) TRACE(61);
           if (LINK && a.link.ranks > 0) {
             // hand-over of the rank state inside the launch.  Dn holds the local part of the border state.
             // The waits for peers below may take longer than any other (a.link.wait_clocks).
@@ -1622,13 +1565,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         mbar_arrive(&mapped);
       }
       wait_or_fault(&st_done, one, &cta, fault, kFaultMmaWait);
-      if (wid == 0) TRACE_TILE(112, 6, i, 0);
       tc_fence_after_sync();
       // row-scaled copy of Q over the state operand (the state products have read it)
       copy_row_pieces<D / 16>(sdn, sq[p], row, half * (D / 16), c * decay_pow(sl2, row), lane);
       fence_async_smem();
       mbar_arrive(&qs_ready);
-      if (wid == 0) TRACE_TILE(112, 6, i, 1);
       // the two state products take their row decay in place (32 columns at a time, dV's blocks then dK's)
       const float kd = decay_pow(sl2, max(len - row, 0));
 #pragma unroll 1
@@ -1640,10 +1581,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       tmem_st_wait();
       tc_fence_before_sync();
       mbar_arrive(&scaled);
-      if (wid == 0) TRACE_TILE(112, 6, i, 2);
       // state: Dn <- lambda^len Dn + L, this thread's half of the columns being the one in T_S or in T_dS
       wait_or_fault(&l_done, one, &cta, fault, kFaultMmaWait);
-      if (wid == 0) TRACE_TILE(112, 6, i, 3);
       tc_fence_after_sync();
       if (row < D) {
         const float lam_len = decay_pow(sl2, len);
@@ -1666,7 +1605,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         if (row < D) write_state_operand<kHalfE>(sdn, D, row, half * kHalfE, Dn);
         fence_async_smem();
         mbar_arrive(&dn_ready);
-        if (wid == 0) TRACE_TILE(112, 6, i, 4);
       } else if constexpr (FUSED) {
         // the state after the first tile of the sequence is the outgoing rank state
         if (a.x_out != nullptr && w.t == 0 && row < D) {
@@ -1679,8 +1617,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (tid == kFirstWorker) TRACE(63);
-  if (tid == kFirstWorker) { GTRACE(58); TRACE_VAL(54, smid()); }
   if (warp == 2) tmem_dealloc(tmem, 512);
   if constexpr (FUSED) {
     if (tid == 0 && a.coop) {
@@ -1701,22 +1637,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// once per kernel and device (the attribute call costs the host about as much as a launch)
-template <auto fn>
-cudaError_t opt_in_smem(size_t bytes) {
-  static bool done[64] = {};
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err == cudaSuccess && dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  if (err == cudaSuccess)
-    err = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (err != cudaSuccess)
-    g_failed_step = "cudaFuncSetAttribute(max dynamic shared memory)";
-  else if (dev >= 0 && dev < 64)
-    done[dev] = true;
-  return err;
-}
-
 cudaError_t seq_map(CUtensorMap* map, const void* base, const Dims& m, int width, int pitch, const char* what) {
   cudaError_t err = make_seq_tile_map(map, base, (uint64_t)m.b * m.h, (uint64_t)m.n, (uint32_t)width, C, (uint32_t)pitch);
   if (err != cudaSuccess) {
@@ -1968,11 +1888,5 @@ cudaError_t walk_bwd_dkv_fused(const Dims& m, const void* q, const void* k, cons
   LASP_DISPATCH_DE(m, LASP_CALL);
 #undef LASP_CALL
 }
-
-#ifdef LASP_TRACE
-extern "C" __attribute__((visibility("default"))) int lasp_b200_debug_trace(long long* host) {
-  return (int)cudaMemcpyFromSymbol(host, g_trace, sizeof(long long) * 160 * kTraceSlots);
-}
-#endif
 
 }  // namespace lasp

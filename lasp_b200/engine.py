@@ -43,6 +43,8 @@ class Plan:
 
     @property
     def path_name(self) -> str:
+        """"simt" is the full-precision path, by the name that the interface has for it: its kernels run on the tensor
+        cores too (csrc/split_kernels.cu)."""
         return "tensor" if self.path == _cabi.PATH_TENSOR else "simt"
 
 
@@ -119,7 +121,7 @@ def make_plan(b: int, h: int, n: int, d: int, e: int, dtype: torch.dtype, path: 
     """``qk_scale`` / ``feature_map`` ("elu1"): the operator is evaluated on qk_scale * map(q), qk_scale * map(k)
     inside the kernels (lasp_problem.qk_map, .qk_scale); raises LaspStatusError when the problem's kernels
     cannot do that.  ``pitch_d`` / ``pitch_e``: row pitch in elements of q,k,dq,dk / v,o,do,dv when they are slices
-    of the head dimension of wider tensors (0: tensors of their own); tensor-core path only."""
+    of the head dimension of wider tensors (0: tensors of their own)."""
     if dtype not in _DTYPES:
         raise TypeError(f"unsupported dtype {dtype}; use float32, bfloat16 or float16")
     name = path or default_path()
