@@ -490,7 +490,7 @@ __device__ __forceinline__ void write_state_operand(uint8_t* tile, int rows, int
 //
 // FUSED = false: the state of every span at its border comes from the scan (a.p0).
 // FUSED = true : one launch does everything.  With more than one span per sequence every CTA has
-//   exactly one span (one CTA per SM at most; each waits for lower block indexes only).  It first sums its own span,
+//   exactly one span (one CTA per SM at most; each waits for the totals of lower block indexes only).  It first sums its own span,
 //   T = sum_c lambda^(span end - c) k_c v_c^T, streaming K and V once through a ring of stages, writes
 //   T to global memory and raises a flag; then it adds up the totals of the spans before it (and the
 //   incoming rank state) with their decays - that is its border state - and walks.  The last span of a sequence
