@@ -129,7 +129,8 @@ def _slice_plan(q, v, wd, we, qk_scale, feature_map, in_place):
 
 
 def _slices_in_place(q, v, qk_scale, feature_map) -> bool:
-    """True when every (q/k slice, v slice) pair of these head dimensions can run on the wide tensors in place."""
+    """True when every (q/k slice, v slice) pair of these head dimensions can run on the wide tensors in place: what the
+    native operator relies on, asked of the plans (csrc/torch_ops.cpp makes the slices itself)."""
     try:
         for d0, d1 in _cuts(q.shape[-1]):
             for e0, e1 in _cuts(v.shape[-1]):
