@@ -85,3 +85,40 @@ def test_saved_tensors_that_are_not_what_they_were_are_refused(change):
             return change(t.view(1, 1, 1, -1) if kind == 1 else t)
         with pytest.raises((RuntimeError, TypeError, ValueError), match="saved"):
             _gradients_through(lambda t: t, back)
+
+
+def test_calls_on_several_streams_at_once():
+    """Threads with a stream each: the CTAs of their launches share the SMs, every launch has its own synchronisation words,
+    and the results are those of the calls one after the other."""
+    import threading
+    from lasp_b200 import engine, lightning_attn
+    shapes = [(2, 12, 2048, 128), (1, 40, 1500, 64), (1, 4, 4096, 128)]
+
+    def inputs(i, rep):
+        b, h, n, d = shapes[i]
+        g = torch.Generator(device=DEV).manual_seed(100 * i + rep)
+        t = [torch.randn(b, h, n, d, generator=g, device=DEV).to(torch.bfloat16) for _ in range(4)]
+        return [x.requires_grad_(j < 3) for j, x in enumerate(t)], torch.full((h, 1, 1), 0.002, device=DEV)
+
+    def call(t, s):
+        o = lightning_attn(*t[:3], s)
+        return [o.detach(), *torch.autograd.grad(o, t[:3], t[3])]
+
+    sets = [[inputs(i, rep) for rep in range(4)] for i in range(len(shapes))]
+    want = [[call(*x) for x in s] for s in sets]
+    got = [[None] * 12 for _ in shapes]
+    torch.cuda.synchronize()
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for k in range(12):
+                got[i][k] = call(*sets[i][k % 4])
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(shapes))]
+    [t.start() for t in threads], [t.join() for t in threads]
+    assert engine.read_status() == 0
+    for i in range(len(shapes)):
+        for k in range(12):
+            for a, b in zip(got[i][k], want[i][k % 4]):
+                assert torch.equal(a, b), (shapes[i], k)
