@@ -126,7 +126,10 @@ int make_dims(const lasp_problem* p, lasp::Dims* m) {
 
 size_t workspace_bytes(const lasp::Dims& m) {
   size_t s = lasp::state_elems(m);
-  if (!m.walk) s = (size_t)m.b * m.h * ((m.n + lasp::kAbiChunk - 1) / lasp::kAbiChunk) * m.d * m.e;
+  if (!m.walk) {   // (two of the ABI's chunks at least: one of the kernels' own)
+    const int chunks = (m.n + lasp::kAbiChunk - 1) / lasp::kAbiChunk;
+    s = (size_t)m.b * m.h * (chunks > 2 ? chunks : 2) * m.d * m.e;
+  }
   size_t bytes = 2 * s * 4;  // local + prefix states
   if (m.walk) bytes += lasp::kWalkSyncBytes;
   return (bytes + 255) & ~(size_t)255;
@@ -241,7 +244,7 @@ int fwd_output(const lasp::Dims& m, const lasp_fwd_args* a, const lasp_call_opti
     return cuda_fail(lasp::walk_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_walk_border(a->ws, m),
                                            opt.sync ? opt.sync : lasp::ws_walk_sync(a->ws), a->o,
                                            (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
-  return cuda_fail(lasp::split_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_prefix(a->ws, m), a->o, opt.alone != 0,
+  return cuda_fail(lasp::split_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_split_prefix(a->ws), a->o, opt.alone != 0,
                                           (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
 }
 
@@ -268,8 +271,8 @@ int bwd_grads(const lasp::Dims& m, const lasp_bwd_args* a, const lasp_call_optio
     return cuda_fail(lasp::walk_bwd_dkv(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->ws, m), a->dk,
                                         a->dv, add_qk, add_v, cs));
   }
-  return cuda_fail(lasp::split_bwd_grads(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_prefix(a->fwd_ws, m),
-                                         lasp::ws_prefix(a->ws, m), a->dq, a->dk, a->dv, opt.alone != 0,
+  return cuda_fail(lasp::split_bwd_grads(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_split_prefix(a->fwd_ws),
+                                         lasp::ws_split_prefix(a->ws), a->dq, a->dk, a->dv, opt.alone != 0,
                                          (opt.accumulate & LASP_ACCUMULATE_QK) != 0,
                                          (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
 }

@@ -13,8 +13,10 @@ namespace lasp {
 // and nc the number of states kept per sequence.  The chunk-state phase writes
 // the LOCAL states, the scan reads them and writes the PREFIX states (exclusive,
 // seeded with the incoming rank state) that the output / gradient kernels read:
-//   FULL PRECISION : one state per 128-token chunk, fp32:
-//                      [0, S*4) prefix states, [S*4, 2*S*4) local states
+//   FULL PRECISION : one state per 128-token chunk, row-major:
+//                      [0, S*6) prefix states, each as the three bf16 matrices that its terms make up
+//                               (state_terms.cuh), as the output kernels' tensor-core operands need them
+//                      [S*6, S*10) local states, fp32
 //   TENSOR path      : one state per SPAN of `span` 128-token tiles (a few per
 //                      sequence; inside a span the state lives on chip):
 //                      [0, 4096)            words the CTAs of the fused kernels
@@ -25,8 +27,8 @@ namespace lasp {
 // The running prefix inside the scan is always fp32.
 constexpr int kTensorTile = 128;  // one tcgen05 M=128 tile
 constexpr int kAbiChunk = 64;     // the reference's block size: the unit in which the C ABI states the chunks of the
-                                  // full-precision path and sizes its workspace.  The kernels' chunks are two of these,
-                                  // so they use half of it; the sizes are part of the interface and stay.
+                                  // full-precision path and sizes its workspace (8 bytes per element of a state; the
+                                  // kernels use 10 per chunk of their own, which are two of these)
 
 struct Dims {
   int b, h, n, d, e;
@@ -49,7 +51,7 @@ int sm_count();
 
 inline size_t state_elems(const Dims& m) { return (size_t)m.b * m.h * m.nc * m.d * m.e; }
 
-// The states in a workspace are kept in "lane order": the float4 holding
+// The states of the tensor path in a workspace are kept in "lane order": the float4 holding
 // columns 4g..4g+3 of row r of a d x e state sits at float4 index g*d + r, so that the 32 rows a warp
 // owns are contiguous for each of its accesses.  Rank states handed in and out by the caller stay
 // row-major.
@@ -67,16 +69,13 @@ inline float* ws_walk_border(void* ws, const Dims& m) {
 inline const float* ws_walk_border(const void* ws, const Dims& m) {
   return reinterpret_cast<const float*>(static_cast<const char*>(ws) + kWalkSyncBytes + state_elems(m) * 4);
 }
-// where the chunk-state phase writes / where the scan writes and the output kernels read
+// where the chunk-state phase writes / where the scan writes and the output kernels read (fp32 on the tensor path, terms
+// on the full-precision path)
 inline float* ws_local(void* ws, const Dims& m) {
-  return m.walk ? ws_walk_totals(ws) : reinterpret_cast<float*>(static_cast<char*>(ws) + state_elems(m) * 4);
+  return m.walk ? ws_walk_totals(ws) : reinterpret_cast<float*>(static_cast<char*>(ws) + state_elems(m) * 6);
 }
-inline float* ws_prefix(void* ws, const Dims& m) {
-  return m.walk ? ws_walk_border(ws, m) : reinterpret_cast<float*>(ws);
-}
-inline const float* ws_prefix(const void* ws, const Dims& m) {
-  return m.walk ? ws_walk_border(ws, m) : reinterpret_cast<const float*>(ws);
-}
+inline void* ws_prefix(void* ws, const Dims& m) { return m.walk ? ws_walk_border(ws, m) : ws; }
+inline const void* ws_split_prefix(const void* ws) { return ws; }
 // bits of the sticky per-device fault word (fault_word.cu owns the word)
 enum : int32_t {
   kFaultNone = 0,
@@ -115,17 +114,17 @@ cudaError_t opt_in_smem(size_t bytes) {
 cudaError_t split_chunk_states(const Dims& m, const void* a, const void* bten, const float* s, float* states,
                                bool backward, bool alone, cudaStream_t st);
 cudaError_t split_fwd_output(const Dims& m, const void* q, const void* k, const void* v, const float* s,
-                             const float* prefix, void* o, bool alone, bool add_o, cudaStream_t st);
+                             const void* prefix, void* o, bool alone, bool add_o, cudaStream_t st);
 cudaError_t split_bwd_grads(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, const float* s,
-                            const float* prefix, const float* suffix, void* dq, void* dk, void* dv, bool alone,
+                            const void* prefix, const void* suffix, void* dq, void* dk, void* dv, bool alone,
                             bool add_qk, bool add_v, cudaStream_t st);
-cudaError_t scan_states(const Dims& m, const float* s, const float* local, float* prefix, const float* x_in,
+cudaError_t scan_states(const Dims& m, const float* s, const float* local, void* prefix, const float* x_in,
                         float* x_out, bool reverse, cudaStream_t st);
 cudaError_t state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
                           const float* x_local, float* x_out, cudaStream_t st);
 
 // state relay (relay_kernels.cu)
-cudaError_t exchange_scan(const Dims& m, const lasp_exchange_args& a, const float* local, float* prefix,
+cudaError_t exchange_scan(const Dims& m, const lasp_exchange_args& a, const float* local, void* prefix,
                           cudaStream_t st);
 
 // tcgen05 path

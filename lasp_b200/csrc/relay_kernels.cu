@@ -21,6 +21,7 @@
 // kFaultRelayWait in the fault word and makes the prefix states it writes NaN.
 #include "common.cuh"
 #include "exchange_layout.h"
+#include "state_terms.cuh"
 
 namespace lasp {
 
@@ -59,7 +60,8 @@ __device__ __forceinline__ bool wait_flag(const uint32_t* flag, uint32_t want, l
 
 struct ExchangeParams {
   const float* local;           // (b,h,nc,d*e) chunk states of this rank (read by both halves of the launch)
-  float* prefix;                // (b,h,nc,d*e) out: exclusive prefix states seeded with the incoming rank state
+  void* prefix;                 // (b,h,nc,d*e) out: exclusive prefix states seeded with the incoming rank state
+  int terms;                    // ... as terms (full-precision path) instead of fp32
   const float* s;               // h decay rates
   const uint2* my_slots;        // local: slots[parity][source][element] of {value, step} words
   uint32_t* src_acks[kMaxRanks];    // peer: ack words [me][slice] in each source's memory
@@ -185,7 +187,7 @@ __global__ void __launch_bounds__(256) k_exchange_scan(const ExchangeParams p) {
       // exclusive scan of the local chunk states seeded with it
       const long long bh = el / p.de;
       const float* base = p.local + (size_t)bh * p.nc * p.de + (el - bh * p.de);
-      float* out = p.prefix + (size_t)bh * p.nc * p.de + (el - bh * p.de);
+      const size_t at = (size_t)(el - bh * p.de);
       const float full = expf(-sh * (float)p.chunk), tail = expf(-sh * (float)last_len);
       constexpr int kBatch = 8;
       for (int i0 = 0; i0 < p.nc; i0 += kBatch) {
@@ -198,7 +200,11 @@ __global__ void __launch_bounds__(256) k_exchange_scan(const ExchangeParams p) {
           if (i0 + u < p.nc) {
             const int c = p.reverse ? p.nc - 1 - (i0 + u) : i0 + u;
             const float dec = (c == p.nc - 1) ? tail : full;
-            *reinterpret_cast<float4*>(out + (size_t)c * p.de) = acc;
+            const size_t state = (size_t)bh * p.nc + c;
+            if (p.terms)
+              store_state_terms(static_cast<__nv_bfloat16*>(p.prefix) + state * 3 * p.de, at, p.de, acc);
+            else
+              *reinterpret_cast<float4*>(static_cast<float*>(p.prefix) + state * p.de + at) = acc;
             acc.x = fmaf(dec, acc.x, loc[u].x), acc.y = fmaf(dec, acc.y, loc[u].y);
             acc.z = fmaf(dec, acc.z, loc[u].z), acc.w = fmaf(dec, acc.w, loc[u].w);
           }
@@ -227,11 +233,12 @@ __global__ void __launch_bounds__(256) k_exchange_scan(const ExchangeParams p) {
 
 }  // namespace
 
-cudaError_t exchange_scan(const Dims& m, const lasp_exchange_args& a, const float* local, float* prefix,
+cudaError_t exchange_scan(const Dims& m, const lasp_exchange_args& a, const float* local, void* prefix,
                           cudaStream_t st) {
   ExchangeParams p;
   p.local = local;
   p.prefix = prefix;
+  p.terms = m.walk ? 0 : 1;
   p.s = a.s;
   p.my_slots = static_cast<const uint2*>(a.my_slots);
   p.my_acks = a.my_acks;

@@ -15,19 +15,26 @@
 //
 // Sequences are cut into 128-token chunks (the last one ragged), everything in parallel over chunks:
 //   k_split_states  T = sum_c w_c a_c b_c^T of every chunk                       (a,b = k,v or q,do)
-//   k_scan          the states at the chunk borders
+//   k_scan          the states at the chunk borders, in terms
 //   k_split_out     OUT = (X Y^T . M) Z + diag(w) X op(P)
 // k_split_out is all of the output kernels: (X,Y,Z,op(P)) = (Q,K,V,P) gives O, (dO,V,K,P^T) dQ, (V,dO,Q,Dn^T) dK and
 // (K,Q,dO,Dn) dV, the last two with the mask transposed; the backward pass runs the three as one launch.  Computing
 // the scores once per result costs one product in nine and makes every chunk three independent tasks.
 //
-// One B200, b=2, h=12, n=2048, forward / backward, before (a CTA of 256 FFMA threads per 64-token chunk) and now:
-// fp32 d=e=128 730 / 1421 -> 82 / 154 us, fp16 d=128, e=64 365 / 869 -> 48 / 86 us, bf16 d=e=96 363 / 920 -> 44 / 79 us;
-// the error against fp64, relative to theirs: fp16 and bf16 results 1.00, rank states of all types 0.5 to 0.97, fp32 results
-// 0.65 to 0.97 of 1.3e-7 to 3.2e-7, but for o and dv without decay beyond a chunk, 1.0 to 1.18 of 1.3e-7 to 1.8e-7 (sums
-// of numbers of one sign, which the tensor cores' accumulation rounds towards zero; the same calls' dq and dk: 0.8).
+// What bounds them: fp32, the shared memory between the fillers' stores and the products (an SS product of 128 x 128 reads
+// 128 bytes a clock, all there is: 48 of a task's 144 MMAs take 87 clocks with A in tensor memory, the others 105 to 125 of
+// 64); 16-bit types, the chain scores - mask - O1 of a task.  In step instead of in roles (sixteen warps loading,
+// splitting, storing and meeting at barriers, results written 16 bytes of 32 rows at a time, the states split once per
+// product) a dQ, dK or dV task of fp32 took 32000 clocks, now 22000; of bf16 16000, now 8400.
+//
+// One B200, b=2, h=12, n=2048, forward / backward in us, in step and now: fp32 d=e=128 82.7 / 160 -> 70.6 / 119, fp16 d=128, e=64
+// 47.8 / 90 -> 43.0 / 68, fp16 d=e=128 57.7 / 111 -> 53.5 / 78, bf16 d=e=96 44.3 / 83 -> 36.9 / 53.  The error against
+// fp64, relative to what it was then: fp32 results 0.79 to 0.87, rank states of all types 0.61 to 0.87, fp16 and bf16 results 1.00
+// (a chunk of 64 elements of K is summed in an accumulator of its own, and the tensor cores' additions round towards zero).
 #include <type_traits>
+#include <utility>
 
+#include "state_terms.cuh"
 #include "tc_common.cuh"
 
 namespace lasp {
@@ -35,8 +42,13 @@ namespace {
 
 using namespace tc;
 
-constexpr int NT = 512;           // sixteen worker warps, one of whose threads issues the MMAs
-constexpr int kPieces = 4;        // 8-element pieces of a 128 x 128 tile per thread
+// Warps in four roles, by warpgroups: control (one warp issues the MMAs, one the TMA loads), readers of the accumulators
+// (mask, split, epilogue), and fillers, which load, split and store operand chunks (two groups of them in the chunk-state
+// kernel, one per chunk).
+constexpr int kFillers = 256;     // threads of one group
+constexpr int kUnit = 16384;      // one term of a chunk: 128 x 64 or 64 x 128 bf16
+constexpr int kBox = 8192;        // what one TMA load brings: 64 x 64
+constexpr int kPieces = 4;        // 8-element pieces of a chunk per filling thread
 
 // terms of the inputs and of intermediate quantities, and the largest i + j of a product that is kept
 template <typename T> struct Terms;
@@ -48,8 +60,6 @@ template <> struct Terms<__nv_bfloat16> { static constexpr int in = 1, mid = 3, 
 template <typename T> struct Raw { uint4 v; };
 template <> struct Raw<float> { uint4 v, w; };
 
-template <typename T> __device__ __forceinline__ void zero_raw(Raw<T>& r) { r.v = make_uint4(0u, 0u, 0u, 0u); }
-template <> __device__ __forceinline__ void zero_raw<float>(Raw<float>& r) { r.v = r.w = make_uint4(0u, 0u, 0u, 0u); }
 __device__ __forceinline__ uint4 ld_nc(const void* p) { return __ldg(static_cast<const uint4*>(p)); }
 template <typename T> __device__ __forceinline__ void load_piece(Raw<T>& r, const T* p) { r.v = ld_nc(p); }
 template <> __device__ __forceinline__ void load_piece<float>(Raw<float>& r, const float* p) {
@@ -87,145 +97,123 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t (&t)[N])
   }
 }
 
-// the terms of eight elements of row `row` from column `col` on, into the operand tiles (one per term,
-// `stride` bytes apart, `rows` rows each)
-template <int N>
-__device__ __forceinline__ void store_terms(uint8_t* tiles, uint32_t stride, int row, int col, int rows, const float (&x)[8]) {
-  uint32_t t[4][N];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) split_pair<N>(x[2 * j], x[2 * j + 1], t[j]);
-  const uint32_t off = tile_offset(row, col, rows);
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-    *reinterpret_cast<uint4*>(tiles + i * stride + off) = make_uint4(t[0][i], t[1][i], t[2][i], t[3][i]);
-}
-
-__device__ __forceinline__ int padded(int w) { return w <= 64 ? 64 : 128; }
-
-// A 128 x wp tile (wp = 64 or 128; rows >= len and columns >= w read as zero): piece p of the tile is row p / (wp/8),
-// columns 8 (p mod wp/8) on, so that a warp reads whole rows and its shared-memory stores hit every bank once.
+// A chunk is 64 elements of a product's K dimension of one operand, all its terms, in units of 16 KB: 128 rows of a
+// K-major operand (X, Y, P^T) or 64 rows of an MN-major one (A, B, Z, P).  States' terms, and 16-bit tiles where they enter
+// a product as they are, come by TMA; everything else through the fillers.  Piece p of a filled chunk is eight elements of
+// a row; pieces run along the rows, so that a warp reads whole rows and its shared-memory stores hit every bank once.
+struct Chunk {
+  const char* src;     // this thread's first piece
+  uint32_t stride;     // bytes from one of its pieces to the next
+  int row0, drow;      // rows of its pieces
+  int col;             // their columns, in eights
+  int rows, live, cols;   // rows of the chunk, those from `live` on being zero; columns in eights
+};
 template <typename T>
-__device__ __forceinline__ void load_tile(Raw<T> (&r)[kPieces], const T* base, int pitch, int len, int w, int wp, int tid) {
-  const int sh = wp == 128 ? 4 : 3;
-#pragma unroll
-  for (int i = 0; i < kPieces; ++i) {
-    const int p = tid + NT * i, row = p >> sh, col = (p & ((1 << sh) - 1)) * 8;
-    zero_raw<T>(r[i]);
-    if (row < len && col < w) load_piece<T>(r[i], base + (size_t)row * pitch + col);
-  }
+__device__ __forceinline__ Chunk tensor_chunk(const T* p, int pitch, int rows, int live, int cols, bool wide, int tid) {
+  const int sh = wide ? 4 : 3, row0 = tid >> sh, col = tid & ((1 << sh) - 1), drow = kFillers >> sh;
+  return {reinterpret_cast<const char*>(p + (size_t)row0 * pitch + 8 * col), (uint32_t)(drow * pitch * (int)sizeof(T)), row0, drow, col, rows, live,
+          cols / 8};
 }
-// ... its terms in shared memory, row `row` multiplied by wt(row) first
-template <typename T, int N, bool WEIGHTED, typename W>
-__device__ __forceinline__ void store_tile(uint8_t* tiles, const Raw<T> (&r)[kPieces], int wp, int tid, W wt) {
-  const int sh = wp == 128 ? 4 : 3;
+
+template <typename T>
+struct RawChunk {   // a thread's pieces on their way
+  Raw<T> piece[kPieces];
+};
+template <typename T>
+__device__ __forceinline__ void load_chunk_piece(RawChunk<T>& r, const Chunk& c, int i) {
+  Raw<T>& e = r.piece[i];
+  e.v = make_uint4(0u, 0u, 0u, 0u);
+  if constexpr (std::is_same<T, float>::value) e.w = e.v;
+  if (c.row0 + i * c.drow < c.live && c.col < c.cols) load_piece<T>(e, reinterpret_cast<const T*>(c.src + (size_t)i * c.stride));
+}
+struct NoWeight {};
+// ... N terms of them in shared memory, units of 16 KB from `units` on, row `row` multiplied by wt(row).  The registers of a
+// piece that is stored take the next chunk's: next(i).
+template <typename T, int N, typename F, typename W = NoWeight>
+__device__ __forceinline__ void store_chunk(uint8_t* units, const RawChunk<T>& r, const Chunk& c, F next, W wt = W()) {
 #pragma unroll
   for (int i = 0; i < kPieces; ++i) {
-    const int p = tid + NT * i, row = p >> sh, col = (p & ((1 << sh) - 1)) * 8;
-    if (row >= C) break;
-    if constexpr (N == 1 && !WEIGHTED) {
-      *reinterpret_cast<uint4*>(tiles + tile_offset(row, col, C)) = r[i].v;   // bf16 is its own only term
-    } else {
+    const int row = c.row0 + i * c.drow;
+    if (row < c.rows && c.col < c.cols) {
+      uint8_t* dst = units + tile_offset(row, 8 * c.col, c.rows);
       float x[8];
-      to_floats<T>(r[i], x);
-      if constexpr (WEIGHTED) {
+      to_floats<T>(r.piece[i], x);
+      if constexpr (!std::is_same<W, NoWeight>::value) {
         const float f = wt(row);
 #pragma unroll
         for (int j = 0; j < 8; ++j) x[j] *= f;
       }
-      store_terms<N>(tiles, C * wp * 2, row, col, C, x);
-    }
-  }
-}
-struct NoWeight {};
-// ... as it is, a 16-bit type
-template <typename T>
-__device__ __forceinline__ void store_raw(uint8_t* tile, const Raw<T> (&r)[kPieces], int wp, int tid) {
-  const int sh = wp == 128 ? 4 : 3;
+      uint32_t t[4][N];
 #pragma unroll
-  for (int i = 0; i < kPieces; ++i) {
-    const int p = tid + NT * i, row = p >> sh, col = (p & ((1 << sh) - 1)) * 8;
-    if (row >= C) break;
-    *reinterpret_cast<uint4*>(tile + tile_offset(row, col, C)) = r[i].v;
+      for (int j = 0; j < 4; ++j) split_pair<N>(x[2 * j], x[2 * j + 1], t[j]);
+#pragma unroll
+      for (int k = 0; k < N; ++k) *reinterpret_cast<uint4*>(dst + k * kUnit) = make_uint4(t[0][k], t[1][k], t[2][k], t[3][k]);
+    }
+    next(i);
   }
 }
 
-// a d x e state in lane order (common.cuh), padded to dp x ep: piece p is row p mod dp, columns 8 (p / dp) on
-__device__ __forceinline__ void load_state(Raw<float> (&r)[kPieces], const float* state, int d, int e, int dp, int ep, int tid) {
-  const int sh = dp == 128 ? 7 : 6;
-#pragma unroll
-  for (int i = 0; i < kPieces; ++i) {
-    const int p = tid + NT * i, row = p & (dp - 1), g = p >> sh;   // columns 8 g .. 8 g + 7
-    zero_raw<float>(r[i]);
-    if (row < d && 8 * g < e) {
-      const float4* src = reinterpret_cast<const float4*>(state) + (size_t)(2 * g) * d + row;
-      r[i].v = ld_nc(src), r[i].w = ld_nc(src + d);
-    }
-  }
-}
-template <int N>
-__device__ __forceinline__ void store_state_terms(uint8_t* tiles, const Raw<float> (&r)[kPieces], int dp, int ep, int tid) {
-  const int sh = dp == 128 ? 7 : 6;
-#pragma unroll
-  for (int i = 0; i < kPieces; ++i) {
-    const int p = tid + NT * i, row = p & (dp - 1), g = p >> sh;
-    if (8 * g >= ep) break;
-    float x[8];
-    to_floats<float>(r[i], x);
-    store_terms<N>(tiles, dp * ep * 2, row, 8 * g, dp, x);
-  }
-}
-
-// One operand of a product in shared memory: its terms lie `stride` bytes apart.
+// One operand of a product over a chunk: descriptors of its terms (16 KB apart) and of the steps of 16 K elements
 struct TermOperand {
-  uint32_t addr, stride, rows;
-  bool mn_major;
-  __device__ __forceinline__ SmemDesc desc(int term) const { return operand_desc(addr + term * stride, rows, mn_major); }
+  SmemDesc first;
+  uint32_t step;   // in units of 16 bytes
+  __device__ __forceinline__ TermOperand(uint32_t addr, uint32_t rows, bool mn_major)
+      : first(operand_desc(addr, rows, mn_major)), step(mn_major ? 128 : 2) {}
+  __device__ __forceinline__ SmemDesc desc(int term, int ks) const { return {first.lo + term * (kUnit / 16) + ks * step, first.hi}; }
 };
-// D[128 x n] = A B: every kept product of terms, the smallest first; issued by one thread
-template <int NA, int NB, int CUT, bool FP16 = false>
-__device__ __forceinline__ void issue_terms(uint32_t d_tmem, const TermOperand& a, const TermOperand& b, uint32_t n, int ksteps) {
-  const uint32_t idesc = umma_idesc(128, n, a.mn_major, b.mn_major, FP16);
-  uint32_t acc = 0;
+// The masked scores' terms in tensor memory, as the readers leave them: K step ks of terms 0 and 1 in the columns of t_s
+// that held the step's sixteen scores, of term 2 in those of t_lo
+struct ScoreOperand {
+  uint32_t t_s, t_lo;
+  __device__ __forceinline__ uint32_t addr(int term, int ks) const { return (term == 2 ? t_lo : t_s + 8 * term) + 16 * ks; }
+};
+// The products of terms whose indexes sum to FROM, FROM - 1, ..., TO, over one chunk.  A whole warp computes what the
+// instructions take (uniform values, so that they live in uniform registers), its lane `leader` issues them.  (One thread
+// in loops took 155 clocks for an MMA of 64, the warp unrolled 100 to 125 with lane 0 as the leader, less with an elected
+// one; the warp in loops 10 % longer for the whole kernel.)
+template <int NA, int NB, int FROM, int TO, typename A>
+__device__ __forceinline__ void issue_terms(uint32_t d_tmem, const A& a, const TermOperand& b, uint32_t idesc, int ksteps, uint32_t& acc,
+                                            bool leader) {
 #pragma unroll
-  for (int sum = CUT; sum >= 0; --sum) {
+  for (int sum = FROM; sum >= TO; --sum) {
 #pragma unroll
     for (int i = 0; i < NA; ++i) {
       const int j = sum - i;
       if (j < 0 || j >= NB) continue;
-      const SmemDesc da = a.desc(i), db = b.desc(j);
-#pragma unroll 1
-      for (int kq = 0; kq < ksteps / 4; ++kq) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          umma(d_tmem, operand_step(da, a.rows, a.mn_major, 4 * kq + u), operand_step(db, b.rows, b.mn_major, 4 * kq + u), idesc, acc);
+      for (int ks = 0; ks < 4; ++ks) {
+        if (ks < ksteps) {
+          if constexpr (std::is_same<A, ScoreOperand>::value)
+            umma_ts(d_tmem, a.addr(i, ks), b.desc(j, ks), idesc, acc, leader);
+          else
+            umma(d_tmem, a.desc(i, ks), b.desc(j, ks), idesc, acc, leader);
           acc = 1;
         }
       }
     }
   }
 }
-// the same with A's terms in tensor memory as mask_terms leaves them: K step ks of terms 0 and 1 in the 32-column block
-// ks / 2 of t_s, of term 2 in t_lo
-template <int NA, int NB, int CUT>
-__device__ __forceinline__ void issue_terms_ts(uint32_t d_tmem, uint32_t t_s, uint32_t t_lo, const TermOperand& b, uint32_t n) {
-  const uint32_t idesc = umma_idesc(128, n, false, b.mn_major);
-  uint32_t acc = 0;
+__device__ __forceinline__ int ksteps_of(int width, int chunk) { return max(min(width - 64 * chunk, 64), 0) / 16; }
+// the same value in every lane, and known to be so
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// Four 16-byte pieces of a row in each of four neighbouring lanes change hands so that piece i of every lane belongs to the
+// i-th of the four rows: stored piece by piece, four lanes then write 64 bytes of one row.  (As they are, the 32 lanes of a
+// store write 16 bytes of 32 rows, a cache line each: 64 KB of results took the load-store unit 5600 clocks, in which the
+// filling warps' loads stood still too.)
+__device__ __forceinline__ void rows_to_lanes(uint4 (&v)[4], int lane) {
 #pragma unroll
-  for (int sum = CUT; sum >= 0; --sum) {
+  for (int s = 1; s <= 2; s *= 2) {
+    const bool high = lane & s;
 #pragma unroll
-    for (int i = 0; i < NA; ++i) {
-      const int j = sum - i;
-      if (j < 0 || j >= NB) continue;
-      const SmemDesc db = b.desc(j);
-#pragma unroll 1
-      for (int kq = 0; kq < C / 64; ++kq) {
+    for (int u = 0; u < 2; ++u) {
+      const int i = s == 1 ? 2 * u : u, j = i + s;   // the pair of pieces of which this lane keeps one and sends the other
+      uint32_t* a = reinterpret_cast<uint32_t*>(&v[i]);
+      uint32_t* b = reinterpret_cast<uint32_t*>(&v[j]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int ks = 4 * kq + u;
-          const uint32_t ta = i == 2 ? t_lo + 8 * ks : t_s + 32 * (ks >> 1) + 8 * (ks & 1) + 16 * i;
-          umma_ts(d_tmem, ta, operand_step(db, b.rows, b.mn_major, ks), idesc, acc);
-          acc = 1;
-        }
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? a[q] : b[q], s);
+        (high ? a[q] : b[q]) = got;
       }
     }
   }
@@ -252,10 +240,10 @@ __device__ __forceinline__ float to_float(__half x) { return __half2float(x); }
 __device__ __forceinline__ float to_float(__nv_bfloat16 x) { return __bfloat162float(x); }
 
 // ---------------------------------------------------------------------------
-// chunk states: T[i][j] = sum_c w_c A[c][i] B[c][j], in lane order
+// chunk states: T[i][j] = sum_c w_c A[c][i] B[c][j], row-major
 //   forward : A = K, B = V,  w_c = lambda^(len-c);   backward: A = Q, B = dO, w_c = lambda^c
-// A task per chunk, persistent CTAs; the next chunk's rows are on their way while the products of this one run.
-// Bound by the loads' latency and the splitting arithmetic (one CTA per SM: 192 KB of operand terms for fp32).
+// A task per chunk of the sequence, persistent CTAs.  The 64 tokens of a chunk of the operands are summed in an accumulator
+// of their own, so that the next task's can follow at once; the readers add the two.
 // ---------------------------------------------------------------------------
 struct StateArgs {
   const void *a, *b;
@@ -266,6 +254,8 @@ struct StateArgs {
   int32_t* fault;
 };
 
+constexpr int kStateReaders = 256, kStateThreads = 128 + kStateReaders + 2 * kFillers;
+
 // The elements of a task's state that are not finite, again
 template <typename T>
 __device__ __forceinline__ void plain_state(const StateArgs& g, int task) {
@@ -274,8 +264,8 @@ __device__ __forceinline__ void plain_state(const StateArgs& g, int task) {
   const T *a = static_cast<const T*>(g.a) + tok * g.pitch_a, *b = static_cast<const T*>(g.b) + tok * g.pitch_b;
   const float sh = g.s[bh % g.h];
   float4* state = reinterpret_cast<float4*>(g.states + (size_t)task * g.d * g.e);
-  for (int p = threadIdx.x; p < g.d * g.e / 4; p += NT) {   // four columns of a row, in lane order
-    const int row = p % g.d, col = p / g.d * 4;
+  for (int p = threadIdx.x - 128; p < g.d * g.e / 4; p += kStateThreads - 128) {   // four columns of a row
+    const int row = p / (g.e / 4), col = p % (g.e / 4) * 4;
     const float4 old = state[p];
     if (isfinite(old.x + old.y + old.z + old.w)) continue;
     float y[4] = {0.f, 0.f, 0.f, 0.f};
@@ -289,84 +279,173 @@ __device__ __forceinline__ void plain_state(const StateArgs& g, int task) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
+struct StatePlan {   // units of 16 KB: A's chunk, then B's, of the first 64 tokens and of the others
+  static constexpr int kChunk = Terms<T>::mid + Terms<T>::in;
+  static constexpr size_t kSmem = (size_t)2 * kChunk * kUnit + 1024;
+  static constexpr bool kTmaB = Terms<T>::in == 1;   // bf16 is its own only term
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kStateThreads, 1) k_split_states(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ StateArgs g) {
   using TT = Terms<T>;
+  using Plan = StatePlan<T>;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t done;
+  __shared__ uint64_t full_a[2], full_b[2], done[2], result[2], acc_free[2];   // by chunk; result, acc_free: by the task's parity
   __shared__ uint32_t tmem_slot;
   __shared__ Health<false> cta;
   __shared__ int look_again;   // a state with an element that is not finite has been written
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int dp = padded(g.d), ep = padded(g.e);
-  uint8_t* sa = align1024(smem_raw);
-  uint8_t* sb = sa + TT::mid * C * dp * 2;   // (with dp = 64 the M = 128 MMA reads on from A into B: valid memory)
+  const int tid = threadIdx.x, warp = (int)uniform(tid >> 5), lane = tid & 31;
+  uint8_t* smem = align1024(smem_raw);
   if (tid == 0) {
     cta.word = look_again = 0;
-    mbar_init(&done, 1);
+    for (int j = 0; j < 2; ++j) {
+      mbar_init(&full_a[j], kFillers / 32);
+      mbar_init(&full_b[j], Plan::kTmaB ? 1 : kFillers / 32);
+      mbar_init(&done[j], 1), mbar_init(&result[j], 1), mbar_init(&acc_free[j], kStateReaders / 32);
+    }
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(&tmem_slot, 128);
+  if (warp == 2) tmem_alloc(&tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = tmem_slot;
-  const int row_l = (warp & 3) * 32 + lane;
-  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-
-  Raw<T> ra[kPieces], rb[kPieces];
-  const auto fetch = [&](int task) {
-    const int bh = task / g.nc, chunk = task - bh * g.nc, len = min(C, g.n - chunk * C);
-    const size_t tok = (size_t)bh * g.n + (size_t)chunk * C;
-    load_tile<T>(ra, static_cast<const T*>(g.a) + tok * g.pitch_a, g.pitch_a, len, g.d, dp, tid);
-    load_tile<T>(rb, static_cast<const T*>(g.b) + tok * g.pitch_b, g.pitch_b, len, g.e, ep, tid);
+  const uint32_t tmem = tmem_slot;   // [parity of the task][chunk], 128 columns each
+  const auto next_task = [&](int t) {
+    while (t < g.tasks && t % g.nc == g.skip) t += gridDim.x;
+    return t;
   };
-  const auto skipped = [&](int task) { return task % g.nc == g.skip; };
-  int task = blockIdx.x;
-  while (task < g.tasks && skipped(task)) task += gridDim.x;
-  if (task < g.tasks) fetch(task);
-  for (int it = 0; task < g.tasks; ++it) {
-    const int bh = task / g.nc, chunk = task - bh * g.nc, len = min(C, g.n - chunk * C);
-    const float sh = g.s[bh % g.h];
-    const bool backward = g.backward != 0;
-    store_tile<T, TT::mid, true>(sa, ra, dp, tid, [&](int row) {
-      return expf(-sh * (float)(backward ? row : max(len - row, 0)));
-    });
-    store_tile<T, TT::in, false>(sb, rb, ep, tid, NoWeight());
-    fence_async_smem();
-    tc_fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after_sync();
-      issue_terms<TT::mid, TT::in, TT::cut>(tmem, TermOperand{smem_u32(sa), (uint32_t)(C * dp * 2), C, true},
-                                            TermOperand{smem_u32(sb), (uint32_t)(C * ep * 2), C, true}, ep, C / 16);
-      umma_commit(&done);
-    }
-    int next = task + gridDim.x;
-    while (next < g.tasks && skipped(next)) next += gridDim.x;
-    if (next < g.tasks) fetch(next);
-    wait_or_fault(&done, it & 1, &cta, g.fault, kFaultMmaWait);
-    tc_fence_after_sync();
-    float4* out = reinterpret_cast<float4*>(g.states + (size_t)task * g.d * g.e);
-    const int per = ep / 4;   // columns of this warp's group
+
+  if (warp < 4) {
+    set_regs_dec<40>();
+    if (warp == 0) {
+      const uint32_t idesc = umma_idesc(128, g.e, true, true), base = uniform(smem_u32(smem)), t_acc = uniform(tmem);
+      const bool leader = elect_one();
+      int it = 0;
+      for (int t = next_task(blockIdx.x); t < g.tasks; t = next_task(t + gridDim.x), ++it) {
+        const int len = min(C, g.n - (t % g.nc) * C);
+        if (it >= 2) wait_or_fault(&acc_free[it & 1], ((it >> 1) - 1) & 1, &cta, g.fault, kFaultMmaWait);
 #pragma unroll 1
-    for (int c0 = (warp >> 2) * per; c0 < ((warp >> 2) + 1) * per; c0 += 16) {
-      uint32_t r[16];
-      tmem_ld16(tmem + lane_base + c0, r);
-      tmem_ld_wait();
-      if (row_l < g.d && c0 < g.e) {
-        if (!all_finite(r)) look_again = 1;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          out[(size_t)(c0 / 4 + q) * g.d + row_l] = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
-                                                               __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+        for (int c = 0; c < 2; ++c) {
+          wait_or_fault(&full_a[c], it & 1, &cta, g.fault, kFaultTmaWait);
+          wait_or_fault(&full_b[c], it & 1, &cta, g.fault, kFaultTmaWait);
+          __syncwarp();
+          tc_fence_after_sync();
+          const uint32_t at = base + c * Plan::kChunk * kUnit;
+          uint32_t acc = 0;
+          issue_terms<TT::mid, TT::in, TT::cut, 0>(t_acc + 256 * (it & 1) + 128 * c, TermOperand(at, 64, true),
+                                                   TermOperand(at + TT::mid * kUnit, 64, true), idesc, ksteps_of(len + 15, c), acc, leader);
+          if (leader) umma_commit(&done[c]);
+        }
+        if (leader) umma_commit(&result[it & 1]);
+        __syncwarp();
+      }
+    } else if (Plan::kTmaB && warp == 1 && lane == 0) {
+      int it = 0;
+      for (int t = next_task(blockIdx.x); t < g.tasks; t = next_task(t + gridDim.x), ++it) {
+        const int bh = t / g.nc, chunk = t - bh * g.nc, slabs = g.e > 64 ? 2 : 1;
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          if (it > 0) wait_or_fault(&done[c], (it - 1) & 1, &cta, g.fault, kFaultMmaWait);
+          mbar_expect_tx(&full_b[c], slabs * kBox);
+          for (int u = 0; u < slabs; ++u)
+            tma_load_3d(smem_u32(smem) + (c * Plan::kChunk + TT::mid) * kUnit + u * kBox, &map_b, &full_b[c], 64 * u, chunk * C + 64 * c, bh);
+        }
       }
     }
-    task = next;
+  } else if (warp < 4 + kStateReaders / 32) {
+    set_regs_inc<88>();
+    const int row = (warp & 3) * 32 + lane, half = (warp >> 2) & 1;   // tensor-memory lanes and columns of this warp
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    int it = 0;
+    for (int t = next_task(blockIdx.x); t < g.tasks; t = next_task(t + gridDim.x), ++it) {
+      const uint32_t acc = tmem + 256 * (it & 1) + lane_base;
+      wait_or_fault(&result[it & 1], (it >> 1) & 1, &cta, g.fault, kFaultMmaWait);
+      __syncwarp();
+      tc_fence_after_sync();
+      const bool two = g.n - (t % g.nc) * C > 64;   // tokens in the second chunk
+      float* out = g.states + ((size_t)t * g.d + (row & ~3)) * g.e + 4 * (lane & 3);
+#pragma unroll 1
+      for (int c0 = 16 * half; c0 < g.e; c0 += 32) {
+        uint32_t r[16], r2[16];
+        tmem_ld16(acc + c0, r);
+        if (two) tmem_ld16(acc + 128 + c0, r2);
+        tmem_ld_wait();
+        if (two) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(r2[j]));
+        }
+        if (row < g.d && !all_finite(r)) look_again = 1;
+        uint4 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+        rows_to_lanes(v, lane);
+        if (row < g.d) {   // (widths are multiples of 16: four neighbouring rows exist together)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(out + (size_t)i * g.e + c0) = v[i];
+        }
+      }
+      tc_fence_before_sync();
+      warp_arrive(&acc_free[it & 1]);
+    }
+  } else {
+    const int c = warp >= 4 + (kStateReaders + kFillers) / 32 ? 1 : 0, ft = tid & (kFillers - 1);   // this group's chunk
+    struct Task {
+      int len;
+      size_t tok;
+      float sh;
+    };
+    const auto task_of = [&](int t) {
+      const int bh = t / g.nc, chunk = t - bh * g.nc;
+      return Task{min(C, g.n - chunk * C), (size_t)bh * g.n + (size_t)chunk * C, g.s[bh % g.h]};
+    };
+    const auto chunk_of = [&](const Task& k, bool is_b) {
+      const int w = is_b ? g.e : g.d, pitch = is_b ? g.pitch_b : g.pitch_a;
+      return tensor_chunk<T>(static_cast<const T*>(is_b ? g.b : g.a) + (k.tok + 64 * c) * pitch, pitch, 64, k.len - 64 * c, w, w > 64, ft);
+    };
+    int t = next_task(blockIdx.x), it = 0;
+    bool is_b = false;
+    if (t < g.tasks) {
+      Task k = task_of(t);
+      Chunk cur = chunk_of(k, false);
+      RawChunk<T> r;
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) load_chunk_piece<T>(r, cur, i);
+      while (true) {
+        const int prev = it - 1, len = k.len;
+        const float sh = k.sh;
+        const bool b_now = is_b;
+        if (Plan::kTmaB || is_b) {
+          is_b = false, ++it;
+          t = next_task(t + gridDim.x);
+          if (t < g.tasks) k = task_of(t);
+        } else {
+          is_b = true;
+        }
+        Chunk next = chunk_of(k, is_b);
+        if (t >= g.tasks) next.cols = 0;
+        if (prev >= 0 && !b_now) wait_or_fault(&done[c], prev & 1, &cta, g.fault, kFaultMmaWait);
+        const auto load_next = [&](int i) { load_chunk_piece<T>(r, next, i); };
+        uint8_t* units = smem + c * Plan::kChunk * kUnit;
+        if (b_now) {
+          store_chunk<T, TT::in>(units + TT::mid * kUnit, r, cur, load_next);
+        } else {
+          const bool backward = g.backward != 0;
+          store_chunk<T, TT::mid>(units, r, cur, load_next, [&](int row) {
+            return expf(-sh * (float)(backward ? 64 * c + row : max(len - 64 * c - row, 0)));
+          });
+        }
+        fence_async_smem();
+        warp_arrive(b_now ? &full_b[c] : &full_a[c]);
+        if (t >= g.tasks) break;
+        cur = next;
+      }
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 128);
-  if (look_again) {   // (after the loop, whose registers hold the next chunk's rows)
+  if (warp == 2) tmem_dealloc(tmem, 512);
+  // (after the loops, whose registers hold the next chunk's rows; the control warps have given theirs away)
+  if (look_again && warp >= 4) {
     for (int u = blockIdx.x; u < g.tasks; u += gridDim.x)
       if (u % g.nc != g.skip) plain_state<T>(g, u);
   }
@@ -375,15 +454,77 @@ __global__ void __launch_bounds__(NT, 1) k_split_states(const StateArgs g) {
 // ---------------------------------------------------------------------------
 // outputs: OUT = (X Y^T . M) Z + diag(w) X op(P)
 //   rev = 0: M_ij = lambda^(i-j) [i >= j], w_i = lambda^i;   rev = 1: M_ij = lambda^(j-i) [j >= i], w_i = lambda^(len-i)
-// Tensor memory: S (terms 0 and 1 of the masked scores over S itself), its term 2, the two products.  Shared memory:
-// two sets of term tiles, X then Z in the first, Y (fp16: Y and X as they are) then P in the second.  A task's steps, each product running
-// under the next step's work (the loads of a step are issued one step earlier):
-//   S = X Y^T | P's terms | O2 = X P | mask, split S; Z's terms | O1 = S_m Z | next task's Y, X terms | next S | epilogue
+// A task - one result of one chunk of the sequence - is up to eight chunks of operands (two of X, Y, P and Z each) and
+// three products:
+//   S = X Y^T (an accumulator per chunk) | O2 = X op(P), while the readers mask and split S | O1 = S_m Z
+// and under the next task's S the readers write OUT.  All of it meets at mbarriers, one phase per task each; every chunk
+// is announced for every task, also one that the task has no use for, so that no barrier gets two phases ahead of a waiter.
 // ---------------------------------------------------------------------------
+enum Kind { kX0, kX1, kY0, kY1, kP0, kP1, kZ0, kZ1 };
+enum Done { kS0, kS, kO2, kO1 };   // products of a task that have read their operands: S of chunk 0, S, O2, O1
+constexpr int kPrev = 4, kAny = 8;  // (of the task before; whatever the same warps have waited for before)
+
+// Where a chunk lies (in units of 16 KB) and what has to have read the chunk that was there before; fill_*: of what the
+// fillers store, where a tile also comes as it is.
+template <typename T> struct OutPlan;
+// fp32: 192 KB hold X and Y and nothing else, so P follows Y, Z follows X and P, and the places of the next task's X and Y are
+// those that are free first: it has them the other way round.
+template <> struct OutPlan<float> {
+  static constexpr int kUnits = 12, kTurn = 6, kReaders = 256, kReaderRegs = 112, kControlRegs = 64;
+  static constexpr bool kFillXZ = true, kFillY = true, kRawXY = false;
+  static constexpr uint32_t kFills = 6, kFillOrder = kX0 | kY0 << 4 | kX1 << 8 | kY1 << 12 | kZ0 << 16 | kZ1 << 20;
+  static constexpr int place(int kind) {
+    return kind == kX0 || kind == kZ0 ? 0 : kind == kX1 ? 6 : kind == kY1 || kind == kP1 ? 9 : 3;
+  }
+  static constexpr int after(int kind) {
+    return kind == kX0 ? kO2 + kPrev : kind == kX1 ? kO1 + kPrev : kind == kP0 ? kS0 : kind == kP1 ? kS : kind == kZ0 || kind == kZ1 ? kO2 : kAny;
+  }
+  static constexpr int fill_place(int kind) { return place(kind); }
+  static constexpr int fill_after(int kind) { return after(kind); }
+};
+// fp16: X as it is, X in two terms, Y as it is, P; Z follows X and Y as they are, which only the scores need
+template <> struct OutPlan<__half> {
+  static constexpr int kUnits = 14, kTurn = 0, kReaders = 256, kReaderRegs = 112, kControlRegs = 64;
+  static constexpr bool kFillXZ = true, kFillY = false, kRawXY = true;
+  static constexpr uint32_t kFills = 4, kFillOrder = kX0 | kX1 << 4 | kZ0 << 8 | kZ1 << 12;
+  static constexpr int place(int kind) {
+    return kind == kX0 || kind == kZ0 ? 0 : kind == kX1 ? 1 : kind == kY0 || kind == kZ1 ? 2 : kind == kY1 ? 3 : kind == kP0 ? 8 : 11;
+  }
+  static constexpr int fill_place(int kind) { return kind == kX0 ? 4 : kind == kX1 ? 6 : place(kind); }
+  static constexpr int after(int kind) { return kind == kX0 ? kO1 + kPrev : kind == kP0 ? kO2 + kPrev : kind == kZ0 || kind == kZ1 ? kS : kAny; }
+  static constexpr int fill_after(int kind) { return kind == kX0 || kind == kX1 ? kO2 + kPrev : kS; }
+};
+// bf16: room for everything
+template <> struct OutPlan<__nv_bfloat16> {
+  static constexpr int kUnits = 12, kTurn = 0, kReaders = 512, kReaderRegs = 104, kControlRegs = 64;
+  static constexpr bool kFillXZ = false, kFillY = false, kRawXY = true;
+  static constexpr int place(int kind) { return kind <= kP0 ? kind : kind == kP1 ? 7 : kind == kZ0 ? 10 : 11; }
+  static constexpr int after(int kind) { return kind == kX0 ? kO2 + kPrev : kind == kZ0 ? kO1 + kPrev : kAny; }
+  static constexpr int fill_place(int kind) { return place(kind); }
+};
+template <typename T>
+constexpr int kOutThreads = 128 + OutPlan<T>::kReaders + (OutPlan<T>::kFillXZ ? kFillers : 0);
+// (looked up at run time: the eight values of a function, four bits each, in a constant)
+template <int (*F)(int)>
+constexpr uint32_t packed_plan() {
+  uint32_t v = 0;
+  for (int k = 0; k < 8; ++k) v |= (uint32_t)F(k) << (4 * k);
+  return v;
+}
+template <int (*F)(int)>
+struct PackedPlan {
+  static constexpr uint32_t value = packed_plan<F>();
+};
+template <int (*F)(int)>
+__device__ __forceinline__ int plan_at(int k) {
+  return (int)(PackedPlan<F>::value >> (4 * k)) & 15;
+}
+
 struct OutRole {
   const void *x, *y, *z;
   void* out;
-  const float* state;      // border states of the chunks in lane order; NULL: all zero
+  const __nv_bfloat16* state;   // border states of the chunks in terms; NULL: all zero
+  int mx, my, mz, mp;      // their tensor maps
   int wx, wz, pitch_x, pitch_z;
   int transposed;          // op(P) = P^T
   int rev;
@@ -394,8 +535,11 @@ struct OutArgs {
   OutRole role[3];
   const float* s;
   int roles, h, n, nc, tasks, d, e;
-  uint32_t set_bytes;      // bytes of the first set of term tiles
   int32_t* fault;
+};
+enum Map { kMapQ, kMapK, kMapV, kMapDo, kMapPrefix, kMapSuffix, kMaps };
+struct OutMaps {
+  CUtensorMap m[kMaps];
 };
 
 __device__ __forceinline__ void put16(float* p, const float (&x)[16], bool add) {
@@ -477,11 +621,12 @@ __device__ __noinline__ void plain_out(const OutArgs* g, int t, int row, int col
       }
     }
     if (!settled && r.state != nullptr && chunk != r.zero_chunk) {
-      const float* p = r.state + ((size_t)bh * g->nc + chunk) * g->d * g->e;   // lane order (common.cuh)
+      const size_t elems = (size_t)g->d * g->e;
+      const __nv_bfloat16* p = r.state + ((size_t)bh * g->nc + chunk) * 3 * elems;
       for (int i = 0; i < r.wx; ++i) {
         for (int j = 0; j < 16; ++j) {
           const int pr = r.transposed ? col + j : i, pc = r.transposed ? i : col + j;
-          inter[j] = fmaf(to_float(x[i]), p[((size_t)(pc / 4) * g->d + pr) * 4 + pc % 4], inter[j]);
+          inter[j] = fmaf(to_float(x[i]), state_of_terms(p, (size_t)pr * g->e + pc, elems), inter[j]);
         }
       }
       const float w_row = expf(-sh * (float)(r.rev ? len - row : row));
@@ -497,7 +642,7 @@ __device__ __noinline__ void plain_out_where_needed(const OutArgs* g, int t) {
   const OutRole& r = g->role[t % g->roles];
   const int u = t / g->roles, bh = u / g->nc, chunk = u - bh * g->nc, len = min(C, g->n - chunk * C);
   const size_t tok = (size_t)bh * g->n + (size_t)chunk * C;
-  for (int p = threadIdx.x; p < C * (r.wz / 16); p += NT) {
+  for (int p = threadIdx.x - 128; p < C * (r.wz / 16); p += blockDim.x - 128) {
     const int row = p % C, col = p / C * 16;
     if (row >= len) continue;
     const T* out = static_cast<const T*>(r.out) + (tok + row) * r.pitch_z + col;
@@ -508,262 +653,423 @@ __device__ __noinline__ void plain_out_where_needed(const OutArgs* g, int t) {
 }
 
 template <typename T, bool ADD>
-__global__ void __launch_bounds__(NT, 1) k_split_out(const __grid_constant__ OutArgs g) {
+__global__ void __launch_bounds__(kOutThreads<T>, 1) k_split_out(const __grid_constant__ OutMaps maps, const __grid_constant__ OutArgs g) {
   using TT = Terms<T>;
+  using Plan = OutPlan<T>;
+  constexpr bool kRawScores = std::is_same<T, __half>::value;   // S of fp16 tiles is one product of the tiles as they are
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t s_done, o2_done, o1_done;
+  __shared__ uint64_t full[8], done[4], sm_ready, acc_free;
   __shared__ uint32_t tmem_slot;
   __shared__ Health<false> cta;
   __shared__ int look_again;   // a result that is not finite has been written
-  __shared__ float decay[C + 1];   // lambda^0 .. lambda^128 of the task's head
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int dp = padded(g.d), ep = padded(g.e);
-  uint8_t* set_a = align1024(smem_raw);
-  uint8_t* set_b = set_a + g.set_bytes;
+  // What the scores of a block of 32 columns on the diagonal take: line[k] = lambda^(31 - k) up to k = 31 and 0 beyond (the
+  // transposed mask: lambda^(k - 31) from k = 31 on and 0 before), of which row r of the block starts at 31 - r.  Four
+  // copies shifted by 0 to 3 elements, so that every row reads 16 bytes at a time, and as far apart as keeps eight
+  // neighbouring rows on different banks.  (With a look-up and a comparison for every element a block on the diagonal took
+  // 2300 clocks, one beside it 600.)
+  __shared__ __align__(16) float line[4][72];
+  __shared__ OutArgs args;   // (for the functions that are called: a parameter whose address is taken is not read as one)
+  const int tid = threadIdx.x, warp = (int)uniform(tid >> 5), lane = tid & 31;
+  uint8_t* smem = align1024(smem_raw);
   if (tid == 0) {
     cta.word = look_again = 0;
-    mbar_init(&s_done, 1);
-    mbar_init(&o2_done, 1);
-    mbar_init(&o1_done, 1);
+    for (int j = 0; j < 8; ++j) {
+      const bool filled = j < kY0 || j >= kZ0 ? Plan::kFillXZ : j < kP0 ? Plan::kFillY : false;
+      const bool loaded = j >= kP0 && j < kZ0 ? true : j >= kZ0 ? !Plan::kFillXZ : Plan::kRawXY;
+      mbar_init(&full[j], (filled ? kFillers / 32 : 0) + (loaded ? 1 : 0));
+    }
+    for (int j = 0; j < 4; ++j) mbar_init(&done[j], 1);
+    mbar_init(&sm_ready, Plan::kReaders / 32);
+    mbar_init(&acc_free, Plan::kReaders / 32);
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(&tmem_slot, 512);
+  if (tid == 32) args = g;
+  if (warp == 2) tmem_alloc(&tmem_slot, 512);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  const uint32_t t_s = tmem, t_lo = tmem + 128, t_o1 = tmem + 192, t_o2 = tmem + 320;
-  const int quarter = warp & 3, group = warp >> 2;     // tensor-memory lanes and columns of this warp
-  const int row_l = quarter * 32 + lane;
-  const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-  const uint32_t addr_a = smem_u32(set_a), addr_b = smem_u32(set_b);
 
   struct Task {
-    const OutRole* r;
+    OutRole r;
     int bh, chunk, len;
     size_t tok;
-    float sh;
     bool has_state;
   };
   const auto task_of = [&](int t) {
     Task k;
-    k.r = &g.role[t % g.roles];
+    k.r = g.role[t % g.roles];
     const int u = t / g.roles;
     k.bh = u / g.nc, k.chunk = u - k.bh * g.nc;
     k.len = min(C, g.n - k.chunk * C);
     k.tok = (size_t)k.bh * g.n + (size_t)k.chunk * C;
-    k.sh = g.s[k.bh % g.h];
-    k.has_state = k.r->state != nullptr && k.chunk != k.r->zero_chunk;
+    k.has_state = k.r.state != nullptr && k.chunk != k.r.zero_chunk;
     return k;
   };
-  const auto load_xy = [&](Raw<T> (&dst)[kPieces], const void* p, const Task& k) {
-    load_tile<T>(dst, static_cast<const T*>(p) + k.tok * k.r->pitch_x, k.r->pitch_x, k.len, k.r->wx, padded(k.r->wx), tid);
+  const auto turned = [&](int unit, int it) {
+    return Plan::kTurn && (it & 1) ? (unit >= Plan::kTurn ? unit - Plan::kTurn : unit + Plan::kTurn) : unit;
   };
-  // the scores' operands: Y and, for fp16, X as they are in the second set, X's terms in the first
-  constexpr bool kRawScores = std::is_same<T, __half>::value;
-  const auto store_y = [&](const Raw<T> (&ry)[kPieces], const Raw<T> (&rx)[kPieces], int wx) {
-    if constexpr (kRawScores) {
-      store_raw<T>(set_b, ry, wx, tid);
-      store_raw<T>(set_b + C * wx * 2, rx, wx, tid);
-    } else {
-      store_tile<T, TT::in, false>(set_b, ry, wx, tid, NoWeight());
-    }
-  };
-  const auto issue_s = [&](const Task& k) {
-    const int wx = padded(k.r->wx);
-    tc_fence_after_sync();
-    if constexpr (kRawScores)
-      issue_terms<1, 1, 0, true>(t_s, TermOperand{addr_b + (uint32_t)(C * wx * 2), 0, C, false}, TermOperand{addr_b, 0, C, false}, C,
-                                 wx / 16);
-    else
-      issue_terms<TT::in, TT::in, TT::cut>(t_s, TermOperand{addr_a, (uint32_t)(C * wx * 2), C, false},
-                                           TermOperand{addr_b, (uint32_t)(C * wx * 2), C, false}, C, wx / 16);
-    umma_commit(&s_done);
+  // (dep: what was in the place of a chunk of the CTA's task `it` has been read)
+  const auto await_place = [&](int dep, int it) {
+    const int of = dep == kAny ? -1 : it - (dep >> 2);
+    if (of >= 0) wait_or_fault(&done[dep & 3], of & 1, &cta, g.fault, kFaultMmaWait);
   };
 
-  int t = blockIdx.x;
-  if (t < g.tasks) {
-    Task k = task_of(t);
-    {
-      Raw<T> rx[kPieces], ry[kPieces];
-      load_xy(rx, k.r->x, k);
-      load_xy(ry, k.r->y, k);
-      if (tid <= C) decay[tid] = expf(-k.sh * (float)tid);
-      store_y(ry, rx, padded(k.r->wx));
-      store_tile<T, TT::in, false>(set_a, rx, padded(k.r->wx), tid, NoWeight());
-    }
-    fence_async_smem();
-    __syncthreads();
-    if (tid == 0) issue_s(k);
-    int o2_uses = 0;
-    for (int it = 0;; ++it) {
-      const int wx = padded(k.r->wx), wz = padded(k.r->wz);
-      const float w_row = decay[k.r->rev ? max(k.len - row_l, 0) : row_l];
-      // ---- P's terms over Y (the scores have read it), O2 = X op(P)
-      if (k.has_state) {
-        Raw<float> rp[kPieces];
-        load_state(rp, k.r->state + ((size_t)k.bh * g.nc + k.chunk) * g.d * g.e, g.d, g.e, dp, ep, tid);
-        wait_or_fault(&s_done, it & 1, &cta, g.fault, kFaultMmaWait);
-        store_state_terms<TT::mid>(set_b, rp, dp, ep, tid);
-        fence_async_smem();
-        tc_fence_before_sync();
-        __syncthreads();
-        if (tid == 0) {
+  if (warp < 4) {
+    set_regs_dec<Plan::kControlRegs>();
+    if (warp == 0) {
+      const bool leader = elect_one();
+      const uint32_t base = uniform(smem_u32(smem)), tm = uniform(tmem);
+      const uint32_t t_s = tm, t_s1 = tm + 128, t_o1 = tm + 256, t_o2 = tm + 384;
+      int it = 0;
+      for (int t = blockIdx.x; t < g.tasks; t += gridDim.x, ++it) {
+        const Task k = task_of(t);
+        const OutRole& r = k.r;
+        const auto await = [&](int kind) {
+          wait_or_fault(&full[kind], it & 1, &cta, g.fault, kFaultTmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          issue_terms<TT::in, TT::mid, TT::cut>(t_o2, TermOperand{addr_a, (uint32_t)(C * wx * 2), C, false},
-                                                TermOperand{addr_b, (uint32_t)(dp * ep * 2), (uint32_t)dp, k.r->transposed == 0},
-                                                wz, wx / 16);
-          umma_commit(&o2_done);
+        };
+        const auto addr = [&](int kind) { return base + turned(plan_at<Plan::place>(kind), it) * kUnit; };
+        const auto addr_terms = [&](int kind) { return base + turned(plan_at<Plan::fill_place>(kind), it) * kUnit; };
+        const int chunks = r.wx > 64 ? 2 : 1;
+        // S; its accumulators hold the masked scores of the task before until O1 has read them
+        if (it > 0) wait_or_fault(&done[kO1], (it - 1) & 1, &cta, g.fault, kFaultMmaWait);
+        const uint32_t idesc_s = umma_idesc(128, C, false, false, kRawScores);
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          await(kX0 + c);
+          await(kY0 + c);
+          if (c < chunks) {
+            uint32_t acc = 0;
+            constexpr int kIn = kRawScores ? 1 : TT::in, kCut = kIn == 1 ? 0 : TT::cut;
+            issue_terms<kIn, kIn, kCut, 0>(c ? t_s1 : t_s, TermOperand(addr(kX0 + c), C, false), TermOperand(addr(kY0 + c), C, false),
+                                           idesc_s, ksteps_of(r.wx, c), acc, leader);
+          }
+          if (leader) umma_commit(&done[c ? kS : kS0]);
         }
-      } else {
-        wait_or_fault(&s_done, it & 1, &cta, g.fault, kFaultMmaWait);
-      }
-      // ---- the masked scores' terms, Z's terms over X, O1 = S_m Z
-      {
-        Raw<T> rz[kPieces];
-        load_tile<T>(rz, static_cast<const T*>(k.r->z) + k.tok * k.r->pitch_z, k.r->pitch_z, k.len, k.r->wz, wz, tid);
-        tc_fence_after_sync();
+        // O2: the smaller products of both chunks, then the largest
+        if (it > 0) wait_or_fault(&acc_free, (it - 1) & 1, &cta, g.fault, kFaultMmaWait);
         {
-          uint32_t hi[16], mid[16], lo[16];
-          const bool none = k.r->rev ? group < quarter : group > quarter;   // the block is all masked (as every lane sees it)
-          if (none) {
+          const bool p_mn = r.transposed == 0;
+          const uint32_t idesc = umma_idesc(128, r.wz, false, p_mn);
+          const int p_rows = p_mn ? 64 : g.d, o2_chunks = k.has_state ? chunks : 0;
+          uint32_t acc = 0;
+#pragma unroll 1
+          for (int c = 0; c < 2; ++c) {
+            await(kP0 + c);
+            if (c < o2_chunks) issue_terms<TT::in, TT::mid, TT::cut, 1>(t_o2, TermOperand(addr_terms(kX0 + c), C, false),
+                                                     TermOperand(addr(kP0 + c), p_rows, p_mn), idesc, ksteps_of(r.wx, c), acc, leader);
+          }
+#pragma unroll 1
+          for (int c = 0; c < o2_chunks; ++c)
+            issue_terms<1, 1, 0, 0>(t_o2, TermOperand(addr_terms(kX0 + c), C, false), TermOperand(addr(kP0 + c), p_rows, p_mn), idesc,
+                                    ksteps_of(r.wx, c), acc, leader);
+        }
+        if (leader) umma_commit(&done[kO2]);
+        // O1
+        wait_or_fault(&sm_ready, it & 1, &cta, g.fault, kFaultMmaWait);
+        {
+          const uint32_t idesc = umma_idesc(128, r.wz, false, true);
+          uint32_t acc = 0;
+          const int zs = k.len > 64 ? 2 : 1;
+#pragma unroll 1
+          for (int c = 0; c < 2; ++c) {
+            await(kZ0 + c);
+            if (c < zs) issue_terms<TT::mid, TT::in, TT::cut, 1>(t_o1, ScoreOperand{t_s + 64 * c, t_s1 + 64 * c}, TermOperand(addr_terms(kZ0 + c), 64, true),
+                                                     idesc, 4, acc, leader);
+          }
+#pragma unroll 1
+          for (int c = 0; c < zs; ++c)
+            issue_terms<1, 1, 0, 0>(t_o1, ScoreOperand{t_s + 64 * c, t_s1 + 64 * c}, TermOperand(addr_terms(kZ0 + c), 64, true), idesc, 4, acc, leader);
+        }
+        if (leader) umma_commit(&done[kO1]);
+        __syncwarp();
+      }
+    } else if (warp == 1 && lane == 0) {
+      // ---- TMA: states' terms, tiles that enter a product as they are
+      int it = 0;
+      for (int t = blockIdx.x; t < g.tasks; t += gridDim.x, ++it) {
+        const Task k = task_of(t);
+        const OutRole& r = k.r;
+        const auto load = [&](int kind, int map, int c0, int rows, int matrix, int row_step, int boxes, int terms) {
+          // `boxes` boxes that lie one behind the other, 64 rows or 64 columns further each, of every term
+          await_place(plan_at<Plan::after>(kind), it);
+          if (boxes == 0) {
+            mbar_arrive(&full[kind]);
+            return;
+          }
+          mbar_expect_tx(&full[kind], boxes * terms * kBox);
+          const uint32_t at = smem_u32(smem) + turned(plan_at<Plan::place>(kind), it) * kUnit;
+          for (int i = 0; i < terms; ++i)
+            for (int u = 0; u < boxes; ++u)
+              tma_load_3d(at + i * kUnit + u * kBox, &maps.m[map], &full[kind], c0 + (64 - row_step) * u, rows + row_step * u, matrix + i);
+        };
+        const int row0 = k.chunk * C, state = 3 * (k.bh * g.nc + k.chunk);
+        const auto load_xy = [&] {
+#pragma unroll 1
+          for (int u = 0; u < 4; ++u) {
+            const int c = u & 1;
+            load((u < 2 ? kX0 : kY0) + c, u < 2 ? r.mx : r.my, 64 * c, row0, k.bh, 64, r.wx > 64 * c ? 2 : 0, 1);
+          }
+        };
+        if (Plan::kRawXY && !Plan::kFillXZ) load_xy();
+#pragma unroll 1
+        for (int c = 0; c < 2; ++c) {
+          const bool live = k.has_state && r.wx > 64 * c;
+          if (r.transposed)
+            load(kP0 + c, r.mp, 64 * c, 0, state, 64, live ? (g.d > 64 ? 2 : 1) : 0, 3);
+          else
+            load(kP0 + c, r.mp, 0, 64 * c, state, 0, live ? (g.e > 64 ? 2 : 1) : 0, 3);
+        }
+        if (Plan::kRawXY && Plan::kFillXZ) load_xy();   // (fp16: they wait for more than P does)
+        if (!Plan::kFillXZ) {
+#pragma unroll 1
+          for (int c = 0; c < 2; ++c) load(kZ0 + c, r.mz, 0, row0 + 64 * c, k.bh, 0, k.len > 64 * c ? (r.wz > 64 ? 2 : 1) : 0, 1);
+        }
+      }
+    }
+  } else if (warp < 4 + Plan::kReaders / 32) {
+    set_regs_inc<Plan::kReaderRegs>();
+    const uint32_t t_s = tmem, t_s1 = tmem + 128, t_o1 = tmem + 256, t_o2 = tmem + 384;
+    const int rid = tid - 128, quarter = warp & 3, part = (rid >> 7);   // tensor-memory lanes and columns of this warp
+    constexpr int kParts = Plan::kReaders / 128;
+    const int row = quarter * 32 + lane;
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const auto decay_of = [&](int t) { return g.s[t / g.roles / g.nc % g.h]; };
+    const auto write_line = [&](int t) {
+      if (rid < 256) {
+        const int k = (rid & 63) + (rid >> 6), dist = g.role[t % g.roles].rev ? k - 31 : 31 - k;
+        line[rid >> 6][rid & 63] = dist >= 0 ? expf(-decay_of(t) * (float)dist) : 0.f;
+      }
+    };
+    write_line(blockIdx.x);
+    int it = 0;
+    for (int t = blockIdx.x; t < g.tasks; t += gridDim.x, ++it) {
+      const Task k = task_of(t);
+      const OutRole& r = k.r;
+      const float sh = decay_of(t);
+      const float w_row = expf(-sh * (float)(r.rev ? max(k.len - row, 0) : row));
+      named_sync(1, Plan::kReaders);
+      // ---- the masked scores' terms over the scores
+      wait_or_fault(&done[kS], it & 1, &cta, g.fault, kFaultMmaWait);
+      tc_fence_after_sync();
+      const bool two = r.wx > 64;
+      // Sixteen columns at a time, in a loop: the code runs once a task, so most of what is straight-line is fetched anew
+      // every time.
+#pragma unroll 1
+      for (int u = 2 * part; u < 8; u = (u & 1) ? u + 2 * kParts - 1 : u + 1) {
+        const int blk = u >> 1;
+        uint32_t hi[8], mid[8], lo[8];
+        const uint32_t at = lane_base + 16 * u;
+        if (r.rev ? blk < quarter : blk > quarter) {   // all masked
 #pragma unroll
-            for (int j = 0; j < 16; ++j) hi[j] = mid[j] = lo[j] = 0u;
-          } else {
-            uint32_t r[32];
-            tmem_ld32(t_s + lane_base + 32 * group, r);
-            tmem_ld_wait();
-            const int rel = k.r->rev ? 32 * group - row_l : row_l - 32 * group;   // distance from the diagonal of column 0
-            const int dir = k.r->rev ? 1 : -1;
+          for (int j = 0; j < 8; ++j) hi[j] = mid[j] = lo[j] = 0u;
+        } else {
+          uint32_t x[16], y[16];
+          tmem_ld16(t_s + at, x);
+          if (two) tmem_ld16(t_s1 + at, y);
+          // lambda^distance: beside the diagonal the row's distance to the block's nearer edge times the column's to it
+          const bool diagonal = blk == quarter;
+          const float edge = diagonal ? 1.f : expf(-sh * (float)(r.rev ? 32 * blk - row : row - 32 * blk - 31));
+          const int first = (diagonal ? 31 - lane : r.rev ? 31 : 0) + 16 * (u & 1);
+          const float4* factors = reinterpret_cast<const float4*>(&line[first & 3][first & ~3]);
+          tmem_ld_wait();
+          if (two) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              float x[2];
-#pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const int dist = rel + dir * (j + u);
-                x[u] = dist >= 0 ? __uint_as_float(r[j + u]) * decay[max(dist, 0)] : 0.f;
-              }
-              uint32_t tt[TT::mid];
-              split_pair<TT::mid>(x[0], x[1], tt);
-              hi[j / 2] = tt[0], mid[j / 2] = tt[1];
-              if constexpr (TT::mid == 3) lo[j / 2] = tt[2];
+            for (int j = 0; j < 16; j += 2) {
+              const F2 sum = fma2(pair(y[j], y[j + 1]), {1.f, 1.f}, pair(x[j], x[j + 1]));
+              x[j] = __float_as_uint(sum.x), x[j + 1] = __float_as_uint(sum.y);
             }
           }
-          tmem_st16(t_s + lane_base + 32 * group, hi);
-          tmem_st16(t_s + lane_base + 32 * group + 16, mid);
-          if constexpr (TT::mid == 3) tmem_st16(t_lo + lane_base + 16 * group, lo);
-          tmem_st_wait();
+          if (diagonal) {   // (a masked score that is not finite must not leave a trace)
+            const uint32_t live = (r.rev ? 0xffffffffu << lane : 0xffffffffu >> (31 - lane)) >> (16 * (u & 1));
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = live & (1u << j) ? x[j] : 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < 16; j += 4) {
+            const float4 f = factors[j / 4];
+#pragma unroll
+            for (int v = 0; v < 4; v += 2) {
+              const F2 m = mul2(pair(x[j + v], x[j + v + 1]), mul2(v ? F2{f.z, f.w} : F2{f.x, f.y}, {edge, edge}));
+              uint32_t tt[3];
+              split_pair<3>(m.x, m.y, tt);
+              hi[(j + v) / 2] = tt[0], mid[(j + v) / 2] = tt[1], lo[(j + v) / 2] = tt[2];
+            }
+          }
         }
-        if (k.has_state) wait_or_fault(&o2_done, o2_uses & 1, &cta, g.fault, kFaultMmaWait);   // O2 has read X
-        store_tile<T, TT::in, false>(set_a, rz, wz, tid, NoWeight());
+        tmem_st8(t_s + at, hi);
+        tmem_st8(t_s + at + 8, mid);
+        tmem_st8(t_s1 + at, lo);
       }
-      fence_async_smem();
+      tmem_st_wait();
       tc_fence_before_sync();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after_sync();
-        issue_terms_ts<TT::mid, TT::in, TT::cut>(t_o1, t_s, t_lo, TermOperand{addr_a, (uint32_t)(C * wz * 2), C, true}, wz);
-        umma_commit(&o1_done);
-      }
-      // ---- the next task's Y and X, its scores
-      const int t_next = t + gridDim.x;
-      const bool more = t_next < g.tasks;
-      Task kn = k;
-      if (more) {
-        kn = task_of(t_next);
-        Raw<T> ry[kPieces], rx[kPieces];
-        load_xy(ry, kn.r->y, kn);
-        load_xy(rx, kn.r->x, kn);
-        if (tid <= C) decay[tid] = expf(-kn.sh * (float)tid);   // this task's masks are done (barrier above)
-        store_y(ry, rx, padded(kn.r->wx));   // O2 has read P
-        wait_or_fault(&o1_done, it & 1, &cta, g.fault, kFaultMmaWait);
-        store_tile<T, TT::in, false>(set_a, rx, padded(kn.r->wx), tid, NoWeight());
-        fence_async_smem();
-        tc_fence_before_sync();
-        __syncthreads();
-        if (tid == 0) issue_s(kn);
-      } else {
-        wait_or_fault(&o1_done, it & 1, &cta, g.fault, kFaultMmaWait);
-      }
-      // ---- epilogue, under the next scores
+      warp_arrive(&sm_ready);
+      named_sync(1, Plan::kReaders);
+      if (t + (int)gridDim.x < g.tasks) write_line(t + gridDim.x);
+      // ---- epilogue
+      wait_or_fault(&done[kO1], it & 1, &cta, g.fault, kFaultMmaWait);
+      __syncwarp();
       tc_fence_after_sync();
-      {
-        const int per = wz / 4;
-        T* out = static_cast<T*>(k.r->out) + (k.tok + row_l) * k.r->pitch_z;
+      const auto result16 = [&](int c0, uint32_t (&a1)[16]) {   // sixteen results of this thread's row from column c0 on
+        uint32_t a2[16];
+        tmem_ld16(t_o1 + lane_base + c0, a1);
+        if (k.has_state) tmem_ld16(t_o2 + lane_base + c0, a2);
+        tmem_ld_wait();
+        if (k.has_state) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) {
+            const F2 x = fma2({w_row, w_row}, pair(a2[j], a2[j + 1]), pair(a1[j], a1[j + 1]));
+            a1[j] = __float_as_uint(x.x), a1[j + 1] = __float_as_uint(x.y);
+          }
+        }
+      };
+      if constexpr (ADD) {
+        T* out = static_cast<T*>(r.out) + (k.tok + row) * r.pitch_z;
         uint32_t again = 0;   // blocks of 16 columns with a result that is not finite
 #pragma unroll 1
-        for (int c0 = group * per; c0 < (group + 1) * per; c0 += 16) {
-          uint32_t a1[16], a2[16];
-          tmem_ld16(t_o1 + lane_base + c0, a1);
-          if (k.has_state) tmem_ld16(t_o2 + lane_base + c0, a2);
-          tmem_ld_wait();
-          if (row_l < k.len && c0 < k.r->wz) {
+        for (int c0 = 16 * part; c0 < r.wz; c0 += 16 * kParts) {
+          uint32_t a1[16];
+          result16(c0, a1);
+          if (row < k.len) {
             float x[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              x[j] = k.has_state ? fmaf(w_row, __uint_as_float(a2[j]), __uint_as_float(a1[j])) : __uint_as_float(a1[j]);
-              a1[j] = __float_as_uint(x[j]);
-            }
-            if constexpr (ADD) {
-              if (all_finite(a1))
-                put16(out + c0, x, k.r->add != 0);
-              else
-                again |= 1u << ((c0 - group * per) / 16);
-            } else {
-              if (!all_finite(a1)) look_again = 1;
-              put16(out + c0, x, false);
-            }
+            for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(a1[j]);
+            if (all_finite(a1))
+              put16(out + c0, x, r.add != 0);
+            else
+              again |= 1u << (c0 / 16);
           }
         }
-        if constexpr (ADD) {
-          if (again) plain_out<T>(&g, t, row_l, group * per, again);   // (here few registers are live)
+        tc_fence_before_sync();
+        warp_arrive(&acc_free);
+        if (again) plain_out<T>(&args, t, row, 0, again);   // (here few registers are live)
+      } else {
+        // 64 bytes of a row at a time: sixteen fp32 results, or two times sixteen
+        constexpr int kCols = 64 / (int)sizeof(T), kPer = 16 / (int)sizeof(T);
+        const int my_col = (lane & 3) * kPer;
+        T* out = static_cast<T*>(r.out) + (k.tok + (row & ~3)) * r.pitch_z + my_col;
+        const int rows_left = k.len - (row & ~3);
+#pragma unroll 1
+        for (int c0 = kCols * part; c0 < r.wz; c0 += kParts * kCols) {
+          uint4 v[4];
+#pragma unroll
+          for (int u = 0; u < kCols / 16; ++u) {
+            uint32_t a1[16];
+            if (u > 0 && c0 + 16 * u >= r.wz) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) a1[j] = 0u;
+            } else {
+              result16(c0 + 16 * u, a1);
+            }
+            if (row < k.len && !all_finite(a1)) look_again = 1;
+            if constexpr (std::is_same<T, float>::value) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) v[q] = make_uint4(a1[4 * q], a1[4 * q + 1], a1[4 * q + 2], a1[4 * q + 3]);
+            } else {
+              uint32_t h[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) h[j] = pack2(__uint_as_float(a1[2 * j]), __uint_as_float(a1[2 * j + 1]), T());
+              v[2 * u] = make_uint4(h[0], h[1], h[2], h[3]), v[2 * u + 1] = make_uint4(h[4], h[5], h[6], h[7]);
+            }
+          }
+          rows_to_lanes(v, lane);
+          if (c0 + my_col < r.wz) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              if (i < rows_left) *reinterpret_cast<uint4*>(out + (size_t)i * r.pitch_z + c0) = v[i];
+          }
         }
+        tc_fence_before_sync();
+        warp_arrive(&acc_free);
       }
-      o2_uses += k.has_state ? 1 : 0;
-      if (!more) break;
-      t = t_next;
-      k = kn;
+    }
+  } else if constexpr (Plan::kFillXZ) {
+    // ---- fillers
+    const int ft = (tid - 128 - Plan::kReaders) & (kFillers - 1);
+    // what a task's chunks are made of: its first token's rows
+    struct Source {
+      const T *x, *y, *z;
+      int pitch_x, pitch_z, wx, wz, len;
+    };
+    const auto source_of = [&](int t) {
+      const Task k = task_of(t);
+      return Source{static_cast<const T*>(k.r.x) + k.tok * k.r.pitch_x, static_cast<const T*>(k.r.y) + k.tok * k.r.pitch_x,
+                    static_cast<const T*>(k.r.z) + k.tok * k.r.pitch_z, k.r.pitch_x, k.r.pitch_z, k.r.wx, k.r.wz, k.len};
+    };
+    const auto chunk_of = [&](const Source& k, int kind) {
+      const int c = kind & 1;
+      if (kind >= kZ0)
+        return tensor_chunk<T>(k.z + (size_t)64 * c * k.pitch_z, k.pitch_z, 64, k.len - 64 * c, k.len > 64 * c ? k.wz : 0, k.wz > 64, ft);
+      return tensor_chunk<T>((kind >= kY0 ? k.y : k.x) + 64 * c, k.pitch_x, C, k.len, min(k.wx - 64 * c, 64), false, ft);
+    };
+    int t = blockIdx.x, it = 0;
+    uint32_t u = 0;
+    if (t < g.tasks) {
+      Source task = source_of(t);
+      Chunk cur = chunk_of(task, Plan::kFillOrder & 15), next;
+      RawChunk<T> r;
+      const auto load_next = [&](int i) { load_chunk_piece<T>(r, next, i); };
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i) load_chunk_piece<T>(r, cur, i);
+      while (true) {
+        const int now = (Plan::kFillOrder >> (4 * u)) & 15, it_now = it;
+        if (++u == Plan::kFills) {
+          u = 0, ++it;
+          t += gridDim.x;
+          if (t < g.tasks) task = source_of(t);
+        }
+        next = chunk_of(task, (Plan::kFillOrder >> (4 * u)) & 15);
+        if (t >= g.tasks) next.cols = 0;
+        await_place(plan_at<Plan::fill_after>(now), it_now);
+        store_chunk<T, TT::in>(smem + turned(plan_at<Plan::fill_place>(now), it_now) * kUnit, r, cur, load_next);
+        fence_async_smem();
+        warp_arrive(&full[now]);
+        if (t >= g.tasks) break;
+        cur = next;
+      }
     }
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, 512);
+  if (warp == 2) tmem_dealloc(tmem, 512);
   if constexpr (!ADD) {
-    if (look_again)   // (after the loop, whose registers are all taken)
-      for (int u = blockIdx.x; u < g.tasks; u += gridDim.x) plain_out_where_needed<T>(&g, u);
+    // (after the loops, whose registers are all taken; the control warps have given theirs away)
+    if (look_again && warp >= 4)
+      for (int u = blockIdx.x; u < g.tasks; u += gridDim.x) plain_out_where_needed<T>(&args, u);
   }
 }
 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-int host_padded(int w) { return w <= 64 ? 64 : 128; }
-
-constexpr size_t kMaxSmem = 6 * 32768 + 1024;
+cudaError_t matrix_map(CUtensorMap* map, const void* base, size_t count, int rows, int width, int pitch) {
+  const cudaError_t err = make_matrix_map(map, base, count, (uint64_t)rows, (uint32_t)width, (uint32_t)pitch);
+  if (err != cudaSuccess) g_failed_step = "tensor map of the full-precision path";
+  return err;
+}
 
 template <typename T>
 cudaError_t launch_states(const Dims& m, const StateArgs& g, cudaStream_t st) {
-  const size_t smem = (size_t)C * 2 * (Terms<T>::mid * host_padded(m.d) + Terms<T>::in * host_padded(m.e)) + 1024;
-  cudaError_t err = opt_in_smem<k_split_states<T>>(kMaxSmem);
-  if (err != cudaSuccess) return err;
-  // (a 64-wide A of the last term reads 16 KB past its tile: the B terms behind it are at least that long)
+  CUtensorMap map_b = {};
+  cudaError_t err;
+  if (StatePlan<T>::kTmaB && (err = matrix_map(&map_b, g.b, (size_t)m.b * m.h, m.n, m.e, m.pitch_e)) != cudaSuccess) return err;
+  if ((err = opt_in_smem<k_split_states<T>>(StatePlan<T>::kSmem)) != cudaSuccess) return err;
   const int grid = g.tasks < sm_count() ? g.tasks : sm_count();
-  k_split_states<T><<<grid, NT, smem, st>>>(g);
+  k_split_states<T><<<grid, kStateThreads, StatePlan<T>::kSmem, st>>>(map_b, g);
   err = cudaGetLastError();
   if (err != cudaSuccess) g_failed_step = "launch of the chunk-state kernel";
   return err;
 }
 
 template <typename T, bool ADD>
-cudaError_t launch_out(const Dims& m, OutArgs& g, cudaStream_t st) {
-  const int dp = host_padded(m.d), ep = host_padded(m.e), widest = dp > ep ? dp : ep;
-  g.set_bytes = (uint32_t)(Terms<T>::in * C * widest * 2);
-  const size_t state = (size_t)Terms<T>::mid * dp * ep * 2;
-  const size_t smem = g.set_bytes + (state > g.set_bytes ? state : g.set_bytes) + 1024;
-  cudaError_t err = opt_in_smem<k_split_out<T, ADD>>(kMaxSmem);
+cudaError_t launch_out(const OutMaps& maps, const OutArgs& g, cudaStream_t st) {
+  constexpr size_t smem = (size_t)OutPlan<T>::kUnits * kUnit + 1024;
+  cudaError_t err = opt_in_smem<k_split_out<T, ADD>>(smem);
   if (err != cudaSuccess) return err;
   const int grid = g.tasks < sm_count() ? g.tasks : sm_count();
-  k_split_out<T, ADD><<<grid, NT, smem, st>>>(g);
+  k_split_out<T, ADD><<<grid, kOutThreads<T>, smem, st>>>(maps, g);
   err = cudaGetLastError();
   if (err != cudaSuccess) g_failed_step = "launch of the output kernel";
   return err;
@@ -793,31 +1099,50 @@ cudaError_t split_chunk_states(const Dims& m, const void* a, const void* bten, c
   return by_dtype(m.dtype, [&](auto t) { return launch_states<decltype(t)>(m, g, st); });
 }
 
-cudaError_t split_fwd_output(const Dims& m, const void* q, const void* k, const void* v, const float* s,
-                             const float* prefix, void* o, bool alone, bool add_o, cudaStream_t st) {
-  OutArgs g = {};
-  g.role[0] = {q, k, v, o, m.nc == 1 && alone ? nullptr : prefix, m.d, m.e, m.pitch_d, m.pitch_e, 0, 0, alone ? 0 : -1, add_o};
-  g.roles = 1;
-  g.s = s, g.h = m.h, g.n = m.n, g.nc = m.nc, g.d = m.d, g.e = m.e, g.tasks = m.b * m.h * m.nc;
-  const cudaError_t err = fault_word_address(&g.fault);
+namespace {
+// the launch of one (o) or three (dq, dk, dv) results; maps only of what the kernels of this type load by TMA
+cudaError_t split_outputs(const Dims& m, OutArgs& g, const void* q, const void* k, const void* v, const void* d_o, const void* prefix,
+                          const void* suffix, cudaStream_t st) {
+  g.h = m.h, g.n = m.n, g.nc = m.nc, g.d = m.d, g.e = m.e, g.tasks = g.roles * m.b * m.h * m.nc;
+  cudaError_t err = fault_word_address(&g.fault);
   if (err != cudaSuccess) return err;
-  return by_dtype(m.dtype, [&](auto t) { return g.role[0].add || g.role[1].add || g.role[2].add ? launch_out<decltype(t), true>(m, g, st) : launch_out<decltype(t), false>(m, g, st); });
+  OutMaps maps = {};
+  const size_t seqs = (size_t)m.b * m.h;
+  for (const auto& [i, p] : {std::pair<int, const void*>{kMapPrefix, prefix}, {kMapSuffix, suffix}})
+    if (p && (err = matrix_map(&maps.m[i], p, seqs * m.nc * 3, m.d, m.e, m.e)) != cudaSuccess) return err;
+  if (m.dtype != LASP_F32) {
+    for (const auto& [i, p] : {std::pair<int, const void*>{kMapQ, q}, {kMapK, k}})
+      if ((err = matrix_map(&maps.m[i], p, seqs, m.n, m.d, m.pitch_d)) != cudaSuccess) return err;
+    for (const auto& [i, p] : {std::pair<int, const void*>{kMapV, v}, {kMapDo, d_o}})
+      if (p && (err = matrix_map(&maps.m[i], p, seqs, m.n, m.e, m.pitch_e)) != cudaSuccess) return err;
+  }
+  const bool add = g.role[0].add || g.role[1].add || g.role[2].add;
+  return by_dtype(m.dtype, [&](auto t) { return add ? launch_out<decltype(t), true>(maps, g, st) : launch_out<decltype(t), false>(maps, g, st); });
+}
+}  // namespace
+
+cudaError_t split_fwd_output(const Dims& m, const void* q, const void* k, const void* v, const float* s,
+                             const void* prefix, void* o, bool alone, bool add_o, cudaStream_t st) {
+  if (m.nc == 1 && alone) prefix = nullptr;
+  OutArgs g = {};
+  g.s = s, g.roles = 1;
+  g.role[0] = {q, k, v, o, static_cast<const __nv_bfloat16*>(prefix), kMapQ, kMapK, kMapV, kMapPrefix, m.d, m.e, m.pitch_d, m.pitch_e,
+               0, 0, alone ? 0 : -1, add_o};
+  return split_outputs(m, g, q, k, v, nullptr, prefix, nullptr, st);
 }
 
 cudaError_t split_bwd_grads(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, const float* s,
-                            const float* prefix, const float* suffix, void* dq, void* dk, void* dv, bool alone,
+                            const void* prefix, const void* suffix, void* dq, void* dk, void* dv, bool alone,
                             bool add_qk, bool add_v, cudaStream_t st) {
-  OutArgs g = {};
-  const int first = alone ? 0 : -1, last = alone ? m.nc - 1 : -1;
   if (m.nc == 1 && alone) prefix = suffix = nullptr;
-  g.role[0] = {d_o, v, k, dq, prefix, m.e, m.d, m.pitch_e, m.pitch_d, 1, 0, first, add_qk};
-  g.role[1] = {v, d_o, q, dk, suffix, m.e, m.d, m.pitch_e, m.pitch_d, 1, 1, last, add_qk};
-  g.role[2] = {k, q, d_o, dv, suffix, m.d, m.e, m.pitch_d, m.pitch_e, 0, 1, last, add_v};
-  g.roles = 3;
-  g.s = s, g.h = m.h, g.n = m.n, g.nc = m.nc, g.d = m.d, g.e = m.e, g.tasks = 3 * m.b * m.h * m.nc;
-  const cudaError_t err = fault_word_address(&g.fault);
-  if (err != cudaSuccess) return err;
-  return by_dtype(m.dtype, [&](auto t) { return g.role[0].add || g.role[1].add || g.role[2].add ? launch_out<decltype(t), true>(m, g, st) : launch_out<decltype(t), false>(m, g, st); });
+  const int first = alone ? 0 : -1, last = alone ? m.nc - 1 : -1;
+  const auto *p = static_cast<const __nv_bfloat16*>(prefix), *dn = static_cast<const __nv_bfloat16*>(suffix);
+  OutArgs g = {};
+  g.s = s, g.roles = 3;
+  g.role[0] = {d_o, v, k, dq, p, kMapDo, kMapV, kMapK, kMapPrefix, m.e, m.d, m.pitch_e, m.pitch_d, 1, 0, first, add_qk};
+  g.role[1] = {v, d_o, q, dk, dn, kMapV, kMapDo, kMapQ, kMapSuffix, m.e, m.d, m.pitch_e, m.pitch_d, 1, 1, last, add_qk};
+  g.role[2] = {k, q, d_o, dv, dn, kMapK, kMapQ, kMapDo, kMapSuffix, m.d, m.e, m.pitch_d, m.pitch_e, 0, 1, last, add_v};
+  return split_outputs(m, g, q, k, v, d_o, prefix, suffix, st);
 }
 
 }  // namespace lasp

@@ -1,6 +1,6 @@
 // Elementwise kernels on the fp32 d x e states: the scan over the chunks (or spans) of a sequence and the update of
 // a rank state.
-#include "common.cuh"
+#include "state_terms.cuh"
 
 namespace lasp {
 namespace {
@@ -8,13 +8,15 @@ namespace {
 // ---------------------------------------------------------------------------
 // scan over chunks, elementwise in (d,e).  forward: exclusive prefix seeded
 // with x_in; reverse: exclusive suffix.  k_scan reads the fp32 local states
-// and writes the prefix states to a second array.  Loads of a batch of chunks are issued before the
+// and writes the prefix states to a second array: fp32 in lane order (tensor path), or row-major in terms
+// (TERMS, full-precision path).  Loads of a batch of chunks are issued before the
 // dependent recurrence so that their latencies overlap.
 // ---------------------------------------------------------------------------
 constexpr int kScanBatch = 8;
 
+template <bool TERMS>
 __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const float* __restrict__ local,
-                                              float* __restrict__ prefix, const float* __restrict__ x_in,
+                                              void* __restrict__ prefix, const float* __restrict__ x_in,
                                               float* __restrict__ x_out, int h,
                                               int n, int de, int nc, int chunk, int reverse, int rows,
                                               int cols) {
@@ -22,7 +24,7 @@ __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const
   const int el = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (el >= de) return;
   // where this float4 of a state in lane order lives in the caller's row-major rank states
-  const int ext = lane_order_to_row_major(el / 4, rows, cols) * 4;
+  const int ext = TERMS ? el : lane_order_to_row_major(el / 4, rows, cols) * 4;
   const float sh = s[bh % h];
   const float full = expf(-sh * (float)chunk);
   const int last_len = n - (nc - 1) * chunk;
@@ -30,7 +32,6 @@ __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
   if (x_in) p = *reinterpret_cast<const float4*>(x_in + (size_t)bh * de + ext);
   const float* base = local + (size_t)bh * nc * de + el;
-  float* out = prefix + (size_t)bh * nc * de + el;
   for (int i0 = 0; i0 < nc; i0 += kScanBatch) {
     float4 loc[kScanBatch];
 #pragma unroll
@@ -44,7 +45,11 @@ __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const
       if (i < nc) {
         const int c = reverse ? nc - 1 - i : i;
         const float dec = (c == nc - 1) ? tail : full;
-        *reinterpret_cast<float4*>(out + (size_t)c * de) = p;
+        const size_t state = (size_t)bh * nc + c;
+        if (TERMS)
+          store_state_terms(static_cast<__nv_bfloat16*>(prefix) + state * 3 * de, el, de, p);
+        else
+          *reinterpret_cast<float4*>(static_cast<float*>(prefix) + state * de + el) = p;
         p.x = fmaf(dec, p.x, loc[u].x);
         p.y = fmaf(dec, p.y, loc[u].y);
         p.z = fmaf(dec, p.z, loc[u].z);
@@ -75,12 +80,12 @@ __global__ void __launch_bounds__(256) k_state_combine(const float* __restrict__
 
 }  // namespace
 
-cudaError_t scan_states(const Dims& m, const float* s, const float* local, float* prefix, const float* x_in,
+cudaError_t scan_states(const Dims& m, const float* s, const float* local, void* prefix, const float* x_in,
                         float* x_out, bool reverse, cudaStream_t st) {
   const int de = m.d * m.e;
   dim3 grid((de / 4 + 255) / 256, m.b * m.h);
-  k_scan<<<grid, 256, 0, st>>>(s, local, prefix, x_in, x_out, m.h, m.n, de, m.nc, m.chunk, reverse ? 1 : 0, m.d,
-                               m.e);
+  auto* kernel = m.walk ? k_scan<false> : k_scan<true>;
+  kernel<<<grid, 256, 0, st>>>(s, local, prefix, x_in, x_out, m.h, m.n, de, m.nc, m.chunk, reverse ? 1 : 0, m.d, m.e);
   return cudaGetLastError();
 }
 
