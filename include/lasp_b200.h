@@ -75,7 +75,11 @@ typedef enum {
  * them would read and write q and k once more in an operator bound by memory traffic.  Only the fused
  * tensor-core launches (forward, backward, the linked forms, bwd_dq, bwd_dkv) take it; every other entry
  * point returns LASP_ERR_PATH when it is requested. */
-typedef enum { LASP_QK_IDENTITY = 0, LASP_QK_ELU1 = 1 /* elu(x) + 1 */ } lasp_qk_map;
+typedef enum {
+  LASP_QK_IDENTITY = 0,
+  LASP_QK_ELU1 = 1,       /* elu(x) + 1 */
+  LASP_QK_ELU1_MAPPED = 2 /* elu(x) + 1, which q and k hold already (lasp_b200_map_qk); dq, dk as with LASP_QK_ELU1 */
+} lasp_qk_map;
 
 typedef struct {
   int32_t b, h, n, d, e;
@@ -89,6 +93,10 @@ typedef struct {
    * of the slice's first column.  Multiples of 8. */
   int32_t pitch_d, pitch_e;
 } lasp_problem;
+
+/* q_out = elu(q) + 1, k_out = elu(k) + 1, bf16, `elements` each (a multiple of 8): what the kernels make of a tile with
+ * LASP_QK_ELU1, once for all launches of a forward and a backward pass instead of once per launch that reads it. */
+LASP_B200_API int lasp_b200_map_qk(const void* q, const void* k, void* q_out, void* k_out, int64_t elements, void* stream);
 
 /* Forward arguments.  ws = workspace of lasp_b200_fwd_workspace_bytes(); after
  * the scan phase it holds the per-chunk prefix states, which the backward

@@ -86,6 +86,7 @@ SIGNATURES = {
     "lasp_b200_bwd_dq": (C.c_int, [_PP, _BP, C.c_void_p]),
     "lasp_b200_bwd_dkv": (C.c_int, [_PP, _BP, C.c_void_p]),
     "lasp_b200_bwd_dkv_walk": (C.c_int, [_PP, _BP, C.c_void_p]),
+    "lasp_b200_map_qk": (C.c_int, [C.c_void_p] * 4 + [C.c_int64, C.c_void_p]),
     "lasp_b200_forward_opt": (C.c_int, [_PP, _FP, C.POINTER(CallOptions), C.c_void_p]),
     "lasp_b200_backward_opt": (C.c_int, [_PP, _BP, C.POINTER(CallOptions), C.c_void_p]),
     "lasp_b200_state_combine": (C.c_int, [C.c_int] * 5 + [C.c_void_p] * 5),

@@ -82,7 +82,7 @@ int make_dims(const lasp_problem* p, lasp::Dims* m) {
   if ((long long)p->b * p->h > 65535) return LASP_ERR_SHAPE;
   m->b = p->b; m->h = p->h; m->n = p->n; m->d = p->d; m->e = p->e;
   m->dtype = p->dtype;
-  if (p->qk_map != LASP_QK_IDENTITY && p->qk_map != LASP_QK_ELU1) return LASP_ERR_SHAPE;
+  if (p->qk_map < LASP_QK_IDENTITY || p->qk_map > LASP_QK_ELU1_MAPPED) return LASP_ERR_SHAPE;
   if (p->pitch_d < 0 || p->pitch_e < 0 || (p->pitch_d && p->pitch_d < p->d) || (p->pitch_e && p->pitch_e < p->e) ||
       p->pitch_d % 8 || p->pitch_e % 8)
     return LASP_ERR_SHAPE;
@@ -281,6 +281,13 @@ int bwd_grads(const lasp::Dims& m, const lasp_bwd_args* a, const lasp_call_optio
 
 extern "C" {
 
+int lasp_b200_map_qk(const void* q, const void* k, void* q_out, void* k_out, int64_t elements, void* stream) {
+  if (!q || !k || !q_out || !k_out) return LASP_ERR_NULL;
+  if (elements <= 0 || elements % 8) return LASP_ERR_SHAPE;
+  if (!aligned16(q) || !aligned16(k) || !aligned16(q_out) || !aligned16(k_out)) return LASP_ERR_ALIGN;
+  return cuda_fail(lasp::map_qk(q, k, q_out, k_out, elements, static_cast<cudaStream_t>(stream)));
+}
+
 // ---- forward --------------------------------------------------------------
 int lasp_b200_fwd_chunk_states(const lasp_problem* p, const lasp_fwd_args* a, void* stream) {
   lasp::Dims m;
@@ -434,7 +441,7 @@ int lasp_b200_linked_ok(const lasp_problem* p) {
   lasp::Dims m;
   int st = make_dims(p, &m);
   if (st != LASP_OK) return st;
-  return (m.walk && !unfused_requested() && m.b * m.h * m.nc <= lasp::sm_count()) ? 1 : 0;
+  return (m.walk && m.qk_map != LASP_QK_ELU1_MAPPED && !unfused_requested() && m.b * m.h * m.nc <= lasp::sm_count()) ? 1 : 0;
 }
 
 int lasp_b200_forward_linked(const lasp_problem* p, const lasp_fwd_args* a, const lasp_exchange_args* x,

@@ -40,7 +40,7 @@ struct Dims {
   int tiles;  // tensor path: 128-token tiles per sequence
   int span;   // tensor path: tiles per span (chunk = span * 128)
   int pitch_d, pitch_e;  // elements between the rows of consecutive tokens in q,k,dq,dk and in v,o,do,dv
-  int qk_map;      // q and k enter as qk_scale * map(x): 0 identity, 1 elu(x) + 1
+  int qk_map;      // q and k enter as qk_scale * map(x): a lasp_qk_map
   float qk_scale;  // (1 when the caller left it 0)
 };
 
@@ -122,6 +122,8 @@ cudaError_t scan_states(const Dims& m, const float* s, const float* local, void*
                         float* x_out, bool reverse, cudaStream_t st);
 cudaError_t state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
                           const float* x_local, float* x_out, cudaStream_t st);
+
+cudaError_t map_qk(const void* q, const void* k, void* q_out, void* k_out, int64_t elements, cudaStream_t st);
 
 // state relay (relay_kernels.cu)
 cudaError_t exchange_scan(const Dims& m, const lasp_exchange_args& a, const float* local, void* prefix,

@@ -1,6 +1,7 @@
-// Elementwise kernels on the fp32 d x e states: the scan over the chunks (or spans) of a sequence and the update of
-// a rank state.
+// Elementwise kernels: on the fp32 d x e states the scan over the chunks (or spans) of a sequence and the update of
+// a rank state; the feature map on q and k.
 #include "state_terms.cuh"
+#include "tc_common.cuh"
 
 namespace lasp {
 namespace {
@@ -78,7 +79,32 @@ __global__ void __launch_bounds__(256) k_state_combine(const float* __restrict__
   *reinterpret_cast<float4*>(x_out + (size_t)bh * de + el) = loc;
 }
 
+// elu(x) + 1 of q (blockIdx.y = 0) and k (1).  Bound by HBM: 8 bytes an element.
+constexpr int kMapPieces = 4;   // 16-byte loads in flight per thread
+__global__ void __launch_bounds__(256) k_map_qk(const uint4* __restrict__ q, const uint4* __restrict__ k, uint4* __restrict__ q_out,
+                                                uint4* __restrict__ k_out, int64_t pieces) {
+  const uint4* in = blockIdx.y ? k : q;
+  uint4* out = blockIdx.y ? k_out : q_out;
+  const int64_t first = (int64_t)blockIdx.x * (256 * kMapPieces) + threadIdx.x;
+  uint4 v[kMapPieces];
+#pragma unroll
+  for (int i = 0; i < kMapPieces; ++i)
+    if (first + 256 * i < pieces) v[i] = __ldg(in + first + 256 * i);
+#pragma unroll
+  for (int i = 0; i < kMapPieces; ++i)
+    if (first + 256 * i < pieces)
+      out[first + 256 * i] = make_uint4(tc::elu1_bf16x2(v[i].x), tc::elu1_bf16x2(v[i].y), tc::elu1_bf16x2(v[i].z), tc::elu1_bf16x2(v[i].w));
+}
+
 }  // namespace
+
+cudaError_t map_qk(const void* q, const void* k, void* q_out, void* k_out, int64_t elements, cudaStream_t st) {
+  const int64_t pieces = elements / 8, blocks = (pieces + 256 * kMapPieces - 1) / (256 * kMapPieces);
+  if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
+  k_map_qk<<<dim3((unsigned)blocks, 2), 256, 0, st>>>(static_cast<const uint4*>(q), static_cast<const uint4*>(k), static_cast<uint4*>(q_out),
+                                                      static_cast<uint4*>(k_out), pieces);
+  return cudaGetLastError();
+}
 
 cudaError_t scan_states(const Dims& m, const float* s, const float* local, void* prefix, const float* x_in,
                         float* x_out, bool reverse, cudaStream_t st) {

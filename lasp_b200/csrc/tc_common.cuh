@@ -201,9 +201,12 @@ __device__ __forceinline__ uint32_t elu1_bf16x2(uint32_t u) {
   const __nv_bfloat162 r = __hadd2(__hmax2(x, __float2bfloat162_rn(0.f)), __hmin2(exp_bf16x2(u), __float2bfloat162_rn(1.f)));
   return *reinterpret_cast<const uint32_t*>(&r);
 }
-// its derivative: 1 for x > 0, exp(x) otherwise = min(exp(x), 1)
+// its derivative: 1 for x > 0, exp(x) otherwise = min(exp(x), 1) = min(elu(x) + 1, 1): from x, or from what the map gave
+// (MAPPED)
+template <bool MAPPED>
 __device__ __forceinline__ float2 elu1_slope_bf16x2(uint32_t u) {
-  return __bfloat1622float2(__hmin2(exp_bf16x2(u), __float2bfloat162_rn(1.f)));
+  const __nv_bfloat162 y = MAPPED ? *reinterpret_cast<const __nv_bfloat162*>(&u) : exp_bf16x2(u);
+  return __bfloat1622float2(__hmin2(y, __float2bfloat162_rn(1.f)));
 }
 
 // Multiplies CHUNKS 16-byte pieces of row `row` of a swizzled tile of C rows by w, in place, starting
@@ -265,6 +268,7 @@ __device__ __forceinline__ void raw_row32(uint4 (&x)[4], const __nv_bfloat16* ra
 #pragma unroll
   for (int j = 0; j < 4; ++j) x[j] = __ldg(reinterpret_cast<const uint4*>(raw + col0) + j);
 }
+template <bool MAPPED>
 __device__ __forceinline__ void stage_row32_chain(uint32_t taddr, uint8_t* tile, int row, int col0,
                                                   const uint4 (&x)[4], float c, bool elu) {
   uint32_t a[32];
@@ -277,7 +281,7 @@ __device__ __forceinline__ void stage_row32_chain(uint32_t taddr, uint8_t* tile,
     for (int t = 0; t < 4; ++t) {
       float sx = c, sy = c;
       if (elu) {
-        const float2 sl = elu1_slope_bf16x2(reinterpret_cast<const uint32_t*>(&x[j])[t]);
+        const float2 sl = elu1_slope_bf16x2<MAPPED>(reinterpret_cast<const uint32_t*>(&x[j])[t]);
         sx *= sl.x, sy *= sl.y;
       }
       m[2 * t] = __uint_as_float(a[8 * j + 2 * t]) * sx;

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <deque>
 #include <mutex>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -211,13 +212,37 @@ std::vector<Tensor> run_forward(const Tensor& q, const Tensor& k, const Tensor& 
   return out;
 }
 
+// Whether q and k go through elu(x) + 1 in a pass of their own, ahead of the kernels, or tile by tile inside them.  The
+// kernels of a training step map a tile up to five times and evaluate the exponential of the chain rule twice more; the pass
+// costs a launch and 8 bytes of memory traffic an element.  Training, 64-wide 4 x 16 x 4096 272 -> 198 us, 2 x 16 x 2048 92 -> 87,
+// 2 x 16 x 1024 83 -> 86; 128-wide 8 x 32 x 2048 754 -> 610, 2 x 16 x 1024 93 -> 87, 1 x 16 x 1024 81 -> 86: from 2^22 elements of q
+// on.  A forward pass alone: v 64 wide 4 x 16 x 4096 80 -> 73, 2 x 16 x 2048 29 -> 28, 2 x 16 x 1024 even; 128 wide 177 -> 195, never.
+bool map_first(const Shape& m, bool train) { return m.b * m.h * m.n * m.d >= (int64_t{1} << 22) && (train || m.e <= 64); }
+
+std::pair<Tensor, Tensor> mapped_qk(const Tensor& q, const Tensor& k) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  Tensor qm = at::empty(q.sizes(), q.options()), km = at::empty(k.sizes(), k.options());
+  check_status("lasp_b200_map_qk", lasp_b200_map_qk(q.data_ptr(), k.data_ptr(), qm.data_ptr(), km.data_ptr(), q.numel(), stream.stream()));
+  return {qm, km};
+}
+
 class Lightning : public torch::autograd::Function<Lightning> {
  public:
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s,
                         double scale, int64_t map) {
     const Shape m{q.size(0), q.size(1), q.size(2), q.size(3), v.size(3)};
-    std::vector<Tensor> out = run_forward(q, k, v, s, m, scale, map, true);
     variable_list saved{q, k, v, s};
+    std::vector<Tensor> out;
+    if (map == LASP_QK_ELU1 && map_first(m, true)) {
+      // the backward pass takes the mapped tensors; the others are saved for what autograd makes of a change to them
+      const auto [qm, km] = mapped_qk(q, k);
+      map = LASP_QK_ELU1_MAPPED;
+      out = run_forward(qm, km, v, s, m, scale, map, true);
+      saved.push_back(qm), saved.push_back(km);
+    } else {
+      out = run_forward(q, k, v, s, m, scale, map, true);
+    }
     saved.insert(saved.end(), out.begin() + 1, out.end());
     ctx->save_for_backward(std::move(saved));
     ctx->saved_data["scale"] = scale;
@@ -230,7 +255,9 @@ class Lightning : public torch::autograd::Function<Lightning> {
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     // What was saved may have been through a saved-tensor hook (offloading, compression): it can come back with other
     // strides, or not as what it was.
-    const Tensor q = saved[0].contiguous(), k = saved[1].contiguous(), v = saved[2].contiguous(), d_o = grads[0].contiguous();
+    const int64_t map = ctx->saved_data["map"].toInt();
+    const size_t qk = map == LASP_QK_ELU1_MAPPED ? 4 : 0, first_ws = map == LASP_QK_ELU1_MAPPED ? 6 : 4;
+    const Tensor q = saved[qk].contiguous(), k = saved[qk + 1].contiguous(), v = saved[2].contiguous(), d_o = grads[0].contiguous();
     TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda() && d_o.is_cuda(), "lasp_b200: a saved tensor is not on a GPU any more");
     TORCH_CHECK_TYPE(q.scalar_type() == d_o.scalar_type() && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
                      "lasp_b200: a saved tensor has changed its dtype");
@@ -245,11 +272,10 @@ class Lightning : public torch::autograd::Function<Lightning> {
     Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options()), dv = at::empty(v.sizes(), v.options());
     const Tensor sync = sync_words(q.device(), stream);
     Tensor ws;
-    const std::vector<Pair> pairs = slice_pairs(m, lasp_dtype_of(q.scalar_type()), ctx->saved_data["scale"].toDouble(),
-                                                ctx->saved_data["map"].toInt());
+    const std::vector<Pair> pairs = slice_pairs(m, lasp_dtype_of(q.scalar_type()), ctx->saved_data["scale"].toDouble(), map);
     for (size_t i = 0; i < pairs.size(); ++i) {
       const Pair& p = pairs[i];
-      const Tensor fwd_ws = saved[4 + i].contiguous();
+      const Tensor fwd_ws = saved[first_ws + i].contiguous();
       TORCH_CHECK(fwd_ws.is_cuda() && fwd_ws.scalar_type() == at::kByte && (size_t)fwd_ws.numel() >= p.ws_bytes,
                   "lasp_b200: the states saved by the forward pass did not come back as the bytes that they are");
       if (!ws.defined() || (size_t)ws.numel() < p.ws_bytes)
@@ -291,6 +317,10 @@ Tensor attention(Tensor q, Tensor k, Tensor v, const Tensor& ed, double scale, i
   // (the decay rates get no gradient, but a result that depends on them through a graph says so)
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad() || s.requires_grad()))
     return Lightning::apply(q, k, v, s, scale, map);
+  if (map == LASP_QK_ELU1 && map_first(m, false)) {
+    std::tie(q, k) = mapped_qk(q, k);
+    map = LASP_QK_ELU1_MAPPED;
+  }
   return run_forward(q, k, v, s, m, scale, map, false)[0];
 }
 

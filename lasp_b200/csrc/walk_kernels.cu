@@ -439,7 +439,7 @@ struct WalkArgs {
   SpanCut cut;
   float qk_scale;      // q and k enter as qk_scale * map(q), qk_scale * map(k)
   int elu;             // map = elu(x) + 1 (otherwise the identity)
-  const void* raw;     // backward with a map or a scale: the raw q (dQ walk) or k (dK/dV walk) for the chain rule
+  const void* raw;     // backward with a map: q (dQ walk) or k (dK/dV walk) for the chain rule, raw or (PRE = 2) mapped
   int raw_pitch;       // ... and its row pitch in elements
   int even;            // the tiles of a sequence are shared out evenly among its spans (see TileWalk); a fused
                        // forward records it in sync[kSyncEven], the dQ walk reads it from the forward's workspace
@@ -498,7 +498,9 @@ __device__ __forceinline__ void write_state_operand(uint8_t* tile, int rows, int
 //   Tokens and totals that the head's decay has brought below 1e-12 are left out of the sums (reach_tiles: the same
 //   line as for the ranks of a group), so on a long sequence only the tiles next to the border are read twice.
 // ---------------------------------------------------------------------------
-template <int D, int E, bool DQ, bool FUSED, bool PRE, bool LINK>
+// PRE: what becomes of q and k - 0 nothing, 1 all of it (the map on tiles in shared memory, the scale, the chain rule),
+// 2 the scale and the chain rule of q and k that are mapped already
+template <int D, int E, bool DQ, bool FUSED, int PRE, bool LINK>
 __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant__ CUtensorMap map_x,
                                                      const __grid_constant__ CUtensorMap map_y,
                                                      const __grid_constant__ CUtensorMap map_z,
@@ -612,9 +614,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
   constexpr int kHalfE = E / 2;
   // q and k enter as c * map(q), c * map(k): the map is applied to the tiles in shared memory, c is folded
   // into factors that exist anyway (dQ: the state already carries k's c)
-  // (PRE = false: instantiations without any of this, for callers who bring q and k as they are)
+  // (PRE = 0: instantiations without any of this, for callers who bring q and k as they are)
   const float c = PRE ? a.qk_scale : 1.f;
-  const bool elu = PRE && a.elu != 0;
+  const bool elu = PRE == 1 && a.elu != 0;           // tiles are mapped here
+  const bool slope = PRE != 0 && a.elu != 0;         // results take the map's derivative
   // brings tile j (buffers of parity j & 1) through the feature map once its loads have landed, each group its share
   auto map_tile = [&](int j, auto group) {
     constexpr int grp = decltype(group)::value;
@@ -734,7 +737,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       //   warp 1  the span total; O2 = X op(P), then O1 = S_m Z on top of the row-scaled O2
       //   warp 2  L = K^T diag(w) V (d x e), the scaled rows being Y's
       //   warp 3  S = X Y^T of the next tile
-      const bool map_xy = PRE && a.elu && !DQ, map_z = PRE && a.elu && DQ;
+      const bool map_xy = PRE == 1 && a.elu && !DQ, map_z = PRE == 1 && a.elu && DQ;
       if (warp == 1 && sums > 0) {
 #pragma unroll 1
         for (int g = 0; g < sums; ++g) {
@@ -837,11 +840,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       mbar_arrive(&sm_ready[p]);
       if (elu && i + 1 < total) map_tile(i + 1, grp);   // the next tile's S can then go out under this tile's work
       // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
-      const bool chain = PRE && DQ && (elu || c != 1.f);
+      const bool chain = PRE && DQ && (slope || c != 1.f);
       const bool live = row < a.n - w.t * C;
       const __nv_bfloat16* raw = nullptr;
       uint4 raw_x[4];
-      if (PRE && DQ && elu) {
+      if (PRE && DQ && slope) {
         raw = static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
         raw_row32(raw_x, raw, half * (WZ / 2));
       }
@@ -853,8 +856,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 #pragma unroll 1
         for (int cc = 0; cc < WZ / 64; ++cc) {
           const int col0 = half * (WZ / 2) + cc * 32;
-          stage_row32_chain(t_o + lane_base + col0, sz[p], row, col0, raw_x, c, elu && live);
-          if (WZ > 64 && cc == 0 && elu) raw_row32(raw_x, raw, col0 + 32);
+          stage_row32_chain<PRE == 2>(t_o + lane_base + col0, sz[p], row, col0, raw_x, c, slope && live);
+          if (WZ > 64 && cc == 0 && slope) raw_row32(raw_x, raw, col0 + 32);
         }
       } else {
 #pragma unroll 1
@@ -1092,7 +1095,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
 // the incoming rank state) and walks; the outgoing rank state is the state after the first tile of the
 // sequence.
 // ---------------------------------------------------------------------------
-template <int D, int E, bool FUSED, bool PRE, bool LINK>
+template <int D, int E, bool FUSED, int PRE, bool LINK>
 __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do,
@@ -1198,9 +1201,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   constexpr int kHalfE = E / 2;
   // q and k enter as c * map(q), c * map(k): the map is applied to the tiles in shared memory, c is folded
   // into factors that exist anyway
-  // (PRE = false: instantiations without any of this, for callers who bring q and k as they are)
+  // (PRE = 0: instantiations without any of this, for callers who bring q and k as they are)
   const float c = PRE ? a.qk_scale : 1.f;
-  const bool elu = PRE && a.elu != 0;
+  const bool elu = PRE == 1 && a.elu != 0;
+  const bool slope = PRE != 0 && a.elu != 0;
   auto span_total = [&](auto group) {
     constexpr int grp = decltype(group)::value;
     if (sums == 0) return;
@@ -1416,7 +1420,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       const bool live = row < a.n - w.t * C;
       const __nv_bfloat16* raw = nullptr;
       uint4 raw_x[4];
-      if (PRE && elu) {
+      if (PRE && slope) {
         raw = static_cast<const __nv_bfloat16*>(a.raw) + ((size_t)w.bh * a.n + (size_t)w.t * C + (live ? row : 0)) * a.raw_pitch;
         raw_row32(raw_x, raw, half * (D / 2));
       }
@@ -1424,17 +1428,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       wait_or_fault(&l_done, one, &cta, fault, kFaultMmaWait);
       wait_or_fault(&b_done, one, &cta, fault, kFaultMmaWait);
       tc_fence_after_sync();
-      if (PRE && (elu || c != 1.f)) {
+      if (PRE && (slope || c != 1.f)) {
 #pragma unroll 1
         for (int cc = 0; cc < D / 64; ++cc) {
           const int col0 = half * (D / 2) + cc * 32;
-          stage_row32_chain(t_dk + lane_base + col0, sq[p], row, col0, raw_x, c, elu && live);
-          if (D > 64 && cc == 0 && elu) raw_row32(raw_x, raw, col0 + 32);
+          stage_row32_chain<PRE == 2>(t_dk + lane_base + col0, sq[p], row, col0, raw_x, c, slope && live);
+          if (D > 64 && cc == 0 && slope) raw_row32(raw_x, raw, col0 + 32);
         }
       }
       // dV's blocks, and dK's too unless the chain rule above has staged them: one loop
 #pragma unroll 1
-      for (int u = (elu || c != 1.f) ? D / 64 : 0; u < D / 64 + E / 64; ++u) {
+      for (int u = (slope || c != 1.f) ? D / 64 : 0; u < D / 64 + E / 64; ++u) {
         const bool dv_part = u >= D / 64;
         const int cc = dv_part ? u - D / 64 : u;
         const int col0 = half * ((dv_part ? E : D) / 2) + cc * 32;
@@ -1691,7 +1695,7 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), int grid, int threads, size_
 
 constexpr long long kFlagWaitClocks = 1000000000LL;   // about half a second
 
-template <int D, int E, bool DQ, bool FUSED, bool PRE, bool LINK>
+template <int D, int E, bool DQ, bool FUSED, int PRE, bool LINK>
 cudaError_t launch_walk_out_pre(const Dims& m, const void* x, const void* y, const void* z, void* out, WalkArgs a,
                             cudaStream_t st) {
   constexpr int WX = DQ ? E : D, WZ = DQ ? D : E;
@@ -1723,7 +1727,7 @@ cudaError_t launch_walk_out_pre(const Dims& m, const void* x, const void* y, con
   return launched(DQ ? "launch of the dq walk kernel" : "launch of the forward walk kernel");
 }
 
-template <int D, int E, bool FUSED, bool PRE, bool LINK>
+template <int D, int E, bool FUSED, int PRE, bool LINK>
 cudaError_t launch_walk_dkv_pre(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, void* dk,
                             void* dv, WalkArgs a, cudaStream_t st) {
   CUtensorMap mq, mk, mv, mdo, mdk, mdv;
@@ -1764,19 +1768,23 @@ cudaError_t launch_walk_out(const Dims& m, const void* x, const void* y, const v
   // ... and the hand-over code only in the launches of a sequence-parallel rank
   const bool linked = a.link.ranks > 0;
   if (has_qk_preprocessing(m)) {
+    const bool map_tiles = m.qk_map == LASP_QK_ELU1;
     if constexpr (FUSED) {
-      return linked ? launch_walk_out_pre<D, E, DQ, true, true, true>(m, x, y, z, out, a, st)
-                    : launch_walk_out_pre<D, E, DQ, true, true, false>(m, x, y, z, out, a, st);
+      if (linked) return launch_walk_out_pre<D, E, DQ, true, 1, true>(m, x, y, z, out, a, st);
+      if (map_tiles) return launch_walk_out_pre<D, E, DQ, true, 1, false>(m, x, y, z, out, a, st);
+      return m.qk_scale == 1.f ? launch_walk_out_pre<D, E, DQ, true, 0, false>(m, x, y, z, out, a, st)   // mapped: nothing is left to do
+                               : launch_walk_out_pre<D, E, DQ, true, 2, false>(m, x, y, z, out, a, st);
     } else if constexpr (DQ) {
-      return launch_walk_out_pre<D, E, true, false, true, false>(m, x, y, z, out, a, st);
+      return map_tiles ? launch_walk_out_pre<D, E, true, false, 1, false>(m, x, y, z, out, a, st)
+                       : launch_walk_out_pre<D, E, true, false, 2, false>(m, x, y, z, out, a, st);
     }
     g_failed_step = "q,k preprocessing is not part of the phase-by-phase schedule";
     return cudaErrorInvalidValue;
   }
   if constexpr (FUSED) {
-    if (linked) return launch_walk_out_pre<D, E, DQ, true, false, true>(m, x, y, z, out, a, st);
+    if (linked) return launch_walk_out_pre<D, E, DQ, true, 0, true>(m, x, y, z, out, a, st);
   }
-  return launch_walk_out_pre<D, E, DQ, FUSED, false, false>(m, x, y, z, out, a, st);
+  return launch_walk_out_pre<D, E, DQ, FUSED, 0, false>(m, x, y, z, out, a, st);
 }
 template <int D, int E, bool FUSED>
 cudaError_t launch_walk_dkv(const Dims& m, const void* q, const void* k, const void* v, const void* d_o, void* dk,
@@ -1784,16 +1792,17 @@ cudaError_t launch_walk_dkv(const Dims& m, const void* q, const void* k, const v
   const bool linked = a.link.ranks > 0;
   if (has_qk_preprocessing(m)) {
     if constexpr (FUSED) {
-      return linked ? launch_walk_dkv_pre<D, E, true, true, true>(m, q, k, v, d_o, dk, dv, a, st)
-                    : launch_walk_dkv_pre<D, E, true, true, false>(m, q, k, v, d_o, dk, dv, a, st);
+      if (linked) return launch_walk_dkv_pre<D, E, true, 1, true>(m, q, k, v, d_o, dk, dv, a, st);
+      return m.qk_map == LASP_QK_ELU1 ? launch_walk_dkv_pre<D, E, true, 1, false>(m, q, k, v, d_o, dk, dv, a, st)
+                                      : launch_walk_dkv_pre<D, E, true, 2, false>(m, q, k, v, d_o, dk, dv, a, st);
     }
     g_failed_step = "q,k preprocessing is not part of the phase-by-phase schedule";
     return cudaErrorInvalidValue;
   }
   if constexpr (FUSED) {
-    if (linked) return launch_walk_dkv_pre<D, E, true, false, true>(m, q, k, v, d_o, dk, dv, a, st);
+    if (linked) return launch_walk_dkv_pre<D, E, true, 0, true>(m, q, k, v, d_o, dk, dv, a, st);
   }
-  return launch_walk_dkv_pre<D, E, FUSED, false, false>(m, q, k, v, d_o, dk, dv, a, st);
+  return launch_walk_dkv_pre<D, E, FUSED, 0, false>(m, q, k, v, d_o, dk, dv, a, st);
 }
 
 }  // namespace
