@@ -124,6 +124,8 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
+// the same value in every lane, and known to be so
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 // registers per thread of the calling warpgroup (all four warps): given back / taken from what the block was
 // launched with.  The warpgroups' shares must add up to no more than that.
 template <int regs>
@@ -228,7 +230,8 @@ __host__ __device__ constexpr uint32_t umma_idesc(uint32_t m, uint32_t n, bool a
 }
 // One MMA of shape M x N x 16; accumulate = 0 overwrites the accumulator.  A descriptor is passed as its two words: the
 // steps of a product differ in the address field of the low one only.  Either one thread calls these, or a whole warp
-// whose lane with `leader` set issues: its operands then come from uniform registers without moves for every instruction.
+// whose elected lane (elect_one) issues: its operands then come from uniform registers without moves for every instruction,
+// which a single thread took two to three times as long to issue as the tensor cores to run.
 struct SmemDesc {
   uint32_t lo, hi;
 };
@@ -274,27 +277,28 @@ __device__ __forceinline__ SmemDesc operand_desc(uint32_t addr, uint32_t rows, b
 __device__ __forceinline__ SmemDesc operand_step(SmemDesc d, uint32_t rows, bool mn_major, uint32_t ks) {
   return {d.lo + (mn_major ? ks * 128 : (ks >> 2) * rows * 8 + (ks & 3) * 2), d.hi};
 }
-// D[128 x N] (+)= A x B over K; issued by ONE thread
+// D[128 x N] (+)= A x B over K; issued by one thread or an elected lane (see umma)
 template <bool A_MN, bool B_MN, int N, int K>
 __device__ __forceinline__ void umma_gemm(uint32_t d_tmem, uint32_t a_addr, uint32_t a_rows, uint32_t b_addr,
-                                          uint32_t b_rows, bool accumulate) {
+                                          uint32_t b_rows, bool accumulate, bool leader = true) {
   constexpr uint32_t idesc = umma_idesc(128, N, A_MN, B_MN);
   const SmemDesc a = operand_desc(a_addr, a_rows, A_MN), b = operand_desc(b_addr, b_rows, B_MN);
 #pragma unroll
   for (uint32_t ks = 0; ks < K / 16; ++ks)
-    umma(d_tmem, operand_step(a, a_rows, A_MN, ks), operand_step(b, b_rows, B_MN, ks), idesc, (accumulate || ks > 0) ? 1u : 0u);
+    umma(d_tmem, operand_step(a, a_rows, A_MN, ks), operand_step(b, b_rows, B_MN, ks), idesc, (accumulate || ks > 0) ? 1u : 0u, leader);
 }
 // D[128 x N] (+)= A x B over 128 K elements with A = a bf16 matrix in tensor memory, K elements 0..63 in columns
 // [0, 32) and 64..127 in columns [SECOND, SECOND + 32) of the region at a_tmem (what packing an fp32 accumulator in
 // place, half by half, leaves)
 template <bool B_MN, int N, int SECOND>
-__device__ __forceinline__ void umma_gemm_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_addr, uint32_t b_rows, bool accumulate) {
+__device__ __forceinline__ void umma_gemm_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_addr, uint32_t b_rows, bool accumulate,
+                                             bool leader = true) {
   constexpr uint32_t idesc = umma_idesc(128, N, false, B_MN);
   const SmemDesc b = operand_desc(b_addr, b_rows, B_MN);
 #pragma unroll
   for (uint32_t ks = 0; ks < 8; ++ks)
     umma_ts(d_tmem, a_tmem + (ks < 4 ? ks * 8 : SECOND + (ks - 4) * 8), operand_step(b, b_rows, B_MN, ks), idesc,
-            (accumulate || ks > 0) ? 1u : 0u);
+            (accumulate || ks > 0) ? 1u : 0u, leader);
 }
 
 // ---------------------------------------------------------------------------
@@ -326,14 +330,15 @@ inline int& last_encode_result() {
 // box = {64, box_rows, width/64, 1}: a tile never crosses from one sequence into the next
 // `pitch`: elements from one token's row to the next (= width for a tensor of its own; larger for a slice of the
 // head dimension of a wider tensor, which is then read and written in place)
+// `box_slabs`: 64-column slabs in a box, where that is not all of them
 inline cudaError_t make_seq_tile_map(CUtensorMap* map, const void* base, uint64_t seqs, uint64_t n, uint32_t width,
-                                     uint32_t box_rows, uint32_t pitch) {
+                                     uint32_t box_rows, uint32_t pitch, uint32_t box_slabs = 0) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return cudaErrorNotSupported;
   if (width % 64 || box_rows > 256 || n == 0 || seqs == 0 || pitch < width || pitch % 8) return cudaErrorInvalidValue;
   const cuuint64_t dims[4] = {64, n, width / 64, seqs};
   const cuuint64_t strides[3] = {(cuuint64_t)pitch * 2, 128, (cuuint64_t)n * pitch * 2};  // bytes, dims 1..3
-  const cuuint32_t box[4] = {64, box_rows, width / 64, 1};
+  const cuuint32_t box[4] = {64, box_rows, box_slabs ? box_slabs : width / 64, 1};
   const cuuint32_t elem[4] = {1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, elem,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

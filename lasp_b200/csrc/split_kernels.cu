@@ -194,30 +194,6 @@ __device__ __forceinline__ void issue_terms(uint32_t d_tmem, const A& a, const T
   }
 }
 __device__ __forceinline__ int ksteps_of(int width, int chunk) { return max(min(width - 64 * chunk, 64), 0) / 16; }
-// the same value in every lane, and known to be so
-__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
-
-// Four 16-byte pieces of a row in each of four neighbouring lanes change hands so that piece i of every lane belongs to the
-// i-th of the four rows: stored piece by piece, four lanes then write 64 bytes of one row.  (As they are, the 32 lanes of a
-// store write 16 bytes of 32 rows, a cache line each: 64 KB of results took the load-store unit 5600 clocks, in which the
-// filling warps' loads stood still too.)
-__device__ __forceinline__ void rows_to_lanes(uint4 (&v)[4], int lane) {
-#pragma unroll
-  for (int s = 1; s <= 2; s *= 2) {
-    const bool high = lane & s;
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int i = s == 1 ? 2 * u : u, j = i + s;   // the pair of pieces of which this lane keeps one and sends the other
-      uint32_t* a = reinterpret_cast<uint32_t*>(&v[i]);
-      uint32_t* b = reinterpret_cast<uint32_t*>(&v[j]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? a[q] : b[q], s);
-        (high ? a[q] : b[q]) = got;
-      }
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------
 // Outside the terms' range.  Infinities, and finite values above bf16's largest, have an infinite first term and a

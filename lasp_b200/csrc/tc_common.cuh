@@ -127,6 +127,28 @@ __device__ __forceinline__ void stage_row32(uint32_t taddr, uint8_t* tile, int r
   }
 }
 
+// Four 16-byte pieces of a row in each of four neighbouring lanes change hands so that piece i of every lane belongs to the
+// i-th of the four rows: stored piece by piece, four lanes then write 64 bytes of one row.  (As they are, the 32 lanes of a
+// store write 16 bytes of 32 rows, a cache line each: 64 KB of results took the load-store unit 5600 clocks, in which the
+// filling warps' loads stood still too.)
+__device__ __forceinline__ void rows_to_lanes(uint4 (&v)[4], int lane) {
+#pragma unroll
+  for (int s = 1; s <= 2; s *= 2) {
+    const bool high = lane & s;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = s == 1 ? 2 * u : u, j = i + s;   // the pair of pieces of which this lane keeps one and sends the other
+      uint32_t* a = reinterpret_cast<uint32_t*>(&v[i]);
+      uint32_t* b = reinterpret_cast<uint32_t*>(&v[j]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, high ? a[q] : b[q], s);
+        (high ? a[q] : b[q]) = got;
+      }
+    }
+  }
+}
+
 // Decay mask.  32 fp32 accumulator columns at `src` (columns col0 .. col0+31 of a score tile, this thread's lane = row)
 // become 16 columns of masked bf16 pairs, which the caller leaves in tensor memory as the A operand of the next MMA.
 // Per group of eight columns the factor is built from the group's live column nearest the diagonal away from it by

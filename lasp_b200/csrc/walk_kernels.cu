@@ -482,7 +482,7 @@ __device__ __forceinline__ void write_state_operand(uint8_t* tile, int rows, int
 // Tensor memory: S (two buffers; the masked scores are packed to bf16 over S itself and feed O1 as its A
 // operand from tensor memory), O (X op(P), rows scaled by lambda^r in place, += S_m Z), L = the state update.
 //   warp 0 (one lane)  producer: loads, and the TMA stores of the finished staging tiles
-//   warps 1-3 (one lane each)  tensor-core issuers
+//   warps 1-3          tensor-core issuers
 //   warps 4-11  (A)    mask of the scores, epilogue
 //   warps 12-19 (B)    the state chain: scaling of Y's rows, of O2's rows, state update
 // Two groups because one group of eight warps doing all of it was the serial chain of a tile: 5300 clocks against
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
   __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x, even_s;
   __shared__ Health<LINK> cta;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)uniform(tid >> 5), lane = tid & 31;
   int32_t* fault = a.fault;
   // Thread 0 is also the producer: it asks for its first tiles before the CTA-wide barrier below, so that their
   // flight overlaps the rest of the set-up (what it issued is remembered in early_*; only its copy matters).
@@ -731,23 +731,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         }
         bulk_wait_all<0>();
       }
-    } else if (lane == 0) {
-      // Three issuing threads, so that no product waits behind another one's issue (eight instructions of 64 tensor
-      // clocks each take the issuing thread about as long) and none of them has to poll for what is ready:
+    } else {
+      // Three issuing warps, so that no product waits behind another one's issue and none of them has to poll for what is
+      // ready.  A whole warp each, an elected lane of which issues (see umma): a thread of its own took 130 to 160 clocks for
+      // an instruction of 64.  8 x 32 x 2048 111 / 108 / 170 -> 99 / 94 / 153 us, 3 x 12 x 3001 36.9 / 26.4 / 47.0 -> 35.1 /
+      // 26.1 / 43.8, 16 x 16384 71.5 / 53.9 / 98 -> 67.4 / 49.7 / 90:
       //   warp 1  the span total; O2 = X op(P), then O1 = S_m Z on top of the row-scaled O2
       //   warp 2  L = K^T diag(w) V (d x e), the scaled rows being Y's
       //   warp 3  S = X Y^T of the next tile
+      const bool leader = elect_one();
       const bool map_xy = PRE == 1 && a.elu && !DQ, map_z = PRE == 1 && a.elu && DQ;
       if (warp == 1 && sums > 0) {
 #pragma unroll 1
         for (int g = 0; g < sums; ++g) {
           const int j = g % R::kStages;
           wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm<true, true, E, C>(t_l, smem_u32(ring.a(j)), C, smem_u32(ring.b(j)), C, g > 0);
-          umma_commit(&ring_empty[j]);
+          umma_gemm<true, true, E, C>(t_l, smem_u32(ring.a(j)), C, smem_u32(ring.b(j)), C, g > 0, leader);
+          if (leader) umma_commit(&ring_empty[j]);
         }
-        umma_commit(&sum_done);
+        if (leader) umma_commit(&sum_done);
       }
       int total = 0;
 #pragma unroll 1
@@ -761,20 +765,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (i >= 1) wait_or_fault(&o_free, one ^ 1, &cta, fault, kFaultMmaWait);
           wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
           if constexpr (!DQ)  // X P: the state tile as [K = d rows] x [N = e columns]
-            umma_gemm<false, true, E, D>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false);
+            umma_gemm<false, true, E, D>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false, leader);
           else                // X P^T: the state tile as [N = d rows] x [K = e columns]
-            umma_gemm<false, false, D, E>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false);
-          umma_commit(&o2_full[p]);
+            umma_gemm<false, false, D, E>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false, leader);
+          if (leader) umma_commit(&o2_full[p]);
           // the masked scores are read from tensor memory
           wait_or_fault(&sm_ready[p], ph, &cta, fault, kFaultMmaWait);
           wait_or_fault(&z_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           wait_or_fault(&o2s_ready, one, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm_ts<true, WZ, 64>(t_o, t_s[p], smem_u32(sz[p]), C, true);
-          umma_commit(&o_full[p]);
+          umma_gemm_ts<true, WZ, 64>(t_o, t_s[p], smem_u32(sz[p]), C, true, leader);
+          if (leader) umma_commit(&o_full[p]);
         }
       } else if (warp == 2) {
 #pragma unroll 1
@@ -784,12 +790,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&l_free, one ^ 1, &cta, fault, kFaultMmaWait);   // the state update has read the previous L
           wait_or_fault(&ys_ready, one, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
           if constexpr (!DQ)
-            umma_gemm<true, true, E, C>(t_l, smem_u32(sy[p]), C, smem_u32(sz[p]), C, false);
+            umma_gemm<true, true, E, C>(t_l, smem_u32(sy[p]), C, smem_u32(sz[p]), C, false, leader);
           else
-            umma_gemm<true, true, E, C>(t_l, smem_u32(sz[p]), C, smem_u32(sy[p]), C, false);
-          umma_commit(&l_full[p]);
+            umma_gemm<true, true, E, C>(t_l, smem_u32(sz[p]), C, smem_u32(sy[p]), C, false, leader);
+          if (leader) umma_commit(&l_full[p]);
         }
       } else {
 #pragma unroll 1
@@ -799,9 +806,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
           wait_or_fault(&y_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm<false, false, C, WX>(t_s[p], smem_u32(sx[p]), C, smem_u32(sy[p]), C, false);
-          umma_commit(&s_full[p]);
+          umma_gemm<false, false, C, WX>(t_s[p], smem_u32(sx[p]), C, smem_u32(sy[p]), C, false, leader);
+          if (leader) umma_commit(&s_full[p]);
         }
       }
     }
@@ -1116,7 +1124,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x;
   __shared__ Health<LINK> cta;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)uniform(tid >> 5), lane = tid & 31;
   int32_t* fault = a.fault;
   // thread 0 is also the producer: its first loads go out before the CTA-wide barrier (see k_walk_out)
   bool early_ring = false, early_q = false;
@@ -1304,17 +1312,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         }
         bulk_wait_all<0>();
       }
-    } else if (lane == 0) {
+    } else {
+      const bool leader = elect_one();   // (see k_walk_out)
       if (warp == 1 && sums > 0) {
 #pragma unroll 1
         for (int g = 0; g < sums; ++g) {
           const int j = g % R::kStages;
           wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm<true, true, E, C>(t_s, smem_u32(ring_buf.a(j)), C, smem_u32(ring_buf.b(j)), C, g > 0);
-          umma_commit(&ring_empty[j]);
+          umma_gemm<true, true, E, C>(t_s, smem_u32(ring_buf.a(j)), C, smem_u32(ring_buf.b(j)), C, g > 0, leader);
+          if (leader) umma_commit(&ring_empty[j]);
         }
-        umma_commit(&sum_done);
+        if (leader) umma_commit(&sum_done);
       }
       int total = 0;
 #pragma unroll 1
@@ -1329,19 +1339,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&dn_ready, one, &cta, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&e_free, one ^ 1, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm<false, false, D, E>(t_dk, smem_u32(sv), C, smem_u32(sdn), D, false);
-          umma_gemm<false, true, E, D>(t_dv, smem_u32(sk), C, smem_u32(sdn), D, false);
-          umma_commit(&st_done);
+          umma_gemm<false, false, D, E>(t_dk, smem_u32(sv), C, smem_u32(sdn), D, false, leader);
+          umma_gemm<false, true, E, D>(t_dv, smem_u32(sk), C, smem_u32(sdn), D, false, leader);
+          if (leader) umma_commit(&st_done);
           // the masked scores' products on top, A operands from tensor memory
           wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&scaled, one, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm_ts<true, E, 96>(t_dv, t_s, smem_u32(sdo[p]), C, true);    // += S_m^T dO
+          umma_gemm_ts<true, E, 96>(t_dv, t_s, smem_u32(sdo[p]), C, true, leader);    // += S_m^T dO
           wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm_ts<true, D, 96>(t_dk, t_ds, smem_u32(sq[p]), C, true);    // += dS_m^T Q
-          umma_commit(&b_done);
+          umma_gemm_ts<true, D, 96>(t_dk, t_ds, smem_u32(sq[p]), C, true, leader);    // += dS_m^T Q
+          if (leader) umma_commit(&b_done);
         }
       } else if (warp == 2) {
 #pragma unroll 1
@@ -1352,11 +1365,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
           if (E > 64) wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&qs_ready, one, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm<true, true, 64, C>(t_s + 32, smem_u32(sdn), C, smem_u32(sdo[p]), C, false);
+          umma_gemm<true, true, 64, C>(t_s + 32, smem_u32(sdn), C, smem_u32(sdo[p]), C, false, leader);
           if constexpr (E > 64)   // columns 64..127 of dO: its second slab
-            umma_gemm<true, true, 64, C>(t_ds + 32, smem_u32(sdn), C, smem_u32(sdo[p]) + C * kSlabRowBytes, C, false);
-          umma_commit(&l_done);
+            umma_gemm<true, true, 64, C>(t_ds + 32, smem_u32(sdn), C, smem_u32(sdo[p]) + C * kSlabRowBytes, C, false, leader);
+          if (leader) umma_commit(&l_done);
         }
       } else {
 #pragma unroll 1
@@ -1369,11 +1383,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&qdo_full[p], (i >> 1) & 1, &cta, fault, kFaultTmaWait);
           wait_or_fault(&kv_full, one, &cta, fault, kFaultTmaWait);
           if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
+          __syncwarp();
           tc_fence_after_sync();
-          umma_gemm<false, false, C, D>(t_s, smem_u32(sk), C, smem_u32(sq[p]), C, false);
-          umma_commit(&s_done);
-          umma_gemm<false, false, C, E>(t_ds, smem_u32(sv), C, smem_u32(sdo[p]), C, false);
-          umma_commit(&ds_done);
+          umma_gemm<false, false, C, D>(t_s, smem_u32(sk), C, smem_u32(sq[p]), C, false, leader);
+          if (leader) umma_commit(&s_done);
+          umma_gemm<false, false, C, E>(t_ds, smem_u32(sv), C, smem_u32(sdo[p]), C, false, leader);
+          if (leader) umma_commit(&ds_done);
         }
       }
     }
