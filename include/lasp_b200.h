@@ -215,6 +215,14 @@ LASP_B200_API int lasp_b200_backward_opt(const lasp_problem* p, const lasp_bwd_a
 
 /* x_out = exp(-s_h n) x_in + x_local on (b,h,d,e) fp32 states; x_in may be NULL.
  * Replaces the torch glue KV = block_decay*KV + kv, lasp/lasp_naive.py:565,614. */
+/* Heads of 256 (d = e = 256) in bf16, n >= 128, without rank states, preprocessing or row pitches: each result in one pass
+ * instead of four 128-wide slice pairs.  wide_ok: 1 where these are the faster way for the forward or the backward pass on
+ * the current device, 0 where the slices are, a negative status where the problem is not of this kind.  The two passes are
+ * independent of one another; kv_in, kv_out, dkv_in, dkv_out must be NULL, the workspaces are not looked at. */
+LASP_B200_API int lasp_b200_wide_ok(const lasp_problem* p, int backward);
+LASP_B200_API int lasp_b200_forward_wide(const lasp_problem* p, const lasp_fwd_args* a, void* stream);
+LASP_B200_API int lasp_b200_backward_wide(const lasp_problem* p, const lasp_bwd_args* a, void* stream);
+
 LASP_B200_API int lasp_b200_state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
                             const float* x_local, float* x_out, void* stream);
 

@@ -89,6 +89,9 @@ SIGNATURES = {
     "lasp_b200_map_qk": (C.c_int, [C.c_void_p] * 4 + [C.c_int64, C.c_void_p]),
     "lasp_b200_forward_opt": (C.c_int, [_PP, _FP, C.POINTER(CallOptions), C.c_void_p]),
     "lasp_b200_backward_opt": (C.c_int, [_PP, _BP, C.POINTER(CallOptions), C.c_void_p]),
+    "lasp_b200_wide_ok": (C.c_int, [_PP, C.c_int]),
+    "lasp_b200_forward_wide": (C.c_int, [_PP, _FP, C.c_void_p]),
+    "lasp_b200_backward_wide": (C.c_int, [_PP, _BP, C.c_void_p]),
     "lasp_b200_state_combine": (C.c_int, [C.c_int] * 5 + [C.c_void_p] * 5),
     "lasp_b200_read_status": (C.c_int, [C.POINTER(C.c_int32), C.c_int, C.c_void_p]),
     "lasp_b200_copy_status_async": (C.c_int, [C.c_void_p, C.c_void_p]),

@@ -19,7 +19,7 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "liblasp_b200.so")
 TORCH_OPS = os.path.join(PKG, "_torch_ops.so")   # the operator as PyTorch calls it, on top of LIB
-SOURCES = ["api.cu", "split_kernels.cu", "state_kernels.cu", "fault_word.cu", "walk_kernels.cu", "relay_kernels.cu", "static_scratch.cu"]
+SOURCES = ["api.cu", "split_kernels.cu", "state_kernels.cu", "fault_word.cu", "walk_kernels.cu", "wide_kernels.cu", "relay_kernels.cu", "static_scratch.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

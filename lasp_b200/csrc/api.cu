@@ -415,6 +415,52 @@ int lasp_b200_backward(const lasp_problem* p, const lasp_bwd_args* a, void* stre
   return lasp_b200_backward_opt(p, a, &kPlainCall, stream);
 }
 
+// ---- 256-wide heads ---------------------------------------------------------
+static int check_wide(const lasp_problem* p) {
+  if (!p) return LASP_ERR_NULL;
+  bind_context_once();
+  if (p->dtype != LASP_BF16) return p->dtype == LASP_F32 || p->dtype == LASP_F16 ? LASP_ERR_PATH : LASP_ERR_DTYPE;
+  if (p->b <= 0 || p->h <= 0 || p->n < lasp::kTensorTile || p->d != 256 || p->e != 256 || (long long)p->b * p->h > 65535) return LASP_ERR_SHAPE;
+  if ((p->pitch_d && p->pitch_d != 256) || (p->pitch_e && p->pitch_e != 256)) return LASP_ERR_SHAPE;
+  if (p->qk_map != LASP_QK_IDENTITY || (p->qk_scale != 0.f && p->qk_scale != 1.f)) return LASP_ERR_PATH;
+  if (p->path != LASP_PATH_AUTO && p->path != LASP_PATH_TENSOR) return LASP_ERR_PATH;
+  return LASP_OK;
+}
+
+int lasp_b200_wide_ok(const lasp_problem* p, int backward) {
+  const int st = check_wide(p);
+  if (st != LASP_OK) return st;
+  // A walk goes over whole sequences, the slices cut them in spans: with few, long sequences those fill the chip and this
+  // does not.  Measured with decay (forward / backward alone, b*h sequences of t tiles): walks 4.4 us a tile and wave of CTAs
+  // plus 10; slices 55 + 0.14 / 140 + 0.24 us per sequence and tile.  64 x 32 tiles 168 / 447 against 306 / 628 us, 24 x 32 153 /
+  // 159 against 149 / 319, 16 x 64 295 / 302 against 195 / 386, 8 x 64 290 / 292 against 133 / 257.
+  const long long seqs = (long long)p->b * p->h, tiles = (p->n + lasp::kTensorTile - 1) / lasp::kTensorTile;
+  const long long waves = ((backward ? 6 : 2) * seqs + lasp::sm_count() - 1) / lasp::sm_count();
+  const long long walk = 440 * tiles * waves + 1000, slices = (backward ? 14000 + 24 * seqs * tiles : 5500 + 14 * seqs * tiles);   // 10 ns
+  return walk < slices ? 1 : 0;
+}
+
+int lasp_b200_forward_wide(const lasp_problem* p, const lasp_fwd_args* a, void* stream) {
+  const int st = check_wide(p);
+  if (st != LASP_OK) return st;
+  if (!a || !a->q || !a->k || !a->v || !a->s || !a->o) return LASP_ERR_NULL;
+  if (a->kv_in || a->kv_out) return LASP_ERR_SHAPE;
+  if (!aligned16(a->q) || !aligned16(a->k) || !aligned16(a->v) || !aligned16(a->o)) return LASP_ERR_ALIGN;
+  return cuda_fail(lasp::wide_forward(p->b, p->h, p->n, a->q, a->k, a->v, a->s, a->o, static_cast<cudaStream_t>(stream)));
+}
+
+int lasp_b200_backward_wide(const lasp_problem* p, const lasp_bwd_args* a, void* stream) {
+  const int st = check_wide(p);
+  if (st != LASP_OK) return st;
+  if (!a || !a->q || !a->k || !a->v || !a->d_o || !a->s || !a->dq || !a->dk || !a->dv) return LASP_ERR_NULL;
+  if (a->dkv_in || a->dkv_out) return LASP_ERR_SHAPE;
+  if (!aligned16(a->q) || !aligned16(a->k) || !aligned16(a->v) || !aligned16(a->d_o) || !aligned16(a->dq) || !aligned16(a->dk) ||
+      !aligned16(a->dv))
+    return LASP_ERR_ALIGN;
+  return cuda_fail(lasp::wide_backward(p->b, p->h, p->n, a->q, a->k, a->v, a->d_o, a->s, a->dq, a->dk, a->dv,
+                                       static_cast<cudaStream_t>(stream)));
+}
+
 int lasp_b200_state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
                             const float* x_local, float* x_out, void* stream) {
   if (!s || !x_local || !x_out) return LASP_ERR_NULL;

@@ -132,6 +132,11 @@ cudaError_t exchange_scan(const Dims& m, const lasp_exchange_args& a, const floa
 // tcgen05 path
 bool tensor_path_supported(const Dims& m);
 
+// 256-wide heads in one pass per result (wide_kernels.cu)
+cudaError_t wide_forward(int b, int h, int n, const void* q, const void* k, const void* v, const float* s, void* o, cudaStream_t st);
+cudaError_t wide_backward(int b, int h, int n, const void* q, const void* k, const void* v, const void* d_o, const float* s, void* dq,
+                          void* dk, void* dv, cudaStream_t st);
+
 // tcgen05 path with the state carried on chip (walk_kernels.cu)
 cudaError_t walk_span_totals(const Dims& m, const void* a, const void* bten, const float* s, float* totals,
                              bool reverse, cudaStream_t st);

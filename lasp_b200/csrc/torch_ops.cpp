@@ -184,11 +184,27 @@ std::vector<Pair> slice_pairs(const Shape& m, int32_t dtype, double scale, int64
 
 char* column(const Tensor& t, int64_t col) { return static_cast<char*>(t.data_ptr()) + col * t.element_size(); }
 
+// Heads of 256: whether each result is made in one pass (1) or slice by slice
+bool in_one_pass(const Shape& m, int32_t dtype, double scale, int64_t map, bool backward, lasp_problem* p) {
+  if (m.d != 256 || m.e != 256) return false;
+  *p = problem_of(m, m.d, m.e, dtype, scale, map, false);
+  return lasp_b200_wide_ok(p, backward ? 1 : 0) == 1;
+}
+
 std::vector<Tensor> run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s, const Shape& m,
                                 double scale, int64_t map, bool keep) {
   const c10::cuda::CUDAGuard guard(q.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   Tensor o = at::empty({m.b, m.h, m.n, m.e}, q.options());
+  lasp_problem wide;
+  if (keep && in_one_pass(m, lasp_dtype_of(q.scalar_type()), scale, map, true, &wide)) keep = false;   // such a backward pass needs no states
+  if (!keep && in_one_pass(m, lasp_dtype_of(q.scalar_type()), scale, map, false, &wide)) {
+    lasp_fwd_args a = {};
+    a.q = q.data_ptr(), a.k = k.data_ptr(), a.v = v.data_ptr(), a.s = s.const_data_ptr<float>(), a.o = o.data_ptr();
+    Range range("lasp_b200_forward");
+    check_status("lasp_b200_forward_wide", lasp_b200_forward_wide(&wide, &a, stream.stream()));
+    return {o};
+  }
   const Tensor sync = sync_words(q.device(), stream);
   std::vector<Tensor> out{o};
   Tensor ws;
@@ -270,6 +286,16 @@ class Lightning : public torch::autograd::Function<Lightning> {
     const c10::cuda::CUDAGuard guard(q.device());
     const auto stream = at::cuda::getCurrentCUDAStream();
     Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options()), dv = at::empty(v.sizes(), v.options());
+    if (saved.size() == first_ws) {   // the forward pass has left no states: each result in one pass
+      lasp_problem wide = problem_of(m, m.d, m.e, lasp_dtype_of(q.scalar_type()), 1.0, LASP_QK_IDENTITY, false);
+      wide.path = LASP_PATH_TENSOR;
+      lasp_bwd_args a = {};
+      a.q = q.data_ptr(), a.k = k.data_ptr(), a.v = v.data_ptr(), a.d_o = d_o.data_ptr(), a.s = s.const_data_ptr<float>();
+      a.dq = dq.data_ptr(), a.dk = dk.data_ptr(), a.dv = dv.data_ptr();
+      Range range("lasp_b200_backward");
+      check_status("lasp_b200_backward_wide", lasp_b200_backward_wide(&wide, &a, stream.stream()));
+      return {dq, dk, dv, Tensor(), Tensor(), Tensor()};
+    }
     const Tensor sync = sync_words(q.device(), stream);
     Tensor ws;
     const std::vector<Pair> pairs = slice_pairs(m, lasp_dtype_of(q.scalar_type()), ctx->saved_data["scale"].toDouble(), map);
