@@ -1121,7 +1121,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   __shared__ uint64_t qdo_full[2], staged[2];
   __shared__ uint64_t kv_full, dn_ready, st_done, s_done, ds_done, sm_ready, dsm_ready, qs_ready, scaled, l_done, l_free, b_done, e_free;
   __shared__ uint64_t mapped;   // with a feature map: the workers have mapped the tile's Q and K in place
-  __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done;   // the span-total phase
+  __shared__ uint64_t ring_full[kMaxRing], ring_scaled[kMaxRing], ring_empty[kMaxRing], sum_done, total_read;   // the span-total phase
   __shared__ uint32_t tmem_slot, step_s, step_x;
   __shared__ Health<LINK> cta;
   const int tid = threadIdx.x, warp = (int)uniform(tid >> 5), lane = tid & 31;
@@ -1154,6 +1154,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     mbar_init(&l_done, 1);
     mbar_init(&b_done, 1);
     mbar_init(&sum_done, 1);
+    mbar_init(&total_read, 2 * kWorkers / 32);
     mbar_init(&dn_ready, kWorkers);
     mbar_init(&sm_ready, kWorkers);
     mbar_init(&dsm_ready, kWorkers);
@@ -1239,6 +1240,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       store_state32<D>(a.totals + (size_t)my_item() * D * E, row, c0, r);
     }
     tc_fence_before_sync();
+    warp_arrive(&total_read);      // (S^T takes the total's place in tensor memory)
     named_sync(2, 2 * kWorkers);   // every worker's part of the total is written ...
     if (tid == kFirstWorker) {
       __threadfence();             // ... and visible to the other CTAs before the flag is
@@ -1379,6 +1381,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           if (i >= 1) {   // the masked scores and L of tile i-1 have been read
             wait_or_fault(&b_done, one ^ 1, &cta, fault, kFaultMmaWait);
             wait_or_fault(&l_free, one ^ 1, &cta, fault, kFaultMmaWait);
+          } else if (sums > 0) {
+            wait_or_fault(&total_read, 0, &cta, fault, kFaultMmaWait);
           }
           wait_or_fault(&qdo_full[p], (i >> 1) & 1, &cta, fault, kFaultTmaWait);
           wait_or_fault(&kv_full, one, &cta, fault, kFaultTmaWait);
