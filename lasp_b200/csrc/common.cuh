@@ -108,6 +108,28 @@ cudaError_t opt_in_smem(size_t bytes) {
   return err;
 }
 
+// The kernels of the full-precision path follow one another closely (states, scan, outputs): each lets the next one's CTAs
+// take an SM as soon as its own have left it, and waits itself, before it touches global memory, for what came before it to
+// be complete.  (A CTA of the next kernel cannot start before all of this one's have: they call this first thing.)
+__device__ __forceinline__ void follow_on() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_following(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // ---- launchers implemented in the .cu files (return cudaError_t) -----------
 // Full-precision path (split_kernels.cu).  `alone`: no rank state comes in or goes out, so the states at the
 // sequence's ends are zero or unread.

@@ -286,6 +286,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) k_split_states(const __grid_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;   // [parity of the task][chunk], 128 columns each
+  follow_on();
   const auto next_task = [&](int t) {
     while (t < g.tasks && t % g.nc == g.skip) t += gridDim.x;
     return t;
@@ -665,6 +666,7 @@ __global__ void __launch_bounds__(kOutThreads<T>, 1) k_split_out(const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
+  follow_on();
 
   struct Task {
     OutRole r;
@@ -1033,8 +1035,7 @@ cudaError_t launch_states(const Dims& m, const StateArgs& g, cudaStream_t st) {
   if (StatePlan<T>::kTmaB && (err = matrix_map(&map_b, g.b, (size_t)m.b * m.h, m.n, m.e, m.pitch_e)) != cudaSuccess) return err;
   if ((err = opt_in_smem<k_split_states<T>>(StatePlan<T>::kSmem)) != cudaSuccess) return err;
   const int grid = g.tasks < sm_count() ? g.tasks : sm_count();
-  k_split_states<T><<<grid, kStateThreads, StatePlan<T>::kSmem, st>>>(map_b, g);
-  err = cudaGetLastError();
+  err = launch_following(k_split_states<T>, dim3(grid), kStateThreads, StatePlan<T>::kSmem, st, map_b, g);
   if (err != cudaSuccess) g_failed_step = "launch of the chunk-state kernel";
   return err;
 }
@@ -1045,8 +1046,7 @@ cudaError_t launch_out(const OutMaps& maps, const OutArgs& g, cudaStream_t st) {
   cudaError_t err = opt_in_smem<k_split_out<T, ADD>>(smem);
   if (err != cudaSuccess) return err;
   const int grid = g.tasks < sm_count() ? g.tasks : sm_count();
-  k_split_out<T, ADD><<<grid, kOutThreads<T>, smem, st>>>(maps, g);
-  err = cudaGetLastError();
+  err = launch_following(k_split_out<T, ADD>, dim3(grid), kOutThreads<T>, smem, st, maps, g);
   if (err != cudaSuccess) g_failed_step = "launch of the output kernel";
   return err;
 }

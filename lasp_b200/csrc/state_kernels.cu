@@ -21,6 +21,7 @@ __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const
                                               float* __restrict__ x_out, int h,
                                               int n, int de, int nc, int chunk, int reverse, int rows,
                                               int cols) {
+  if (TERMS) follow_on();
   const int bh = blockIdx.y;
   const int el = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (el >= de) return;
@@ -110,8 +111,10 @@ cudaError_t scan_states(const Dims& m, const float* s, const float* local, void*
                         float* x_out, bool reverse, cudaStream_t st) {
   const int de = m.d * m.e;
   dim3 grid((de / 4 + 255) / 256, m.b * m.h);
-  auto* kernel = m.walk ? k_scan<false> : k_scan<true>;
-  kernel<<<grid, 256, 0, st>>>(s, local, prefix, x_in, x_out, m.h, m.n, de, m.nc, m.chunk, reverse ? 1 : 0, m.d, m.e);
+  if (!m.walk)
+    return launch_following(k_scan<true>, grid, 256, 0, st, s, local, prefix, x_in, x_out, m.h, m.n, de, m.nc, m.chunk, reverse ? 1 : 0, m.d,
+                            m.e);
+  k_scan<false><<<grid, 256, 0, st>>>(s, local, prefix, x_in, x_out, m.h, m.n, de, m.nc, m.chunk, reverse ? 1 : 0, m.d, m.e);
   return cudaGetLastError();
 }
 
