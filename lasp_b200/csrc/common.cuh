@@ -110,7 +110,8 @@ cudaError_t opt_in_smem(size_t bytes) {
 
 // The kernels of the full-precision path follow one another closely (states, scan, outputs): each lets the next one's CTAs
 // take an SM as soon as its own have left it, and waits itself, before it touches global memory, for what came before it to
-// be complete.  (A CTA of the next kernel cannot start before all of this one's have: they call this first thing.)
+// be complete.  (A CTA of the next kernel cannot start before all of this one's have: they call this first thing.)  Training
+// passes of 2 x 12 x 2048: fp32 219 -> 212 us, fp16 122 -> 116.5; the walk kernels' passes got 1 to 2 % longer with it.
 __device__ __forceinline__ void follow_on() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -27,8 +27,8 @@
 // splitting, storing and meeting at barriers, results written 16 bytes of 32 rows at a time, the states split once per
 // product) a dQ, dK or dV task of fp32 took 32000 clocks, now 22000; of bf16 16000, now 8400.
 //
-// One B200, b=2, h=12, n=2048, forward / backward in us, in step and now: fp32 d=e=128 82.7 / 160 -> 70.6 / 119, fp16 d=128, e=64
-// 47.8 / 90 -> 43.0 / 68, fp16 d=e=128 57.7 / 111 -> 53.5 / 78, bf16 d=e=96 44.3 / 83 -> 36.9 / 53.  The error against
+// One B200, b=2, h=12, n=2048, forward / backward in us, in step and now: fp32 d=e=128 82.7 / 160 -> 69.5 / 119, fp16 d=128, e=64
+// 47.8 / 90 -> 44 / 72, fp16 d=e=128 57.7 / 111 -> 53.4 / 82, bf16 d=e=96 44.3 / 83 -> 36.8 / 55.  The error against
 // fp64, relative to what it was then: fp32 results 0.79 to 0.87, rank states of all types 0.61 to 0.87, fp16 and bf16 results 1.00
 // (a chunk of 64 elements of K is summed in an accumulator of its own, and the tensor cores' additions round towards zero).
 #include <type_traits>

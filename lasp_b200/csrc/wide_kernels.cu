@@ -18,7 +18,9 @@
 // at the ends of the sequences.
 //
 // What bounds it: the chain of a tile (S, mask, O1, state update and operand, all tiles of a step in single buffers: X, Y,
-// the state operand 64 KB each, Z 32 KB), then HBM.  Tensor work of a tile is 3584 clocks, its bytes 192 KB.
+// the state operand 64 KB each, Z 32 KB), then HBM.  A tile takes 5400 clocks, 3584 of them tensor work, for 192 KB.  b=4, h=16,
+// n=4096, no decay, slices and now: forward 326 -> 138 us, training 984 -> 476 (1044 -> 544 under the power cap); with decay 306 -> 162
+// and 934 -> 556.  Error against fp64 2.4e-3 to 3.2e-3 -> 1.8e-3 to 2.7e-3.  The next tile's X, Y, Z asked into L2 ahead: 8 % slower.
 #include <stdio.h>
 
 #include "tc_common.cuh"
@@ -218,8 +220,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
       wait_or_fault(&o_done, ph, &cta, fault, kFaultMmaWait);
       __syncwarp();
       tc_fence_after_sync();
-      // Straight to memory, four lanes 64 bytes of a row: through a staging tile over Z and a TMA store, Z's next tile, and
-      // with it L, Y and S, came 2000 clocks later (7000 of a tile in all, now 5500).
+      // Straight to memory, four lanes 64 bytes of a row, so that Z's buffer is free for the next tile at once.  (Through a
+      // staging tile over Z and a TMA store, no decay: 4 x 16 x 4096 training 505 instead of 476 us, 2 x 24 x 2048 215 instead
+      // of 197; with decay, where the scaling of rows is longer than Z's way, even.)
       const int row4 = w.t * C + (row & ~3);
       __nv_bfloat16* out = a.out[w.r.out] + ((size_t)w.bh * a.n + row4) * W + N * w.half + 8 * (lane & 3);
 #pragma unroll 1
