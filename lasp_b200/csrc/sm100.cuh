@@ -118,8 +118,9 @@ template <int pending>
 __device__ __forceinline__ void bulk_wait_all() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(pending) : "memory");
 }
-// named barrier over `count` threads (count a multiple of 32); id 1..15
+// named barrier over `count` threads (count a multiple of 32); id 1..15.  A warp arrives as one, its lanes together.
 __device__ __forceinline__ void named_sync(int id, int count) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 // true in one lane of the (whole) calling warp, and known to be so: what a single thread issues needs no code for several
@@ -160,6 +161,12 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t ncols) {
 }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// ... for a whole warp whose lanes have waited each for itself and may have left the wait one by one: what follows (tensor-
+// memory loads and stores, MMAs by an elected lane) is for all of them together, and undefined otherwise
+__device__ __forceinline__ void tc_fence_after_wait() {
+  __syncwarp();
+  tc_fence_after_sync();
+}
 
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base lane + t)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {

@@ -305,8 +305,7 @@ __global__ void __launch_bounds__(kStateThreads, 1) k_split_states(const __grid_
         for (int c = 0; c < 2; ++c) {
           wait_or_fault(&full_a[c], it & 1, &cta, g.fault, kFaultTmaWait);
           wait_or_fault(&full_b[c], it & 1, &cta, g.fault, kFaultTmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           const uint32_t at = base + c * Plan::kChunk * kUnit;
           uint32_t acc = 0;
           issue_terms<TT::mid, TT::in, TT::cut, 0>(t_acc + 256 * (it & 1) + 128 * c, TermOperand(at, 64, true),
@@ -337,13 +336,13 @@ __global__ void __launch_bounds__(kStateThreads, 1) k_split_states(const __grid_
     for (int t = next_task(blockIdx.x); t < g.tasks; t = next_task(t + gridDim.x), ++it) {
       const uint32_t acc = tmem + 256 * (it & 1) + lane_base;
       wait_or_fault(&result[it & 1], (it >> 1) & 1, &cta, g.fault, kFaultMmaWait);
-      __syncwarp();
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       const bool two = g.n - (t % g.nc) * C > 64;   // tokens in the second chunk
       float* out = g.states + ((size_t)t * g.d + (row & ~3)) * g.e + 4 * (lane & 3);
 #pragma unroll 1
       for (int c0 = 16 * half; c0 < g.e; c0 += 32) {
         uint32_t r[16], r2[16];
+        __syncwarp();   // (rows that do not exist are not stored)
         tmem_ld16(acc + c0, r);
         if (two) tmem_ld16(acc + 128 + c0, r2);
         tmem_ld_wait();
@@ -705,8 +704,7 @@ __global__ void __launch_bounds__(kOutThreads<T>, 1) k_split_out(const __grid_co
         const OutRole& r = k.r;
         const auto await = [&](int kind) {
           wait_or_fault(&full[kind], it & 1, &cta, g.fault, kFaultTmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
         };
         const auto addr = [&](int kind) { return base + turned(plan_at<Plan::place>(kind), it) * kUnit; };
         const auto addr_terms = [&](int kind) { return base + turned(plan_at<Plan::fill_place>(kind), it) * kUnit; };
@@ -838,7 +836,7 @@ __global__ void __launch_bounds__(kOutThreads<T>, 1) k_split_out(const __grid_co
       named_sync(1, Plan::kReaders);
       // ---- the masked scores' terms over the scores
       wait_or_fault(&done[kS], it & 1, &cta, g.fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       const bool two = r.wx > 64;
       // Sixteen columns at a time, in a loop: the code runs once a task, so most of what is straight-line is fetched anew
       // every time.
@@ -895,10 +893,10 @@ __global__ void __launch_bounds__(kOutThreads<T>, 1) k_split_out(const __grid_co
       if (t + (int)gridDim.x < g.tasks) write_line(t + gridDim.x);
       // ---- epilogue
       wait_or_fault(&done[kO1], it & 1, &cta, g.fault, kFaultMmaWait);
-      __syncwarp();
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       const auto result16 = [&](int c0, uint32_t (&a1)[16]) {   // sixteen results of this thread's row from column c0 on
         uint32_t a2[16];
+        __syncwarp();   // (rows past the end are not stored)
         tmem_ld16(t_o1 + lane_base + c0, a1);
         if (k.has_state) tmem_ld16(t_o2 + lane_base + c0, a2);
         tmem_ld_wait();

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(320, 1) k_span_totals(const __grid_constant__ 
       if (!w.last_of_item()) continue;
       ++li;
       wait_or_fault(&acc_full[li & 1], (li >> 1) & 1, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       if (row < D) {
 #pragma unroll
         for (int c0 = 0; c0 < E; c0 += 32) {
@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       warp_arrive(&ring_scaled[j]);
     }
     wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);
-    tc_fence_after_sync();
+    tc_fence_after_wait();
     const int c0 = half * kHalfE + grp * 32;
     if (row < D && grp * 32 < kHalfE) {
       uint32_t r[32];
@@ -746,8 +746,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         for (int g = 0; g < sums; ++g) {
           const int j = g % R::kStages;
           wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<true, true, E, C>(t_l, smem_u32(ring.a(j)), C, smem_u32(ring.b(j)), C, g > 0, leader);
           if (leader) umma_commit(&ring_empty[j]);
         }
@@ -765,8 +764,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (i >= 1) wait_or_fault(&o_free, one ^ 1, &cta, fault, kFaultMmaWait);
           wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           if constexpr (!DQ)  // X P: the state tile as [K = d rows] x [N = e columns]
             umma_gemm<false, true, E, D>(t_o, smem_u32(sx[p]), C, smem_u32(sp), D, false, leader);
           else                // X P^T: the state tile as [N = d rows] x [K = e columns]
@@ -777,8 +775,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           wait_or_fault(&z_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           wait_or_fault(&o2s_ready, one, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm_ts<true, WZ, 64>(t_o, t_s[p], smem_u32(sz[p]), C, true, leader);
           if (leader) umma_commit(&o_full[p]);
         }
@@ -790,8 +787,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           if (map_z) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&l_free, one ^ 1, &cta, fault, kFaultMmaWait);   // the state update has read the previous L
           wait_or_fault(&ys_ready, one, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           if constexpr (!DQ)
             umma_gemm<true, true, E, C>(t_l, smem_u32(sy[p]), C, smem_u32(sz[p]), C, false, leader);
           else
@@ -806,8 +802,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           wait_or_fault(&x_full[p], ph, &cta, fault, kFaultTmaWait);
           wait_or_fault(&y_full[p], ph, &cta, fault, kFaultTmaWait);
           if (map_xy) wait_or_fault(&mapped[p], ph, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<false, false, C, WX>(t_s[p], smem_u32(sx[p]), C, smem_u32(sy[p]), C, false, leader);
           if (leader) umma_commit(&s_full[p]);
         }
@@ -835,7 +830,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
         lam = exp2f(-sl2);
       }
       wait_or_fault(&s_full[p], ph, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       // masked scores, packed to bf16 in place: they are the A operand of O1 straight from tensor memory
 #pragma unroll 1
       for (int cc = 0; cc < 2; ++cc) {
@@ -859,7 +854,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       // epilogue: OUT staged in Z's buffer, once L and O1 have read it
       wait_or_fault(&l_full[p], ph, &cta, fault, kFaultMmaWait);
       wait_or_fault(&o_full[p], ph, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       if (chain) {
 #pragma unroll 1
         for (int cc = 0; cc < WZ / 64; ++cc) {
@@ -1009,7 +1004,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       }
       // O2's rows take their decay lambda^row in tensor memory; O1 then accumulates on top
       wait_or_fault(&o2_full[p], ph, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       {
         const float qd = c_o2 * decay_pow(sl2, row);
 #pragma unroll 1
@@ -1020,7 +1015,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       mbar_arrive(&o2s_ready);
       // state: P <- lambda^len P + L
       wait_or_fault(&l_full[p], ph, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       if (row < D) {
         const float lam_c = decay_pow(sl2, len);
 #pragma unroll
@@ -1231,7 +1226,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       warp_arrive(&ring_scaled[j]);
     }
     wait_or_fault(&sum_done, 0, &cta, fault, kFaultMmaWait);
-    tc_fence_after_sync();
+    tc_fence_after_wait();
     const int c0 = half * kHalfE + grp * 32;
     if (row < D && grp * 32 < kHalfE) {
       uint32_t r[32];
@@ -1322,8 +1317,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         for (int g = 0; g < sums; ++g) {
           const int j = g % R::kStages;
           wait_or_fault(&ring_scaled[j], (g / R::kStages) & 1, &cta, fault, kFaultTmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<true, true, E, C>(t_s, smem_u32(ring_buf.a(j)), C, smem_u32(ring_buf.b(j)), C, g > 0, leader);
           if (leader) umma_commit(&ring_empty[j]);
         }
@@ -1342,20 +1336,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&dn_ready, one, &cta, fault, kFaultMmaWait);
           if (i >= 1) wait_or_fault(&e_free, one ^ 1, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<false, false, D, E>(t_dk, smem_u32(sv), C, smem_u32(sdn), D, false, leader);
           umma_gemm<false, true, E, D>(t_dv, smem_u32(sk), C, smem_u32(sdn), D, false, leader);
           if (leader) umma_commit(&st_done);
           // the masked scores' products on top, A operands from tensor memory
           wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&scaled, one, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm_ts<true, E, 96>(t_dv, t_s, smem_u32(sdo[p]), C, true, leader);    // += S_m^T dO
           wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm_ts<true, D, 96>(t_dk, t_ds, smem_u32(sq[p]), C, true, leader);    // += dS_m^T Q
           if (leader) umma_commit(&b_done);
         }
@@ -1368,8 +1359,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&sm_ready, one, &cta, fault, kFaultMmaWait);
           if (E > 64) wait_or_fault(&dsm_ready, one, &cta, fault, kFaultMmaWait);
           wait_or_fault(&qs_ready, one, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<true, true, 64, C>(t_s + 32, smem_u32(sdn), C, smem_u32(sdo[p]), C, false, leader);
           if constexpr (E > 64)   // columns 64..127 of dO: its second slab
             umma_gemm<true, true, 64, C>(t_ds + 32, smem_u32(sdn), C, smem_u32(sdo[p]) + C * kSlabRowBytes, C, false, leader);
@@ -1388,8 +1378,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           wait_or_fault(&qdo_full[p], (i >> 1) & 1, &cta, fault, kFaultTmaWait);
           wait_or_fault(&kv_full, one, &cta, fault, kFaultTmaWait);
           if (elu) wait_or_fault(&mapped, one, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<false, false, C, D>(t_s, smem_u32(sk), C, smem_u32(sq[p]), C, false, leader);
           if (leader) umma_commit(&s_done);
           umma_gemm<false, false, C, E>(t_ds, smem_u32(sv), C, smem_u32(sdo[p]), C, false, leader);
@@ -1423,7 +1412,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       for (int u = 0; u < 4; ++u) {
         if ((u & 1) == 0) {
           wait_or_fault(u == 0 ? &s_done : &ds_done, one, &cta, fault, kFaultMmaWait);
-          tc_fence_after_sync();
+          tc_fence_after_wait();
         }
         const int blk = half == 0 ? (u & 1) : 3 - (u & 1);
         const uint32_t t = (u < 2 ? t_s : t_ds) + lane_base;
@@ -1447,7 +1436,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       // epilogue: dK and dV staged over Q and dO, which every product has read
       wait_or_fault(&l_done, one, &cta, fault, kFaultMmaWait);
       wait_or_fault(&b_done, one, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       if (PRE && (slope || c != 1.f)) {
 #pragma unroll 1
         for (int cc = 0; cc < D / 64; ++cc) {
@@ -1589,7 +1578,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
         mbar_arrive(&mapped);
       }
       wait_or_fault(&st_done, one, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       // row-scaled copy of Q over the state operand (the state products have read it)
       copy_row_pieces<D / 16>(sdn, sq[p], row, half * (D / 16), c * decay_pow(sl2, row), lane);
       fence_async_smem();
@@ -1607,7 +1596,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       mbar_arrive(&scaled);
       // state: Dn <- lambda^len Dn + L, this thread's half of the columns being the one in T_S or in T_dS
       wait_or_fault(&l_done, one, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       if (row < D) {
         const float lam_len = decay_pow(sl2, len);
         const uint32_t t_l = lane_base + 32 + (E > 64 ? (half ? t_ds : t_s) : t_s + half * 32);

@@ -146,8 +146,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
           wait_or_fault(&x_full, ph, &cta, fault, kFaultTmaWait);
           wait_or_fault(&y_full, ph, &cta, fault, kFaultTmaWait);
           if (i > 0) wait_or_fault(&o_done, ph ^ 1, &cta, fault, kFaultMmaWait);   // O1 has read the masked scores
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<false, false, C, W>(t_s, x, C, y, C, false, leader);
           if (leader) umma_commit(&s_done);
           __syncwarp();
@@ -159,16 +158,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
           wait_or_fault(&x_full, ph, &cta, fault, kFaultTmaWait);
           wait_or_fault(&g_ready, ph, &cta, fault, kFaultMmaWait);
           if (i > 0) wait_or_fault(&o_free, ph ^ 1, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<false, false, N, W>(t_o, x, C, g, N, false, leader);
           if (leader) umma_commit(&o2_done);
           __syncwarp();
           wait_or_fault(&z_full, ph, &cta, fault, kFaultTmaWait);
           wait_or_fault(&o2_scaled, ph, &cta, fault, kFaultMmaWait);
           wait_or_fault(&sm_ready, ph, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm_ts<true, N, 32>(t_o, t_s, z, C, true, leader);
           if (leader) umma_commit(&o_done);
           __syncwarp();
@@ -180,8 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
           wait_or_fault(&z_full, ph, &cta, fault, kFaultTmaWait);
           wait_or_fault(&ys_ready, ph, &cta, fault, kFaultMmaWait);
           if (i > 0) wait_or_fault(&l_free, ph ^ 1, &cta, fault, kFaultMmaWait);
-          __syncwarp();
-          tc_fence_after_sync();
+          tc_fence_after_wait();
           umma_gemm<true, true, W, C>(t_l, z, C, y, C, false, leader);
           if (leader) umma_commit(&l_done);
           __syncwarp();
@@ -203,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
         lam = exp2f(-sl2);
       }
       wait_or_fault(&s_done, ph, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       // packed from left to right: sixteen columns for the thirty-two that have been read
 #pragma unroll 1
       for (int b = 0; b < 4; ++b) {
@@ -218,8 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
       tc_fence_before_sync();
       mbar_arrive(&sm_ready);
       wait_or_fault(&o_done, ph, &cta, fault, kFaultMmaWait);
-      __syncwarp();
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       // Straight to memory, four lanes 64 bytes of a row, so that Z's buffer is free for the next tile at once.  (Through a
       // staging tile over Z and a TMA store, no decay: 4 x 16 x 4096 training 505 instead of 476 us, 2 x 24 x 2048 215 instead
       // of 197; with decay, where the scaling of rows is longer than Z's way, even.)
@@ -228,6 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
 #pragma unroll 1
       for (int c0 = 0; c0 < N; c0 += 32) {
         uint32_t r[32];
+        __syncwarp();   // (rows past the end are not stored)
         tmem_ld32(t_o + lane_base + c0, r);
         tmem_ld_wait();
         uint4 v[4];
@@ -284,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
       mbar_arrive(&ys_ready);
       wait_or_fault(&o2_done, ph, &cta, fault, kFaultMmaWait);
       if (decays) {
-        tc_fence_after_sync();
+        tc_fence_after_wait();
         const float wt = decay_pow(sl2, w.r.backwards ? from_end : row);
 #pragma unroll 1
         for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) scale_tmem32(t_o + lane_base + c0, wt);
@@ -293,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_wide(const __grid_constant
       }
       mbar_arrive(&o2_scaled);
       wait_or_fault(&l_done, ph, &cta, fault, kFaultMmaWait);
-      tc_fence_after_sync();
+      tc_fence_after_wait();
       const float lam_len = decay_pow(sl2, len);
 #pragma unroll
       for (int c0 = 0; c0 < 128; c0 += 16) {
