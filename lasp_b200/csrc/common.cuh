@@ -110,12 +110,20 @@ cudaError_t opt_in_smem(size_t bytes) {
 
 // The kernels of the full-precision path follow one another closely (states, scan, outputs): each lets the next one's CTAs
 // take an SM as soon as its own have left it, and waits itself, before it touches global memory, for what came before it to
-// be complete.  (A CTA of the next kernel cannot start before all of this one's have: they call this first thing.)  Training
-// passes of 2 x 12 x 2048: fp32 219 -> 212 us, fp16 122 -> 116.5; the walk kernels' passes got 1 to 2 % longer with it.
-__device__ __forceinline__ void follow_on() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// be complete.  Training passes of 2 x 12 x 2048: fp32 219 -> 212 us, fp16 122 -> 116.5; the walk kernels' passes got 1 to 2 %
+// longer with it.
+//   after_previous   every thread, before its first access to global memory, and after the CTA has its tensor memory: a CTA
+//                    that waited for columns while it kept the CTA that holds them from starting would wait for good.
+//                    Tiles that a kernel wrote with ordinary stores are read by TMA, another proxy: hence the fence.
+//   let_next_start   behind after_previous: whatever starts early finds everything but this kernel complete - a kernel of a
+//                    caller's that reads what it takes for long written ahead of its own wait, and the L1 of its SM.  A
+//                    kernel whose stores the next one's TMA reads calls it behind them and their fence.
+__device__ __forceinline__ void fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  fence_async_global();
 }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... KArgs, typename... Args>
 cudaError_t launch_following(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
   cudaLaunchAttribute attr = {};

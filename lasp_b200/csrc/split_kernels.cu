@@ -60,10 +60,11 @@ template <> struct Terms<__nv_bfloat16> { static constexpr int in = 1, mid = 3, 
 template <typename T> struct Raw { uint4 v; };
 template <> struct Raw<float> { uint4 v, w; };
 
-__device__ __forceinline__ uint4 ld_nc(const void* p) { return __ldg(static_cast<const uint4*>(p)); }
-template <typename T> __device__ __forceinline__ void load_piece(Raw<T>& r, const T* p) { r.v = ld_nc(p); }
+// (not by the read-only path: the kernel before may write them while this one's CTAs are there already)
+__device__ __forceinline__ uint4 ld16(const void* p) { return *static_cast<const uint4*>(p); }
+template <typename T> __device__ __forceinline__ void load_piece(Raw<T>& r, const T* p) { r.v = ld16(p); }
 template <> __device__ __forceinline__ void load_piece<float>(Raw<float>& r, const float* p) {
-  r.v = ld_nc(p), r.w = ld_nc(p + 4);
+  r.v = ld16(p), r.w = ld16(p + 4);
 }
 template <typename T> __device__ __forceinline__ void to_floats(const Raw<T>& r, float (&x)[8]);
 template <> __device__ __forceinline__ void to_floats<float>(const Raw<float>& r, float (&x)[8]) {
@@ -286,7 +287,8 @@ __global__ void __launch_bounds__(kStateThreads, 1) k_split_states(const __grid_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;   // [parity of the task][chunk], 128 columns each
-  follow_on();
+  after_previous();
+  let_next_start();
   const auto next_task = [&](int t) {
     while (t < g.tasks && t % g.nc == g.skip) t += gridDim.x;
     return t;
@@ -665,7 +667,8 @@ __global__ void __launch_bounds__(kOutThreads<T>, 1) k_split_out(const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = tmem_slot;
-  follow_on();
+  after_previous();
+  let_next_start();
 
   struct Task {
     OutRole r;

@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const
                                               float* __restrict__ x_out, int h,
                                               int n, int de, int nc, int chunk, int reverse, int rows,
                                               int cols) {
-  if (TERMS) follow_on();
+  if (TERMS) after_previous();
   const int bh = blockIdx.y;
   const int el = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (el >= de) return;
@@ -32,14 +32,15 @@ __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const
   const int last_len = n - (nc - 1) * chunk;
   const float tail = expf(-sh * (float)last_len);
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (x_in) p = *reinterpret_cast<const float4*>(x_in + (size_t)bh * de + ext);
+  // (around the read-only path: the kernel before writes these while this one's CTAs may be there already)
+  if (x_in) p = __ldcg(reinterpret_cast<const float4*>(x_in + (size_t)bh * de + ext));
   const float* base = local + (size_t)bh * nc * de + el;
   for (int i0 = 0; i0 < nc; i0 += kScanBatch) {
     float4 loc[kScanBatch];
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u) {
       const int i = i0 + u;
-      if (i < nc) loc[u] = *reinterpret_cast<const float4*>(base + (size_t)(reverse ? nc - 1 - i : i) * de);
+      if (i < nc) loc[u] = __ldcg(reinterpret_cast<const float4*>(base + (size_t)(reverse ? nc - 1 - i : i) * de));
     }
 #pragma unroll
     for (int u = 0; u < kScanBatch; ++u) {
@@ -60,6 +61,10 @@ __global__ void __launch_bounds__(256) k_scan(const float* __restrict__ s, const
     }
   }
   if (x_out) *reinterpret_cast<float4*>(x_out + (size_t)bh * de + ext) = p;
+  if (TERMS) {   // (the output kernels read the terms by TMA)
+    fence_async_global();
+    let_next_start();
+  }
 }
 
 __global__ void __launch_bounds__(256) k_state_combine(const float* __restrict__ s, const float* __restrict__ x_in,
