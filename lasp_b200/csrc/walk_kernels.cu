@@ -231,11 +231,21 @@ __device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t* p) {
 __device__ __forceinline__ void st_volatile_u32(uint32_t* p, uint32_t v) {
   asm volatile("st.volatile.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// A flag between CTAs of a launch: what its writer's CTA wrote ahead of a barrier before the release is there for everyone
+// behind a barrier after the acquire.
+__device__ __forceinline__ void st_release_u32(uint32_t* p, uint32_t v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 // spins until *flag == want or `limit` clocks pass
 __device__ __forceinline__ bool wait_flag_eq(const uint32_t* flag, uint32_t want, long long limit) {
-  if (ld_volatile_u32(flag) == want) return true;
+  if (ld_acquire_u32(flag) == want) return true;
   const long long t0 = clock64();
-  while (ld_volatile_u32(flag) != want) {
+  while (ld_acquire_u32(flag) != want) {
     if (clock64() - t0 > limit) return false;
   }
   return true;
@@ -661,10 +671,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
     }
     tc_fence_before_sync();
     named_sync(2, 2 * kWorkers);   // every worker's part of the total is written ...
-    if (tid == kFirstWorker) {
-      __threadfence();             // ... and visible to the other CTAs before the flag is
-      st_volatile_u32(a.sync + kSyncFlags + blockIdx.x, step_s);
-    }
+    if (tid == kFirstWorker) st_release_u32(a.sync + kSyncFlags + blockIdx.x, step_s);   // ... and visible before the flag is
   };
   // The three kinds of warps part for good here: each branch sets its registers and is compiled for them.
   if (warp < kFirstWorker / 32) {
@@ -956,10 +963,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
                   link_make_total<kHalfE, D>(a.totals + (size_t)owner * D * E, row, half * kHalfE,
                                              decay_pow(sl2, a.n - w.t0 * C), P);
                 named_sync(1, kWorkers);
-                if (wid == 0) {
-                  __threadfence();
-                  st_volatile_u32(ready, step_s);
-                }
+                if (wid == 0) st_release_u32(ready, step_s);
               }
               if (far || w.it == owner) {
                 // the readers of the ranks after this one have acknowledged the slots' previous use
@@ -1241,7 +1245,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     // the forward pass, whose totals are further from its first tile's work, 24.0 -> 24.1.)
     __threadfence();
     named_sync(2, 2 * kWorkers);
-    if (tid == kFirstWorker) st_volatile_u32(a.sync + kSyncFlags + my_item(), step_s);
+    if (tid == kFirstWorker) st_release_u32(a.sync + kSyncFlags + my_item(), step_s);
   };
 
   if (warp < kFirstWorker / 32) {
@@ -1526,10 +1530,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
                   link_make_total<kHalfE, D>(a.totals + (size_t)owner * D * E, row, half * kHalfE,
                                              decay_pow(sl2, span_end), Dn);
                 named_sync(1, kWorkers);
-                if (wid == 0) {
-                  __threadfence();
-                  st_volatile_u32(ready, step_s);
-                }
+                if (wid == 0) st_release_u32(ready, step_s);
               }
               if (far || sp_idx == 0) {
                 // the readers of the ranks after this one in the chain order (the ranks BEFORE it in the
