@@ -321,8 +321,9 @@ def _slice_like(q, v):
 
 def lightning_attn_fused(q, k, v, s, qk_scale: float = 1.0, feature_map=None):
     """``lightning_attn(c * map(q), c * map(k), v, s)`` with the preprocessing of q and k folded into the
-    kernels' load path (and its chain rule into their epilogues); in large calls the map goes ahead of the kernels, in one
-    pass over q and k whose results the backward pass takes too.  ``feature_map``: None or "elu1" (elu(x) + 1); ``qk_scale``: c.  Problems whose kernels cannot
+    kernels' load path (and its chain rule into their epilogues).  From 2^22 elements of q on the map goes ahead of the
+    kernels, in one pass over q and k; a training call then saves the mapped copies (as much memory as q and k) for its
+    backward pass, and not q and k.  ``feature_map``: None or "elu1" (elu(x) + 1); ``qk_scale``: c.  Problems whose kernels cannot
     do this (fp32 path, head dims other than 64 / 128 per slice, more spans than SMs) get the same result from
     torch operations in front of the operator."""
     return lightning(q, k, v, s, qk_scale, feature_map)

@@ -10,6 +10,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAGraphsUtils.cuh>
 #include <c10/cuda/CUDAGuard.h>
@@ -243,6 +244,23 @@ std::pair<Tensor, Tensor> mapped_qk(const Tensor& q, const Tensor& k) {
   return {qm, km};
 }
 
+// What autograd asks of a saved tensor when it is taken out again, for q and k whose mapped copies are saved in their place:
+// that nobody has written to them since.  (Saving them beside the copies would hold twice the memory until the backward
+// pass.)  Under saved-tensor hooks it does not ask, what they have packed being theirs.
+struct Unwritten : torch::CustomClassHolder {
+  c10::VariableVersion counter[2];
+  uint32_t at[2];
+  Unwritten(const Tensor& q, const Tensor& k)
+      : counter{torch::autograd::impl::version_counter(q), torch::autograd::impl::version_counter(k)},
+        at{counter[0].current_version(), counter[1].current_version()} {}
+  void check() const {
+    for (int i = 0; i < 2; ++i)
+      TORCH_CHECK(counter[i].current_version() == at[i],
+                  "one of the variables needed for gradient computation has been modified by an inplace operation: ", i ? "k" : "q",
+                  " of lasp_b200 attention is at version ", counter[i].current_version(), "; expected version ", at[i], " instead");
+  }
+};
+
 class Lightning : public torch::autograd::Function<Lightning> {
  public:
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& s,
@@ -251,11 +269,14 @@ class Lightning : public torch::autograd::Function<Lightning> {
     variable_list saved{q, k, v, s};
     std::vector<Tensor> out;
     if (map == LASP_QK_ELU1 && map_first(m, true)) {
-      // the backward pass takes the mapped tensors; the others are saved for what autograd makes of a change to them
-      const auto [qm, km] = mapped_qk(q, k);
+      for (const Tensor* t : {&q, &k})   // (as for a tensor that is saved)
+        TORCH_CHECK(!t->is_inference(), "Inference tensors cannot be saved for backward. To work around you can make a clone to get a "
+                                        "normal tensor and use it in autograd.");
+      if (!at::SavedTensorDefaultHooks::get_hooks())
+        ctx->saved_data["unwritten"] = c10::IValue::make_capsule(c10::make_intrusive<Unwritten>(q, k));
+      std::tie(saved[0], saved[1]) = mapped_qk(q, k);   // all that the backward pass takes
       map = LASP_QK_ELU1_MAPPED;
-      out = run_forward(qm, km, v, s, m, scale, map, true);
-      saved.push_back(qm), saved.push_back(km);
+      out = run_forward(saved[0], saved[1], v, s, m, scale, map, true);
     } else {
       out = run_forward(q, k, v, s, m, scale, map, true);
     }
@@ -268,12 +289,14 @@ class Lightning : public torch::autograd::Function<Lightning> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const variable_list saved = ctx->get_saved_variables();
+    const auto unwritten = ctx->saved_data.find("unwritten");
+    if (unwritten != ctx->saved_data.end()) c10::static_intrusive_pointer_cast<Unwritten>(unwritten->second.toCapsule())->check();
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
     // What was saved may have been through a saved-tensor hook (offloading, compression): it can come back with other
     // strides, or not as what it was.
     const int64_t map = ctx->saved_data["map"].toInt();
-    const size_t qk = map == LASP_QK_ELU1_MAPPED ? 4 : 0, first_ws = map == LASP_QK_ELU1_MAPPED ? 6 : 4;
-    const Tensor q = saved[qk].contiguous(), k = saved[qk + 1].contiguous(), v = saved[2].contiguous(), d_o = grads[0].contiguous();
+    constexpr size_t first_ws = 4;
+    const Tensor q = saved[0].contiguous(), k = saved[1].contiguous(), v = saved[2].contiguous(), d_o = grads[0].contiguous();
     TORCH_CHECK(q.is_cuda() && k.is_cuda() && v.is_cuda() && d_o.is_cuda(), "lasp_b200: a saved tensor is not on a GPU any more");
     TORCH_CHECK_TYPE(q.scalar_type() == d_o.scalar_type() && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
                      "lasp_b200: a saved tensor has changed its dtype");
