@@ -37,7 +37,7 @@
 extern "C" {
 #endif
 
-#define LASP_B200_ABI_VERSION 3
+#define LASP_B200_ABI_VERSION 4
 
 /* the library is built with hidden visibility; only the entry points below are exported */
 #if defined(__GNUC__)
@@ -68,13 +68,13 @@ typedef enum {
   LASP_PATH_TENSOR = 2  /* tcgen05/TMEM/TMA kernels: bf16, d,e in {64,128}, n >= 128 (a ragged tail is fine) */
 } lasp_path;
 
-/* Preprocessing of q and k folded into the kernels' load path: the operator is evaluated on
- * qk_scale * map(q) and qk_scale * map(k), and dq, dk are the gradients with respect to the RAW q and k
- * (chain rule applied in the epilogues).  Replaces the caller-side passes `q, k = elu(q) + 1, elu(k) + 1`
- * and `q, k *= d ** -0.5` in front of lightning_attn / lasp_* (lasp/lightning_attention.py:510); each of
- * them would read and write q and k once more in an operator bound by memory traffic.  Only the fused
- * tensor-core launches (forward, backward, the linked forms, bwd_dq, bwd_dkv) take it; every other entry
- * point returns LASP_ERR_PATH when it is requested. */
+/* Preprocessing of q and k folded into the kernels: the operator is evaluated on qk_scale * map(q) and
+ * qk_scale * map(k), and dq, dk are the gradients with respect to the RAW q and k (chain rule applied in the
+ * epilogues).  q and k come raw, and are mapped tile by tile where they are loaded; with LASP_QK_ELU1_MAPPED they come
+ * mapped.  Replaces the caller-side passes `q, k = elu(q) + 1, elu(k) + 1` and `q, k *= d ** -0.5` in front of
+ * lightning_attn / lasp_* (lasp/lightning_attention.py:510).  Only the fused tensor-core launches take it: forward,
+ * backward, bwd_dq, bwd_dkv and, except for LASP_QK_ELU1_MAPPED, the linked forms; every other entry point returns
+ * LASP_ERR_PATH when it is requested. */
 typedef enum {
   LASP_QK_IDENTITY = 0,
   LASP_QK_ELU1 = 1,       /* elu(x) + 1 */
@@ -213,8 +213,6 @@ LASP_B200_API int lasp_b200_forward_opt(const lasp_problem* p, const lasp_fwd_ar
 LASP_B200_API int lasp_b200_backward_opt(const lasp_problem* p, const lasp_bwd_args* a, const lasp_call_options* opt,
                                          void* stream);
 
-/* x_out = exp(-s_h n) x_in + x_local on (b,h,d,e) fp32 states; x_in may be NULL.
- * Replaces the torch glue KV = block_decay*KV + kv, lasp/lasp_naive.py:565,614. */
 /* Heads of 256 (d = e = 256) in bf16, n >= 128, without rank states, preprocessing or row pitches: each result in one pass
  * instead of four 128-wide slice pairs.  wide_ok: 1 where these are the faster way for the forward or the backward pass on
  * the current device, 0 where the slices are, a negative status where the problem is not of this kind.  The two passes are
@@ -223,6 +221,8 @@ LASP_B200_API int lasp_b200_wide_ok(const lasp_problem* p, int backward);
 LASP_B200_API int lasp_b200_forward_wide(const lasp_problem* p, const lasp_fwd_args* a, void* stream);
 LASP_B200_API int lasp_b200_backward_wide(const lasp_problem* p, const lasp_bwd_args* a, void* stream);
 
+/* x_out = exp(-s_h n) x_in + x_local on (b,h,d,e) fp32 states; x_in may be NULL.
+ * Replaces the torch glue KV = block_decay*KV + kv, lasp/lasp_naive.py:565,614. */
 LASP_B200_API int lasp_b200_state_combine(int b, int h, int d, int e, int n, const float* s, const float* x_in,
                             const float* x_local, float* x_out, void* stream);
 

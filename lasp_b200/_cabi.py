@@ -10,7 +10,7 @@ import ctypes as C
 import os
 
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "liblasp_b200.so")
-ABI_VERSION = 3
+ABI_VERSION = 4
 
 # lasp_dtype / lasp_path / lasp_status of include/lasp_b200.h
 F32, BF16, F16 = 0, 1, 2

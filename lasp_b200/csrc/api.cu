@@ -244,7 +244,7 @@ int fwd_output(const lasp::Dims& m, const lasp_fwd_args* a, const lasp_call_opti
     return cuda_fail(lasp::walk_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_walk_border(a->ws, m),
                                            opt.sync ? opt.sync : lasp::ws_walk_sync(a->ws), a->o,
                                            (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
-  return cuda_fail(lasp::split_fwd_output(m, a->q, a->k, a->v, a->s, lasp::ws_split_prefix(a->ws), a->o, opt.alone != 0,
+  return cuda_fail(lasp::split_fwd_output(m, a->q, a->k, a->v, a->s, a->ws, a->o, opt.alone != 0,
                                           (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
 }
 
@@ -271,8 +271,8 @@ int bwd_grads(const lasp::Dims& m, const lasp_bwd_args* a, const lasp_call_optio
     return cuda_fail(lasp::walk_bwd_dkv(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_walk_border(a->ws, m), a->dk,
                                         a->dv, add_qk, add_v, cs));
   }
-  return cuda_fail(lasp::split_bwd_grads(m, a->q, a->k, a->v, a->d_o, a->s, lasp::ws_split_prefix(a->fwd_ws),
-                                         lasp::ws_split_prefix(a->ws), a->dq, a->dk, a->dv, opt.alone != 0,
+  return cuda_fail(lasp::split_bwd_grads(m, a->q, a->k, a->v, a->d_o, a->s, a->fwd_ws,
+                                         a->ws, a->dq, a->dk, a->dv, opt.alone != 0,
                                          (opt.accumulate & LASP_ACCUMULATE_QK) != 0,
                                          (opt.accumulate & LASP_ACCUMULATE_V) != 0, cs));
 }

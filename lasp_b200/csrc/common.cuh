@@ -75,7 +75,6 @@ inline float* ws_local(void* ws, const Dims& m) {
   return m.walk ? ws_walk_totals(ws) : reinterpret_cast<float*>(static_cast<char*>(ws) + state_elems(m) * 6);
 }
 inline void* ws_prefix(void* ws, const Dims& m) { return m.walk ? ws_walk_border(ws, m) : ws; }
-inline const void* ws_split_prefix(const void* ws) { return ws; }
 // bits of the sticky per-device fault word (fault_word.cu owns the word)
 enum : int32_t {
   kFaultNone = 0,

@@ -282,8 +282,8 @@ __device__ __forceinline__ void copy_row_pieces(uint8_t* dst, const uint8_t* src
 }
 
 // stage_row32 with the chain rule of the folded q,k preprocessing x' = c * map(x): the 32 accumulator values
-// (a gradient with respect to x') are multiplied by c * map'(x) on their way to the staging tile.  x comes from the raw
-// tensor (`raw` points at column 0 of this thread's row): raw_row32, which the caller issues ahead of its wait for the
+// (a gradient with respect to x') are multiplied by c * map'(x) on their way to the staging tile.  x, or with MAPPED
+// map(x), comes from the q or k that the launch was given (`raw` points at column 0 of this thread's row): raw_row32, which the caller issues ahead of its wait for the
 // accumulator, because these loads go through L2 (with the loads behind the wait a dQ walk over 64-wide heads took 86 us - now 79 -
 // for 4 x 16 x 4096 tokens, against 35 us without a map).
 __device__ __forceinline__ void raw_row32(uint4 (&x)[4], const __nv_bfloat16* raw, int col0) {

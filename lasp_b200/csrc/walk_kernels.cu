@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
       tc_fence_before_sync();
       mbar_arrive(&sm_ready[p]);
       if (elu && i + 1 < total) map_tile(i + 1, grp);   // the next tile's S can then go out under this tile's work
-      // dq = dq' * c * map'(q), q read from the raw tensor (rows past the end of the sequence are not stored)
+      // dq = dq' * c * map'(q), q (PRE = 2: mapped) read from its tensor (rows past the end of the sequence are not stored)
       const bool chain = PRE && DQ && (slope || c != 1.f);
       const bool live = row < a.n - w.t * C;
       const __nv_bfloat16* raw = nullptr;
@@ -1429,7 +1429,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           mbar_arrive(u == 1 ? &sm_ready : &dsm_ready);
         }
       }
-      // dk = dk' * c * map'(k), k read from the raw tensor (rows past the end of the sequence are not stored)
+      // dk = dk' * c * map'(k), k (PRE = 2: mapped) read from its tensor (rows past the end of the sequence are not stored)
       const bool live = row < a.n - w.t * C;
       const __nv_bfloat16* raw = nullptr;
       uint4 raw_x[4];
