@@ -241,6 +241,9 @@ __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void red_release_inc(uint32_t* p) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+}
 // spins until *flag == want or `limit` clocks pass
 __device__ __forceinline__ bool wait_flag_eq(const uint32_t* flag, uint32_t want, long long limit) {
   if (ld_acquire_u32(flag) == want) return true;
@@ -464,6 +467,12 @@ struct WalkArgs {
 };
 constexpr int kSyncEven = 2;
 constexpr int kSyncFlags = 32;
+// A span's flag counts the parts of its total that are there, the launch's number above the count: no launch takes another's
+// for its own until the number has gone round, which is 2^27 launches.
+constexpr uint32_t kTotalParts = 2 * kWorkers / 32;
+__device__ __forceinline__ uint32_t nothing_published(uint32_t step) { return step * 32; }
+__device__ __forceinline__ uint32_t published(uint32_t step) { return step * 32 + kTotalParts; }
+static_assert(kTotalParts < 32, "the count's bits");
 constexpr int kSyncSecondBank = 480;   // [kSyncFlags + kSyncSecondBank + sequence]: "the sequence's total is written"
 
 // bf16 image of this thread's part of the state (row `row`, columns [col0, col0 + N)) in the operand tile
@@ -671,7 +680,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
     }
     tc_fence_before_sync();
     named_sync(2, 2 * kWorkers);   // every worker's part of the total is written ...
-    if (tid == kFirstWorker) st_release_u32(a.sync + kSyncFlags + blockIdx.x, step_s);   // ... and visible before the flag is
+    if (tid == kFirstWorker) st_release_u32(a.sync + kSyncFlags + blockIdx.x, published(step_s));   // ... and visible before the flag is
   };
   // The three kinds of warps part for good here: each branch sets its registers and is compiled for them.
   if (warp < kFirstWorker / 32) {
@@ -933,7 +942,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_out(const __grid_constant_
           int first = sp_idx;
           while (first > 0 && w.t0 - w.span_t0(first) < reach) --first;
           if (wid < sp_idx && wid >= first && !cta.gave_up()) {
-            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + wid, step_s, a.wait_clocks)) {
+            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + wid, published(step_s), a.wait_clocks)) {
               cta.give_up();
               atomicOr(fault, kFaultFlagWait);
             }
@@ -1125,6 +1134,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
   __shared__ Health<LINK> cta;
   const int tid = threadIdx.x, warp = (int)uniform(tid >> 5), lane = tid & 31;
   int32_t* fault = a.fault;
+  // this CTA's span among all spans (the places of a sequence count down, see span_of_place)
+  const auto item_of = [&](int bh) { return (2 * bh + 1) * a.cut.nspans - 1 - (int)blockIdx.x; };
   // thread 0 is also the producer: its first loads go out before the CTA-wide barrier (see k_walk_out)
   bool early_ring = false, early_q = false;
   if (tid == 0) {
@@ -1176,6 +1187,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     if (w0.start()) {
       const bool ring = FUSED && a.coop && (w0.sp > 0 || a.all_totals);
       const int t = ring ? w0.t0 : w0.t;   // first stage of the span-total ring, or Q, dO of the walk's first tile
+      if (ring) st_volatile_u32(a.sync + kSyncFlags + item_of(w0.bh), nothing_published(step_s));
       uint64_t* bar = ring ? &ring_full[0] : &qdo_full[0];
       mbar_expect_tx(bar, C * (D + E) * 2);
       tma_load_4d(sq[0], &map_q, bar, 0, t * C, 0, w0.bh);   // (where the first ring stage begins too)
@@ -1200,8 +1212,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
       if (w.sp > 0 || a.all_totals) sums = min(w.t1 - w.t0, reach_tiles(a.s[my_bh % a.h]));
     }
   }
-  // this CTA's span among all spans (the places of a sequence count down, see span_of_place), not kept in a register
-  const auto my_item = [&] { return (2 * my_bh + 1) * a.cut.nspans - 1 - (int)blockIdx.x; };
+  const auto my_item = [&] { return item_of(my_bh); };   // (not kept in a register)
   const int row = (warp & 3) * 32 + lane;      // workers: tensor-memory lane quarter of this warp
   const int wid = (tid - kFirstWorker) & (kWorkers - 1);   // 0..255 inside the group
   const int half = wid >> 7;
@@ -1240,12 +1251,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
     }
     tc_fence_before_sync();
     warp_arrive(&total_read);      // (S^T takes the total's place in tensor memory)
-    // Every worker's part of the total is written and visible to the other CTAs before the flag is.  (A fence of each thread
-    // behind its own stores instead of one behind the barrier: 24 x 2048 tokens 28.4 -> 27.8 us, 36 x 3001 43.5 -> 43.0;
-    // the forward pass, whose totals are further from its first tile's work, 24.0 -> 24.1.)
-    __threadfence();
+    // Every warp releases its own part, so that they wait for their stores side by side: the flag is complete with the last
+    // one.  24 x 2048 tokens, 128/128 and 128/64, 25.2 / 21.4 us; released by one thread behind a fence of each and a barrier 26.0 /
+    // 23.0; behind the barrier alone 26.6 / 22.8; a fence of each, a barrier and a plain store, which is no release, 25.4 / 22.0.
+    // (The forward pass, whose totals are further from its first tile's work: even.)  The barrier orders nothing: without it the
+    // compiler spills more in the 64-wide kernels with a chain rule (64 x 4096 tokens 71.4 -> 78.9 us).
+    __syncwarp();
+    if (lane == 0) red_release_inc(a.sync + kSyncFlags + my_item());
     named_sync(2, 2 * kWorkers);
-    if (tid == kFirstWorker) st_release_u32(a.sync + kSyncFlags + my_item(), step_s);
   };
 
   if (warp < kFirstWorker / 32) {
@@ -1500,7 +1513,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_walk_dkv(
           int past = sp_idx + 1;
           while (past < a.cut.nspans && w.span_t0(past) - w.t1 < reach) ++past;
           if (wid < past - 1 - sp_idx && !cta.gave_up()) {
-            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + sp_idx + 1 + wid, step_s, a.wait_clocks)) {
+            if (!wait_flag_eq(a.sync + kSyncFlags + w.bh * a.cut.nspans + sp_idx + 1 + wid, published(step_s), a.wait_clocks)) {
               cta.give_up();
               atomicOr(fault, kFaultFlagWait);
             }
