@@ -433,7 +433,10 @@ int lasp_b200_wide_ok(const lasp_problem* p, int backward) {
   // A walk goes over whole sequences, the slices cut them in spans: with few, long sequences those fill the chip and this
   // does not.  Measured with decay (forward / backward alone, b*h sequences of t tiles): walks 4.4 us a tile and wave of CTAs
   // plus 10; slices 55 + 0.14 / 140 + 0.24 us per sequence and tile.  64 x 32 tiles 168 / 447 against 306 / 628 us, 24 x 32 153 /
-  // 159 against 149 / 319, 16 x 64 295 / 302 against 195 / 386, 8 x 64 290 / 292 against 133 / 257.
+  // 159 against 149 / 319, 16 x 64 295 / 302 against 195 / 386, 8 x 64 290 / 292 against 133 / 257.  Without decay the walks are
+  // a sixth faster and the slices (kept on by a scale next to 1) even: 126 / 352 against 316 / 638, 117 / 125 against 155 / 336,
+  // 209 / 212 against 185 / 429, 205 / 205 against 139 / 279.  The decay rates are not known here: the rule is right for both but
+  // for the last of these backward passes, which it leaves to the slices.
   const long long seqs = (long long)p->b * p->h, tiles = (p->n + lasp::kTensorTile - 1) / lasp::kTensorTile;
   const long long waves = ((backward ? 6 : 2) * seqs + lasp::sm_count() - 1) / lasp::sm_count();
   const long long walk = 440 * tiles * waves + 1000, slices = (backward ? 14000 + 24 * seqs * tiles : 5500 + 14 * seqs * tiles);   // 10 ns

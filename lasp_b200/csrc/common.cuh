@@ -109,7 +109,8 @@ cudaError_t opt_in_smem(size_t bytes) {
 
 // The kernels of the full-precision path follow one another closely (states, scan, outputs): each lets the next one's CTAs
 // take an SM as soon as its own have left it, and waits itself, before it touches global memory, for what came before it to
-// be complete.  Training passes of 2 x 12 x 2048: fp32 219 -> 212 us, fp16 122 -> 116.5; the walk kernels' passes got 1 to 2 %
+// be complete.  Training passes of 2 x 12 x 2048: fp32 219 -> 212 us, fp16 122 -> 116.5 (with the
+// next one let in ahead of the wait; behind it 213.7 -> 211.2 and 116.6 -> 114.8); the walk kernels' passes got 1 to 2 %
 // longer with it.
 //   after_previous   every thread, before its first access to global memory, and after the CTA has its tensor memory: a CTA
 //                    that waited for columns while it kept the CTA that holds them from starting would wait for good.

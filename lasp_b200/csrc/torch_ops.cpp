@@ -231,9 +231,13 @@ std::vector<Tensor> run_forward(const Tensor& q, const Tensor& k, const Tensor& 
 
 // Whether q and k go through elu(x) + 1 in a pass of their own, ahead of the kernels, or tile by tile inside them.  The
 // kernels of a training step map a tile up to five times and evaluate the exponential of the chain rule twice more; the pass
-// costs a launch and 8 bytes of memory traffic an element.  Training, 64-wide 4 x 16 x 4096 272 -> 198 us, 2 x 16 x 2048 92 -> 87,
-// 2 x 16 x 1024 83 -> 86; 128-wide 8 x 32 x 2048 754 -> 610, 2 x 16 x 1024 93 -> 87, 1 x 16 x 1024 81 -> 86: from 2^22 elements of q
-// on.  A forward pass alone: v 64 wide 4 x 16 x 4096 80 -> 73, 2 x 16 x 2048 29 -> 28, 2 x 16 x 1024 even; 128 wide 177 -> 195, never.
+// costs a launch and 8 bytes of memory traffic an element.  Passes through the operator, training, 64-wide 4 x 16 x 4096 272 -> 198
+// us, 2 x 16 x 2048 92 -> 87, 2 x 16 x 1024 83 -> 86; 128-wide 8 x 32 x 2048 754 -> 610, 2 x 16 x 1024 93 -> 87, 1 x 16 x 1024 81 -> 86:
+// from 2^22 elements of q on.  A forward pass alone: v 64 wide 4 x 16 x 4096 80 -> 73, 2 x 16 x 2048 29 -> 28, 2 x 16 x 1024 even; 128
+// wide never.  Those are without decay; with it tiles next to a span's border alone are read twice, which moves the line
+// little.  Launches alone, inside -> ahead, without / with decay: training 64-wide 4 x 16 x 4096 251 -> 180 / 241 -> 176, 2 x 16 x 1024
+// 52 -> 45 / 52 -> 44, 128-wide 8 x 32 x 2048 699 -> 543 / 700 -> 535, 1 x 16 x 16384 394 -> 311 / 372 -> 287; forward 64-wide 4 x 16 x 4096
+// 71 -> 64 / 67 -> 62, 128-wide 8 x 32 x 2048 174 -> 174 / 172 -> 176.
 bool map_first(const Shape& m, bool train) { return m.b * m.h * m.n * m.d >= (int64_t{1} << 22) && (train || m.e <= 64); }
 
 std::pair<Tensor, Tensor> mapped_qk(const Tensor& q, const Tensor& k) {

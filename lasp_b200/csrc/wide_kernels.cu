@@ -20,7 +20,7 @@
 // What bounds it: the chain of a tile (S, mask, O1, state update and operand, all tiles of a step in single buffers: X, Y,
 // the state operand 64 KB each, Z 32 KB), then HBM.  A tile takes 5400 clocks, 3584 of them tensor work, for 192 KB.  b=4, h=16,
 // n=4096, no decay, slices and now: forward 326 -> 138 us, training 984 -> 476 (1044 -> 544 under the power cap); with decay 306 -> 162
-// and 934 -> 556.  Error against fp64 2.4e-3 to 3.2e-3 -> 1.8e-3 to 2.7e-3.  The next tile's X, Y, Z asked into L2 ahead: 8 % slower.
+// and 934 -> 556.  Error against fp64 2.3e-3 to 3.1e-3 -> 1.7e-3 to 2.4e-3.  The next tile's X, Y, Z asked into L2 ahead: 8 % slower.
 #include "tc_common.cuh"
 
 namespace lasp {
